@@ -51,13 +51,13 @@ def listed():
     whole = dict(vocab=151936)
     return [
         # one user, a short exchange with a small model: launches and latency
-        dict(case("qwen3", "1b", 4, "decode", 1, 77), name="decode 1x77, 4 layers"),
+        dict(case("qwen3", "1b", 4, "decode", 1, 77), name="decode 1x77 in 4 layers"),
         # one user of the 4B model after a page of text: weights read once for one token
         dict(case("qwen3", "4b", 36, "decode", 1, 2048, **whole), name="decode 1x2048"),
         # the benchmark's headline: eight requests near the end of their context
         dict(case("qwen3", "4b", 36, "decode", 8, 8100, **whole), name="decode 8x8100"),
         # a loaded server that draws its tokens
-        dict(case("qwen3", "4b", 36, "decode", 64, 2048, sample=True, **whole), name="decode 64x2048, sampled"),
+        dict(case("qwen3", "4b", 36, "decode", 64, 2048, sample=True, **whole), name="decode 64x2048 sampled"),
         # an odd number of requests, each at another place of its text
         dict(case("qwen3", "4b", 36, "decode", 13, 5003, ragged=True, **whole), name="decode 13 ragged"),
         # the benchmark's prompt
