@@ -262,6 +262,10 @@ template <int TILE_T, int TILE_F> struct Cfg {
     static constexpr int STAGES = (TILE_T >= 128 || TILE_F > 128)
                                       ? (192 * 1024) / STAGE_BYTES
                                       : (NARROW_RING_BYTES / STAGE_BYTES > 8 ? 8 : NARROW_RING_BYTES / STAGE_BYTES);
+    // Resident CTAs per SM, told to the compiler as well: left alone it gave the 64-token kernel 144
+    // registers a thread for the activations of its epilogue, so that one CTA fitted where the ring
+    // is cut for two (a decode step of 64 tokens, 2,048 keys, tokens drawn: 7,903 us, 7,104 with two); at 96 registers nothing spills.
+    static constexpr int CTAS = (TILE_T >= 128 || TILE_F > 128) ? 1 : 2;
     static constexpr int ACC_COLS = TILE_T * HALVES;
     static constexpr int TMEM_COLS = ACC_COLS < 32 ? 32 : ACC_COLS;   // 32, 64, 128, 256 or 512
     // epilogue warp groups: two groups of four warps split the token columns
@@ -423,7 +427,7 @@ __device__ __forceinline__ void epilogue_chunk(const Params& p, float* v, int t_
 }
 
 template <int TILE_T, int TILE_F>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, Cfg<TILE_T, TILE_F>::CTAS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                const Params p) {
     using C = Cfg<TILE_T, TILE_F>;
