@@ -6,8 +6,24 @@
 // one output row per block and one token per launch (matvec_kernel,
 // cuda/kipp_kernels.cu:93; src/kipp.c:2233-2243).
 //
-// The sum over k runs in the same order for every output element whatever M
-// is, so a token's result does not depend on what else is in the batch.
+// The sum over k runs in the same order for every output element whatever M is, so a token's result does
+// not depend on what else is in the batch: K is cut into at most 16 runs whose length depends on K alone
+// (run_length), a run is one chain of FMAs in the order of k, and the runs are added in their order.  The
+// runs are what lets a few tokens be multiplied by many threads at once.
+//
+// Three kernels, chosen by shape alone, with that one order:
+//   few   float32, up to FEW_MAX tokens: bound by the weights' bytes (a token is 2 operations per 4 bytes).  A
+//         block holds 16 features, a thread one feature and one run, so a 2,048-feature matrix still
+//         gives 128 blocks of 256 chains; the weights travel by asynchronous copies, five chunks of 64 bytes
+//         per thread on their way, the first of them before the wait for the kernel before.  12,288 x 2,048 with
+//         1, 3 and 16 tokens: 24, 34 and 94 us (100 MB: 15 us of copy rate; the kernel below, which ran before: 334, 339
+//         and 353); 2,048 x 6,144 with 3: 30 us (543).  At 32 tokens its two passes still win where the features are
+//         few (2,048 x 2,048: 31 us against 88 in tiles) and tie where they are many (12,288: 176 against 174).
+//   tile  float32, more tokens: bound by the FMA pipes.  64 x 64 outputs per block of 128 threads, 8 x 4 per
+//         thread, operands in shared memory as they lie in memory (16 bytes of k per row and
+//         thread), three stages of asynchronous copies.  407 tokens, 12,288 x 2,048: 608 us (34 TFLOP/s; 943 us before), 2,048 x 6,144: 540 us (866).
+//   any   what is left: bfloat16 operands of shapes that the tensor-core kernels refuse, and float32 rows that do
+//         not start on 16 bytes.
 //
 // Epilogues:
 //   STORE   C[m,n]    = acc                 (C in float32 or bfloat16)
@@ -23,6 +39,22 @@
 namespace {
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
+// K in runs: at most MAX_RUNS of them, each of a length that is a multiple of BK.
+constexpr int MAX_RUNS = 16;
+__host__ __device__ inline int run_length(int K) {
+    const int per = (K + MAX_RUNS - 1) / MAX_RUNS;
+    return (per + BK - 1) / BK * BK;
+}
+
+// One finished sum per element, or a gate and up pair of it, into C.
+template <typename TC, int EPI>
+__device__ __forceinline__ void put(TC* C, int ldc, int m, int n, float v) {
+    const size_t idx = (size_t)m * ldc + n;
+    if (EPI == EPI_ADD) C[idx] = from_f32<TC>(to_f32(C[idx]) + v);
+    else C[idx] = from_f32<TC>(v);
+}
+__device__ __forceinline__ float swiglu(float g, float u) { return g / (1.0f + expf(-g)) * u; }
+
 template <typename TA, typename TW, typename TC, int EPI>
 __global__ void __launch_bounds__(256)
 gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restrict__ W,
@@ -34,11 +66,12 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[TM][TN];
+    const int run = run_length(K);
+    float acc[TM][TN], sum[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) acc[i][j] = sum[i][j] = 0.f;
 
     // 64x16 tile = 1024 elements, 256 threads -> 4 each; thread loads row
     // (tid / 4), k columns (tid % 4) * 4 .. + 3.
@@ -65,32 +98,233 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
                 for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
         __syncthreads();
+        if ((k0 + BK) % run == 0 || k0 + BK >= K) {
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) {
+                    sum[i][j] += acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+        }
     }
 
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int m = m0 + ty * TM + i;
         if (m >= M) continue;
-        if (EPI == EPI_SWIGLU) {
 #pragma unroll
-            for (int j = 0; j < TN; j += 2) {
-                const int n = n0 + tx * TN + j;
-                if (n + 1 < N) {
-                    const float g = acc[i][j], u = acc[i][j + 1];
-                    C[(size_t)m * ldc + (n >> 1)] = from_f32<TC>(g / (1.0f + expf(-g)) * u);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const int n = n0 + tx * TN + j;
-                if (n >= N) continue;
-                const size_t idx = (size_t)m * ldc + n;
-                if (EPI == EPI_ADD) C[idx] = from_f32<TC>(to_f32(C[idx]) + acc[i][j]);
-                else C[idx] = from_f32<TC>(acc[i][j]);
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + tx * TN + j;
+            if (EPI == EPI_SWIGLU) {
+                if ((j & 1) == 0 && n + 1 < N) put<TC, EPI_STORE>(C, ldc, m, n >> 1, swiglu(sum[i][j], sum[i][j + 1]));
+            } else if (n < N) {
+                put<TC, EPI>(C, ldc, m, n, sum[i][j]);
             }
         }
     }
+}
+
+// ---------------------------------------------------------------------------------------
+// Few tokens (see the head of the file).  Warp w of a block holds runs 2w and 2w + 1 of the block's 16
+// features; a warp copies only what its own lanes read, so its ring needs no block-wide barrier.
+constexpr int FEW_F = 16, FEW_STAGES = 5, FEW_THREADS = 16 * MAX_RUNS, FEW_MAX = 32;
+constexpr int FEW_CHUNK = BK * 4 + 16;              // 64 bytes of a feature's row, padded against bank conflicts
+constexpr int FEW_SMEM = (FEW_THREADS / 32) * FEW_STAGES * 32 * FEW_CHUNK;
+
+template <int MT, int EPI>
+__global__ void __launch_bounds__(FEW_THREADS)
+gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
+                int M, int N, int K, int lda, int ldw, int ldc) {
+    extern __shared__ __align__(16) uint8_t ring[];
+    __shared__ float parts[MAX_RUNS][MT][FEW_F + 1];
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n0 = blockIdx.x * FEW_F, m0 = blockIdx.y * MT;
+    const int run = run_length(K), steps = run / BK;
+    uint8_t* mine = ring + (size_t)warp * FEW_STAGES * 32 * FEW_CHUNK;
+    // copy j of a step: 16 bytes (lane & 3) of chunk 8 j + lane / 4; chunk c is feature c & 15 of run 2 warp + c / 16
+    auto fetch = [&](int step, int stage) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int c = 8 * j + (lane >> 2), n = n0 + (c & 15);
+            const int k = (2 * warp + (c >> 4)) * run + step * BK + (lane & 3) * 4;
+            const bool in = n < N && k < K;
+            cp_async16(smem_address(mine + (size_t)(stage * 32 + c) * FEW_CHUNK + (lane & 3) * 16),
+                       in ? W + (size_t)n * ldw + k : W, in ? 16 : 0);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < FEW_STAGES - 1; ++s) {
+        if (s < steps) fetch(s, s);
+        cp_async_commit();
+    }
+    pdl_wait();
+    const int r = 2 * warp + (lane >> 4);                 // this thread's run of feature lane & 15
+    const float* x[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) x[m] = A + (size_t)min(m0 + m, M - 1) * lda;
+    float acc[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) acc[m] = 0.f;
+    for (int step = 0; step < steps; ++step) {
+        cp_async_wait<FEW_STAGES - 2>();
+        __syncwarp();
+        const int k0 = r * run + step * BK;
+        const uint8_t* chunk = mine + (size_t)((step % FEW_STAGES) * 32 + lane) * FEW_CHUNK;
+#pragma unroll
+        for (int q = 0; q < BK / 4; ++q) {
+            if (k0 + 4 * q >= K) break;                   // whole quarters: K is a multiple of 4
+            const float4 w = *reinterpret_cast<const float4*>(chunk + 16 * q);
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float4 v = *reinterpret_cast<const float4*>(x[m] + k0 + 4 * q);
+                acc[m] = fmaf(v.x, w.x, acc[m]);
+                acc[m] = fmaf(v.y, w.y, acc[m]);
+                acc[m] = fmaf(v.z, w.z, acc[m]);
+                acc[m] = fmaf(v.w, w.w, acc[m]);
+            }
+        }
+        __syncwarp();                                     // the stage before this one is read: fill it again
+        if (step + FEW_STAGES - 1 < steps) fetch(step + FEW_STAGES - 1, (step + FEW_STAGES - 1) % FEW_STAGES);
+        cp_async_commit();
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int m = 0; m < MT; ++m) parts[r][m][lane & 15] = acc[m];
+    __syncthreads();
+    const int runs = (K + run - 1) / run;
+    for (int i = threadIdx.x; i < MT * FEW_F; i += FEW_THREADS) {
+        const int f = i % FEW_F, m = i / FEW_F, n = n0 + f;
+        if (m0 + m >= M) break;
+        float v = 0.f, u = 0.f;
+        if (EPI == EPI_SWIGLU) {
+            if ((f & 1) || n + 1 >= N) continue;
+            for (int s = 0; s < runs; ++s) { v += parts[s][m][f]; u += parts[s][m][f + 1]; }
+            put<float, EPI_STORE>(C, ldc, m0 + m, n >> 1, swiglu(v, u));
+        } else if (n < N) {
+            for (int s = 0; s < runs; ++s) v += parts[s][m][f];
+            put<float, EPI>(C, ldc, m0 + m, n, v);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// Many tokens.  Thread (tx, ty) has the outputs of tokens ty + 8 i and features tx + 16 j: the
+// rows that a warp reads together lie next to one another, 80 bytes apart, so 16-byte reads meet
+// every bank once.
+constexpr int TILE_M = 64, TILE_N = 64, TILE_STAGES = 3, TILE_THREADS = 128, TILE_ROW = BK + 4;
+constexpr int TILE_SMEM = TILE_STAGES * (TILE_M + TILE_N) * TILE_ROW * 4;
+
+template <int EPI>
+__global__ void __launch_bounds__(TILE_THREADS)
+gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
+                 int M, int N, int K, int lda, int ldw, int ldc) {
+    extern __shared__ __align__(16) float tiles[];        // [stage][A rows, W rows][TILE_ROW]
+    pdl_launch_dependents();
+    pdl_wait();
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int m0 = blockIdx.y * TILE_M, n0 = blockIdx.x * TILE_N;
+    const int run = run_length(K), steps = (K + BK - 1) / BK;
+    auto fetch = [&](int step, int stage) {
+        float* to = tiles + (size_t)stage * (TILE_M + TILE_N) * TILE_ROW;
+#pragma unroll
+        for (int j = 0; j < (TILE_M + TILE_N) * 4 / TILE_THREADS; ++j) {
+            const int c = j * TILE_THREADS + tid, row = c >> 2, k = step * BK + (c & 3) * 4;
+            const bool of_a = row < TILE_M;
+            const int at = of_a ? m0 + row : n0 + row - TILE_M;
+            const bool in = k < K && at < (of_a ? M : N);
+            const float* src = of_a ? A + (size_t)at * lda + k : W + (size_t)at * ldw + k;
+            cp_async16(smem_address(to + row * TILE_ROW + (c & 3) * 4), in ? src : W, in ? 16 : 0);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < TILE_STAGES - 1; ++s) {
+        if (s < steps) fetch(s, s);
+        cp_async_commit();
+    }
+    float acc[8][4], sum[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = sum[i][j] = 0.f;
+    for (int step = 0; step < steps; ++step) {
+        cp_async_wait<TILE_STAGES - 2>();
+        __syncthreads();                                  // this stage has landed, the one before is read by all
+        if (step + TILE_STAGES - 1 < steps) fetch(step + TILE_STAGES - 1, (step + TILE_STAGES - 1) % TILE_STAGES);
+        cp_async_commit();
+        const float* a = tiles + (size_t)(step % TILE_STAGES) * (TILE_M + TILE_N) * TILE_ROW;
+        const float* b = a + TILE_M * TILE_ROW;
+#pragma unroll
+        for (int q = 0; q < BK / 4; ++q) {
+            float4 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(b + (tx + 16 * j) * TILE_ROW + 4 * q);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 v = *reinterpret_cast<const float4*>(a + (ty + 8 * i) * TILE_ROW + 4 * q);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[i][j] = fmaf(v.x, w[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(v.y, w[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(v.z, w[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(v.w, w[j].w, acc[i][j]);
+                }
+            }
+        }
+        if (((step + 1) * BK) % run == 0 || step + 1 == steps) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    sum[i][j] += acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+        }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + ty + 8 * i;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + tx + 16 * j;
+            if (EPI == EPI_SWIGLU) {
+                const float u = __shfl_xor_sync(0xffffffffu, sum[i][j], 1);      // an even lane's neighbour has the up row
+                if ((tx & 1) == 0 && m < M && n + 1 < N) put<float, EPI_STORE>(C, ldc, m, n >> 1, swiglu(sum[i][j], u));
+            } else if (m < M && n < N) {
+                put<float, EPI>(C, ldc, m, n, sum[i][j]);
+            }
+        }
+    }
+}
+
+template <int MT, int EPI>
+int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    return kipp_launch(gemm_few_kernel<MT, EPI>, dim3((N + FEW_F - 1) / FEW_F, (M + MT - 1) / MT), dim3(FEW_THREADS),
+                       FEW_SMEM, s, 1, C, A, W, M, N, K, lda, ldw, ldc);
+}
+
+// float32 rows that start on 16 bytes and hold whole groups of four: the kernels that copy 16 bytes at a time.
+template <int EPI>
+int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+    if (M <= FEW_MAX) {
+        // tokens of a block: as many as there are, up to 16 (the accumulators of a thread)
+        if (M == 1) return launch_few<1, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
+        if (M == 2) return launch_few<2, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
+        if (M <= 4) return launch_few<4, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
+        if (M <= 8) return launch_few<8, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
+        return launch_few<16, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
+    }
+    const dim3 grid((N + TILE_N - 1) / TILE_N, (M + TILE_M - 1) / TILE_M);
+    if (grid.y > 65535) return KIPP_ERR_ARG;
+    return kipp_launch(gemm_tile_kernel<EPI>, grid, dim3(TILE_THREADS), TILE_SMEM, s, 1, C, A, W, M, N, K, lda, ldw, ldc);
 }
 
 template <typename TA, typename TW, typename TC>
@@ -123,6 +357,13 @@ extern "C" int kipp_gemm_simt(void* C, int out_dtype, const void* A, const void*
     if (K <= 0) return KIPP_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     if (epilogue == EPI_ADD && out_dtype != KIPP_DT_F32) return KIPP_ERR_DTYPE;
+    const bool vectors = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    if (in_dtype == KIPP_DT_F32 && out_dtype == KIPP_DT_F32 && vectors) {
+        if (epilogue == EPI_STORE) return launch_f32<EPI_STORE>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, s);
+        if (epilogue == EPI_ADD) return launch_f32<EPI_ADD>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, s);
+        if (epilogue == EPI_SWIGLU && N % 2 == 0)
+            return launch_f32<EPI_SWIGLU>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, s);
+    }
     if (in_dtype == KIPP_DT_F32 && out_dtype == KIPP_DT_F32)
         return launch<float, float, float>(C, A, W, M, N, K, lda, ldw, ldc, epilogue, s);
     if (in_dtype == KIPP_DT_BF16 && out_dtype == KIPP_DT_F32)

@@ -105,6 +105,34 @@ def test_gemm_simt(dtype, shape, epilogue):
 
 
 @pytest.mark.parametrize("epilogue", ["store", "add", "swiglu"])
+@pytest.mark.parametrize("shape", [(130, 20), (18, 136), (66, 260), (2, 1028), (34, 2064)])
+def test_gemm_32_bit_kernels_agree(shape, epilogue):
+    """The 32-bit product's three kernels add in one order: the rows of a batch have the same bits whether 1, 3,
+    16, 17, 32 (the kernel for few tokens, at its block sizes and the last count it takes), 33 or 70 of them (tiles)
+    are multiplied at once, and where rows do not start on 16 bytes.  The K reach from one run of 16 to runs that
+    end inside a tile; the error against float64 stays under that of one chain of K roundings, K eps |a| |w|."""
+    N, K = shape
+    M = 70
+    g = torch.Generator().manual_seed(N + K)
+    a, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    base = torch.randn(M, N // 2 if epilogue == "swiglu" else N, generator=g).to(DEV)
+    whole = base.clone()
+    ops().gemm(whole, a, w, epilogue, impl="simt")
+    if epilogue != "swiglu":
+        bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()) + 2.0 ** -23 * whole.double().abs()
+        assert ((whole.double().cpu() - gemm_ref(a, w, epilogue, base)).abs() <= bound.cpu()).all()
+    for m in (1, 2, 3, 5, 16, 17, 32, 33):
+        some = base[:m].clone()
+        ops().gemm(some, a[:m], w, epilogue, impl="simt")
+        assert torch.equal(some, whole[:m]), m
+    odd = torch.zeros(M, K + 1, device=DEV)[:, :K]
+    odd.copy_(a)
+    some = base.clone()
+    ops().gemm(some, odd, w, epilogue, impl="simt")
+    assert torch.equal(some, whole)
+
+
+@pytest.mark.parametrize("epilogue", ["store", "add", "swiglu"])
 @pytest.mark.parametrize("shape", [(1, 128, 64), (8, 256, 128), (17, 250, 192), (64, 1000, 136),
                                    (100, 384, 2568), (300, 640, 520), (5, 2560, 1216), (40, 14400, 136),
                                    (100, 14400, 72)])
@@ -525,7 +553,8 @@ LAYOUTS = [[(0, 70), (130, 1), (5, 2), (63, 66), (300, 1)],
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("window", [None, 37])
 @pytest.mark.parametrize("shape", [dict(D=16, nq=4, nkv=2, page=16), dict(D=48, nq=6, nkv=3, page=8),
-                                   dict(D=128, nq=8, nkv=1, page=4), dict(D=256, nq=2, nkv=2, page=32)])
+                                   dict(D=128, nq=8, nkv=1, page=4), dict(D=256, nq=2, nkv=2, page=32),
+                                   dict(D=20, nq=10, nkv=1, page=16), dict(D=7, nq=3, nkv=1, page=8)])
 def test_attention_simt(shape, window, dtype):
     D, nq, nkv, page = shape["D"], shape["nq"], shape["nkv"], shape["page"]
     for li, layout in enumerate(LAYOUTS[:2] + LAYOUTS[3:]):
@@ -756,6 +785,39 @@ def test_sample_rows_draws_the_plain_sampler_tokens(vocab):
                              torch.tensor(uni, dtype=torch.float64, device=DEV)).cpu().tolist()
         assert got == want, (trial, got, want)
         state = state * 7 + 13
+
+
+def test_sample_rows_with_buckets_longer_than_a_blocks_list():
+    """Rows whose candidates share one value or a few (more than the 4,096 that a block lists, so the passes
+    after the first go over the whole row again), a top-k just under, at and above that number, and a set that empties
+    but for its first: the tokens of the plain sampler."""
+    from kipp_b200.kernels import sampling as ks
+    n = 40000
+    logits = torch.zeros(6, n)
+    logits[1, ::2] = 1e-7                                       # two values a rounding apart
+    logits[2] = torch.arange(n) % 3 * 0.5
+    logits[3:] = torch.randn(3, n, generator=torch.Generator().manual_seed(3)) * 1e-3
+    k = [0, 9000, 0, 4095, 4096, 4097]
+    top_p, min_p = [0.7, 1.0, 0.3, 0.9, 1.0, 0.9], [0.0, 0.0, 1.0, 0.0, 0.5, 0.0]
+    for u in (0.0, 0.3, 0.999):
+        want = []
+        for r in range(6):
+            # the uniform number comes from the state's first draw: look for the token by its definition instead
+            order = np.lexsort((np.arange(n), -logits[r].numpy().astype(np.float64)))
+            order = order[: k[r] or n]
+            w = np.exp((logits[r].numpy()[order] - logits[r].numpy()[order[0]]).astype(np.float32)).astype(np.float64)
+            keep = w >= min_p[r]
+            order, w = order[keep], w[keep]
+            c = np.cumsum(w)
+            last = int(np.searchsorted(c, top_p[r] * c[-1])) if top_p[r] < 1 else len(w) - 1
+            want.append((order, c, u * c[min(last, len(w) - 1)]))
+        got = ks.sample_rows(logits.to(DEV), torch.ones(6, device=DEV), torch.tensor(k, dtype=torch.int32, device=DEV),
+                             torch.tensor(top_p, device=DEV), torch.tensor(min_p, device=DEV),
+                             torch.full((6,), u, dtype=torch.float64, device=DEV)).cpu().tolist()
+        for r, (order, c, draw) in enumerate(want):
+            # the running sums of 40,000 weights are exact to 2^-23 of their unit: the token or its neighbour
+            at = int(np.nonzero(order == got[r])[0][0])
+            assert c[at] >= draw - 1e-2 and (at == 0 or c[at - 1] <= draw + 1e-2), (u, r, got[r])
 
 
 def test_penalties_and_bias_match_the_reference_sampler():
