@@ -22,6 +22,15 @@
 // reference keeps a running double sum, so a draw that lies within 2^-23 of a
 // boundary may pick the neighbour.
 //
+// A pass over the row is what costs (a 151,936-entry row is 600 KB, and each of its entries takes some
+// forty instructions in a pass that adds weights), so there are few: the first pass of a selection also
+// gives the total that its target is a share of; its second pass, which looks at one bucket of the
+// first, puts that bucket's elements into a list in shared memory, and the passes after it walk the
+// list; and what top-k leaves is listed once for everything that follows.  64 rows of 151,936, half of
+// them with top-k 50, top-p 0.95: 588 us (934 with all passes over the rows
+// and the loads one at a time); a single such row by eight blocks: 170 us (221).  What is left is the aggregation
+// of equal buckets within a warp.
+//
 // Also here: the penalties and logit bias the reference applies before
 // sampling (apply_bias_and_penalties, src/kipp.c:3386-3431).
 #include "common.cuh"
@@ -58,14 +67,17 @@ __device__ __forceinline__ float team_ld_f32(const void* p, int rank) {
 __device__ __forceinline__ unsigned long long team_ld_u64(const void* p, int rank) {
     unsigned long long v; asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(team_addr(p, rank)) : "memory"); return v;
 }
-__device__ __forceinline__ double team_ld_f64(const void* p, int rank) {
-    double v; asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(team_addr(p, rank)) : "memory"); return v;
-}
+
+constexpr int LIST_CAP = 4096;  // elements a block lists: 16 KB
+constexpr int COPIES = 4;       // histograms of a block, one for every fourth warp: most elements of a first pass meet a
+                                // handful of buckets, and atomics on one word run one after the other
 
 struct RowCtx {
     const float* v;
     int n;
     int lo, hi;                 // this block's part of the row
+    int* list;                  // [LIST_CAP] in shared memory
+    int listed;                 // >= 0: the elements to walk are the first `listed` of the list
     float inv_t, smax, cutoff;
     // filters
     bool has_topk;   unsigned topk_key, topk_tok;
@@ -77,23 +89,27 @@ __device__ __forceinline__ bool before_or_at(unsigned key, unsigned tok, unsigne
     return key < bkey || (key == bkey && tok <= btok);
 }
 
-// Whether element i is in the current candidate set; gives its key and weight.
-__device__ __forceinline__ bool member(const RowCtx& c, int i, unsigned& key, float& w) {
-    const float scaled = c.v[i] * c.inv_t;
+// Whether element i of value x passes every filter but min-p, which wants the weight; gives its key.
+__device__ __forceinline__ bool candidate(const RowCtx& c, int i, float x, unsigned& key) {
+    const float scaled = x * c.inv_t;
     if (!(scaled >= c.cutoff)) return false;
     key = desc_key(scaled);
     if (c.has_topk && !before_or_at(key, (unsigned)i, c.topk_key, c.topk_tok)) return false;
-    w = expf(scaled - c.smax);
-    if (c.has_minp && (double)w < c.minp_threshold) return false;
-    if (c.has_nucleus && !before_or_at(key, (unsigned)i, c.nuc_key, c.nuc_tok)) return false;
-    return true;
+    return !c.has_nucleus || before_or_at(key, (unsigned)i, c.nuc_key, c.nuc_tok);
+}
+__device__ __forceinline__ bool weighs(const RowCtx& c, float x, float& w) {
+    w = expf(x * c.inv_t - c.smax);
+    return !c.has_minp || !((double)w < c.minp_threshold);
 }
 
 struct Shared {
-    unsigned cnt[256];          // this block's part of the row
-    unsigned long long wfix[256];   // weight sums in units of 2^-40 (see weight_units)
+    unsigned cnt[COPIES][256];  // this block's part of the row
+    unsigned long long wfix[COPIES][256];   // weight sums in units of 2^-40 (see weight_units)
     unsigned cnt_all[256];      // the team's: the blocks' parts added in block order
     double wsum_all[256];
+    unsigned long long units_all[256];
+    int listed;                 // elements appended to the list
+    double total;
     float red_val[32];
     int red_idx[32];
     double red_d[32];
@@ -124,20 +140,52 @@ __device__ __forceinline__ unsigned long long peers_sum(unsigned peers, unsigned
     return ((unsigned long long)hi << 20) + lo;
 }
 
-// One histogram pass.  level 0..3: value key digits (high to low); level 4..7:
-// token digits among elements whose key == prefix_key.
-__device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned prefix_key,
-                               unsigned prefix_tok) {
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) { sh.cnt[b] = 0; sh.wfix[b] = 0ull; }
-    __syncthreads();
-    // whole warps walk the part (every lane makes every round): the lanes of a round that fall
-    // into one bucket are found with match.any and add as one
+// Calls f(i, x, there) for every element of this block's part (or list), by whole warps: all lanes
+// of a warp together, `there` false where a lane has none.  Several loads are on their way at a time.
+template <typename F> __device__ __forceinline__ void walk(const RowCtx& c, F f) {
+    constexpr int AT_ONCE = 8;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const bool list = c.listed >= 0;
+    const int n = list ? c.listed : c.hi - c.lo;
+    for (int base = warp * 32; base < n; base += warps * 32 * AT_ONCE) {
+        int i[AT_ONCE]; float x[AT_ONCE];
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) {
+            const int at = base + 32 * warps * u + lane;
+            i[u] = at >= n ? -1 : list ? c.list[at] : c.lo + at;
+            x[u] = i[u] < 0 ? 0.f : c.v[i[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) {
+            if (base + 32 * warps * u >= n) break;
+            f(i[u], x[u], i[u] >= 0);
+        }
+    }
+}
+// Appends the lanes' elements to the block's list (the caller knows that they fit; whole warps).
+__device__ __forceinline__ void append(const RowCtx& c, Shared& sh, int i, bool there) {
     const int lane = threadIdx.x & 31;
-    for (int base = c.lo + (int)(threadIdx.x - lane); base < c.hi; base += blockDim.x) {
-        const int i = base + lane;
+    const unsigned who = __ballot_sync(0xffffffffu, there);
+    if (who == 0) return;
+    int at = 0;
+    if (lane == __ffs(who) - 1) at = atomicAdd(&sh.listed, __popc(who));
+    at = __shfl_sync(0xffffffffu, at, __ffs(who) - 1) + __popc(who & ((1u << lane) - 1u));
+    if (there) c.list[at] = i;
+}
+
+// One histogram pass.  level 0..3: value key digits (high to low); level 4..7:
+// token digits among elements whose key == prefix_key.  `gather`: what lies under the prefix is listed too.
+__device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned prefix_key,
+                               unsigned prefix_tok, bool gather) {
+    for (int b = threadIdx.x; b < COPIES * 256; b += blockDim.x) { (&sh.cnt[0][0])[b] = 0; (&sh.wfix[0][0])[b] = 0ull; }
+    if (threadIdx.x == 0) sh.listed = 0;
+    __syncthreads();
+    // the lanes of a round that fall into one bucket are found with match.any and add as one
+    const int lane = threadIdx.x & 31, copy = (threadIdx.x >> 5) % COPIES;
+    walk(c, [&](int i, float x, bool there) {
         unsigned key = 0; float w = 0.f;
         unsigned digit = 256u;                                  // no bucket: not in the set at this level
-        if (i < c.hi && member(c, i, key, w)) {
+        if (there && candidate(c, i, x, key)) {
             if (level < 4) {
                 const int shift = 24 - 8 * level;
                 if (level == 0 || (key >> (shift + 8)) == (prefix_key >> (shift + 8))) digit = (key >> shift) & 0xffu;
@@ -146,15 +194,22 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
                 const unsigned tok = (unsigned)i;
                 if (level == 4 || (tok >> (shift + 8)) == (prefix_tok >> (shift + 8))) digit = (tok >> shift) & 0xffu;
             }
+            if (digit < 256u && !weighs(c, x, w)) digit = 256u;
         }
+        if (gather) append(c, sh, i, digit < 256u);
+        if (!__any_sync(0xffffffffu, digit < 256u)) return;
         const unsigned peers = __match_any_sync(0xffffffffu, digit);
         const unsigned long long units = peers_sum(peers, digit < 256u ? weight_units(w) : 0ull);
         if (digit < 256u && lane == __ffs(peers) - 1) {
-            atomicAdd(&sh.cnt[digit], (unsigned)__popc(peers));
-            atomicAdd(&sh.wfix[digit], units);
+            atomicAdd(&sh.cnt[copy][digit], (unsigned)__popc(peers));
+            atomicAdd(&sh.wfix[copy][digit], units);
         }
-    }
+    });
     __syncthreads();
+    for (int b = threadIdx.x; b < 256; b += blockDim.x) {
+#pragma unroll
+        for (int k = 1; k < COPIES; ++k) { sh.cnt[0][b] += sh.cnt[k][b]; sh.wfix[0][b] += sh.wfix[k][b]; }
+    }
     // the team's histogram: every block adds the blocks' parts in block order
     team_sync();
     const int blocks = team_size();
@@ -162,13 +217,13 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
         unsigned n8[8]; unsigned long long w8[8];    // all loads first: they travel together
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-            n8[r] = r < blocks ? team_ld_u32(&sh.cnt[b], r) : 0u;
-            w8[r] = r < blocks ? team_ld_u64(&sh.wfix[b], r) : 0ull;
+            n8[r] = r < blocks ? team_ld_u32(&sh.cnt[0][b], r) : 0u;
+            w8[r] = r < blocks ? team_ld_u64(&sh.wfix[0][b], r) : 0ull;
         }
         unsigned n = 0; unsigned long long w = 0ull;
 #pragma unroll
         for (int r = 0; r < 8; ++r) { n += n8[r]; w += w8[r]; }
-        sh.cnt_all[b] = n; sh.wsum_all[b] = (double)w * WEIGHT_UNIT;
+        sh.cnt_all[b] = n; sh.wsum_all[b] = (double)w * WEIGHT_UNIT; sh.units_all[b] = w;
     }
     team_sync();                                   // nobody clears its part while another still reads it
 }
@@ -177,16 +232,31 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
 //   MODE_COUNT: the element with 1-based rank `target_count`;
 //   MODE_W_GE : the first element whose inclusive weight sum >= target_w;
 //   MODE_W_GT : the first element whose inclusive weight sum >  target_w.
+// With `of_total` target_w is a share of the set's total weight, which `total` gives in any case.
 // If no element qualifies, the last element of the set is returned.
 // Outputs (uniform over the block): key, token, inclusive weight sum at it.
-__device__ void select(const RowCtx& c, Shared& sh, int mode, unsigned long long target_count,
-                       double target_w, unsigned& out_key, unsigned& out_tok, double& out_cum) {
+__device__ void select(RowCtx& c, Shared& sh, int mode, unsigned long long target_count, double target_w, bool of_total,
+                       unsigned& out_key, unsigned& out_tok, double& out_cum, double& total) {
+    const int listed_before = c.listed;
+    unsigned part_cnt = 0;                            // elements of this block's part under the prefix
     unsigned prefix_key = 0, prefix_tok = 0;
     unsigned long long cnt_before = 0;
     double w_before = 0.0;
     for (int level = 0; level < 8; ++level) {
-        histogram_pass(c, sh, level, prefix_key, prefix_tok);
+        const bool gather = level > 0 && c.listed < 0 && part_cnt <= LIST_CAP;
+        histogram_pass(c, sh, level, prefix_key, prefix_tok, gather);
+        if (gather) c.listed = sh.listed;
         if (threadIdx.x < 32) {
+            if (level == 0) {
+                unsigned long long all = 0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) all += sh.units_all[8 * threadIdx.x + j];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+                const double sum = (double)all * WEIGHT_UNIT;
+                if (of_total) target_w *= sum;
+                if (threadIdx.x == 0) sh.total = sum;
+            }
             // The first bucket (in order) at which the running count or weight reaches the target,
             // else the last bucket that is not empty.  One warp: a lane walks over its eight
             // buckets from the sums of the lanes before it (one thread alone took 256 dependent
@@ -245,37 +315,50 @@ __device__ void select(const RowCtx& c, Shared& sh, int mode, unsigned long long
         cnt_before = sh.sel_cnt_before; w_before = sh.sel_w_before;
         const double cum_incl = sh.d_val;
         const unsigned bucket_cnt = sh.sel_bucket_cnt;
+        if (level == 0) total = sh.total;
+        part_cnt = chosen < 0 ? 0 : sh.cnt[0][chosen];
         __syncthreads();
-        if (chosen < 0) { out_key = 0xffffffffu; out_tok = 0; out_cum = w_before; return; }  // empty set
+        if (chosen < 0) { out_key = 0xffffffffu; out_tok = 0; out_cum = w_before; break; }  // empty set
         const int shift = 24 - 8 * (level & 3);
         if (level < 4) prefix_key |= (unsigned)chosen << shift;
         else prefix_tok |= (unsigned)chosen << shift;
-        if (level == 7) { out_key = prefix_key; out_tok = prefix_tok; out_cum = cum_incl; return; }
+        if (level == 7) { out_key = prefix_key; out_tok = prefix_tok; out_cum = cum_incl; break; }
         if (level == 3 && bucket_cnt == 1) {
             // One element has this value: find its token in one pass.
             if (threadIdx.x == 0) sh.i_val = 0x7fffffff;
             __syncthreads();
-            for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
+            walk(c, [&](int i, float x, bool there) {
                 unsigned key; float w;
-                if (member(c, i, key, w) && key == prefix_key) atomicMin(&sh.i_val, i);
-            }
+                if (there && candidate(c, i, x, key) && key == prefix_key && weighs(c, x, w)) atomicMin(&sh.i_val, i);
+            });
             __syncthreads();
             team_sync();
             int first = 0x7fffffff;
             for (int r = 0; r < team_size(); ++r) first = min(first, (int)team_ld_u32(&sh.i_val, r));
             team_sync();
             out_key = prefix_key; out_tok = (unsigned)first; out_cum = cum_incl;
-            return;
+            break;
         }
     }
+    c.listed = listed_before;
 }
 
 // best_i = 0x7fffffff when the row holds no number (NaN only)
 __device__ void block_argmax_raw(const float* v, int n, Shared& sh, float& best_v, int& best_i) {
     float bv = -INFINITY; int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const float x = v[i];
-        if (x > bv || (x == bv && i < bi)) { bv = x; bi = i; }
+    constexpr int AT_ONCE = 8;                        // loads on their way
+    for (int i0 = threadIdx.x; i0 < n; i0 += AT_ONCE * blockDim.x) {
+        float x[AT_ONCE];
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) {
+            const int i = i0 + u * (int)blockDim.x;
+            x[u] = i < n ? v[i] : -INFINITY;
+        }
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u) {
+            const int i = i0 + u * (int)blockDim.x;
+            if (i < n && (x[u] > bv || (x[u] == bv && i < bi))) { bv = x[u]; bi = i; }
+        }
     }
     // A row of NaNs or -inf leaves bi unset in some threads; index 0 then wins
     // as in the reference (argmax starts at 0 and only '>' replaces it).
@@ -359,36 +442,13 @@ __global__ void argmax_merge_kernel(const ArgmaxPart* __restrict__ parts, int n_
     if (threadIdx.x == 0) out[blockIdx.x] = bi == 0x7fffffff ? 0 : bi;
 }
 
-// The sum of the weights of the current set: the blocks' sums added in block order.
-__device__ double team_weight_sum(const RowCtx& c, Shared& sh) {
-    unsigned long long local = 0ull;
-    for (int i = c.lo + threadIdx.x; i < c.hi; i += blockDim.x) {
-        unsigned kk; float w;
-        if (member(c, i, kk, w)) local += weight_units(w);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-    if ((threadIdx.x & 31) == 0) sh.red_u[threadIdx.x >> 5] = local;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long t = 0ull;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh.red_u[w];
-        sh.u_val = t;
-    }
-    __syncthreads();
-    team_sync();
-    unsigned long long total = 0ull;
-    for (int b = 0; b < team_size(); ++b) total += team_ld_u64(&sh.u_val, b);
-    team_sync();
-    return (double)total * WEIGHT_UNIT;
-}
-
 __global__ void __launch_bounds__(THREADS)
 sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
                    const float* __restrict__ temperature, const int* __restrict__ top_k,
                    const float* __restrict__ top_p, const float* __restrict__ min_p,
                    const double* __restrict__ uniform, int* __restrict__ out) {
     __shared__ Shared sh;
+    __shared__ int list[LIST_CAP];
     pdl_launch_dependents();
     pdl_wait();
     const int blocks = team_size(), rank = team_rank();
@@ -416,7 +476,7 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
         return;
     }
     RowCtx c;
-    c.v = v; c.n = n; c.lo = lo; c.hi = hi;
+    c.v = v; c.n = n; c.lo = lo; c.hi = hi; c.list = list; c.listed = -1;
     c.inv_t = 1.0f / T;
     c.smax = v[best_i] * c.inv_t;
     c.cutoff = c.smax - 20.0f;
@@ -424,12 +484,23 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
     c.topk_key = c.topk_tok = c.nuc_key = c.nuc_tok = 0;
     c.minp_threshold = 0.0;
 
-    unsigned key, tok; double cum;
+    unsigned key, tok; double cum, total;
     const int k = top_k[r];
     if (k > 0) {
         // rank k in the order, or the last candidate when there are fewer
-        select(c, sh, MODE_COUNT, (unsigned long long)k, 0.0, key, tok, cum);
+        select(c, sh, MODE_COUNT, (unsigned long long)k, 0.0, false, key, tok, cum, total);
         c.has_topk = true; c.topk_key = key; c.topk_tok = tok;
+        if (k <= LIST_CAP) {                           // what is left is k elements at most
+            if (threadIdx.x == 0) sh.listed = 0;
+            __syncthreads();
+            walk(c, [&](int i, float x, bool there) {
+                unsigned kk;
+                append(c, sh, i, there && candidate(c, i, x, kk));
+            });
+            __syncthreads();
+            c.listed = sh.listed;
+            __syncthreads();                           // read by all before the next pass counts anew
+        }
     }
     const float mp = min_p[r];
     if (mp > 0.0f) {
@@ -437,19 +508,18 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
         c.has_minp = true;
         c.minp_threshold = (double)mp * (double)expf(0.0f);
     }
-    // total weight of the set (and, with a nucleus, the prefix that is kept)
+    // with a nucleus, the prefix that is kept, and a share of its weight; else a share of the set's
     const float tp = top_p[r];
     double kept;
     if (tp < 1.0f) {
-        const double total = team_weight_sum(c, sh);
-        select(c, sh, MODE_W_GE, 0, (double)tp * total, key, tok, cum);
+        select(c, sh, MODE_W_GE, 0, (double)tp, true, key, tok, cum, total);
         c.has_nucleus = true; c.nuc_key = key; c.nuc_tok = tok;
         kept = cum;
+        select(c, sh, MODE_W_GT, 0, uniform[r] * kept, false, key, tok, cum, total);
     } else {
-        kept = team_weight_sum(c, sh);
+        select(c, sh, MODE_W_GT, 0, uniform[r], true, key, tok, cum, total);
+        kept = total;
     }
-    const double draw = uniform[r] * kept;
-    select(c, sh, MODE_W_GT, 0, draw, key, tok, cum);
     if (threadIdx.x == 0 && rank == 0) out[r] = (key == 0xffffffffu && tok == 0 && kept == 0.0) ? best_i : (int)tok;
 }
 
