@@ -5,6 +5,7 @@ again; keys far away and at the edges of pages; the sink; the first tokens; a st
 that remembers the first token through long decoding; long decoding through
 graphs; drawn configurations; greedy generation through the scheduler; the command
 line and the trace program."""
+import ctypes
 import json
 import math
 import os
@@ -137,6 +138,42 @@ def test_state_space_alone(name, layer, dtype):
         at += n
     assert at == T
     close(out, want, dtype, f"{name} layer {layer}")
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("state,vdim,heads,groups", [(128, 64, 4, 2), (68, 36, 12, 2), (100, 72, 6, 1)])
+def test_state_space_by_chunks(state, vdim, heads, groups, dtype):
+    """Prompts long enough for the form by chunks of 128 tokens: whole and partial chunks, one of a single token, an entry
+    that ends on a chunk's edge, columns in two slices, heads that share their group's pairs; two steps, so that the
+    second starts from the state that the first left.  Then the same step with one token fewer than the form asks for."""
+    from kipp_b200.config import config_from_dict
+    from kipp_b200.config.registry import get_architecture
+    from kipp_b200.csrc.build import library_path
+    from kipp_b200.engine import Engine, StepEntry
+    from kipp_b200.weights.random_init import random_tensors
+    mixer = {"heads": heads, "groups": groups, "vdim": vdim, "state": state, "conv": 4, "norm_groups": 1}
+    cfg = {"architecture": "Zunilorn", "vocab": 64, "width": 64, "norm": {"eps": 1e-6},
+           "layers": [{"type": "mamba2", "mixer": mixer, "mlp": None}]}
+    spec = get_architecture("Zunilorn").build(config_from_dict(cfg))
+    tensors = dict(random_tensors(spec.tensor_specs(), 5, sigma=0.1, dtype=torch.float32))
+    if dtype == "bfloat16":                            # matrices lie in bfloat16 (the convolution stays 32-bit)
+        tensors = {k: v.bfloat16().float() if v.dim() == 2 and "conv" not in k else v for k, v in tensors.items()}
+    eng = Engine(spec, tensors, dtype=dtype, cache_tokens=4096, max_requests=4, max_batch_tokens=1024, cuda_graphs=False)
+    w = {k: v.double() for k, v in tensors.items()}
+    steps = [[("a", 385), ("b", 1), ("c", 256)], [("b", 300), ("a", 128), ("c", 200)], [("a", 191)]]
+    total = {r: sum(n for st in steps for q, n in st if q == r) for r in "abc"}
+    h = {r: torch.randn(n, 64, generator=torch.Generator().manual_seed(ord(r))).to("cuda", eng.dtype) for r, n in total.items()}
+    want = {r: P.mamba2(mixer, w, "l0.mix.", x.double().cpu(), 1e-6) for r, x in h.items()}
+    at = dict.fromkeys("abc", 0)
+    lib = ctypes.CDLL(library_path("recurrent"))
+    assert [lib.kipp_ssd_by_chunks(len(st), sum(n for _, n in st), heads, groups, state, vdim) for st in steps] == [1, 1, 0]
+    for st in steps:
+        rows = torch.cat([h[r][at[r]:at[r] + n] for r, n in st]).contiguous()
+        out = torch.zeros(len(rows), 64, device="cuda")
+        eng.run_part([StepEntry(r, [0] * n, []) for r, n in st], 0, "mixer", input=rows, residual=out)
+        close(out, torch.cat([want[r][at[r]:at[r] + n] for r, n in st]), dtype, str(st))
+        for r, n in st:
+            at[r] += n
 
 
 def test_the_convolution_starts_from_zeros_in_a_slot_used_again():
