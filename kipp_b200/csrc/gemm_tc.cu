@@ -200,7 +200,8 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
 // true in one lane of the (converged) warp.  The warps that issue copies and products walk
 // their loops and wait as whole warps and let one elected lane issue: with a single lane in a
 // branch of its own the operands of every product come out of that lane's registers, and a
-// product was measured to take 60 to 80 cycles to issue instead of about 40.
+// product was measured to take 60 to 80 cycles to issue instead of about 40.  (2,048 tokens, 2,560 features: the residual
+// add with two products of 144 features per step 62.6 -> 54.5 us on average of K = 4,096 and 9,728, gate/up 163 -> 150.)
 __device__ __forceinline__ bool elect_one() {
     uint32_t chosen;
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(chosen));
@@ -312,6 +313,29 @@ struct Params {
     const float* glu_bias;
     const float* glu_row_gate;
 };
+
+// A token's sum of squares out of its partial sums, in slot order (see Params::ssq_in).  Forty values are on their way
+// at a time: with the compiler's four or eight, the 80 slots of a 2,560-wide row were 10 to 20 trips to the L2, which
+// stood before the cluster's reduction of a few-token product and behind the last tile of a prompt's.
+__device__ __forceinline__ float token_ssq(const Params& p, int t) {
+    const float* row = p.ssq_in + (size_t)t * p.ssq_in_slots;
+    const int n = p.ssq_in_slots;
+    float sum = 0.f;
+    int i = 0;
+    if ((n & 3) == 0 && ((uintptr_t)p.ssq_in & 15) == 0) {
+        constexpr int AT_ONCE = 10;
+        for (; i + 4 * AT_ONCE <= n; i += 4 * AT_ONCE) {
+            float4 v[AT_ONCE];
+#pragma unroll
+            for (int j = 0; j < AT_ONCE; ++j) v[j] = *reinterpret_cast<const float4*>(row + i + 4 * j);
+#pragma unroll
+            for (int j = 0; j < AT_ONCE; ++j) sum = sum + v[j].x + v[j].y + v[j].z + v[j].w;
+        }
+    }
+#pragma unroll 8
+    for (; i < n; ++i) sum += row[i];
+    return sum;
+}
 
 constexpr int GLU_GELU_TANH = 2;      // the code of kipp_activation
 
@@ -550,11 +574,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             // 256 epilogue threads sums token t0 + i's partial sums in slot order
             for (int j = threadIdx.x - 64; j < TILE_T; j += 256) {
                 float sum = 0.f;
-                if (t0 + j < p.tokens) {
-                    const float* row = p.ssq_in + (size_t)(t0 + j) * p.ssq_in_slots;
-#pragma unroll 8
-                    for (int i = 0; i < p.ssq_in_slots; ++i) sum += row[i];
-                }
+                if (t0 + j < p.tokens) sum = token_ssq(p, t0 + j);
                 rstd_s[j] = 1.0f / sqrtf(sum * p.inv_n + p.eps);
             }
             asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -925,12 +945,18 @@ __device__ __forceinline__ void sink_head(const Params& p, uint32_t taddr_head, 
     }
 }
 
+// The factor token t still lacks (see Params::ssq_in), or 1.
+__device__ __forceinline__ float token_rstd(const Params& p, int t) {
+    return p.ssq_in != nullptr && t < p.tokens ? 1.0f / sqrtf(token_ssq(p, t) * p.inv_n + p.eps) : 1.0f;
+}
+
 // Epilogue of one 128-token x TILE_N tile by one warp: its 32 tokens (tensor-memory
-// lanes of `taddr`), its share `cg` (0 or 1) of the feature columns.
+// lanes of `taddr`; `rstd`: this lane's token_rstd, formed while the products run), its share `cg` (0 or 1)
+// of the feature columns.
 template <int TILE_N, bool REDUCE, bool HEADS = false>
 __device__ __forceinline__ void tokm_epilogue_tile(const Params& p, const CUtensorMap* map_c, uint32_t taddr,
                                                    uint8_t* box, int t_warp, int f0, int cg, int lane, bool ok,
-                                                   bf16* head_dst = nullptr) {
+                                                   float rstd, bf16* head_dst = nullptr) {
     constexpr int HALF = (TILE_N / 2 + 15) / 16 * 16;
     const int t = t_warp + lane;
     if constexpr (REDUCE) {
@@ -953,14 +979,6 @@ __device__ __forceinline__ void tokm_epilogue_tile(const Params& p, const CUtens
             }
         }
     } else {
-        // the factor this thread's token still lacks (see Params::ssq_in), summed in slot order
-        float rstd = 1.0f;
-        if (p.ssq_in != nullptr && t < p.tokens) {
-            const float* row = p.ssq_in + (size_t)t * p.ssq_in_slots;
-            float sum = 0.f;
-            for (int i = 0; i < p.ssq_in_slots; ++i) sum += row[i];
-            rstd = 1.0f / sqrtf(sum * p.inv_n + p.eps);
-        }
         if constexpr (HEADS) {
             static_assert(TILE_N == 2 * SINK_HEAD, "a head per half of the tile's columns");
             sink_head(p, taddr + cg * SINK_HEAD, t, f0 / SINK_HEAD + cg, rstd, ok ? head_dst : nullptr);
@@ -1076,28 +1094,32 @@ gemm_tc_tokm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        // ---------------------------------------------------------------- MMA issuer (converged, see elect_one)
+        {
             constexpr uint32_t idesc = umma_idesc(UMMA_M, TILE_N);
             int it = 0, tile_iter = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++tile_iter) {
                 const int b = tile_iter & 1, use = tile_iter >> 1;
-                if (tile_iter >= 2 && !mbar_wait(&acc_empty[b], (use & 1) ^ 1, abort_flag)) { ok = false; break; }
+                if (tile_iter >= 2 && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[b], (use & 1) ^ 1, abort_flag))) break;
                 tcgen05_fence_after();
                 const uint32_t acc = tmem_base + b * C::TMEM_COLS;
                 for (int i = 0; i < n_kb; ++i, ++it) {
                     const int s = it % C::STAGES;
-                    if (!mbar_wait(&full[s], (it / C::STAGES) & 1, abort_flag)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (it / C::STAGES) & 1, abort_flag))) { ok = false; break; }
                     tcgen05_fence_after();
                     const uint32_t xa = smem_u32(tiles + (size_t)s * C::STAGE_BYTES);
                     const uint64_t xd = umma_smem_desc(xa), wd = umma_smem_desc(xa + C::X_BYTES);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < TILE_K / UMMA_K; ++k)
-                        umma_bf16(acc, xd + 2 * k, wd + 2 * k, idesc, (i | k) ? 1u : 0u);
-                    umma_commit(&empty[s]);
+                        for (int k = 0; k < TILE_K / UMMA_K; ++k)
+                            umma_bf16(acc, xd + 2 * k, wd + 2 * k, idesc, (i | k) ? 1u : 0u);
+                        umma_commit(&empty[s]);
+                    }
+                    __syncwarp();
                 }
-                if (ok) umma_commit(&acc_full[b]);
+                if (ok && elect_one()) umma_commit(&acc_full[b]);
+                __syncwarp();
             }
         }
     } else {
@@ -1106,15 +1128,20 @@ gemm_tc_tokm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const int cg = (warp - 2) >> 2;            // half of the feature columns
         pdl_wait();
         uint8_t* box = staging + (size_t)(warp - 2) * RED_BYTES;
-        int tile_iter = 0;
+        int tile_iter = 0, rstd_of = -1;
+        float rstd = 1.0f;
         bool ok = true;
         for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++tile_iter) {
             const int b = tile_iter & 1, use = tile_iter >> 1;
             const int t_warp = (tile % m_tiles) * UMMA_M + q * 32, f0 = (tile / m_tiles) * TILE_N;
+            if (!REDUCE && t_warp != rstd_of) {
+                rstd = token_rstd(p, t_warp + lane);
+                rstd_of = t_warp;
+            }
             if (ok && !mbar_wait(&acc_full[b], use & 1, abort_flag)) ok = false;
             tcgen05_fence_after();
             const uint32_t taddr = tmem_base + b * C::TMEM_COLS + ((uint32_t)(q * 32) << 16);
-            tokm_epilogue_tile<TILE_N, REDUCE>(p, &map_c, taddr, box, t_warp, f0, cg, lane, ok);
+            tokm_epilogue_tile<TILE_N, REDUCE>(p, &map_c, taddr, box, t_warp, f0, cg, lane, ok, rstd);
             // this warp has read its part of the accumulator: hand it back
             tcgen05_fence_before();
             __syncwarp();
@@ -1253,33 +1280,37 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            // ------------------------------------------------------------ MMA issuer (first CTA)
+        if (rank == 0) {
+            // ------------------------------------------------------------ MMA issuer (first CTA; converged, see elect_one)
             constexpr uint32_t idesc = umma_idesc(2 * UMMA_M, C::SUB_N);
             int it = 0, tile_iter = 0;
             bool ok = true;
             for (int tile = pair; tile < total_tiles && ok; tile += n_pairs, ++tile_iter) {
                 const int b = tile_iter % C::ACCS, use = tile_iter / C::ACCS;
-                if (tile_iter >= C::ACCS && !mbar_wait(&acc_empty[b], (use & 1) ^ 1, abort_flag)) { ok = false; break; }
+                if (tile_iter >= C::ACCS && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[b], (use & 1) ^ 1, abort_flag))) break;
                 tcgen05_fence_after();
                 const uint32_t acc = tmem_base + b * C::TMEM_COLS;
                 for (int i = 0; i < n_kb; ++i, ++it) {
                     const int s = it % C::STAGES;
                     const uint32_t ph = (it / C::STAGES) & 1;
-                    if (!mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
                     tcgen05_fence_after();
                     const uint32_t xa = smem_u32(tiles + (size_t)s * C::STAGE_BYTES);
                     const uint64_t xd = umma_smem_desc(xa), wd = umma_smem_desc(xa + C::X_BYTES);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < TILE_K / UMMA_K; ++k) {
+                        for (int k = 0; k < TILE_K / UMMA_K; ++k) {
 #pragma unroll
-                        for (int j = 0; j < C::SUBS; ++j)
-                            umma_bf16_pair(acc + j * C::SUB_N, xd + 2 * k, wd + j * (C::SUB_BYTES >> 4) + 2 * k, idesc,
-                                           (i | k) ? 1u : 0u);
+                            for (int j = 0; j < C::SUBS; ++j)
+                                umma_bf16_pair(acc + j * C::SUB_N, xd + 2 * k, wd + j * (C::SUB_BYTES >> 4) + 2 * k, idesc,
+                                               (i | k) ? 1u : 0u);
+                        }
+                        umma_commit_pair(&empty[s]);
                     }
-                    umma_commit_pair(&empty[s]);
+                    __syncwarp();
                 }
-                if (ok) umma_commit_pair(&acc_full[b]);
+                if (ok && elect_one()) umma_commit_pair(&acc_full[b]);
+                __syncwarp();
             }
         }
         __syncwarp();
@@ -1289,7 +1320,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const int cg = (warp - 2) >> 2;            // half of the feature columns
         pdl_wait();
         uint8_t* box = staging + (size_t)(warp - 2) * RED_BYTES;
-        int tile_iter = 0;
+        int tile_iter = 0, rstd_of = -1;
+        float rstd = 1.0f;
         bool ok = true;
         for (int tile = pair; tile < total_tiles; tile += n_pairs, ++tile_iter) {
             const int b = tile_iter % C::ACCS, use = tile_iter / C::ACCS;
@@ -1297,10 +1329,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const int f0 = (tile / m_tiles) * TILE_N;
             bf16* head_dst = nullptr;
             if constexpr (HEADS) head_dst = sink_dst(p, t_warp + lane, f0 / SINK_HEAD + cg);
+            if (!REDUCE && t_warp != rstd_of) {
+                rstd = token_rstd(p, t_warp + lane);
+                rstd_of = t_warp;
+            }
             if (ok && !mbar_wait(&acc_full[b], use & 1, abort_flag)) ok = false;
             tcgen05_fence_after();
             const uint32_t taddr = tmem_base + b * C::TMEM_COLS + ((uint32_t)(q * 32) << 16);
-            tokm_epilogue_tile<TILE_N, REDUCE, HEADS>(p, &map_c, taddr, box, t_warp, f0, cg, lane, ok, head_dst);
+            tokm_epilogue_tile<TILE_N, REDUCE, HEADS>(p, &map_c, taddr, box, t_warp, f0, cg, lane, ok, rstd, head_dst);
             // this warp has read its part of the accumulator: hand it back to the first CTA
             tcgen05_fence_before();
             __syncwarp();
