@@ -349,62 +349,6 @@ __device__ __forceinline__ void warp_norm_rope(float (&x)[D / 32], const void* n
     }
 }
 
-// out[:] = sum_s o_s * 2^(m_s - m) / sum_s l_s * 2^(m_s - m) of one head, splits in order, by one
-// warp.  `ml` [n_splits][2], `po` [n_splits][D]; `weight` is 64 floats of shared memory of this warp.
-__device__ __forceinline__ void warp_merge_head(bf16* __restrict__ dst, const float* ml, const float* po,
-                                                int n_splits, int head_dim, float* weight, int lane) {
-    float m[2], l[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int s = lane + 32 * i;
-        m[i] = s < n_splits ? __ldcg(ml + 2 * s) : -INFINITY;
-        l[i] = s < n_splits ? __ldcg(ml + 2 * s + 1) : 0.f;
-    }
-    const float mx = warp_max(fmaxf(m[0], m[1]));
-    float total = 0.f;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float w = (m[i] == -INFINITY) ? 0.f : exp2f(m[i] - mx);
-        weight[lane + 32 * i] = w;
-        total += l[i] * w;
-    }
-    // sum in split order would need a serial loop; lanes hold splits s and s + 32,
-    // a fixed tree over lanes keeps the order the same for every token
-    total = warp_sum(total);
-    const float inv_sum = total > 0.f ? 1.f / total : 0.f;
-    __syncwarp();
-    // a lane takes four neighbouring values (head sizes are multiples of 16); the loads of eight
-    // splits are issued together, then added in split order
-    for (int d = 4 * lane; d < head_dim; d += 128) {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int s0 = 0; s0 < n_splits; s0 += 8) {
-            float4 v[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                // a split with no key in reach (wholly behind a window) has weight 0 and wrote no
-                // partial output: what lies in the scratch there is not read (0 x garbage may be NaN)
-                const bool live = s0 + i < n_splits && weight[s0 + i] != 0.f;
-                v[i] = live ? __ldcg(reinterpret_cast<const float4*>(po + (size_t)(s0 + i) * head_dim + d))
-                            : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float w = s0 + i < n_splits ? weight[s0 + i] : 0.f;
-                if (w != 0.f) {
-                    acc[0] += v[i].x * w; acc[1] += v[i].y * w; acc[2] += v[i].z * w; acc[3] += v[i].w * w;
-                }
-            }
-        }
-        __nv_bfloat162 lo = __floats2bfloat162_rn(acc[0] * inv_sum, acc[1] * inv_sum);
-        __nv_bfloat162 hi = __floats2bfloat162_rn(acc[2] * inv_sum, acc[3] * inv_sum);
-        uint2 packed;
-        packed.x = *reinterpret_cast<uint32_t*>(&lo);
-        packed.y = *reinterpret_cast<uint32_t*>(&hi);
-        *reinterpret_cast<uint2*>(dst + d) = packed;
-    }
-    __syncwarp();
-}
-
 // Keys per split for a context of kv_len keys: the step's split length, or
 // longer when max_splits of them would not cover the context.
 __host__ __device__ __forceinline__ int decode_split_keys(int kv_len, int max_splits, int split_keys_min) {
@@ -752,10 +696,15 @@ attn_decode_stream_kernel(const DecodeParams p, int n_tokens) {
     // (a CTA without a run leaves without the dependency wait: it touched nothing but the lists)
 }
 
-// The merge of a token's splits: a warp per head, WARPS heads per block.  (Merging inside the
-// split kernel, by the CTA that finishes a token's last split, was measured and is no faster:
+// The merge of a token's splits: a warp per head, WARPS heads per block, four neighbouring values per lane.  All a trip
+// to the L2 each is what it lasts: so the step's lists are read before the dependency wait (as in the split kernel),
+// and the first MERGE_AHEAD splits' results are on their way beside the maxima and sums that say how they count.  (With
+// a thread per value and 32 splits at a time, one token of 2,048 keys merged its 33 splits in 4.0 us instead of 5.1, but
+// 8 tokens of 8,100 keys took 6.5 instead of 4.5 and 64 of 2,048 8.7 instead of 4.3: four times the blocks.)  (Merging
+// inside the split kernel, by the CTA that finishes a token's last split, was measured and is no faster:
 // one CTA then does behind a fence what this launch spreads over many while the next kernel
 // already prefetches its weights.)
+constexpr int MERGE_AHEAD = 16;
 __global__ void __launch_bounds__(THREADS)
 attn_decode_merge_kernel(bf16* __restrict__ out, const float* __restrict__ part_o,
                          const float* __restrict__ part_ml, const int* __restrict__ rows,
@@ -763,25 +712,75 @@ attn_decode_merge_kernel(bf16* __restrict__ out, const float* __restrict__ part_
                          int n_q, int head_dim, int max_splits,
                          const int* __restrict__ split_keys_ptr, int split_stride,
                          const int* __restrict__ n_splits_info, int n_kv) {
-    __shared__ float weight[WARPS * 64];           // max_splits <= 64 checked by the launcher
+    __shared__ float weights[WARPS][64];           // max_splits <= 64 checked by the launcher
     pdl_launch_dependents();
-    pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = blockIdx.y, h = blockIdx.x * WARPS + warp;
     if (h >= n_q) return;
-    const int entry = rows[n];
-    int n_splits;
-    if (n_splits_info != nullptr) {                // the stream cut noted the pair's splits
-        n_splits = n_splits_info[n * n_kv + h / (n_q / n_kv)];
-    } else {
+    const int entry = rows[n], token = q_start[entry];
+    int n_splits = 0;
+    if (n_splits_info == nullptr) {
         const int kv_len = context_len[entry] + 1;
         const int split_keys = decode_split_keys(kv_len, max_splits, __ldg(split_keys_ptr + n * split_stride));
         n_splits = (kv_len + split_keys - 1) / split_keys;
     }
+    pdl_wait();
+    if (n_splits_info != nullptr) n_splits = n_splits_info[n * n_kv + h / (n_q / n_kv)];      // the stream cut noted the pair's splits
     if (n_splits == 1) return;                     // the split kernel wrote the result itself
     const size_t head = (size_t)n * n_q + h;
-    warp_merge_head(out + ((size_t)q_start[entry] * n_q + h) * head_dim, part_ml + head * max_splits * 2,
-                    part_o + head * max_splits * head_dim, n_splits, head_dim, weight + warp * 64, lane);
+    const float* ml = part_ml + head * max_splits * 2;
+    const float* po = part_o + head * max_splits * head_dim;
+    bf16* dst = out + ((size_t)token * n_q + h) * head_dim;
+    float* weight = weights[warp];
+    int d = 4 * lane;                              // (head sizes are multiples of 16)
+    float4 v[MERGE_AHEAD];
+    auto load = [&](int s0) {
+#pragma unroll
+        for (int i = 0; i < MERGE_AHEAD; ++i)
+            if (s0 + i < n_splits && d < head_dim) v[i] = __ldcg(reinterpret_cast<const float4*>(po + (size_t)(s0 + i) * head_dim + d));
+    };
+    float m[2], l[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int s = lane + 32 * i;
+        m[i] = s < n_splits ? __ldcg(ml + 2 * s) : -INFINITY;
+        l[i] = s < n_splits ? __ldcg(ml + 2 * s + 1) : 0.f;
+    }
+    load(0);
+    const float mx = warp_max(fmaxf(m[0], m[1]));
+    float total = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float w = (m[i] == -INFINITY) ? 0.f : exp2f(m[i] - mx);
+        weight[lane + 32 * i] = w;
+        total += l[i] * w;
+    }
+    // sum in split order would need a serial loop; lanes hold splits s and s + 32,
+    // a fixed tree over lanes keeps the order the same for every token
+    total = warp_sum(total);
+    const float inv_sum = total > 0.f ? 1.f / total : 0.f;
+    __syncwarp();
+    for (; d < head_dim; d += 128) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s0 = 0; s0 < n_splits; s0 += MERGE_AHEAD) {
+            if (s0 > 0 || d >= 128) load(s0);
+            // in split order; a split with no key in reach (wholly behind a window) has weight 0 and wrote no
+            // partial output: what lies in the scratch there does not count (0 x garbage may be NaN)
+#pragma unroll
+            for (int i = 0; i < MERGE_AHEAD; ++i) {
+                const float w = s0 + i < n_splits ? weight[s0 + i] : 0.f;
+                if (w != 0.f) {
+                    acc[0] += v[i].x * w; acc[1] += v[i].y * w; acc[2] += v[i].z * w; acc[3] += v[i].w * w;
+                }
+            }
+        }
+        __nv_bfloat162 lo = __floats2bfloat162_rn(acc[0] * inv_sum, acc[1] * inv_sum);
+        __nv_bfloat162 hi = __floats2bfloat162_rn(acc[2] * inv_sum, acc[3] * inv_sum);
+        uint2 packed;
+        packed.x = *reinterpret_cast<uint32_t*>(&lo);
+        packed.y = *reinterpret_cast<uint32_t*>(&hi);
+        *reinterpret_cast<uint2*>(dst + d) = packed;
+    }
 }
 
 template <int D> int launch_prefill(const PrefillParams& p, int items, cudaStream_t s) {

@@ -941,6 +941,20 @@ def test_decode_attention_dealt_out_as_a_stream(shape, window):
     assert st.tolist() == [0, 0, 0, 0]
 
 
+@pytest.mark.parametrize("context,D", [(63, 128), (64, 64), (1022, 128), (1030, 64), (4094, 128)])
+def test_decode_merge_at_its_edges(context, D):
+    """One decoded token whose keys are cut into 1, 2, 16, 17 and 64 splits of a tile each: the merge fetches 16 splits
+    at a time, in heads of half a warp and of a whole one.  What lies in the scratch beforehand must not matter."""
+    from kipp_b200.kernels import attention_bf16
+    nq, nkv, page, layout = 8, 2, 16, [(context, 1)]
+    meta, table, q, kp, vp = attention_case(context, D, nq, nkv, page, layout, torch.bfloat16)
+    out, st = torch.full_like(q, 9.0), status()
+    attention_bf16.decode_scratch(torch.device(DEV), 1, nq, D).fill_(float("nan"))
+    attention_bf16.run("mma", out, q, kp, vp, meta, meta.block_tables[0], page, nq, nkv, D, 1 / math.sqrt(D), None, st, stream=False)
+    ref = attention_ref(meta, table, q, kp, vp, layout, page, None, 1 / math.sqrt(D))
+    assert st.tolist() == [0, 0, 0, 0] and torch.allclose(out.double().cpu(), ref, rtol=2e-2, atol=2e-2)
+
+
 def test_a_bounded_wait_runs_out_and_reports():
     """The give-up branch of the mbarrier wait every tensor-core kernel uses
     (csrc/mbarrier.cuh), run by a probe kernel on a barrier nothing arrives at, with
