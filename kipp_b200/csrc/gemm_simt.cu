@@ -8,8 +8,9 @@
 //
 // The sum over k runs in the same order for every output element whatever M is, so a token's result does
 // not depend on what else is in the batch: K is cut into at most 16 runs whose length depends on K alone
-// (run_length), a run is one chain of FMAs in the order of k, and the runs are added in their order.  The
-// runs are what lets a few tokens be multiplied by many threads at once.
+// (run_length), a run is one chain of FMAs in the order of k, the sums of four neighbouring runs are added in
+// their order, and so are then the up to four sums of those.  The runs are what lets a few tokens be multiplied by
+// many threads at once, the groups of four what lets a small product of many tokens be shared by more blocks.
 //
 // Three kernels, chosen by shape alone, with that one order:
 //   few   float32, up to FEW_MAX tokens: bound by the weights' bytes (a token is 2 operations per 4 bytes).  A
@@ -19,9 +20,12 @@
 //         1, 3 and 16 tokens: 24, 34 and 94 us (100 MB: 15 us of copy rate; the kernel below, which ran before: 334, 339
 //         and 353); 2,048 x 6,144 with 3: 30 us (543).  At 32 tokens its two passes still win where the features are
 //         few (2,048 x 2,048: 31 us against 88 in tiles) and tie where they are many (12,288: 176 against 174).
-//   tile  float32, more tokens: bound by the FMA pipes.  64 x 64 outputs per block of 128 threads, 8 x 4 per
-//         thread, operands in shared memory as they lie in memory (16 bytes of k per row and
-//         thread), three stages of asynchronous copies.  407 tokens, 12,288 x 2,048: 608 us (34 TFLOP/s; 943 us before), 2,048 x 6,144: 540 us (866).
+//   tile  float32, more tokens: bound by the FMA pipes.  128 features x 64 tokens per block of 128 threads, 8 x 8 per
+//         thread in float32 pairs, operands in shared memory with k outermost, so that a k's 16 values cost a
+//         thread four 16-byte reads (with four bytes copied at a time: 24 copies per 1,024 FMAs); the groups of runs
+//         are blocks of their own, a cluster that meets in its shared memory.
+//         407 tokens, 12,288 x 2,048: 608 us (943 before), 2,048 x 6,144: 392 us (866; 540 with
+//         tiles of 64 x 64, 8 x 4 per thread and k innermost); 64 tokens, 12,288 x 2,048: 106 us (387; 181).
 //   any   what is left: bfloat16 operands of shapes that the tensor-core kernels refuse, and float32 rows that do
 //         not start on 16 bytes.
 //
@@ -39,8 +43,8 @@
 namespace {
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
-// K in runs: at most MAX_RUNS of them, each of a length that is a multiple of BK.
-constexpr int MAX_RUNS = 16;
+// K in runs: at most MAX_RUNS of them, each of a length that is a multiple of BK, in groups of GROUP_RUNS.
+constexpr int MAX_RUNS = 16, GROUP_RUNS = 4;
 __host__ __device__ inline int run_length(int K) {
     const int per = (K + MAX_RUNS - 1) / MAX_RUNS;
     return (per + BK - 1) / BK * BK;
@@ -67,11 +71,11 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
     const int tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int run = run_length(K);
-    float acc[TM][TN], sum[TM][TN];
+    float acc[TM][TN], group[TM][TN], sum[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = sum[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) acc[i][j] = group[i][j] = sum[i][j] = 0.f;
 
     // 64x16 tile = 1024 elements, 256 threads -> 4 each; thread loads row
     // (tid / 4), k columns (tid % 4) * 4 .. + 3.
@@ -99,12 +103,17 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
         }
         __syncthreads();
         if ((k0 + BK) % run == 0 || k0 + BK >= K) {
+            const bool whole = (k0 + BK) % (GROUP_RUNS * run) == 0 || k0 + BK >= K;
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) {
-                    sum[i][j] += acc[i][j];
+                    group[i][j] += acc[i][j];
                     acc[i][j] = 0.f;
+                    if (whole) {
+                        sum[i][j] += group[i][j];
+                        group[i][j] = 0.f;
+                    }
                 }
         }
     }
@@ -167,6 +176,17 @@ gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
     float acc[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) acc[m] = 0.f;
+    // (the tokens' next four values are asked for while the present ones are multiplied; left to itself the compiler
+    // held back the loads of four tokens to save registers: 39 us against 34 for 3 tokens of 12,288 x 2,048)
+    constexpr bool AHEAD = MT <= 8;
+    float4 next[AHEAD ? MT : 1];
+    auto load_next = [&](int k) {
+        if constexpr (AHEAD) {
+#pragma unroll
+            for (int m = 0; m < MT; ++m) next[m] = k < K ? *reinterpret_cast<const float4*>(x[m] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    load_next(r * run);
     for (int step = 0; step < steps; ++step) {
         cp_async_wait<FEW_STAGES - 2>();
         __syncwarp();
@@ -176,9 +196,15 @@ gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
         for (int q = 0; q < BK / 4; ++q) {
             if (k0 + 4 * q >= K) break;                   // whole quarters: K is a multiple of 4
             const float4 w = *reinterpret_cast<const float4*>(chunk + 16 * q);
+            float4 now[AHEAD ? MT : 1];
+            if constexpr (AHEAD) {
+#pragma unroll
+                for (int m = 0; m < MT; ++m) now[m] = next[m];
+                load_next(k0 + 4 * q + 4);
+            }
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                const float4 v = *reinterpret_cast<const float4*>(x[m] + k0 + 4 * q);
+                const float4 v = AHEAD ? now[AHEAD ? m : 0] : *reinterpret_cast<const float4*>(x[m] + k0 + 4 * q);
                 acc[m] = fmaf(v.x, w.x, acc[m]);
                 acc[m] = fmaf(v.y, w.y, acc[m]);
                 acc[m] = fmaf(v.z, w.z, acc[m]);
@@ -197,45 +223,71 @@ gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
     for (int i = threadIdx.x; i < MT * FEW_F; i += FEW_THREADS) {
         const int f = i % FEW_F, m = i / FEW_F, n = n0 + f;
         if (m0 + m >= M) break;
-        float v = 0.f, u = 0.f;
+        auto total = [&](int at) {
+            float v = 0.f;
+            for (int s0 = 0; s0 < runs; s0 += GROUP_RUNS) {
+                float group = 0.f;
+                for (int s = s0; s < min(runs, s0 + GROUP_RUNS); ++s) group += parts[s][m][at];
+                v += group;
+            }
+            return v;
+        };
         if (EPI == EPI_SWIGLU) {
             if ((f & 1) || n + 1 >= N) continue;
-            for (int s = 0; s < runs; ++s) { v += parts[s][m][f]; u += parts[s][m][f + 1]; }
-            put<float, EPI_STORE>(C, ldc, m0 + m, n >> 1, swiglu(v, u));
+            put<float, EPI_STORE>(C, ldc, m0 + m, n >> 1, swiglu(total(f), total(f + 1)));
         } else if (n < N) {
-            for (int s = 0; s < runs; ++s) v += parts[s][m][f];
-            put<float, EPI>(C, ldc, m0 + m, n, v);
+            put<float, EPI>(C, ldc, m0 + m, n, total(f));
         }
     }
 }
 
 // ---------------------------------------------------------------------------------------
-// Many tokens.  Thread (tx, ty) has the outputs of tokens ty + 8 i and features tx + 16 j: the
-// rows that a warp reads together lie next to one another, 80 bytes apart, so 16-byte reads meet
-// every bank once.
-constexpr int TILE_M = 64, TILE_N = 64, TILE_STAGES = 3, TILE_THREADS = 128, TILE_ROW = BK + 4;
-constexpr int TILE_SMEM = TILE_STAGES * (TILE_M + TILE_N) * TILE_ROW * 4;
+// Many tokens.  Thread (r, c) has features r .. r + 3 and 64 + r .. of the block's 128, tokens c .. c + 3 and 32 + c .. of
+// its 64.  A block has one group of runs; the blocks of the groups are a cluster along z, and each of them finishes a
+// share of the tokens.  A group's sums lie in shared memory (one word per thread and value: 64 registers fewer).
+constexpr int TILE_F = 128, TILE_T = 64, TILE_K = 16, TILE_STAGES = 3, TILE_THREADS = 128;
+constexpr int TILE_W = TILE_F + 4, TILE_X = TILE_T + 4;               // padded: eight k's of four rows meet every bank once
+constexpr int TILE_STAGE = TILE_K * (TILE_W + TILE_X), TILE_VALUES = 64;
+constexpr int TILE_SMEM = (TILE_STAGES * TILE_STAGE + TILE_VALUES * TILE_THREADS) * 4;
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int src_bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+          "l"(reinterpret_cast<const unsigned long long&>(c)));
+    return d;
+}
 
 template <int EPI>
-__global__ void __launch_bounds__(TILE_THREADS)
+__global__ void __launch_bounds__(TILE_THREADS, 3)
 gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
                  int M, int N, int K, int lda, int ldw, int ldc) {
-    extern __shared__ __align__(16) float tiles[];        // [stage][A rows, W rows][TILE_ROW]
+    extern __shared__ __align__(16) float tiles[];        // [stage][W by k, X by k], then [value][thread]: a group's sum
+    float* sums = tiles + TILE_STAGES * TILE_STAGE;
     pdl_launch_dependents();
     pdl_wait();
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * TILE_M, n0 = blockIdx.x * TILE_N;
-    const int run = run_length(K), steps = (K + BK - 1) / BK;
+    const int tid = threadIdx.x;
+    const int m0 = blockIdx.y * TILE_T, n0 = blockIdx.x * TILE_F;
+    const int run = run_length(K), per_group = GROUP_RUNS * run;
+    const int k_begin = (int)blockIdx.z * per_group, k_end = min(K, k_begin + per_group);
+    const int steps = (k_end - k_begin + TILE_K - 1) / TILE_K;
+    // copy j of a step: k = (tid & 7) + 8 (j & 1), row (tid >> 3) + 16 (j >> 1): eight neighbouring k of a row are one sector
+    const int ck = tid & 7, crow = tid >> 3;
     auto fetch = [&](int step, int stage) {
-        float* to = tiles + (size_t)stage * (TILE_M + TILE_N) * TILE_ROW;
+        float* to = tiles + stage * TILE_STAGE;
 #pragma unroll
-        for (int j = 0; j < (TILE_M + TILE_N) * 4 / TILE_THREADS; ++j) {
-            const int c = j * TILE_THREADS + tid, row = c >> 2, k = step * BK + (c & 3) * 4;
-            const bool of_a = row < TILE_M;
-            const int at = of_a ? m0 + row : n0 + row - TILE_M;
-            const bool in = k < K && at < (of_a ? M : N);
-            const float* src = of_a ? A + (size_t)at * lda + k : W + (size_t)at * ldw + k;
-            cp_async16(smem_address(to + row * TILE_ROW + (c & 3) * 4), in ? src : W, in ? 16 : 0);
+        for (int j = 0; j < TILE_F / 8; ++j) {
+            const int k = ck + 8 * (j & 1), row = crow + 16 * (j >> 1), at = k_begin + step * TILE_K + k;
+            const bool in = at < k_end && n0 + row < N;
+            cp_async4(smem_address(to + k * TILE_W + row), in ? W + (size_t)(n0 + row) * ldw + at : W, in ? 4 : 0);
+        }
+#pragma unroll
+        for (int j = 0; j < TILE_T / 8; ++j) {
+            const int k = ck + 8 * (j & 1), row = crow + 16 * (j >> 1), at = k_begin + step * TILE_K + k;
+            const bool in = at < k_end && m0 + row < M;
+            cp_async4(smem_address(to + TILE_K * TILE_W + k * TILE_X + row), in ? A + (size_t)(m0 + row) * lda + at : A, in ? 4 : 0);
         }
     };
 #pragma unroll
@@ -243,60 +295,101 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
         if (s < steps) fetch(s, s);
         cp_async_commit();
     }
-    float acc[8][4], sum[8][4];
+    // acc[i][j]: features 2 i, 2 i + 1 of the thread's eight, token j of its eight
+    float2 acc[4][8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = sum[i][j] = 0.f;
+        for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    // value v of a thread: token v / 8, feature v % 8
+#pragma unroll
+    for (int v = 0; v < TILE_VALUES; ++v) sums[v * TILE_THREADS + tid] = 0.f;
+    const int r = (tid >> 3) * 4, c = (tid & 7) * 4;
     for (int step = 0; step < steps; ++step) {
         cp_async_wait<TILE_STAGES - 2>();
         __syncthreads();                                  // this stage has landed, the one before is read by all
         if (step + TILE_STAGES - 1 < steps) fetch(step + TILE_STAGES - 1, (step + TILE_STAGES - 1) % TILE_STAGES);
         cp_async_commit();
-        const float* a = tiles + (size_t)(step % TILE_STAGES) * (TILE_M + TILE_N) * TILE_ROW;
-        const float* b = a + TILE_M * TILE_ROW;
+        const float* w = tiles + (step % TILE_STAGES) * TILE_STAGE;
+        const float* x = w + TILE_K * TILE_W;
+#pragma unroll 4
+        for (int k = 0; k < TILE_K; ++k) {
+            const float4 w0 = *reinterpret_cast<const float4*>(w + k * TILE_W + r), w1 = *reinterpret_cast<const float4*>(w + k * TILE_W + 64 + r);
+            const float4 x0 = *reinterpret_cast<const float4*>(x + k * TILE_X + c), x1 = *reinterpret_cast<const float4*>(x + k * TILE_X + 32 + c);
+            const float2 f[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+            const float t[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-        for (int q = 0; q < BK / 4; ++q) {
-            float4 w[4];
+            for (int j = 0; j < 8; ++j)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const float4*>(b + (tx + 16 * j) * TILE_ROW + 4 * q);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float4 v = *reinterpret_cast<const float4*>(a + (ty + 8 * i) * TILE_ROW + 4 * q);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc[i][j] = fmaf(v.x, w[j].x, acc[i][j]);
-                    acc[i][j] = fmaf(v.y, w[j].y, acc[i][j]);
-                    acc[i][j] = fmaf(v.z, w[j].z, acc[i][j]);
-                    acc[i][j] = fmaf(v.w, w[j].w, acc[i][j]);
-                }
-            }
+                for (int i = 0; i < 4; ++i) acc[i][j] = fma_pair(f[i], make_float2(t[j], t[j]), acc[i][j]);
         }
-        if (((step + 1) * BK) % run == 0 || step + 1 == steps) {
+        const int done = k_begin + (step + 1) * TILE_K;
+        if (done % run == 0 || step + 1 == steps) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int j = 0; j < 8; ++j)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sum[i][j] += acc[i][j];
-                    acc[i][j] = 0.f;
+                for (int i = 0; i < 4; ++i) {
+                    float* at = sums + (8 * j + 2 * i) * TILE_THREADS + tid;
+                    at[0] += acc[i][j].x;
+                    at[TILE_THREADS] += acc[i][j].y;
+                    acc[i][j] = make_float2(0.f, 0.f);
                 }
         }
     }
     cp_async_wait<0>();
+    const int groups = (int)gridDim.z;
+    if (groups > 1)                                       // all blocks' sums are there
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    uint32_t of[MAX_RUNS / GROUP_RUNS];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + ty + 8 * i;
+    for (int z = 0; z < MAX_RUNS / GROUP_RUNS; ++z)
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(of[z]) : "r"(smem_address(sums + tid)), "r"(z < groups ? z : 0));
+    const int per = (8 + groups - 1) / groups, j0 = (int)blockIdx.z * per, j1 = min(8, j0 + per);
+    const bool vectors = (EPI == EPI_SWIGLU ? ldc % 2 == 0 && ((uintptr_t)C & 7) == 0 : ldc % 4 == 0 && ((uintptr_t)C & 15) == 0);
+    for (int j = j0; j < j1; ++j) {
+        float g[8][MAX_RUNS / GROUP_RUNS];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx + 16 * j;
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int z = 0; z < MAX_RUNS / GROUP_RUNS; ++z) {
+                g[i][z] = 0.f;
+                if (z < groups)
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(g[i][z]) : "r"(of[z] + (uint32_t)((8 * j + i) * TILE_THREADS * 4)) : "memory");
+            }
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            v[i] = 0.f;
+#pragma unroll
+            for (int z = 0; z < MAX_RUNS / GROUP_RUNS; ++z) v[i] += g[i][z];
+        }
+        const int m = m0 + (j < 4 ? c + j : 28 + c + j);
+        if (m >= M) continue;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int n = n0 + 64 * half + r;
+            const float* q = v + 4 * half;
             if (EPI == EPI_SWIGLU) {
-                const float u = __shfl_xor_sync(0xffffffffu, sum[i][j], 1);      // an even lane's neighbour has the up row
-                if ((tx & 1) == 0 && m < M && n + 1 < N) put<float, EPI_STORE>(C, ldc, m, n >> 1, swiglu(sum[i][j], u));
-            } else if (m < M && n < N) {
-                put<float, EPI>(C, ldc, m, n, sum[i][j]);
+                float* at = C + (size_t)m * ldc + (n >> 1);
+                if (vectors && n + 3 < N) {
+                    *reinterpret_cast<float2*>(at) = make_float2(swiglu(q[0], q[1]), swiglu(q[2], q[3]));
+                } else {
+                    if (n + 1 < N) at[0] = swiglu(q[0], q[1]);
+                    if (n + 3 < N) at[1] = swiglu(q[2], q[3]);
+                }
+            } else if (vectors && n + 3 < N) {
+                float4* at = reinterpret_cast<float4*>(C + (size_t)m * ldc + n);
+                float4 o = EPI == EPI_ADD ? *at : make_float4(0.f, 0.f, 0.f, 0.f);
+                *at = EPI == EPI_ADD ? make_float4(o.x + q[0], o.y + q[1], o.z + q[2], o.w + q[3]) : make_float4(q[0], q[1], q[2], q[3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (n + i < N) put<float, EPI>(C, ldc, m, n + i, q[i]);
             }
         }
     }
+    if (groups > 1)                                       // nobody's sums may go away while a neighbour reads them
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
 template <int MT, int EPI>
@@ -322,9 +415,16 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, in
         if (M <= 8) return launch_few<8, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
         return launch_few<16, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
     }
-    const dim3 grid((N + TILE_N - 1) / TILE_N, (M + TILE_M - 1) / TILE_M);
+    const int groups = (K + GROUP_RUNS * run_length(K) - 1) / (GROUP_RUNS * run_length(K));
+    const dim3 grid((N + TILE_F - 1) / TILE_F, (M + TILE_T - 1) / TILE_T, groups);
     if (grid.y > 65535) return KIPP_ERR_ARG;
-    return kipp_launch(gemm_tile_kernel<EPI>, grid, dim3(TILE_THREADS), TILE_SMEM, s, 1, C, A, W, M, N, K, lda, ldw, ldc);
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_tile_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    return kipp_launch(gemm_tile_kernel<EPI>, grid, dim3(TILE_THREADS), TILE_SMEM, s, groups, C, A, W, M, N, K, lda, ldw, ldc);
 }
 
 template <typename TA, typename TW, typename TC>
