@@ -51,16 +51,24 @@ __device__ __forceinline__ void load4(float (&x)[4], const bf16* row, int i) {
 // The order of a token's sums depends on the sizes only, not on TOK or on the other tokens.
 // Then warp j chooses for token j.
 template <typename T, int TOK>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(TOK == 1 ? 1024 : 256)
 moe_route_kernel(int* __restrict__ expert_of, float* __restrict__ weight_of, const T* __restrict__ h, long long ldh,
                  const float* __restrict__ router, const float* __restrict__ bias, int tokens, int hidden, int experts,
                  int top, int vec, int by_scores, int renormalize, int real_experts, float weight_scale) {
     // by_scores: 0 the logits choose, 1 softmax scores, 2 sigmoid scores
-    extern __shared__ float z_all[];                      // [TOK][experts], and [TOK][experts] scores when by_scores
+    // [TOK][experts], [TOK][experts] scores when by_scores, [TOK][top] chosen weights
+    extern __shared__ float z_all[];
     pdl_launch_dependents();
-    pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    if (TOK == 1) {
+        // few tokens: the router's rows come from memory, and a warp asks for its own before the wait
+        for (int e = warp; e < experts; e += warps)
+            for (int i = 32 * lane; i < hidden; i += 1024)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(router + (size_t)e * hidden + i));
+    }
+    pdl_wait();
     const int t0 = blockIdx.x * TOK;
+    float* chosen_all = z_all + (size_t)(by_scores ? 2 : 1) * TOK * experts;
     const T* rows[TOK];
 #pragma unroll
     for (int j = 0; j < TOK; ++j) rows[j] = h + (size_t)min(t0 + j, tokens - 1) * ldh;
@@ -70,7 +78,7 @@ moe_route_kernel(int* __restrict__ expert_of, float* __restrict__ weight_of, con
 #pragma unroll
         for (int j = 0; j < TOK; ++j) acc[j] = 0.f;
         if (vec) {
-#pragma unroll 4
+#pragma unroll TOK == 1 ? 8 : 4
             for (int i = 4 * lane; i < hidden; i += 128) {
                 float wv[4];
                 load4(wv, w, i);
@@ -102,6 +110,7 @@ moe_route_kernel(int* __restrict__ expert_of, float* __restrict__ weight_of, con
         if (t >= tokens) continue;
         float* z = z_all + (size_t)j * experts;
         float* score = z_all + (size_t)(TOK + j) * experts;
+        float* chosen = chosen_all + (size_t)j * top;
         if (by_scores == 2) {
             // (without a correction the logits are compared: the order is the same, and scores that
             // round to 1 do not tie)
@@ -148,25 +157,17 @@ moe_route_kernel(int* __restrict__ expert_of, float* __restrict__ weight_of, con
             if (lane == 0) {
                 // an identity expert (an output behind the real experts) is marked by a negative id
                 expert_of[(size_t)t * top + k] = idx < real_experts ? idx : -1 - (idx - real_experts);
-                weight_of[(size_t)t * top + k] = by_scores ? score[idx] : best;
+                chosen[k] = by_scores ? score[idx] : best;
                 z[idx] = -INFINITY;
             }
             __syncwarp();
         }
-        if (lane == 0 && by_scores) {
-            float* w = weight_of + (size_t)t * top;
-            float sum = 0.f;
-            for (int k = 0; k < top; ++k) sum += w[k];
-            const float f = renormalize ? weight_scale / (sum + 1e-20f) : weight_scale;
-            for (int k = 0; k < top; ++k) w[k] *= f;
-        } else if (lane == 0) {
-            float* w = weight_of + (size_t)t * top;
-            const float m = w[0];                            // the largest of the chosen
-            float sum = 0.f;
-            for (int k = 0; k < top; ++k) { w[k] = expf(w[k] - m); sum += w[k]; }
-            const float inv = 1.0f / sum;
-            for (int k = 0; k < top; ++k) w[k] *= inv;
-        }
+        // (every lane forms the sum, in the order of the choices)
+        float sum = 0.f;
+        const float m = chosen[0];                           // the largest of the chosen logits
+        for (int k = 0; k < top; ++k) sum += by_scores ? chosen[k] : expf(chosen[k] - m);
+        const float f = !by_scores ? 1.0f / sum : renormalize ? weight_scale / (sum + 1e-20f) : weight_scale;
+        for (int k = lane; k < top; k += 32) weight_of[(size_t)t * top + k] = (by_scores ? chosen[k] : expf(chosen[k] - m)) * f;
     }
 }
 
@@ -335,47 +336,59 @@ moe_gemm_kernel(const GemmArgs g) {
     }
 }
 
+// y[t, :] += sum over k, in order, of weight x row (weight_of null: rows that carry their weight), W neighbouring elements
+// per thread at a time: 4 where the rows go by fours and start on 16 bytes (2,048 tokens x 2,048, top 4: 32 us an element
+// at a time, 24 so).  IDENTITY: some pairs are identity experts (expert_of < 0), whose row is weight x the token's
+// input (weighted: the other rows carry their weight already).
+__device__ __forceinline__ void load_row(float (&x)[1], const float* row, int i) { x[0] = row[i]; }
+__device__ __forceinline__ void load_row(float (&x)[1], const bf16* row, int i) { x[0] = to_f32(row[i]); }
+__device__ __forceinline__ void load_row(float (&x)[4], const float* row, int i) { load4(x, row, i); }
+__device__ __forceinline__ void load_row(float (&x)[4], const bf16* row, int i) { load4(x, row, i); }
+template <typename T, bool IDENTITY, int W>
 __global__ void __launch_bounds__(512)
-moe_combine_kernel(float* __restrict__ y, const float* __restrict__ rows, const float* __restrict__ weight_of, int hidden,
-                   int top, const int* __restrict__ place_of_pair) {
+moe_combine_kernel(float* __restrict__ y, const float* __restrict__ rows, const float* __restrict__ weight_of,
+                   const int* __restrict__ expert_of, const T* __restrict__ h, long long ldh, int hidden, int top,
+                   const int* __restrict__ place_of_pair, int weighted) {
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x;
-    const float* w = weight_of ? weight_of + (size_t)t * top : nullptr;      // null: rows that carry their weight
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        float acc = 0.f;
+    const float* w = weight_of ? weight_of + (size_t)t * top : nullptr;
+    const int* ex = IDENTITY ? expert_of + (size_t)t * top : nullptr;
+    for (int i = W * threadIdx.x; i < hidden; i += W * blockDim.x) {
+        float old[W], acc[W];
+        load_row(old, y + (size_t)t * hidden, i);
+#pragma unroll
+        for (int j = 0; j < W; ++j) acc[j] = 0.f;
+#pragma unroll 4
         for (int k = 0; k < top; ++k) {
-            const size_t row = place_of_pair ? (size_t)place_of_pair[(size_t)t * top + k] : (size_t)t * top + k;
-            acc = weight_of ? fmaf(w[k], rows[row * hidden + i], acc) : acc + rows[row * hidden + i];
-        }
-        y[(size_t)t * hidden + i] += acc;
-    }
-}
-
-// The combine where some pairs are identity experts (expert_of < 0): their row is weight x the token's input
-// (weighted: the other rows carry their weight already).
-template <typename T>
-__global__ void __launch_bounds__(512)
-moe_combine_identity_kernel(float* __restrict__ y, const float* __restrict__ rows, const float* __restrict__ weight_of,
-                            const int* __restrict__ expert_of, const T* __restrict__ h, long long ldh, int hidden, int top,
-                            const int* __restrict__ place_of_pair, int weighted) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int t = blockIdx.x;
-    const float* w = weight_of + (size_t)t * top;
-    const int* ex = expert_of + (size_t)t * top;
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        float acc = 0.f;
-        for (int k = 0; k < top; ++k) {
-            if (ex[k] < 0) {
-                acc = fmaf(w[k], to_f32(h[(size_t)t * ldh + i]), acc);
+            float x[W];
+            const bool own = IDENTITY && ex[k] < 0;
+            if (own) {
+                load_row(x, h + (size_t)t * ldh, i);
             } else {
                 const size_t row = place_of_pair ? (size_t)place_of_pair[(size_t)t * top + k] : (size_t)t * top + k;
-                acc = weighted ? acc + rows[row * hidden + i] : fmaf(w[k], rows[row * hidden + i], acc);
+                load_row(x, rows + row * hidden, i);
             }
+            const bool plain = w == nullptr || (weighted && !own);
+#pragma unroll
+            for (int j = 0; j < W; ++j) acc[j] = plain ? acc[j] + x[j] : fmaf(w[k], x[j], acc[j]);
         }
-        y[(size_t)t * hidden + i] += acc;
+#pragma unroll
+        for (int j = 0; j < W; ++j) acc[j] += old[j];
+        if constexpr (W == 4) *reinterpret_cast<float4*>(y + (size_t)t * hidden + i) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        else y[(size_t)t * hidden + i] = acc[0];
     }
+}
+template <typename T, bool IDENTITY>
+int launch_combine(float* y, const float* rows, const float* weight_of, const int* expert_of, const T* h, long long ldh, int tokens,
+                   int hidden, int top, const int* place_of_pair, int weighted, cudaStream_t s) {
+    const bool fours = hidden % 4 == 0 && (((uintptr_t)y | (uintptr_t)rows) & 15) == 0 &&
+                       (!IDENTITY || (ldh % 4 == 0 && (uintptr_t)h % (4 * sizeof(T)) == 0));
+    // (an element's steps wait for one another: one step per thread where a block of 512 allows)
+    const int at_once = fours ? hidden / 4 : hidden;
+    const dim3 block(at_once >= 512 ? 512 : at_once >= 256 ? 256 : 128);
+    return kipp_launch(fours ? moe_combine_kernel<T, IDENTITY, 4> : moe_combine_kernel<T, IDENTITY, 1>, dim3((unsigned)tokens), block, 0, s, 1,
+                       y, rows, weight_of, expert_of, h, ldh, hidden, top, place_of_pair, weighted);
 }
 }  // namespace
 
@@ -391,11 +404,23 @@ static int moe_route_any(int* expert_of, float* weight_of, const void* h, long l
     cudaStream_t s = (cudaStream_t)stream;
     const size_t es = dtype == KIPP_DT_F32 ? 4 : 2;
     const int vec = hidden % 4 == 0 && ldh % 4 == 0 && ((uintptr_t)h % (4 * es)) == 0 && ((uintptr_t)router & 15) == 0;
-    // many tokens: four per block share a read of the router; few: a warp per expert, up to sixteen
+    // many tokens: four per block share a read of the router
     const int tok = tokens >= 256 ? 4 : 1;
-    const int warps = tok == 4 ? 8 : (experts >= 16 ? 16 : experts > 8 ? 8 : 4);
+    // few: a warp an expert, up to 32 (8 tokens, 18 outputs, 2,560 wide: 23 us with sixteen warps, whose last two outputs were a
+    // round of their own, the router's rows asked for behind the wait and the weights normalised in global memory;
+    // 9 us so)
+    const int warps = tok == 4 ? 8 : experts > 32 ? 32 : experts < 4 ? 4 : experts;
     const dim3 grid((unsigned)((tokens + tok - 1) / tok)), block((unsigned)(32 * warps));
-    const size_t smem = (size_t)(by_scores ? 2 : 1) * tok * experts * sizeof(float);
+    const size_t scores = (size_t)(by_scores ? 2 : 1) * tok * experts * sizeof(float), smem = scores + (size_t)tok * top * sizeof(float);
+    if (smem > 48 * 1024 && scores <= 48 * 1024) {
+        // (the chosen weights must not be what a size fails for)
+        const void* kernels[] = {(const void*)moe_route_kernel<float, 1>, (const void*)moe_route_kernel<float, 4>,
+                                 (const void*)moe_route_kernel<bf16, 1>, (const void*)moe_route_kernel<bf16, 4>};
+        for (const void* k : kernels) {
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return (int)e;
+        }
+    }
     if (dtype == KIPP_DT_F32) {
         if (tok == 4)
             return kipp_launch(moe_route_kernel<float, 4>, grid, block, smem, s, 1, expert_of, weight_of, (const float*)h,
@@ -466,9 +491,7 @@ extern "C" int kipp_moe_combine(float* y, const float* rows, const float* weight
                                 const int* place_of_pair, void* stream) {
     if (tokens <= 0) return 0;
     if (hidden <= 0 || top <= 0) return KIPP_ERR_ARG;
-    // (an element's steps wait for one another, the loads behind the store before them: few elements per thread)
-    return kipp_launch(moe_combine_kernel, dim3((unsigned)tokens), dim3(hidden >= 2048 ? 512 : hidden >= 512 ? 256 : 128), 0,
-                       (cudaStream_t)stream, 1, y, rows, weight_of, hidden, top, place_of_pair);
+    return launch_combine<float, false>(y, rows, weight_of, nullptr, nullptr, 0, tokens, hidden, top, place_of_pair, 0, (cudaStream_t)stream);
 }
 
 // The same where pairs with expert_of < 0 stand for the token's own input h [tokens, ldh] (`dtype`).
@@ -478,11 +501,11 @@ extern "C" int kipp_moe_combine_identity(float* y, const float* rows, const floa
     if (tokens <= 0) return 0;
     if (hidden <= 0 || top <= 0 || expert_of == nullptr || h == nullptr) return KIPP_ERR_ARG;
     if (dtype == KIPP_DT_F32)
-        return kipp_launch(moe_combine_identity_kernel<float>, dim3((unsigned)tokens), dim3(hidden >= 2048 ? 512 : hidden >= 512 ? 256 : 128), 0, (cudaStream_t)stream, 1, y,
-                           rows, weight_of, expert_of, (const float*)h, ldh, hidden, top, place_of_pair, weighted);
+        return launch_combine<float, true>(y, rows, weight_of, expert_of, (const float*)h, ldh, tokens, hidden, top, place_of_pair, weighted,
+                                           (cudaStream_t)stream);
     if (dtype == KIPP_DT_BF16)
-        return kipp_launch(moe_combine_identity_kernel<bf16>, dim3((unsigned)tokens), dim3(hidden >= 2048 ? 512 : hidden >= 512 ? 256 : 128), 0, (cudaStream_t)stream, 1, y,
-                           rows, weight_of, expert_of, (const bf16*)h, ldh, hidden, top, place_of_pair, weighted);
+        return launch_combine<bf16, true>(y, rows, weight_of, expert_of, (const bf16*)h, ldh, tokens, hidden, top, place_of_pair, weighted,
+                                          (cudaStream_t)stream);
     return KIPP_ERR_DTYPE;
 }
 
