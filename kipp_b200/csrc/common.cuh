@@ -97,6 +97,14 @@ __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Asks for a weight vector before pdl_wait(): a step of few tokens reads every weight once and finds none of
+// them in the L2, and a small kernel that first meets its weights behind the wait adds that trip to the step's
+// chain.  The first blocks ask for all of it.
+__device__ __forceinline__ void prefetch_weights(const void* p, size_t bytes) {
+    if (p == nullptr || blockIdx.x >= 4 || blockIdx.y > 0) return;
+    for (size_t i = (size_t)threadIdx.x * 128; i < bytes; i += (size_t)blockDim.x * 128)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(p) + i));
+}
 
 // ---------------------------------------------------------------------------
 // Asynchronous 16-byte copies from global to shared memory: src_bytes of 0 writes zeros (the
