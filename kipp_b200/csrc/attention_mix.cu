@@ -334,8 +334,12 @@ attention_mix_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __re
 
 // The runs of a token merged in run order: o = sum_r acc_r e^(m_r - M) / sum_r l_r e^(m_r - M).  A block
 // takes MERGE_HEADS heads of a token: a warp per head forms the runs' weights once, then every
-// thread sums its elements over the runs.
-constexpr int MERGE_HEADS = 2;
+// thread sums its elements over the runs.  What such a launch lasts is its trips to the L2, one after the other: so the
+// token's position comes before the dependency wait (it lies in the step's lists, which a copy brought before any kernel
+// of the step started), and a thread's first values, MERGE_AHEAD runs of them, are on their way beside the maxima and
+// sums (with the position behind the wait, maxima, sums and values in turn, and the values of fewer than eight runs
+// one by one: 8.5 us a launch at one token of 300 keys, 5.1 so).
+constexpr int MERGE_HEADS = 2, MERGE_AHEAD = 8;
 template <typename T>
 __global__ void __launch_bounds__(THREADS)
 attention_mix_merge_kernel(T* __restrict__ out, const float* __restrict__ partial, const int* __restrict__ positions,
@@ -345,37 +349,51 @@ attention_mix_merge_kernel(T* __restrict__ out, const float* __restrict__ partia
     float* wts = merged + MERGE_HEADS * v_dim;
     float* fac = wts + MERGE_HEADS * max_runs;
     pdl_launch_dependents();
-    pdl_wait();
     const int t = blockIdx.x, pos = positions[t], h_first = blockIdx.y * MERGE_HEADS;
+    pdl_wait();
     const int nh = min(MERGE_HEADS, n_q - h_first);
     int first, kept;
     visible_runs(pos, window, keep_first, ex.chunk, first, kept);
     const int n_tiles = (kept + KT - 1) / KT + pos / KT - first / KT + 1;
     const int runs = min(max_runs, (n_tiles + SPLIT_TILES - 1) / SPLIT_TILES);
     const float* src = partial + (size_t)t * max_runs * n_q * (v_dim + 2);
+    const size_t run_stride = (size_t)n_q * (v_dim + 2);
     const int lane = threadIdx.x & 31;
+    auto values_of = [&](int e) { return src + (size_t)(h_first + e / v_dim) * (v_dim + 2) + 2 + e % v_dim; };
+    float ahead[MERGE_AHEAD];
+    auto load = [&](const float* p, int r0) {
+#pragma unroll
+        for (int i = 0; i < MERGE_AHEAD; ++i) ahead[i] = r0 + i < runs ? p[(size_t)(r0 + i) * run_stride] : 0.f;
+    };
+    if ((int)threadIdx.x < nh * v_dim) load(values_of(threadIdx.x), 0);
     for (int hl = threadIdx.x >> 5; hl < nh; hl += THREADS / 32) {
         const int h = h_first + hl;
-        float m = -INFINITY;
-        for (int r = lane; r < runs; r += 32) m = fmaxf(m, src[((size_t)r * n_q + h) * (v_dim + 2)]);
+        const float* p = src + (size_t)h * (v_dim + 2);
+        const float m0 = lane < runs ? p[(size_t)lane * run_stride] : -INFINITY, l0 = lane < runs ? p[(size_t)lane * run_stride + 1] : 0.f;
+        float m = m0;
+        for (int r = lane + 32; r < runs; r += 32) m = fmaxf(m, p[(size_t)r * run_stride]);
         m = warp_max(m);
         float l = 0.f;
         for (int r = lane; r < runs; r += 32) {
-            const float* p = src + ((size_t)r * n_q + h) * (v_dim + 2);
-            const float w = p[0] == -INFINITY ? 0.f : expf(p[0] - m);
+            const float mr = r == lane ? m0 : p[(size_t)r * run_stride], lr = r == lane ? l0 : p[(size_t)r * run_stride + 1];
+            const float w = mr == -INFINITY ? 0.f : expf(mr - m);
             wts[hl * max_runs + r] = w;
-            l = fmaf(p[1], w, l);
+            l = fmaf(lr, w, l);
         }
         l = warp_sum(l);
         if (lane == 0) fac[hl] = softmax_factor(m, l, ex.sink, h);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < nh * v_dim; e += THREADS) {
-        const int hl = e / v_dim, d = e % v_dim;
-        const float* p = src + (size_t)(h_first + hl) * (v_dim + 2) + 2 + d;
+        const int hl = e / v_dim;
+        const float* p = values_of(e);
         float o = 0.f;
-#pragma unroll 8
-        for (int r = 0; r < runs; ++r) o = fmaf(p[(size_t)r * n_q * (v_dim + 2)], wts[hl * max_runs + r], o);
+        for (int r0 = 0; r0 < runs; r0 += MERGE_AHEAD) {
+            if (r0 > 0 || e >= THREADS) load(p, r0);
+#pragma unroll
+            for (int i = 0; i < MERGE_AHEAD; ++i)
+                if (r0 + i < runs) o = fmaf(ahead[i], wts[hl * max_runs + r0 + i], o);
+        }
         merged[e] = o * fac[hl];
     }
     __syncthreads();

@@ -62,7 +62,8 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
     pdl_launch_dependents();
-    pdl_wait();
+    // (positions and the block table come with the step's lists, which a copy brought before any kernel of the step
+    // started: a head's place is looked up before the wait, and its weights are asked for)
     const int lane = threadIdx.x & 31;
     const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wg >= (long long)a.tokens * a.total_heads) return;
@@ -93,6 +94,10 @@ head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
               (size_t)within * D;
         into_cache = true;
     }
+
+    if (lane < 4 && g.norm_w != nullptr && t < 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(g.norm_w + min(32 * lane, D - 1)));
+    if (lane < 4 && bias != nullptr && t < 8) asm volatile("prefetch.global.L2 [%0];" ::"l"(bias + min(32 * lane, D - 1)));
+    pdl_wait();
 
     float inv = 1.f;
     const float* norm_w = g.norm_w;
@@ -305,7 +310,6 @@ head_matmul_mma_kernel(bf16* __restrict__ C, const bf16* __restrict__ A, const b
     __shared__ __align__(16) bf16 A_stage[H_STAGES][HM * HLD];
     __shared__ __align__(16) bf16 W_stage[H_STAGES][HN * HLD];
     pdl_launch_dependents();
-    pdl_wait();
     const int h = blockIdx.z;
     A += (size_t)h * a_head;
     W += (size_t)h * w_head;
@@ -316,25 +320,45 @@ head_matmul_mma_kernel(bf16* __restrict__ C, const bf16* __restrict__ A, const b
 #pragma unroll
     for (int j = 0; j < HN / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
     // 64 rows x 4 chunks of 8 elements for each operand: 256 chunks, two per thread and operand
-    auto fetch = [&](int k0, int stage) {
+    auto fetch_a = [&](int k0, int stage) {
 #pragma unroll
         for (int i = tid; i < HM * (HK / 8); i += 128) {
             const int r = i >> 2, c = (i & 3) * 8;
-            const bool ka = k0 + c < K;
-            const bool oa = ka && m0 + r < M, ow = ka && n0 + r < N;
+            const bool oa = k0 + c < K && m0 + r < M;
             cp_async16(smem_address(A_stage[stage] + r * HLD + c), oa ? A + (size_t)(m0 + r) * lda + k0 + c : A, oa ? 16 : 0);
+        }
+    };
+    auto fetch_w = [&](int k0, int stage) {
+#pragma unroll
+        for (int i = tid; i < HN * (HK / 8); i += 128) {
+            const int r = i >> 2, c = (i & 3) * 8;
+            const bool ow = k0 + c < K && n0 + r < N;
             cp_async16(smem_address(W_stage[stage] + r * HLD + c), ow ? W + (size_t)(n0 + r) * K + k0 + c : W, ow ? 16 : 0);
         }
     };
+    // The weights do not depend on the kernel before: their first stages are on their way, and of what follows the lines are
+    // asked for, before the wait.
+#pragma unroll
+    for (int s = 0; s < H_STAGES - 1; ++s)
+        if (s * HK < K) fetch_w(s * HK, s);
+    if (M <= HM)
+        for (int i = tid; i < HN * ((K + 63) / 64); i += 128) {
+            const int r = i % HN, k = (i / HN) * 64;
+            if (n0 + r < N && k >= (H_STAGES - 1) * HK) asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (size_t)(n0 + r) * K + k));
+        }
+    pdl_wait();
 #pragma unroll
     for (int s = 0; s < H_STAGES - 1; ++s) {
-        if (s * HK < K) fetch(s * HK, s);
+        if (s * HK < K) fetch_a(s * HK, s);
         cp_async_commit();
     }
     for (int k0 = 0, s = 0; k0 < K; k0 += HK, s = (s + 1) % H_STAGES) {
         cp_async_wait<H_STAGES - 2>();
         __syncthreads();                                            // this step's tiles are there, those of the step before are read
-        if (k0 + (H_STAGES - 1) * HK < K) fetch(k0 + (H_STAGES - 1) * HK, (s + H_STAGES - 1) % H_STAGES);
+        if (k0 + (H_STAGES - 1) * HK < K) {
+            fetch_a(k0 + (H_STAGES - 1) * HK, (s + H_STAGES - 1) % H_STAGES);
+            fetch_w(k0 + (H_STAGES - 1) * HK, (s + H_STAGES - 1) % H_STAGES);
+        }
         cp_async_commit();
         const bf16 *As = A_stage[s], *Ws = W_stage[s];
 #pragma unroll
