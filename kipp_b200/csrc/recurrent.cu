@@ -1266,8 +1266,8 @@ int launch_scan_chunk(const ScanArgs& b, const float* vec, float* o_raw, int sli
 // time by neighbouring lanes.  CHUNK: at 64 the chunks' states are 67 MB written and read three times for
 // 2,048 tokens of 64 heads, at 256 the pairs (t, s) cost as much as the states save.
 //
-// 2,048 tokens, 64 heads of 128 x 64, one sequence: 192 us (28 + 48 + 10 + 106) against 477 us for the scan in
-// order, whose 128 blocks walk 0.23 us a token.
+// 2,048 tokens, 64 heads of 128 x 64, one sequence: 164 us (19 + 48 + 10 + 87) against 477 us for the scan in
+// order, whose 128 blocks walk 0.23 us a token; the whole layer for four sequences of 511: 261 us against 412.
 constexpr int CHUNK = 128, CHUNK_COLS = 64, CHUNK_SLICE = 32;
 struct ChunkScratch {
     float* states;      // [chunks][heads][dim][v_dim]: (2) leaves the chunk's own share, (3) the state before the chunk
@@ -1294,7 +1294,7 @@ __device__ __forceinline__ bool chunk_at(const ScanArgs& a, int i, int& row0, in
     return false;
 }
 
-// (1) blockIdx.y 3 g + z: the 64 x 64 part (s half, t half) = (0, 0), (0, 1), (1, 1) of group g; the last y: the decays.
+// (1) blockIdx.y 1 + 3 g + z: the 64 x 64 part (s half, t half) = (0, 0), (0, 1), (1, 1) of group g; y 0: the decays.
 constexpr int PAIRS_ROW = CHUNK_SLICE + 4;
 __global__ void __launch_bounds__(128)
 ssd_chunk_pairs_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* __restrict__ dts, const ChunkScratch w) {
@@ -1304,26 +1304,33 @@ ssd_chunk_pairs_kernel(const ScanArgs a, const float* __restrict__ conv, const f
     const int ci = blockIdx.x, tid = threadIdx.x, D = a.dim;
     int row0, n;
     if (!chunk_at(a, ci, row0, n)) return;
-    if ((int)blockIdx.y == 3 * a.groups) {
+    if (blockIdx.y == 0) {                                            // (first: its loops are the longest)
         float* up = w.up_to + (size_t)ci * CHUNK * a.heads;
         float* down = w.after + (size_t)ci * CHUNK * a.heads;
         for (int h = tid; h < a.heads; h += 128) {
             const float2* d = dts + (size_t)row0 * a.heads + h;
             float p = 1.f, q = 1.f;
-#pragma unroll 8
-            for (int t = 0; t < CHUNK; ++t) {
-                if (t < n) p *= d[(size_t)t * a.heads].x;
-                up[(size_t)t * a.heads + h] = p;
+            for (int t0 = 0; t0 < CHUNK; t0 += 32) {                  // (32 loads on their way at a time)
+                float x[32];
+#pragma unroll
+                for (int k = 0; k < 32; ++k) x[k] = t0 + k < n ? d[(size_t)(t0 + k) * a.heads].x : 1.f;
+#pragma unroll
+                for (int k = 0; k < 32; ++k) up[(size_t)(t0 + k) * a.heads + h] = p *= x[k];
             }
-#pragma unroll 8
-            for (int s = CHUNK - 1; s >= 0; --s) {
-                down[(size_t)s * a.heads + h] = q;
-                if (s < n) q *= d[(size_t)s * a.heads].x;
+            for (int t0 = CHUNK - 32; t0 >= 0; t0 -= 32) {
+                float x[32];
+#pragma unroll
+                for (int k = 0; k < 32; ++k) x[k] = t0 + k < n ? d[(size_t)(t0 + k) * a.heads].x : 1.f;
+#pragma unroll
+                for (int k = 31; k >= 0; --k) {
+                    down[(size_t)(t0 + k) * a.heads + h] = q;
+                    q *= x[k];
+                }
             }
         }
         return;
     }
-    const int g = blockIdx.y / 3, z = blockIdx.y % 3, s0 = z == 2 ? 64 : 0, t0 = z == 0 ? 0 : 64;
+    const int part = blockIdx.y - 1, g = part / 3, z = part % 3, s0 = z == 2 ? 64 : 0, t0 = z == 0 ? 0 : 64;
     const int inner = a.heads * a.v_dim, slices = (D + CHUNK_SLICE - 1) / CHUNK_SLICE;
     if (n <= t0) return;                                              // (rows past the last token are read by nobody)
     auto fetch = [&](int slice, int buf) {
@@ -1519,8 +1526,9 @@ ssd_chunk_carry_kernel(const ScanArgs a, const ChunkScratch w) {
     *slot = s;
 }
 
-// (4) the outputs.  Thread t makes row t of l_ts (C_t . B_s), a slice of s at a time from the last to the first, so that
-// l grows by one factor per step.
+// (4) the outputs.  Thread t makes row t of l_ts (C_t . B_s) in place, a slice of s at a time from the last to the first,
+// so that l grows by one factor per step.  (With the pairs read from global memory at that place, a trip for
+// every eight of them, the kernel took 106 us; 87 so.)
 __global__ void __launch_bounds__(128)
 ssd_chunk_output_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* __restrict__ dts, const ChunkScratch w,
                         float* __restrict__ o_raw) {
@@ -1538,7 +1546,7 @@ ssd_chunk_output_kernel(const ScanArgs a, const float* __restrict__ conv, const 
     up[tid] = w.up_to[((size_t)ci * CHUNK + tid) * a.heads + h];
     const float* ct = w.c_rows + ((size_t)ci * a.groups + g) * D * CHUNK;
     const float* s_in = w.states + ((size_t)ci * a.heads + h) * D * V + v0;
-    const float* pairs = w.pairs + ((size_t)ci * a.groups + g) * CHUNK * CHUNK + tid;
+    const float* pairs = w.pairs + ((size_t)ci * a.groups + g) * CHUNK * CHUNK;
     constexpr int BUF = CHUNK_SLICE * (CHUNK + CHUNK_COLS);
     auto fetch = [&](int sl, int buf) {
         float* to = smem + buf * BUF;
@@ -1578,26 +1586,23 @@ ssd_chunk_output_kernel(const ScanArgs a, const float* __restrict__ conv, const 
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = mul2(acc[i][j], p);
     }
-    // slices of s from the last that holds a token; thread t's row of a slice, s from high to low
+    // slices of s from the last that holds a token, the next one's pairs and x on their way
     const int last = (n - 1) / CHUNK_SLICE;
     float l = 1.f;
     for (int sl = last; sl >= 0; --sl) {
         float* rows = smem + (sl & 1) * BUF;
         float* x = rows + CHUNK_SLICE * CHUNK;
-        chunk_fetch_x(a, conv, x, row0, n, sl * CHUNK_SLICE, h, v0);
-        cp_async_commit();
+        // thread t's column, s from high to low (above the diagonal lies what nobody wrote)
 #pragma unroll 8
         for (int k = CHUNK_SLICE - 1; k >= 0; --k) {
             const int s = sl * CHUNK_SLICE + k;
             float m = 0.f;
-            if (s <= tid && tid < n) {
-                m = l * pairs[(size_t)s * CHUNK];
+            if (s <= tid) {
+                m = l * rows[k * CHUNK + tid];
                 l *= decay[s];
             }
             rows[k * CHUNK + tid] = m;
         }
-        cp_async_wait<0>();
-        __syncthreads();
         chunk_scale_x(x, [&](int k) { return dt[sl * CHUNK_SLICE + k]; });
         __syncthreads();
         if (sl * CHUNK_SLICE >= 64) chunk_products<2>(acc, rows, x, r, c);      // the rows below 64 see none of these
@@ -1618,13 +1623,14 @@ ssd_chunk_output_kernel(const ScanArgs a, const float* __restrict__ conv, const 
 }
 
 // Whether the form by chunks pays: heads whose rows and columns fill most of the products' tiles, 192 tokens an
-// entry on average (a partial chunk costs what a whole one does), few enough entries to look through.  What it keeps lies where the records of the general form
-// would; groups that are hardly shared by heads may not fit there.
+// entry on average (a partial chunk costs what a whole one does) and 320 in all (300 tokens of one sequence: 117 us the
+// layer against 111), few enough entries to look through.  What it keeps lies where the records of the general
+// form would; groups that are hardly shared by heads may not fit there.
 inline long long chunk_room(int tokens, int heads, int dim, int v_dim) {
     return (long long)tokens * heads * (2LL * dim + 4 + v_dim) - (2LL * tokens * heads + 3) / 4 * 4;
 }
 inline bool by_chunks(int entries, int tokens, int heads, int groups, int dim, int v_dim) {
-    return dim <= CHUNK && dim > CHUNK / 2 && v_dim > CHUNK_COLS / 2 && tokens >= 192 * entries && entries <= 64 && heads <= 65535 &&
+    return dim <= CHUNK && dim > CHUNK / 2 && v_dim > CHUNK_COLS / 2 && tokens >= 192 * entries && tokens >= 320 && entries <= 64 && heads <= 65535 &&
            chunk_floats(tokens, entries, heads, groups, dim, v_dim) <= chunk_room(tokens, heads, dim, v_dim);
 }
 inline int launch_ssd_chunks(const ScanArgs& a, const float* conv, const float2* dts, float* scratch, float* o_raw, int tokens,
@@ -1837,8 +1843,23 @@ extern "C" int kipp_retention_scan(void* out, long long ld_out, const void* proj
     a.k_scale = k_scale; a.eps = eps; a.out_scale = out_scale; a.gate = gate;
     if (dtype == KIPP_DT_F32) return launch_scan<float, RETENTION>(a, entries, tokens, scratch, (cudaStream_t)stream);
     if (dtype == KIPP_DT_BF16) return launch_scan<bf16, RETENTION>(a, entries, tokens, scratch, (cudaStream_t)stream);
+    auto fetch_pairs = [&](int sl) {
+        float* to = smem + (sl & 1) * BUF;
+#pragma unroll
+        for (int j = 0; j < CHUNK_SLICE * CHUNK / 4 / 128; ++j) {
+            const int i = 4 * (j * 128 + tid);
+            cp_async16(smem_address(to + i), pairs + (size_t)sl * CHUNK_SLICE * CHUNK + i, 16);
+        }
+        chunk_fetch_x(a, conv, to + CHUNK_SLICE * CHUNK, row0, n, sl * CHUNK_SLICE, h, v0);
+        cp_async_commit();
+    };
+    fetch_pairs(last);
     return KIPP_ERR_DTYPE;
 }
+        if (sl > 0) fetch_pairs(sl - 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
 
 extern "C" int kipp_delta_rule_scan(void* out, long long ld_out, const void* proj, long long ld_proj, int dtype,
                                     int r_off, int k_off, int v_off, int g_off, int a_off, const void* w_raw,
@@ -1859,6 +1880,7 @@ extern "C" int kipp_delta_rule_scan(void* out, long long ld_out, const void* pro
     if (dtype == KIPP_DT_BF16) return launch_scan<bf16, DELTA_RULE>(a, entries, tokens, scratch, (cudaStream_t)stream);
     return KIPP_ERR_DTYPE;
 }
+        __syncthreads();
 
 // The gated matrix memory (see the head of this file): q, k [heads, dim], v and the output gate
 // [heads, v_dim] and the two gates' pre-activations [heads] are columns of proj; the state of a slot
