@@ -880,11 +880,161 @@ ssd_scan_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* 
     }
 }
 
-// The gated delta rule: a thread owns R rows of one column.  The decayed state meets k and q in one pass and both
-// sums travel through the same shuffles; the token's own write then joins the output as (q . k) u.
+// The gated delta rule: a thread owns 4 columns x R rows, as above.  The decayed state meets k; the four columns' sums
+// over P lanes meet with every exchange halving the columns a lane is responsible for, the lane that ends up with a
+// column forms its u = beta (v - S^T k), and three more exchanges hand the four u to everybody.  The sums with q travel
+// while the next token is worked on, and the token's own write joins the output as (q . k) u.
+// (With one column per thread, as below, a token costs ten shuffles and three 16-byte reads of shared memory for FOUR
+// elements of the state, and many blocks on an SM are bound by those: sequences of 1,277, 700 and 753 tokens, 16 heads:
+// 712 us so, 431 us here.)
 template <int P, int R, int WARPS, bool EXACT>
 __global__ void __launch_bounds__(32 * WARPS)
 gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* __restrict__ o_raw, int v_slices, int tokens) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int COLS = SCAN_COLS * 32 * WARPS / P;
+    const int D = a.dim, V = a.v_dim, nvd = 3 * D + 4, rec = nvd + V;
+    const TokenBatch tb = token_batch(nvd + COLS);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int tid = threadIdx.x, p = tid % P, slice = blockIdx.x % v_slices, eh = blockIdx.x / v_slices;
+    const int e = eh / a.heads, h = eh % a.heads;
+    const int row0 = a.q_start[e], n_tok = a.q_start[e + 1] - row0;
+    const int cl = tid / P * SCAN_COLS, col = slice * COLS + cl;
+    const bool live = col < V;                                      // (V is a multiple of 4: a group is whole or absent)
+    const bool odd_lane = p & 1, second = p & 2;
+    const int mine = 2 * (p & 1) + (p >> 1 & 1);                    // the column whose sums end up in this lane
+    float* S_slot = a.state + (size_t)a.slots[e] * (size_t)a.slot_stride + (size_t)h * D * V;
+    const float* recs = vec + ((size_t)h * tokens + row0) * rec;
+    auto fetch = [&](int t0, float* buf) {
+        const int nb = min(tb.tokens, n_tok - t0), n4 = nvd / 4, per = n4 + COLS / 4;
+        for (int t = tid >> 5; t < nb; t += WARPS) {
+            const float* src = recs + (size_t)(t0 + t) * rec;
+            const uint32_t to = smem_address(buf + (size_t)t * tb.floats);
+            for (int c = tid & 31; c < per; c += 32) {
+                const int x = slice * COLS + 4 * (c - n4);
+                const bool ok = c < n4 || x < V;
+                cp_async16(to + 16 * c, src + (c < n4 ? 4 * c : ok ? nvd + x : 0), ok ? 16 : 0);
+            }
+        }
+        cp_async_commit();
+    };
+    float2 S[R / 2][SCAN_COLS];             // pairs of neighbouring rows
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = 4 * (p + P * (i >> 2)) + (i & 3);
+        const float4 s4 = live && r < D ? *reinterpret_cast<const float4*>(S_slot + (size_t)r * V + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float x[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+        for (int c = 0; c < SCAN_COLS; ++c) (i & 1 ? S[i >> 1][c].y : S[i >> 1][c].x) = x[c];
+    }
+    struct Token { float2 q[R / 2], k[R / 2], g[R / 2]; float beta, qk, v; };
+    auto take = [&](const float* tok, Token& n) {
+#pragma unroll
+        for (int q = 0; q < R / 4; ++q) {
+            const int r = 4 * (p + P * q);
+            float4 q4 = make_float4(0.f, 0.f, 0.f, 0.f), k4 = q4, g4 = q4;
+            if (EXACT || r < D) {
+                q4 = *reinterpret_cast<const float4*>(tok + r);
+                k4 = *reinterpret_cast<const float4*>(tok + D + r);
+                g4 = *reinterpret_cast<const float4*>(tok + 2 * D + r);
+            }
+            n.q[2 * q] = make_float2(q4.x, q4.y); n.q[2 * q + 1] = make_float2(q4.z, q4.w);
+            n.k[2 * q] = make_float2(k4.x, k4.y); n.k[2 * q + 1] = make_float2(k4.z, k4.w);
+            n.g[2 * q] = make_float2(g4.x, g4.y); n.g[2 * q + 1] = make_float2(g4.z, g4.w);
+        }
+        const float2 bq = *reinterpret_cast<const float2*>(tok + 3 * D);
+        n.beta = bq.x;
+        n.qk = bq.y;
+        n.v = tok[nvd + cl + mine];
+    };
+    // the four columns' sums over the P lanes: each lane gets column `mine`
+    auto meet = [&](const float (&o)[SCAN_COLS]) {
+        float k0 = odd_lane ? o[2] : o[0], k1 = odd_lane ? o[3] : o[1];
+        k0 += __shfl_xor_sync(0xffffffffu, odd_lane ? o[0] : o[2], 1);
+        k1 += __shfl_xor_sync(0xffffffffu, odd_lane ? o[1] : o[3], 1);
+        float y = (second ? k1 : k0) + __shfl_xor_sync(0xffffffffu, second ? k0 : k1, 2);
+#pragma unroll
+        for (int x = 4; x < P; x <<= 1) y += __shfl_xor_sync(0xffffffffu, y, x);
+        return y;
+    };
+    fetch(0, smem);
+    int buf = 0;
+    for (int t0 = 0; t0 < n_tok; t0 += tb.tokens, buf ^= 1) {
+        const int nb = min(tb.tokens, n_tok - t0);
+        if (t0 + tb.tokens < n_tok) fetch(t0 + tb.tokens, smem + (size_t)(buf ^ 1) * tb.tokens * tb.floats);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* toks = smem + (size_t)buf * tb.tokens * tb.floats;
+        float* out = o_raw + (size_t)(row0 + t0) * (a.heads * V) + h * V + col + mine;
+        const bool writes = live && p < SCAN_COLS;
+        Token even, odd;
+        float last[SCAN_COLS] = {0.f, 0.f, 0.f, 0.f}, last_qk = 0.f, last_u = 0.f;      // the token before: its sums with q, q . k, u
+        // one token from `now`; `next` is fetched meanwhile (the last token of a batch fetches itself again)
+        auto step = [&](int t, const Token& now, Token& next) {
+            float2 us[SCAN_COLS];
+#pragma unroll
+            for (int i = 0; i < R / 2; ++i)
+#pragma unroll
+                for (int c = 0; c < SCAN_COLS; ++c) {
+                    S[i][c] = mul2(S[i][c], now.g[i]);
+                    us[c] = i == 0 ? mul2(now.k[i], S[i][c]) : fma2(now.k[i], S[i][c], us[c]);
+                }
+            float sum[SCAN_COLS];
+#pragma unroll
+            for (int c = 0; c < SCAN_COLS; ++c) sum[c] = us[c].x + us[c].y;
+            const float uy = meet(sum);
+            const float y = fmaf(last_qk, last_u, meet(last));
+            if (writes && t > 0) {
+                *out = y;
+                out += a.heads * V;
+            }
+            float2 os[SCAN_COLS];
+#pragma unroll
+            for (int i = 0; i < R / 2; ++i)
+#pragma unroll
+                for (int c = 0; c < SCAN_COLS; ++c) os[c] = i == 0 ? mul2(now.q[i], S[i][c]) : fma2(now.q[i], S[i][c], os[c]);
+            take(toks + (size_t)min(t + 1, nb - 1) * tb.floats, next);
+            const float u = now.beta * (now.v - uy);
+            const float over2 = __shfl_xor_sync(0xffffffffu, u, 2);
+            const float lo = second ? over2 : u, hi = second ? u : over2;                 // the pair of columns of this parity
+            const float lo1 = __shfl_xor_sync(0xffffffffu, lo, 1), hi1 = __shfl_xor_sync(0xffffffffu, hi, 1);
+            const float2 u2[SCAN_COLS] = {both(odd_lane ? lo1 : lo), both(odd_lane ? hi1 : hi), both(odd_lane ? lo : lo1),
+                                          both(odd_lane ? hi : hi1)};
+#pragma unroll
+            for (int i = 0; i < R / 2; ++i)
+#pragma unroll
+                for (int c = 0; c < SCAN_COLS; ++c) S[i][c] = fma2(now.k[i], u2[c], S[i][c]);
+            last_qk = now.qk;
+            last_u = u;
+#pragma unroll
+            for (int c = 0; c < SCAN_COLS; ++c) last[c] = os[c].x + os[c].y;
+        };
+        take(toks, even);
+        int t = 0;
+        for (; t + 1 < nb; t += 2) {
+            step(t, even, odd);
+            step(t + 1, odd, even);
+        }
+        if (t < nb) step(t, even, odd);
+        const float y = fmaf(last_qk, last_u, meet(last));
+        if (writes) *out = y;
+        __syncthreads();                    // the buffer is free for the batch after the next
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int r = 4 * (p + P * (i >> 2)) + (i & 3);
+        auto at = [&](int c) { return i & 1 ? S[i >> 1][c].y : S[i >> 1][c].x; };
+        if (live && r < D) *reinterpret_cast<float4*>(S_slot + (size_t)r * V + col) = make_float4(at(0), at(1), at(2), at(3));
+    }
+}
+
+// The same with one column per thread, the same sums in the same order: more blocks, whose tokens wait for a shorter chain
+// (five exchanges instead of seven, a quarter of the arithmetic).  For grids that leave no SM more than one of its
+// blocks (see launch_gated_delta_scan): 8 heads of 128 x 128, one sequence of 2,048 tokens: 0.19 us a token against 0.27.
+template <int P, int R, int WARPS, bool EXACT>
+__global__ void __launch_bounds__(32 * WARPS)
+gated_delta_column_kernel(const ScanArgs a, const float* __restrict__ vec, float* __restrict__ o_raw, int v_slices, int tokens) {
     extern __shared__ __align__(16) float smem[];
     constexpr int COLS = 32 * WARPS / P;
     const int D = a.dim, V = a.v_dim, nvd = 3 * D + 4, rec = nvd + V;
@@ -950,21 +1100,20 @@ gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* 
         Token even, odd;
         // one token from `now`; `next` is fetched meanwhile (the last token of a batch fetches itself again)
         auto step = [&](int t, const Token& now, Token& next) {
-            // (two sums per product, so that no chain is longer than a quarter of the rows)
-            float2 us[2], os[2];
+            float2 us, os;
 #pragma unroll
             for (int i = 0; i < R / 2; ++i) {
                 S[i] = mul2(S[i], now.g[i]);
-                us[i & 1] = i < 2 ? mul2(now.k[i], S[i]) : fma2(now.k[i], S[i], us[i & 1]);
+                us = i == 0 ? mul2(now.k[i], S[i]) : fma2(now.k[i], S[i], us);
             }
-            float uy = (us[0].x + us[0].y) + (us[1].x + us[1].y);
+            float uy = us.x + us.y;
 #pragma unroll
-            for (int x = P / 2; x > 0; x >>= 1) uy += __shfl_xor_sync(0xffffffffu, uy, x);
+            for (int x = 1; x < P; x <<= 1) uy += __shfl_xor_sync(0xffffffffu, uy, x);
 #pragma unroll
-            for (int i = 0; i < R / 2; ++i) os[i & 1] = i < 2 ? mul2(now.q[i], S[i]) : fma2(now.q[i], S[i], os[i & 1]);
-            float oy = (os[0].x + os[0].y) + (os[1].x + os[1].y);
+            for (int i = 0; i < R / 2; ++i) os = i == 0 ? mul2(now.q[i], S[i]) : fma2(now.q[i], S[i], os);
+            float oy = os.x + os.y;
 #pragma unroll
-            for (int x = P / 2; x > 0; x >>= 1) oy += __shfl_xor_sync(0xffffffffu, oy, x);
+            for (int x = 1; x < P; x <<= 1) oy += __shfl_xor_sync(0xffffffffu, oy, x);
             take(toks + (size_t)min(t + 1, nb - 1) * tb.floats, next);
             const float u = now.beta * (now.v - uy);
             const float2 u2 = both(u);
@@ -1093,10 +1242,26 @@ int launch_ssd_scan(const ScanArgs& a, const float* conv, const float2* dts, flo
                        dim3((unsigned)(entries * a.heads * slices)), dim3(32 * WARPS), (size_t)2 * tb.tokens * tb.floats * sizeof(float),
                        stream, a, conv, dts, o_raw, slices);
 }
-// (8 columns a block: the more blocks, the fewer warps share an SM, and a token's chain is what this scan is bound by)
+// 16 columns a block, or, where its blocks of 8 columns are no more than the SMs, a thread per column (measured with layers
+// of 128 x 128, the whole layer: one sequence of 2,048 tokens, 8 heads: 478 us against 623; 16 heads, 256 blocks: 697
+// against 661; four sequences of 511, 16 heads: 581 against 356).  The bits are the same.
 template <int P, int R>
 int launch_gated_delta_scan(const ScanArgs& a, const float* vec, float* o_raw, int entries, int tokens, cudaStream_t stream) {
-    constexpr int WARPS = P / 4, COLS = 32 * WARPS / P;
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    }
+    constexpr int CHAINS = P / 4, CHAIN_COLS = 32 * CHAINS / P;
+    const int chain_slices = (a.v_dim + CHAIN_COLS - 1) / CHAIN_COLS;
+    if ((long long)entries * a.heads * chain_slices <= sms) {
+        const TokenBatch tb = token_batch(3 * a.dim + 4 + CHAIN_COLS);
+        return launch_walk(a, tokens, a.dim == P * R ? gated_delta_column_kernel<P, R, CHAINS, true> : gated_delta_column_kernel<P, R, CHAINS, false>,
+                           dim3((unsigned)(entries * a.heads * chain_slices)), dim3(32 * CHAINS),
+                           (size_t)2 * tb.tokens * tb.floats * sizeof(float), stream, a, vec, o_raw, chain_slices, tokens);
+    }
+    constexpr int WARPS = P / 8, COLS = SCAN_COLS * 32 * WARPS / P;
     const TokenBatch tb = token_batch(3 * a.dim + 4 + COLS);
     const int slices = (a.v_dim + COLS - 1) / COLS;
     return launch_walk(a, tokens, a.dim == P * R ? gated_delta_scan_kernel<P, R, WARPS, true> : gated_delta_scan_kernel<P, R, WARPS, false>,

@@ -141,6 +141,27 @@ def test_state_space_alone(name, layer, dtype):
     close(_in_portions(eng, layer, "mixer", h_dev, (1, 2, 1, 1, 3, 17, 2, 39)), want, dtype, f"{name} layer {layer}")
 
 
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (36, 20), (64, 132), (200, 64)])
+def test_the_two_gated_delta_scans_agree(tmp_path, dim, vdim):
+    """A sequence alone runs with a thread per column, among so many that their blocks are more than the SMs with four
+    columns per thread: the same bits in 32-bit, and float64's values, over a batch of tokens and a half."""
+    from kipp_b200.engine import Engine, StepEntry
+    cfg = {"architecture": "Nogavik", "vocab": 50, "width": 32, "norm": {"eps": 1e-5},
+           "layers": [parallel_layer(left(1, 1, 8, 8, 0.5), right(2, 2, dim, vdim, 4, 6, 4), None)]}
+    folder = write_folder(str(tmp_path / "m"), cfg, dict(seed=6, sigma=0.3, norm_jitter=0.1))
+    many, n = 75, 21
+    eng = Engine.from_folder(folder, dtype="float32", page_size=16, cache_tokens=4096, max_requests=many + 1, max_batch_tokens=2048,
+                             cuda_graphs=False)
+    assert 2 * many * -(-vdim // 8) > 148 >= 2 * -(-vdim // 8)
+    h = torch.randn(many * n, 32, generator=torch.Generator().manual_seed(2)).cuda()
+    alone, among = torch.zeros(n, 32, device="cuda"), torch.zeros(many * n, 32, device="cuda")
+    eng.run_part([StepEntry("alone", [0] * n, [])], 0, "mixer/1", input=h[n:2 * n].contiguous(), residual=alone)
+    eng.run_part([StepEntry(i, [0] * n, []) for i in range(many)], 0, "mixer/1", input=h, residual=among)
+    assert torch.equal(alone, among[n:2 * n])
+    want = P.gated_delta(cfg["layers"][0]["mixer"]["right"], f64(read_weights(folder)), "l0.mix.right.", h[n:2 * n].double().cpu(), 1e-5)
+    close(alone, want, "float32", "alone")
+
+
 def test_decays_and_write_rates_far_from_the_middle(tmp_path):
     """Decays from almost nothing kept to almost all, write rates near 0 and 1, softplus at both of its
     ends: the state follows the equations over 80 tokens."""
