@@ -1845,8 +1845,23 @@ ssd_chunk_output_kernel(const ScanArgs a, const float* __restrict__ conv, const 
     }
     // slices of s from the last that holds a token, the next one's pairs and x on their way
     const int last = (n - 1) / CHUNK_SLICE;
+    auto fetch_pairs = [&](int sl) {
+        float* to = smem + (sl & 1) * BUF;
+#pragma unroll
+        for (int j = 0; j < CHUNK_SLICE * CHUNK / 4 / 128; ++j) {
+            const int i = 4 * (j * 128 + tid);
+            cp_async16(smem_address(to + i), pairs + (size_t)sl * CHUNK_SLICE * CHUNK + i, 16);
+        }
+        chunk_fetch_x(a, conv, to + CHUNK_SLICE * CHUNK, row0, n, sl * CHUNK_SLICE, h, v0);
+        cp_async_commit();
+    };
+    fetch_pairs(last);
     float l = 1.f;
     for (int sl = last; sl >= 0; --sl) {
+        if (sl > 0) fetch_pairs(sl - 1);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
         float* rows = smem + (sl & 1) * BUF;
         float* x = rows + CHUNK_SLICE * CHUNK;
         // thread t's column, s from high to low (above the diagonal lies what nobody wrote)
@@ -1864,6 +1879,7 @@ ssd_chunk_output_kernel(const ScanArgs a, const float* __restrict__ conv, const 
         __syncthreads();
         if (sl * CHUNK_SLICE >= 64) chunk_products<2>(acc, rows, x, r, c);      // the rows below 64 see none of these
         else chunk_products<0>(acc, rows, x, r, c);
+        __syncthreads();
     }
     float* out = o_raw + (size_t)row0 * inner + h * V + v0;
 #pragma unroll
@@ -2106,23 +2122,8 @@ extern "C" int kipp_retention_scan(void* out, long long ld_out, const void* proj
     a.k_scale = k_scale; a.eps = eps; a.out_scale = out_scale; a.gate = gate;
     if (dtype == KIPP_DT_F32) return launch_scan<float, RETENTION>(a, entries, tokens, scratch, (cudaStream_t)stream);
     if (dtype == KIPP_DT_BF16) return launch_scan<bf16, RETENTION>(a, entries, tokens, scratch, (cudaStream_t)stream);
-    auto fetch_pairs = [&](int sl) {
-        float* to = smem + (sl & 1) * BUF;
-#pragma unroll
-        for (int j = 0; j < CHUNK_SLICE * CHUNK / 4 / 128; ++j) {
-            const int i = 4 * (j * 128 + tid);
-            cp_async16(smem_address(to + i), pairs + (size_t)sl * CHUNK_SLICE * CHUNK + i, 16);
-        }
-        chunk_fetch_x(a, conv, to + CHUNK_SLICE * CHUNK, row0, n, sl * CHUNK_SLICE, h, v0);
-        cp_async_commit();
-    };
-    fetch_pairs(last);
     return KIPP_ERR_DTYPE;
 }
-        if (sl > 0) fetch_pairs(sl - 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
 
 extern "C" int kipp_delta_rule_scan(void* out, long long ld_out, const void* proj, long long ld_proj, int dtype,
                                     int r_off, int k_off, int v_off, int g_off, int a_off, const void* w_raw,
@@ -2143,7 +2144,6 @@ extern "C" int kipp_delta_rule_scan(void* out, long long ld_out, const void* pro
     if (dtype == KIPP_DT_BF16) return launch_scan<bf16, DELTA_RULE>(a, entries, tokens, scratch, (cudaStream_t)stream);
     return KIPP_ERR_DTYPE;
 }
-        __syncthreads();
 
 // The gated matrix memory (see the head of this file): q, k [heads, dim], v and the output gate
 // [heads, v_dim] and the two gates' pre-activations [heads] are columns of proj; the state of a slot
