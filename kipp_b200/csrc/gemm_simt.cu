@@ -13,13 +13,14 @@
 // many threads at once, the groups of four what lets a small product of many tokens be shared by more blocks.
 //
 // Three kernels, chosen by shape alone, with that one order:
-//   few   float32, up to FEW_MAX tokens: bound by the weights' bytes (a token is 2 operations per 4 bytes).  A
+//   few   float32, up to FEW_MAX tokens (16 of many features): bound by the weights' bytes (a token is 2 operations per 4 bytes).  A
 //         block holds 16 features, a thread one feature and one run, so a 2,048-feature matrix still
 //         gives 128 blocks of 256 chains; the weights travel by asynchronous copies, five chunks of 64 bytes
 //         per thread on their way, the first of them before the wait for the kernel before.  12,288 x 2,048 with
-//         1, 3 and 16 tokens: 24, 34 and 94 us (100 MB: 15 us of copy rate; the kernel below, which ran before: 334, 339
-//         and 353); 2,048 x 6,144 with 3: 30 us (543).  At 32 tokens its two passes still win where the features are
-//         few (2,048 x 2,048: 31 us against 88 in tiles) and tie where they are many (12,288: 176 against 174).
+//         1, 3 and 16 tokens: 24, 28 and 95 us (100 MB: 15 us of copy rate; the kernel below, which ran before: 334, 339
+//         and 353); 2,048 x 6,144 with 3: 24 us (543).  From 17 tokens on it needs two passes, which still win where the
+//         features are few (32 tokens, 2,048 and 3,072 x 2,048: 31 and 48 us against 58 and 74 in tiles) and lose where
+//         they are many (12,288 and 32,000: 180 and 442 us against 104 and 260): from MANY_F on those are tiles'.
 //   tile  float32, more tokens: bound by the FMA pipes.  128 features x 64 tokens per block of 128 threads, 8 x 8 per
 //         thread in float32 pairs, operands in shared memory with k outermost, so that a k's 16 values cost a
 //         thread four 16-byte reads (with four bytes copied at a time: 24 copies per 1,024 FMAs); the groups of runs
@@ -137,34 +138,41 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
 // ---------------------------------------------------------------------------------------
 // Few tokens (see the head of the file).  Warp w of a block holds runs 2w and 2w + 1 of the block's 16
 // features; a warp copies only what its own lanes read, so its ring needs no block-wide barrier.
-constexpr int FEW_F = 16, FEW_STAGES = 5, FEW_THREADS = 16 * MAX_RUNS, FEW_MAX = 32;
+// PAIR: a thread has two features (f and f + 16 of the block's 32), so that a token's values, which every lane of a
+// run reads, serve both: of several tokens those reads are what an SM is busy with.
+constexpr int FEW_F = 16, FEW_THREADS = 16 * MAX_RUNS, FEW_MAX = 32, MANY_F = 64 * 148;
 constexpr int FEW_CHUNK = BK * 4 + 16;              // 64 bytes of a feature's row, padded against bank conflicts
-constexpr int FEW_SMEM = (FEW_THREADS / 32) * FEW_STAGES * 32 * FEW_CHUNK;
+template <bool PAIR> struct Few {
+    static constexpr int PER = PAIR ? 2 : 1, F = FEW_F * PER, STAGES = PAIR ? 4 : 5, CHUNKS = 32 * PER;
+    static constexpr int SMEM = (FEW_THREADS / 32) * STAGES * CHUNKS * FEW_CHUNK;
+};
 
-template <int MT, int EPI>
+template <int MT, int EPI, bool PAIR>
 __global__ void __launch_bounds__(FEW_THREADS)
 gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
                 int M, int N, int K, int lda, int ldw, int ldc) {
+    using Form = Few<PAIR>;
     extern __shared__ __align__(16) uint8_t ring[];
-    __shared__ float parts[MAX_RUNS][MT][FEW_F + 1];
+    __shared__ float parts[MAX_RUNS][MT][Form::F + 1];
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n0 = blockIdx.x * FEW_F, m0 = blockIdx.y * MT;
+    const int n0 = blockIdx.x * Form::F, m0 = blockIdx.y * MT;
     const int run = run_length(K), steps = run / BK;
-    uint8_t* mine = ring + (size_t)warp * FEW_STAGES * 32 * FEW_CHUNK;
-    // copy j of a step: 16 bytes (lane & 3) of chunk 8 j + lane / 4; chunk c is feature c & 15 of run 2 warp + c / 16
+    uint8_t* mine = ring + (size_t)warp * Form::STAGES * Form::CHUNKS * FEW_CHUNK;
+    // copy j of a step: 16 bytes (lane & 3) of chunk 8 j + lane / 4; chunk c is feature c & 15 (the second 32: 16 + c & 15)
+    // of run 2 warp + c / 16 & 1
     auto fetch = [&](int step, int stage) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = 8 * j + (lane >> 2), n = n0 + (c & 15);
-            const int k = (2 * warp + (c >> 4)) * run + step * BK + (lane & 3) * 4;
+        for (int j = 0; j < 4 * Form::PER; ++j) {
+            const int c = 8 * j + (lane >> 2), n = n0 + (c & 15) + (c >> 5) * FEW_F;
+            const int k = (2 * warp + (c >> 4 & 1)) * run + step * BK + (lane & 3) * 4;
             const bool in = n < N && k < K;
-            cp_async16(smem_address(mine + (size_t)(stage * 32 + c) * FEW_CHUNK + (lane & 3) * 16),
+            cp_async16(smem_address(mine + (size_t)(stage * Form::CHUNKS + c) * FEW_CHUNK + (lane & 3) * 16),
                        in ? W + (size_t)n * ldw + k : W, in ? 16 : 0);
         }
     };
 #pragma unroll
-    for (int s = 0; s < FEW_STAGES - 1; ++s) {
+    for (int s = 0; s < Form::STAGES - 1; ++s) {
         if (s < steps) fetch(s, s);
         cp_async_commit();
     }
@@ -173,9 +181,11 @@ gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
     const float* x[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) x[m] = A + (size_t)min(m0 + m, M - 1) * lda;
-    float acc[MT];
+    float acc[Form::PER][MT];
 #pragma unroll
-    for (int m = 0; m < MT; ++m) acc[m] = 0.f;
+    for (int f = 0; f < Form::PER; ++f)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) acc[f][m] = 0.f;
     // (the tokens' next four values are asked for while the present ones are multiplied; left to itself the compiler
     // held back the loads of four tokens to save registers: 39 us against 34 for 3 tokens of 12,288 x 2,048)
     constexpr bool AHEAD = MT <= 8;
@@ -188,14 +198,16 @@ gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
     };
     load_next(r * run);
     for (int step = 0; step < steps; ++step) {
-        cp_async_wait<FEW_STAGES - 2>();
+        cp_async_wait<Form::STAGES - 2>();
         __syncwarp();
         const int k0 = r * run + step * BK;
-        const uint8_t* chunk = mine + (size_t)((step % FEW_STAGES) * 32 + lane) * FEW_CHUNK;
+        const uint8_t* chunk = mine + (size_t)((step % Form::STAGES) * Form::CHUNKS + lane) * FEW_CHUNK;
 #pragma unroll
         for (int q = 0; q < BK / 4; ++q) {
             if (k0 + 4 * q >= K) break;                   // whole quarters: K is a multiple of 4
-            const float4 w = *reinterpret_cast<const float4*>(chunk + 16 * q);
+            float4 w[Form::PER];
+#pragma unroll
+            for (int f = 0; f < Form::PER; ++f) w[f] = *reinterpret_cast<const float4*>(chunk + 32 * f * FEW_CHUNK + 16 * q);
             float4 now[AHEAD ? MT : 1];
             if constexpr (AHEAD) {
 #pragma unroll
@@ -205,23 +217,24 @@ gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const float4 v = AHEAD ? now[AHEAD ? m : 0] : *reinterpret_cast<const float4*>(x[m] + k0 + 4 * q);
-                acc[m] = fmaf(v.x, w.x, acc[m]);
-                acc[m] = fmaf(v.y, w.y, acc[m]);
-                acc[m] = fmaf(v.z, w.z, acc[m]);
-                acc[m] = fmaf(v.w, w.w, acc[m]);
+#pragma unroll
+                for (int f = 0; f < Form::PER; ++f)
+                    acc[f][m] = fmaf(v.w, w[f].w, fmaf(v.z, w[f].z, fmaf(v.y, w[f].y, fmaf(v.x, w[f].x, acc[f][m]))));
             }
         }
         __syncwarp();                                     // the stage before this one is read: fill it again
-        if (step + FEW_STAGES - 1 < steps) fetch(step + FEW_STAGES - 1, (step + FEW_STAGES - 1) % FEW_STAGES);
+        if (step + Form::STAGES - 1 < steps) fetch(step + Form::STAGES - 1, (step + Form::STAGES - 1) % Form::STAGES);
         cp_async_commit();
     }
     cp_async_wait<0>();
 #pragma unroll
-    for (int m = 0; m < MT; ++m) parts[r][m][lane & 15] = acc[m];
+    for (int f = 0; f < Form::PER; ++f)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) parts[r][m][(lane & 15) + FEW_F * f] = acc[f][m];
     __syncthreads();
     const int runs = (K + run - 1) / run;
-    for (int i = threadIdx.x; i < MT * FEW_F; i += FEW_THREADS) {
-        const int f = i % FEW_F, m = i / FEW_F, n = n0 + f;
+    for (int i = threadIdx.x; i < MT * Form::F; i += FEW_THREADS) {
+        const int f = i % Form::F, m = i / Form::F, n = n0 + f;
         if (m0 + m >= M) break;
         auto total = [&](int at) {
             float v = 0.f;
@@ -392,22 +405,31 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
-template <int MT, int EPI>
-int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+template <int MT, int EPI, bool PAIR>
+int launch_few_form(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+    using F = Few<PAIR>;
     static bool configured = false;
     if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM);
+        const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MT, EPI, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    return kipp_launch(gemm_few_kernel<MT, EPI>, dim3((N + FEW_F - 1) / FEW_F, (M + MT - 1) / MT), dim3(FEW_THREADS),
-                       FEW_SMEM, s, 1, C, A, W, M, N, K, lda, ldw, ldc);
+    return kipp_launch(gemm_few_kernel<MT, EPI, PAIR>, dim3((N + F::F - 1) / F::F, (M + MT - 1) / MT), dim3(FEW_THREADS),
+                       F::SMEM, s, 1, C, A, W, M, N, K, lda, ldw, ldc);
+}
+template <int MT, int EPI>
+int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
+    // pairs of features where they still make two blocks for each SM (12,288 x 2,048 with 3 and 8 tokens: 28.3 and 37.9 us,
+    // one feature per thread 32.9 and 47.2; 32,000: 59 and 88 against 78 and 106)
+    constexpr bool MAY_PAIR = MT >= 2 && MT <= 8;
+    if (MAY_PAIR && N >= MANY_F) return launch_few_form<MT, EPI, MAY_PAIR>(C, A, W, M, N, K, lda, ldw, ldc, s);
+    return launch_few_form<MT, EPI, false>(C, A, W, M, N, K, lda, ldw, ldc, s);
 }
 
 // float32 rows that start on 16 bytes and hold whole groups of four: the kernels that copy 16 bytes at a time.
 template <int EPI>
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
-    if (M <= FEW_MAX) {
+    if (M <= (N >= MANY_F ? FEW_MAX / 2 : FEW_MAX)) {
         // tokens of a block: as many as there are, up to 16 (the accumulators of a thread)
         if (M == 1) return launch_few<1, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
         if (M == 2) return launch_few<2, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);

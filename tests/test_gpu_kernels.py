@@ -105,11 +105,12 @@ def test_gemm_simt(dtype, shape, epilogue):
 
 
 @pytest.mark.parametrize("epilogue", ["store", "add", "swiglu"])
-@pytest.mark.parametrize("shape", [(130, 20), (18, 136), (66, 260), (2, 1028), (34, 2064)])
+@pytest.mark.parametrize("shape", [(130, 20), (18, 136), (66, 260), (2, 1028), (34, 2064), (9470, 36), (9474, 260)])
 def test_gemm_32_bit_kernels_agree(shape, epilogue):
     """The 32-bit product's three kernels add in one order: the rows of a batch have the same bits whether 1, 3,
     16, 17, 32 (the kernel for few tokens, at its block sizes and the last count it takes), 33 or 70 of them (tiles)
-    are multiplied at once, and where rows do not start on 16 bytes.  The K reach from one run of 16 to runs that
+    are multiplied at once, and where rows do not start on 16 bytes; from 9,472 features on a thread of the kernel for
+    few tokens has two of them, and tiles take over at 17 tokens.  The K reach from one run of 16 to runs that
     end inside a tile; the error against float64 stays under that of one chain of K roundings, K eps |a| |w|."""
     N, K = shape
     M = 70
