@@ -974,3 +974,54 @@ def test_a_bounded_wait_runs_out_and_reports():
     assert rc == 0
     assert st.tolist() == [0, 1, 0, 0]
     assert limit <= int(waited) < 200 * limit
+
+
+@pytest.mark.parametrize("interleaved", [0, 1])
+@pytest.mark.parametrize("D,rot_off,rot", [(64, 0, 64), (192, 128, 64), (192, 0, 16), (40, 8, 32), (72, 8, 24), (192, 128, 6), (48, 4, 40),
+                                           (320, 24, 256)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_head_segments_rotated(dtype, D, rot_off, rot, interleaved):
+    """A rotated segment with a norm, in whole vectors where its rotated dims are that and an element at a time
+    elsewhere (rotated parts that start or end inside a vector, rows or a rotation table off a 16-byte boundary), against
+    float64: the value is rounded once to the result's type, and float32 on its way (a sum of D squares, three
+    products and a sum)."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+
+    class Segment(ctypes.Structure):
+        _fields_ = ([(n, ctypes.c_int) for n in ("src_off", "heads", "dim", "src_stride", "rot_off", "rot", "target", "dst_off", "dst_stride",
+                                                 "heads_per_row", "norm_all", "interleaved", "unit_norm")]
+                    + [(n, ctypes.c_void_p) for n in ("bias", "norm_w", "cos_sin", "dst")] + [("ld_dst", ctypes.c_longlong)])
+
+    fn = load_library("head_ops").kipp_head_segments
+    p, i, ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
+    fn.argtypes = [p, ll, i, p, i, p, p, i, i, i, p, p, p, i, i, i, i, ctypes.c_float, p, p]
+    T, H, eps = 5, 3, 1e-6
+    g = torch.Generator().manual_seed(D + rot)
+    x = torch.randn(T, H, D, generator=g).to(dtype)
+    w = torch.randn(D, generator=g)
+    angle = torch.rand(T, rot // 2, generator=g) * 6
+    cs = torch.stack([angle.cos(), angle.sin()], -1).contiguous()
+    v = x.double()
+    v = v / (v.square().mean(-1, keepdim=True) + eps).sqrt() * w.double()
+    c, s = cs.double()[:, None, :, 0], cs.double()[:, None, :, 1]
+    r = v[..., rot_off:rot_off + rot].clone()
+    lo, hi = (r[..., 0::2], r[..., 1::2]) if interleaved else (r[..., :rot // 2], r[..., rot // 2:])
+    turned = (lo * c - hi * s, hi * c + lo * s)
+    v[..., rot_off:rot_off + rot] = torch.stack(turned, -1).flatten(-2) if interleaved else torch.cat(turned, -1)
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
+    bound = ulp * v.abs() + (D + 8) * 2.0 ** -24 * v.abs().amax()
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    for src_shift, w_shift, cs_shift in ((0, 0, 0), (0, 1, 0), (0, 0, 2), (1, 0, 0)):
+        held = torch.zeros(src_shift + x.numel(), dtype=dtype, device=DEV)
+        held[src_shift:] = x.flatten()
+        norm, table = torch.zeros(w_shift + D, device=DEV), torch.zeros(cs_shift + cs.numel(), device=DEV)
+        norm[w_shift:], table[cs_shift:] = w, cs.flatten()
+        out = torch.zeros(T, H, D, dtype=dtype, device=DEV)
+        seg = Segment(src_off=0, heads=H, dim=D, src_stride=D, rot_off=rot_off, rot=rot, target=0, dst_stride=D, interleaved=interleaved,
+                      norm_w=norm[w_shift:].data_ptr(), cos_sin=table[cs_shift:].data_ptr(), dst=out.data_ptr(), ld_dst=H * D)
+        rc = fn(held[src_shift:].data_ptr(), H * D, 0 if dtype == torch.float32 else 1, ctypes.byref(seg), 1, None, None, 0, 0, 0, None, None,
+                None, 0, 1, T, 0, eps, status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0 and status.item() == 0
+        assert ((out.double().cpu() - v).abs() <= bound).all(), (src_shift, w_shift, cs_shift)
