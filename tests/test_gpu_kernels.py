@@ -81,6 +81,25 @@ def test_rmsnorm_deferred(size):
     assert torch.equal(out.cpu(), (x.cpu()[[6, 0, 3]] * w.float().cpu()).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("rows", [591, 592, 593, 1300])
+@pytest.mark.parametrize("size", [256, 2052, 4096])
+def test_rmsnorm_of_many_rows(size, rows):
+    """From 593 rows on a block has several: each row's result has the bits it has alone."""
+    g = torch.Generator().manual_seed(size + rows)
+    x, w = torch.randn(rows, size, generator=g).to(DEV), torch.randn(size, generator=g).to(DEV)
+    out, ssq, normed = torch.empty(rows, size, dtype=torch.bfloat16, device=DEV), torch.empty(rows, device=DEV), torch.empty(rows, size, device=DEV)
+    ops().rmsnorm_deferred(out, ssq, x, w)
+    ops().rmsnorm(normed, x, w, 1e-5)
+    assert torch.equal(out, (x * w).bfloat16())
+    for r in (0, 1, rows // 2, rows - 2, rows - 1):
+        one, s, n = torch.empty(1, size, dtype=torch.bfloat16, device=DEV), torch.empty(1, device=DEV), torch.empty(1, size, device=DEV)
+        ops().rmsnorm_deferred(one, s, x[r:r + 1], w)
+        ops().rmsnorm(n, x[r:r + 1], w, 1e-5)
+        assert torch.equal(s, ssq[r:r + 1]) and torch.equal(n, normed[r:r + 1])
+    assert torch.allclose(ssq.double(), (x.double() ** 2).sum(-1), rtol=size * 2.0 ** -24)
+    assert torch.allclose(normed.double().cpu(), P.plain_rmsnorm(x.cpu(), w.cpu(), 1e-5), **tol(torch.float32))
+
+
 # ------------------------------------------------------------------ matrix products
 def gemm_ref(a, w, epilogue, base):
     p = a.double().cpu() @ w.double().cpu().t()
