@@ -717,6 +717,179 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     if (warp == 9) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
+// ------------------------------------------------------------------------ keys and values out of cached latents
+// The keys and values of every head from the latents a step's entries have cached (what this file's kernels read as pages
+// of keys and values of heads of their own; head_ops.cu has the form for other page sizes, and the layout's words).
+// A contraction of 128 tokens x 256 features per CTA on tcgen05.mma, K in steps of 64 through two stages of 48 KB: a box
+// per page of latents and one of weights; two CTAs an SM, so that one's products run beside the other's way out.
+// The result leaves through shared memory a token's row at a time, 512 neighbouring bytes per warp.  Latents past the
+// columns a row has are multiplied by weights the unit fills with zeros, tokens past the entry's last become zeros at
+// the end.  (2,730 tokens, 8,192 features of 512: 97 us on mma.sync, 45 so.)
+constexpr int X_TOK = 128, X_FEAT = 256, X_STAGES = 2, X_THREADS = 128, X_PAGE = 64;
+constexpr int X_A_BYTES = X_TOK * 128, X_W_BYTES = X_FEAT * 128, X_STAGE_BYTES = X_A_BYTES + X_W_BYTES;
+constexpr int X_ROW = X_FEAT * 2 + 16;                       // bytes of a result row in shared memory: 4 banks on per row
+constexpr size_t X_SMEM = (size_t)X_STAGES * X_STAGE_BYTES + 64;
+static_assert((size_t)X_TOK * X_ROW <= (size_t)X_STAGES * X_STAGE_BYTES, "the result fits where the stages were");
+struct ExpandArgs {
+    const bf16* pages;                       // [page][page_size][row] latents
+    const int* block_table; int table_width, page_size, row;
+    const int* q_start; const int* context_len;
+    int rank, dim, rot, v_dim, heads;
+    bf16* k_out; bf16* v_out; int* table_out;
+    int pages_per_entry, k_tiles, v_tiles;
+    int box_rows, rows_total;                // rows of a box of latents; a row coordinate from rows_total on reads zeros
+    int* status;
+};
+__global__ void __launch_bounds__(X_THREADS)
+latent_expand_tc_kernel(const __grid_constant__ CUtensorMap map_pages, const __grid_constant__ CUtensorMap map_wk,
+                        const __grid_constant__ CUtensorMap map_wv, const ExpandArgs a) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (lists first: a burst's steps move them on.  The tensor memory is asked for after the wait too, when no earlier
+    // kernel holds any, and the next kernel is let in once this CTA has it: nobody waits for one who waits.)
+    pdl_wait();
+    const int e = blockIdx.z, t0 = blockIdx.y * X_TOK;
+    const int ft = (int)blockIdx.x - 1;                                // (the copy first: it is one block's work)
+    const int len = a.context_len[e] + a.q_start[e + 1] - a.q_start[e];
+    const int rows_end = (len + X_PAGE - 1) / X_PAGE * X_PAGE;          // rows to write: whole pages
+    const bool shared_part = ft < 0;
+    if (shared_part && blockIdx.y == 0)
+        for (int j = tid; j < a.pages_per_entry; j += X_THREADS) a.table_out[(size_t)e * a.pages_per_entry + j] = e * a.pages_per_entry + j;
+    if (t0 >= rows_end) { pdl_launch_dependents(); return; }
+    const int* table = a.block_table + (size_t)e * a.table_width;
+    const int k_row = a.dim + a.rot;
+    // the pool's row of token t, or -1 where the entry has no such token
+    auto cached = [&](int t) -> int {
+        if (t >= len) return -1;
+        const int slot = t / a.page_size, page = slot < a.table_width ? table[slot] : -1;
+        if (page < 0) {
+            atomicExch(a.status, 3);                                    // a needed key is not mapped
+            return -1;
+        }
+        return page * a.page_size + t % a.page_size;
+    };
+    auto out_row = [&](bf16* base, int t, int h, int width) {
+        return base + ((((size_t)e * a.pages_per_entry + t / X_PAGE) * a.heads + h) * X_PAGE + t % X_PAGE) * width;
+    };
+    if (shared_part) {
+        pdl_launch_dependents();
+        const int chunks = a.rot / 8;
+        for (int i = tid; i < X_TOK * chunks; i += X_THREADS) {
+            const int t = t0 + i / chunks, c = i % chunks;
+            if (t >= rows_end) break;
+            const int src = cached(t);
+            const uint4 v = src >= 0 ? *reinterpret_cast<const uint4*>(a.pages + (size_t)src * a.row + a.rank + c * 8)
+                                     : make_uint4(0u, 0u, 0u, 0u);
+            for (int h = 0; h < a.heads; ++h) *reinterpret_cast<uint4*>(out_row(a.k_out, t, h, k_row) + a.dim + c * 8) = v;
+        }
+        return;
+    }
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + X_STAGES * X_STAGE_BYTES);
+    uint64_t *full = bars, *empty = bars + X_STAGES, *done = bars + 2 * X_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * X_STAGES + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const uint32_t stages = smem_u32(smem);
+    if (tid == 0) {
+        for (int s = 0; s < X_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(done, 1);
+        *abort_flag = (stages & 1023u) ? 1 : 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, X_FEAT);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_launch_dependents();
+    const uint32_t tmem = *tmem_slot;
+    const bool keys = ft < a.k_tiles;
+    const int per_head = keys ? a.dim : a.v_dim, features = a.heads * per_head, n0 = (keys ? ft : ft - a.k_tiles) * X_FEAT;
+    const int steps = (a.rank + 63) / 64;
+    bool ok = *abort_flag == 0;
+    if (warp == 0) {
+        // lane l brings the rows [l * box_rows, + box_rows) of the tile: they lie in one page
+        const int boxes = X_TOK / a.box_rows;
+        int coord = a.rows_total;
+        if (lane < boxes) {
+            const int at = cached(t0 + lane * a.box_rows);
+            if (at >= 0) coord = at;
+        }
+        const CUtensorMap* map_w = keys ? &map_wk : &map_wv;
+        for (int s = 0; s < steps; ++s) {
+            const int b = s % X_STAGES;
+            if (s >= X_STAGES && ok && !mbar_wait(&empty[b], (s / X_STAGES - 1) & 1, abort_flag)) ok = false;
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            if (lane == 0) mbar_expect_tx(&full[b], X_STAGE_BYTES);
+            __syncwarp();
+            const uint32_t at = stages + b * X_STAGE_BYTES;
+            if (lane < boxes) tma_load_2d(at + lane * a.box_rows * 128, &map_pages, &full[b], s * 64, coord);
+            if (lane == 31) tma_load_2d(at + X_A_BYTES, map_w, &full[b], s * 64, n0);
+            __syncwarp();
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t IDESC = idesc(X_TOK, X_FEAT, 0);
+        for (int s = 0; s < steps; ++s) {
+            const int b = s % X_STAGES;
+            if (ok && !mbar_wait(&full[b], (s / X_STAGES) & 1, abort_flag)) ok = false;
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+                const uint64_t ad = smem_desc(stages + b * X_STAGE_BYTES, 0, 1024);
+                const uint64_t wd = smem_desc(stages + b * X_STAGE_BYTES + X_A_BYTES, 0, 1024);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) umma_bf16(tmem, ad + 2 * k, wd + 2 * k, IDESC, (s | k) ? 1u : 0u);
+                umma_commit(&empty[b]);
+                if (s == steps - 1) umma_commit(done);
+            }
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+    if (ok && !mbar_wait(done, 0, abort_flag)) ok = false;
+    ok = __all_sync(0xffffffffu, ok);
+    tc_fence_after();
+    // a warp has the 32 tokens of its quarter of the tensor memory's lanes
+    uint8_t* rows = smem + warp * 32 * X_ROW;
+#pragma unroll 1
+    for (int c = 0; c < X_FEAT; c += 32) {
+        float v[32];
+        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + c, v);
+        if (t0 + warp * 32 + lane >= len) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) v[k] = 0.f;
+        }
+        if (ok) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                uint4 q;
+                uint32_t* w = reinterpret_cast<uint32_t*>(&q);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[8 * k + 2 * j], v[8 * k + 2 * j + 1]);
+                    w[j] = *reinterpret_cast<const uint32_t*>(&h2);
+                }
+                *reinterpret_cast<uint4*>(rows + lane * X_ROW + (c + 8 * k) * 2) = q;
+            }
+        }
+    }
+    __syncwarp();
+    const int n = n0 + lane * 8;                              // (heads are multiples of 8: a piece lies in one head)
+    if (ok && n < features) {
+        const int h = n / per_head;
+        for (int r = 0; r < 32; ++r) {
+            const int t = t0 + warp * 32 + r;
+            if (t >= rows_end) break;
+            bf16* dst = keys ? out_row(a.k_out, t, h, k_row) : out_row(a.v_out, t, h, a.v_dim);
+            *reinterpret_cast<uint4*>(dst + n % per_head) = *reinterpret_cast<const uint4*>(rows + r * X_ROW + lane * 16);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0 && *abort_flag) atomicExch(&a.status[1], 1);
+    if (warp == 1) tmem_dealloc(tmem, X_FEAT);
+}
+
 // ------------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -946,4 +1119,43 @@ extern "C" int kipp_attn_prefill_tc_ex(void* out, const void* q, int tokens, con
     if (ex->gate != nullptr && ex->gate_dims && ((((uintptr_t)ex->gate + 2 * (size_t)ex->gate_off) & 15) || (ex->ld_gate & 7))) return -3;
     return prefill_tc(out, q, tokens, k_pages, v_pages, n_pages, q_start, context_len, block_table, table_width, page_size, work,
                       items, n_q, n_kv, head_dim, v_dim, scale, window, out_scale, ex, status, stream);
+}
+
+// kipp_latent_expand (head_ops.cu) for page sizes whose boxes fill whole swizzle groups (kipp_attn_prefill_tc_page_ok):
+// the same arguments and results, and the number of the pool's pages.
+extern "C" int kipp_latent_expand_tc(const void* pages, int n_pages, const int* block_table, int table_width, int page_size, int row,
+                                     const int* q_start, const int* context_len, int entries, const void* w_k, const void* w_v,
+                                     int rank, int dim, int rot, int v_dim, int heads, void* k_out, void* v_out, int* table_out,
+                                     int pages_per_entry, int* status, void* stream) {
+    if (entries <= 0) return 0;
+    if (rank <= 0 || dim <= 0 || rot < 0 || v_dim <= 0 || heads <= 0 || ((rank | dim | rot | v_dim) & 7) || row != rank + rot ||
+        !kipp_attn_prefill_tc_page_ok(page_size) || n_pages <= 0 || table_width <= 0 ||
+        (long long)pages_per_entry * X_PAGE < (long long)table_width * page_size || entries > 65535 || status == nullptr ||
+        (long long)n_pages * page_size + X_TOK > 0x7fffffffLL)
+        return KIPP_ERR_ARG;
+    if ((((uintptr_t)pages | (uintptr_t)w_k | (uintptr_t)w_v | (uintptr_t)k_out | (uintptr_t)v_out) & 15) != 0) return -3;
+    ExpandArgs a = {};
+    a.pages = (const bf16*)pages; a.block_table = block_table; a.table_width = table_width; a.page_size = page_size; a.row = row;
+    a.q_start = q_start; a.context_len = context_len;
+    a.rank = rank; a.dim = dim; a.rot = rot; a.v_dim = v_dim; a.heads = heads;
+    a.k_out = (bf16*)k_out; a.v_out = (bf16*)v_out; a.table_out = table_out; a.pages_per_entry = pages_per_entry; a.status = status;
+    a.k_tiles = (heads * dim + X_FEAT - 1) / X_FEAT;
+    a.v_tiles = (heads * v_dim + X_FEAT - 1) / X_FEAT;
+    a.box_rows = page_size < 64 ? page_size : 64;
+    a.rows_total = n_pages * page_size;
+    CUtensorMap mp, mk, mv;
+    int rc = pool_map(&mp, pages, a.rows_total, row, a.box_rows);
+    if (rc == 0) rc = pool_map(&mk, w_k, (long long)heads * dim, rank, X_FEAT);
+    if (rc == 0) rc = pool_map(&mv, w_v, (long long)heads * v_dim, rank, X_FEAT);
+    if (rc) return rc;
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t err = cudaFuncSetAttribute(latent_expand_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)X_SMEM);
+        if (err != cudaSuccess) { cudaGetLastError(); return (int)err; }
+        configured = true;
+    }
+    const int tiles = (pages_per_entry * X_PAGE + X_TOK - 1) / X_TOK;
+    if (tiles > 65535) return KIPP_ERR_ARG;
+    return kipp_launch(latent_expand_tc_kernel, dim3((unsigned)(a.k_tiles + a.v_tiles + 1), (unsigned)tiles, (unsigned)entries),
+                       dim3(X_THREADS), X_SMEM, (cudaStream_t)stream, 1, mp, mk, mv, a);
 }

@@ -437,9 +437,21 @@ public:
         v.v_pages = workspace->buffer("latent_values", rows * v_dim * 2);
         int* table = workspace->get<int>("latent_table", (size_t)v.n_pages);
         v.block_table = table;
-        run(f(cache.k_pages, cache.block_table, cache.table_width, cache.page_size, rank + rot, q_start, context_len, entries, w_k, w_v,
-              rank, dim, rot, v_dim, heads, v.k_pages, v.v_pages, table, v.table_width, status, stream),
-            "latent_expand");
+        // on tcgen05 where a box of the pool's rows lies in one page, as the attention kernel itself needs it (attention_tc.cu)
+        using Pages = int (*)(int);
+        static Pages page_ok = kernel_symbol<Pages>("attention_tc", "kipp_attn_prefill_tc_page_ok");
+        if (page_ok(cache.page_size)) {
+            using Ft = int (*)(const void*, int, const int*, int, int, int, const int*, const int*, int, const void*, const void*, int, int,
+                               int, int, int, void*, void*, int*, int, int*, void*);
+            static Ft ft = kernel_symbol<Ft>("attention_tc", "kipp_latent_expand_tc");
+            run(ft(cache.k_pages, cache.n_pages, cache.block_table, cache.table_width, cache.page_size, rank + rot, q_start, context_len,
+                   entries, w_k, w_v, rank, dim, rot, v_dim, heads, v.k_pages, v.v_pages, table, v.table_width, status, stream),
+                "latent_expand");
+        } else {
+            run(f(cache.k_pages, cache.block_table, cache.table_width, cache.page_size, rank + rot, q_start, context_len, entries, w_k,
+                  w_v, rank, dim, rot, v_dim, heads, v.k_pages, v.v_pages, table, v.table_width, status, stream),
+                "latent_expand");
+        }
         ++latent_expansions;
         return v;
     }

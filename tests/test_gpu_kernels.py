@@ -1044,3 +1044,64 @@ def test_head_segments_rotated(dtype, D, rot_off, rot, interleaved):
         torch.cuda.synchronize()
         assert rc == 0 and status.item() == 0
         assert ((out.double().cpu() - v).abs() <= bound).all(), (src_shift, w_shift, cs_shift)
+
+
+@pytest.mark.parametrize("page", [8, 16, 64, 192, 24])
+@pytest.mark.parametrize("sizes", [(72, 40, 8, 24, 3), (512, 128, 64, 128, 5), (40, 16, 0, 16, 2), (200, 64, 16, 256, 2)])
+def test_latent_expand(sizes, page):
+    """The heads' keys and values out of cached latents, on tcgen05 where the page sizes allow it and on mma.sync at any:
+    entries of 1 token, of a page of the result less, exactly and plus one, and of several tiles, in pages of the pool that follow no
+    order; ranks and features that end inside a step or tile.  Every value is a sum of `rank` products, in float32 (error
+    under rank 2^-23 sum |c||w|), rounded once; the shared part is copied, rows past an entry's last token are zeros, and the
+    rest of the result's pages stays untouched."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    rank, dim, rot, v_dim, heads = sizes
+    lens = [1, 63, 64, 65, 300]
+    g = torch.Generator().manual_seed(rank + page)
+    per = -(-max(lens) // page)
+    n_pages = per * len(lens) + 3
+    pool = torch.randn(n_pages, page, rank + rot, generator=g).bfloat16()
+    order = torch.randperm(n_pages, generator=g)
+    table = torch.full((len(lens), per), -1, dtype=torch.int32)
+    at = 0
+    for e, n in enumerate(lens):
+        need = -(-n // page)
+        table[e, :need] = order[at:at + need].int()
+        at += need
+    wk = (torch.randn(heads * dim, rank, generator=g) * 0.1).bfloat16()
+    wv = (torch.randn(heads * v_dim, rank, generator=g) * 0.1).bfloat16()
+    new = torch.tensor([1, 10, 64, 1, 299])                                   # tokens of the step, the others are cached before
+    q_start = torch.cat([torch.zeros(1, dtype=torch.int64), new.cumsum(0)]).int().to(DEV)
+    context = (torch.tensor(lens) - new).int().to(DEV)
+    width = -(-per * page // 64)
+    p, i = ctypes.c_void_p, ctypes.c_int
+    rest = [p, i, i, i, p, p, i, p, p, i, i, i, i, i, p, p, p, i, p, p]
+    dev = [x.to(DEV).contiguous() for x in (pool, table, wk, wv)]
+    on_tc = load_library("attention_tc").kipp_attn_prefill_tc_page_ok(page)
+    assert bool(on_tc) == (page != 24)
+    for tc in ([True, False] if on_tc else [False]):
+        fn = load_library("attention_tc").kipp_latent_expand_tc if tc else load_library("head_ops").kipp_latent_expand
+        fn.argtypes = [p] + ([i] if tc else []) + rest
+        ko = torch.full((len(lens), width, heads, 64, dim + rot), 7.0, dtype=torch.bfloat16, device=DEV)
+        vo = torch.full((len(lens), width, heads, 64, v_dim), 7.0, dtype=torch.bfloat16, device=DEV)
+        to = torch.zeros(len(lens), width, dtype=torch.int32, device=DEV)
+        status = torch.zeros(8, dtype=torch.int32, device=DEV)
+        rc = fn(dev[0].data_ptr(), *([n_pages] if tc else []), dev[1].data_ptr(), per, page, rank + rot, q_start.data_ptr(),
+                context.data_ptr(), len(lens), dev[2].data_ptr(), dev[3].data_ptr(), rank, dim, rot, v_dim, heads, ko.data_ptr(),
+                vo.data_ptr(), to.data_ptr(), width, status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0 and status.abs().sum().item() == 0
+        assert torch.equal(to.cpu().flatten(), torch.arange(len(lens) * width, dtype=torch.int32))
+        for e, n in enumerate(lens):
+            rows = torch.cat([pool[table[e, j]] for j in range(-(-n // page))])[:n]
+            c = rows[:, :rank].double()
+            end = -(-n // 64) * 64
+            for out, w, size in ((ko, wk, dim), (vo, wv, v_dim)):
+                got = out[e].cpu().double().transpose(1, 2).reshape(width * 64, heads, -1)
+                ref = (c @ w.double().t()).reshape(n, heads, size)
+                slack = (rank * 2.0 ** -23 * (c.abs() @ w.double().abs().t())).reshape(n, heads, size)
+                assert ((got[:n, :, :size] - ref).abs() <= 2.0 ** -8 * ref.abs() + slack).all(), (tc, e)
+                if out is ko:
+                    assert (got[:n, :, size:] == rows[:, None, rank:].double()).all(), (tc, e)
+                assert (got[n:end] == 0).all() and (got[end:] == 7).all(), (tc, e)
