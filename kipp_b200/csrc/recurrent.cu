@@ -56,8 +56,10 @@
 // on the sizes only.
 //
 // Two kinds have scans of their own for the sizes that divide by four: ssd_scan_kernel (straight from the
-// convolved rows, no records) and gated_delta_scan_kernel.  There a thread works on pairs of float32 and the
-// shuffles of one token's sums travel while the next token is worked on.  For steps of one token per request
+// convolved rows, no records), and for the gated delta rule gated_delta_scan_kernel (four columns a thread) and
+// gated_delta_column_kernel (one, where few blocks make the chain of a token what counts).  There a thread works on pairs of
+// float32 and the shuffles of one token's sums travel while the next token is worked on.  State space prompts go by
+// chunks of tokens instead where that pays (by_chunks): products within a chunk, the state from chunk to chunk.  For steps of one token per request
 // ssd_token_kernel and gated_delta_token_kernel do the convolution, the state and the output in one launch.
 // A scan of many tokens starts when the kernel before it has left the GPU (kipp_launch_spread): blocks that
 // were placed early share few multiprocessors, and a scan lasts as long as its most crowded one.
@@ -1141,17 +1143,19 @@ gated_delta_column_kernel(const ScanArgs a, const float* __restrict__ vec, float
 // The convolution for channels that go by eights (four in 32-bit) and up to 4 taps: a thread takes 16 bytes of
 // channels over a run of CONV_RUN tokens and reads every input once (the last taps - 1 stay in registers; they come
 // anew where a run or an entry starts).  The order of a channel's sum is ssd_conv_kernel's.  The last row of
-// blocks forms the state space layer's decays and step sizes, dts [tokens][heads] (null: none).
+// blocks forms the state space layer's decays and step sizes, dts [tokens][heads] (null: none).  Bound by the trips of a
+// run's tokens, one after the other: the next token's input is on its way, the weights come 16 bytes at a time before
+// the wait (2,048 tokens of 6,144 channels: 35 us a launch, 27 so).
 constexpr int CONV_RUN = 8, CONV_THREADS = 128;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(CONV_THREADS)
 conv_run_kernel(const ScanArgs a, float* __restrict__ conv_out, float2* __restrict__ dts, int tokens) {
     constexpr int VEC = 16 / (int)sizeof(T);
     pdl_launch_dependents();
-    pdl_wait();
     const int r0 = blockIdx.x * CONV_RUN, r1 = min(tokens, r0 + CONV_RUN);
     const T* proj = static_cast<const T*>(a.proj);
     if (dts != nullptr && blockIdx.y == gridDim.y - 1) {
+        pdl_wait();
         for (int i = threadIdx.x; i < (r1 - r0) * a.heads; i += CONV_THREADS) {
             const int row = r0 + i / a.heads, h = i % a.heads;
             const float raw = to_f32(proj[(size_t)row * a.ld_proj + a.dt_off + h]) + a.dt_bias[h];
@@ -1163,18 +1167,34 @@ conv_run_kernel(const ScanArgs a, float* __restrict__ conv_out, float2* __restri
     const int c = (blockIdx.y * CONV_THREADS + threadIdx.x) * VEC;
     if (c >= a.channels) return;
     float w[VEC][TAPS], bias[VEC], in[TAPS][VEC];              // in[TAPS - 1]: the current token's
+    // (weights before the wait)
+    if (((uintptr_t)a.conv_w & 15) == 0 && ((uintptr_t)a.conv_b & 15) == 0) {
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-        bias[i] = a.conv_b != nullptr ? a.conv_b[c + i] : 0.f;
+        for (int i = 0; i < VEC; i += 4) {
+            const float4 b = a.conv_b != nullptr ? *reinterpret_cast<const float4*>(a.conv_b + c + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            bias[i] = b.x; bias[i + 1] = b.y; bias[i + 2] = b.z; bias[i + 3] = b.w;
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) w[i][j] = a.conv_w[(size_t)j * a.channels + c + i];
+            for (int j = 0; j < TAPS; ++j) {
+                const float4 q = *reinterpret_cast<const float4*>(a.conv_w + (size_t)j * a.channels + c + i);
+                w[i][j] = q.x; w[i + 1][j] = q.y; w[i + 2][j] = q.z; w[i + 3][j] = q.w;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+            bias[i] = a.conv_b != nullptr ? a.conv_b[c + i] : 0.f;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) w[i][j] = a.conv_w[(size_t)j * a.channels + c + i];
+        }
     }
-    auto load = [&](int row, float* to) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(proj + (size_t)row * a.ld_proj + a.xbc_off + c);
+    pdl_wait();
+    auto at = [&](int row) { return *reinterpret_cast<const uint4*>(proj + (size_t)row * a.ld_proj + a.xbc_off + c); };
+    auto values = [&](const uint4& raw, float* to) {
         const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
         for (int i = 0; i < VEC; ++i) to[i] = to_f32(e[i]);
     };
+    uint4 now = at(r0), next = now;                            // the next token's input is on its way
     int end = r0;                                              // where the entry of the run's next token ends
     for (int row = r0; row < r1; ++row) {
         if (row == end || row == r0) {
@@ -1185,14 +1205,16 @@ conv_run_kernel(const ScanArgs a, float* __restrict__ conv_out, float2* __restri
             for (int j = 0; j < TAPS - 1; ++j) {
                 const int r = row - (TAPS - 1 - j);
                 if (r >= first) {
-                    load(r, in[j]);
+                    values(at(r), in[j]);
                 } else {
 #pragma unroll
                     for (int i = 0; i < VEC; ++i) in[j][i] = kept[(size_t)(TAPS - 1 + r - first) * a.channels + c + i];
                 }
             }
         }
-        load(row, in[TAPS - 1]);
+        if (row + 1 < r1) next = at(row + 1);
+        values(now, in[TAPS - 1]);
+        now = next;
         float y[VEC];
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
