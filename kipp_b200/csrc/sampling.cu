@@ -18,7 +18,7 @@
 // that order is found by radix selection over the (value, token) keys, with
 // per-bucket counts and weight sums, four 8-bit passes over the value and,
 // only among equal values, four over the token id.  Bucket sums add the same
-// float32 weights as integers in units of 2^-40 (see weight_units) where the
+// float32 weights as integers in units of 2^-40 (see peers_units) where the
 // reference keeps a running double sum, so a draw that lies within 2^-23 of a
 // boundary may pick the neighbour.
 //
@@ -26,9 +26,10 @@
 // forty instructions in a pass that adds weights), so there are few: the first pass of a selection also
 // gives the total that its target is a share of; its second pass, which looks at one bucket of the
 // first, puts that bucket's elements into a list in shared memory, and the passes after it walk the
-// list; and what top-k leaves is listed once for everything that follows.  64 rows of 151,936, half of
-// them with top-k 50, top-p 0.95: 588 us (934 with all passes over the rows
-// and the loads one at a time); a single such row by eight blocks: 170 us (221).  What is left is the aggregation
+// list; what top-k leaves is listed once for everything that follows; a rank is looked for without weights; and the
+// draw within a nucleus takes its first pass from the selection that found the nucleus.  64 rows of 151,936, half of
+// them with top-k 50, top-p 0.95: 488 us (588 without the last two; 934 with all passes over the rows
+// and the loads one at a time); a single such row by eight blocks: 143 us (170; 221).  What is left is the aggregation
 // of equal buckets within a warp.
 //
 // Also here: the penalties and logit bias the reference applies before
@@ -104,10 +105,12 @@ __device__ __forceinline__ bool weighs(const RowCtx& c, float x, float& w) {
 
 struct Shared {
     unsigned cnt[COPIES][256];  // this block's part of the row
-    unsigned long long wfix[COPIES][256];   // weight sums in units of 2^-40 (see weight_units)
+    unsigned long long wfix[COPIES][256];   // weight sums in units of 2^-40 (see peers_units)
     unsigned cnt_all[256];      // the team's: the blocks' parts added in block order
     double wsum_all[256];
     unsigned long long units_all[256];
+    unsigned cnt_first[256], part_first[256];   // cnt_all, cnt[0] and wsum_all after the first pass of a selection by share
+    double wsum_first[256];
     int listed;                 // elements appended to the list
     double total;
     float red_val[32];
@@ -130,13 +133,13 @@ enum { MODE_COUNT = 0, MODE_W_GE = 1, MODE_W_GT = 2 };
 // so it keeps eleven bits and more; a row's sums stay below 2^58.  Against the reference's
 // running float64 sum a draw within 2^-23 of a boundary may pick the neighbour.
 constexpr double WEIGHT_UNIT = 1.0 / 1099511627776.0;      // 2^-40
-__device__ __forceinline__ unsigned long long weight_units(float w) {
-    return (unsigned long long)((double)w * 1099511627776.0);
-}
-// Sum of `v` over the lanes of `peers` (all of them call this with the same mask; v < 2^41).
-__device__ __forceinline__ unsigned long long peers_sum(unsigned peers, unsigned long long v) {
-    const unsigned lo = __reduce_add_sync(peers, (unsigned)(v & 0xfffffu));          // 32 x 2^20 < 2^32
-    const unsigned hi = __reduce_add_sync(peers, (unsigned)(v >> 20));               // 32 x 2^21 < 2^32
+// Sum of the units of `w` (0 <= w <= 1, cut to a whole number of them) over the lanes of `peers` (all of them call this
+// with the same mask).  The units leave the float in two pieces of 20 bits, every step exact.
+__device__ __forceinline__ unsigned long long peers_units(unsigned peers, float w) {
+    const float scaled = w * 1048576.0f;
+    const unsigned whole = (unsigned)scaled;
+    const unsigned hi = __reduce_add_sync(peers, whole);                                                    // 32 x 2^20 < 2^32
+    const unsigned lo = __reduce_add_sync(peers, (unsigned)((scaled - (float)whole) * 1048576.0f));
     return ((unsigned long long)hi << 20) + lo;
 }
 
@@ -175,8 +178,9 @@ __device__ __forceinline__ void append(const RowCtx& c, Shared& sh, int i, bool 
 
 // One histogram pass.  level 0..3: value key digits (high to low); level 4..7:
 // token digits among elements whose key == prefix_key.  `gather`: what lies under the prefix is listed too.
+// Without `weigh` only the counts are formed (no min-p is in force then).
 __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned prefix_key,
-                               unsigned prefix_tok, bool gather) {
+                               unsigned prefix_tok, bool gather, bool weigh) {
     for (int b = threadIdx.x; b < COPIES * 256; b += blockDim.x) { (&sh.cnt[0][0])[b] = 0; (&sh.wfix[0][0])[b] = 0ull; }
     if (threadIdx.x == 0) sh.listed = 0;
     __syncthreads();
@@ -194,15 +198,15 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
                 const unsigned tok = (unsigned)i;
                 if (level == 4 || (tok >> (shift + 8)) == (prefix_tok >> (shift + 8))) digit = (tok >> shift) & 0xffu;
             }
-            if (digit < 256u && !weighs(c, x, w)) digit = 256u;
+            if (weigh && digit < 256u && !weighs(c, x, w)) { digit = 256u; w = 0.f; }
         }
         if (gather) append(c, sh, i, digit < 256u);
         if (!__any_sync(0xffffffffu, digit < 256u)) return;
         const unsigned peers = __match_any_sync(0xffffffffu, digit);
-        const unsigned long long units = peers_sum(peers, digit < 256u ? weight_units(w) : 0ull);
+        const unsigned long long units = weigh ? peers_units(peers, w) : 0ull;
         if (digit < 256u && lane == __ffs(peers) - 1) {
             atomicAdd(&sh.cnt[copy][digit], (unsigned)__popc(peers));
-            atomicAdd(&sh.wfix[copy][digit], units);
+            if (weigh) atomicAdd(&sh.wfix[copy][digit], units);
         }
     });
     __syncthreads();
@@ -234,9 +238,13 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
 //   MODE_W_GT : the first element whose inclusive weight sum >  target_w.
 // With `of_total` target_w is a share of the set's total weight, which `total` gives in any case.
 // If no element qualifies, the last element of the set is returned.
+// `again`: the set is the nucleus that the selection before has found in its own set (`nuc_key`).  It is a prefix of
+// that set's order, so the counts and sums of the first pass are those found then: exactly in the buckets before
+// the one where the nucleus ends, in that one too much, which decides nothing (it is the last either way),
+// and none after it.
 // Outputs (uniform over the block): key, token, inclusive weight sum at it.
 __device__ void select(RowCtx& c, Shared& sh, int mode, unsigned long long target_count, double target_w, bool of_total,
-                       unsigned& out_key, unsigned& out_tok, double& out_cum, double& total) {
+                       bool again, unsigned& out_key, unsigned& out_tok, double& out_cum, double& total) {
     const int listed_before = c.listed;
     unsigned part_cnt = 0;                            // elements of this block's part under the prefix
     unsigned prefix_key = 0, prefix_tok = 0;
@@ -244,8 +252,21 @@ __device__ void select(RowCtx& c, Shared& sh, int mode, unsigned long long targe
     double w_before = 0.0;
     for (int level = 0; level < 8; ++level) {
         const bool gather = level > 0 && c.listed < 0 && part_cnt <= LIST_CAP;
-        histogram_pass(c, sh, level, prefix_key, prefix_tok, gather);
+        if (level == 0 && again) {
+            for (int b = threadIdx.x; b < 256; b += blockDim.x) {
+                sh.cnt_all[b] = b <= (int)(c.nuc_key >> 24) ? sh.cnt_first[b] : 0u;
+                sh.wsum_all[b] = b <= (int)(c.nuc_key >> 24) ? sh.wsum_first[b] : 0.0;
+                sh.cnt[0][b] = sh.part_first[b];
+            }
+            __syncthreads();
+        } else {
+            histogram_pass(c, sh, level, prefix_key, prefix_tok, gather, mode != MODE_COUNT);
+        }
         if (gather) c.listed = sh.listed;
+        if (level == 0 && mode == MODE_W_GE)                      // (a bucket's own thread has formed all three)
+            for (int b = threadIdx.x; b < 256; b += blockDim.x) {
+                sh.cnt_first[b] = sh.cnt_all[b]; sh.part_first[b] = sh.cnt[0][b]; sh.wsum_first[b] = sh.wsum_all[b];
+            }
         if (threadIdx.x < 32) {
             if (level == 0) {
                 unsigned long long all = 0;
@@ -488,7 +509,7 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
     const int k = top_k[r];
     if (k > 0) {
         // rank k in the order, or the last candidate when there are fewer
-        select(c, sh, MODE_COUNT, (unsigned long long)k, 0.0, false, key, tok, cum, total);
+        select(c, sh, MODE_COUNT, (unsigned long long)k, 0.0, false, false, key, tok, cum, total);
         c.has_topk = true; c.topk_key = key; c.topk_tok = tok;
         if (k <= LIST_CAP) {                           // what is left is k elements at most
             if (threadIdx.x == 0) sh.listed = 0;
@@ -512,12 +533,12 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
     const float tp = top_p[r];
     double kept;
     if (tp < 1.0f) {
-        select(c, sh, MODE_W_GE, 0, (double)tp, true, key, tok, cum, total);
+        select(c, sh, MODE_W_GE, 0, (double)tp, true, false, key, tok, cum, total);
         c.has_nucleus = true; c.nuc_key = key; c.nuc_tok = tok;
         kept = cum;
-        select(c, sh, MODE_W_GT, 0, uniform[r] * kept, false, key, tok, cum, total);
+        select(c, sh, MODE_W_GT, 0, uniform[r] * kept, false, true, key, tok, cum, total);
     } else {
-        select(c, sh, MODE_W_GT, 0, uniform[r], true, key, tok, cum, total);
+        select(c, sh, MODE_W_GT, 0, uniform[r], true, false, key, tok, cum, total);
         kept = total;
     }
     if (threadIdx.x == 0 && rank == 0) out[r] = (key == 0xffffffffu && tok == 0 && kept == 0.0) ? best_i : (int)tok;

@@ -840,6 +840,38 @@ def test_sample_rows_with_buckets_longer_than_a_blocks_list():
             assert c[at] >= draw - 1e-2 and (at == 0 or c[at - 1] <= draw + 1e-2), (u, r, got[r])
 
 
+@pytest.mark.parametrize("vocab", [700, 151936])
+def test_sample_rows_at_the_ends_of_a_nucleus(vocab):
+    """The draw takes its first pass from the selection that found the nucleus: 0 gives the nucleus's first token and the
+    largest number below 1 its last, never one behind it, with and without top-k and min-p, where the nucleus ends in the
+    first bucket of values, in a later one or with the set."""
+    from kipp_b200.kernels import sampling as ks
+    g = torch.Generator().manual_seed(vocab)
+    cases = [(0, 0.02, 0.0), (0, 0.5, 0.0), (0, 0.9999, 0.0), (50, 0.6, 0.0), (0, 0.7, 0.3), (300, 0.99, 0.01), (1, 0.5, 0.0)]
+    rows = len(cases)
+    logits = torch.randn(rows, vocab, generator=g) * 2.5
+    logits[:, 100:104] += 12.0                                                       # few tokens with most of the weight
+    logits[1, 100:104] -= 12.0
+    last, first = [], []
+    for r, (k, p, mp) in enumerate(cases):
+        v = logits[r].numpy()
+        order = np.lexsort((np.arange(vocab), -v.astype(np.float64)))[: k or vocab]
+        w = np.exp((v[order] - v[order[0]]).astype(np.float32)).astype(np.float64)
+        order, w = order[(w >= mp) & (v[order] >= v[order[0]] - 20)], w[(w >= mp) & (v[order] >= v[order[0]] - 20)]
+        c = np.cumsum(w)
+        at = min(int(np.searchsorted(c, np.float64(np.float32(p)) * c[-1])), len(w) - 1)
+        # sums are exact to 2^-23 of the top weight each: the tokens whose inclusive sums lie that near the boundary
+        slack = len(w) * 2.0 ** -22
+        last.append(set(order[(c >= c[at] - w[at] - slack - 1e-9) & (c - w <= c[at] + slack)].tolist()) if slack > w[at] else {int(order[at])})
+        first.append(int(order[0]))
+    f = lambda j, dt: torch.tensor([c[j] for c in cases], dtype=dt, device=DEV)      # noqa: E731
+    for u in (0.0, 1.0 - 2.0 ** -53):
+        got = ks.sample_rows(logits.to(DEV), torch.ones(rows, device=DEV), f(0, torch.int32), f(1, torch.float32), f(2, torch.float32),
+                             torch.full((rows,), u, dtype=torch.float64, device=DEV)).cpu().tolist()
+        for r in range(rows):
+            assert got[r] == first[r] if u == 0.0 else got[r] in last[r], (u, r, got[r])
+
+
 def test_penalties_and_bias_match_the_reference_sampler():
     import json
     import os
