@@ -854,16 +854,17 @@ int launch_mix_mma(size_t smem, int items, int head_blocks, cudaStream_t s, Args
 // finish (sink, gate, scale) from their registers.
 constexpr int SK_ROWS = 16, SK_THREADS = 128;
 
+constexpr size_t SK_SMEM_MAX = 200 * 1024;
 struct SharedKeySmem {
     int ldq, lds, ldp;
     size_t qs, ks, phi, plo, sraw, m_run, l_run, corr, pg, bytes;
-    __host__ __device__ SharedKeySmem(int head_dim) {
+    __host__ __device__ SharedKeySmem(int head_dim, int stages) {
         ldq = head_dim + 8;
         lds = KT + 1;
         ldp = KT + 8;
         size_t at = 0;
         qs = at; at += (size_t)SK_ROWS * ldq * 2;
-        ks = at; at += (size_t)KT * ldq * 2;
+        ks = at; at += (size_t)stages * KT * ldq * 2;
         phi = at; at += (size_t)SK_ROWS * ldp * 2;
         plo = at; at += (size_t)SK_ROWS * ldp * 2;
         sraw = at; at += (size_t)SK_ROWS * lds * 4;
@@ -962,12 +963,11 @@ __global__ void __launch_bounds__(SK_THREADS)
 attention_shared_key_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, const bf16* __restrict__ k_pages,
                             const int* __restrict__ positions, const int* __restrict__ entry_of_token,
                             const int* __restrict__ block_table, int table_width, int page_size, int n_q,
-                            int head_dim, int v_dim, float scale, int window, float out_scale, int split,
+                            int head_dim, int v_dim, float scale, int window, float out_scale, int split, int stages,
                             float* __restrict__ partial, int* __restrict__ status, const MixExtras ex) {
     extern __shared__ __align__(16) unsigned char raw[];
-    const SharedKeySmem L(head_dim);
+    const SharedKeySmem L(head_dim, stages);
     bf16* qs = reinterpret_cast<bf16*>(raw + L.qs);
-    bf16* ks = reinterpret_cast<bf16*>(raw + L.ks);
     bf16* phi = reinterpret_cast<bf16*>(raw + L.phi);
     bf16* plo = reinterpret_cast<bf16*>(raw + L.plo);
     float* sraw = reinterpret_cast<float*>(raw + L.sraw);
@@ -975,10 +975,9 @@ attention_shared_key_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
     float* l_run = reinterpret_cast<float*>(raw + L.l_run);
     float* corr = reinterpret_cast<float*>(raw + L.corr);
     int* pg = reinterpret_cast<int*>(raw + L.pg);
-    int* sl = pg + KT;
     const int ldq = L.ldq, lds = L.lds, ldp = L.ldp;
     pdl_launch_dependents();
-    pdl_wait();
+    // (positions and tables come with the step's lists, which a copy brought before any kernel of the step started)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gid = lane >> 2, tig = lane & 3;
     const int t = blockIdx.x, h0 = blockIdx.y * SK_ROWS;
@@ -990,48 +989,58 @@ attention_shared_key_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
     if (it0 >= n_tiles) return;
     const int it1 = split ? min(n_tiles, it0 + SPLIT_TILES) : n_tiles;
     const int* table = block_table + (size_t)entry_of_token[t] * table_width;
-
     const int chunks = head_dim / 8;
+    // four threads per key row of a tile; -1 where the tile has no such key, -2 where its page is missing
+    auto page_of = [&](int it) {
+        const int j = (win0 + it) * KT + (tid >> 2);
+        if (j < first || j > pos) return -1;
+        const int page = j / page_size < table_width ? table[j / page_size] : -1;
+        return page < 0 ? -2 : page;
+    };
+    auto fetch = [&](int it, int page, int stage) {
+        const int rr = tid >> 2, j = (win0 + it) * KT + rr;
+        if (page == -2 && (tid & 3) == 0) atomicExch(status, 3);
+        const bool ok = page >= 0;
+        const bf16* src = ok ? k_pages + ((size_t)page * page_size + j % page_size) * head_dim : k_pages;
+        const uint32_t dst = smem_address(reinterpret_cast<bf16*>(raw + L.ks) + (size_t)(stage * KT + rr) * ldq);
+        for (int c = tid & 3; c < chunks; c += 4) cp_async16(dst + c * 16, ok ? src + c * 8 : src, ok ? 16 : 0);
+        if ((tid & 3) == 0) pg[stage * KT + rr] = page;
+    };
+    static_assert(SK_THREADS / 4 == KT, "four threads per row of a tile");
+    const int page0 = page_of(it0);
+    if (tid < SK_ROWS) { m_run[tid] = -INFINITY; l_run[tid] = 0.f; corr[tid] = 1.f; }
+    pdl_wait();
+    fetch(it0, page0, 0);
     for (int i = tid; i < SK_ROWS * chunks; i += SK_THREADS) {
         const int c = i % chunks, r = i / chunks;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (h0 + r < n_q) v = *reinterpret_cast<const uint4*>(q + ((size_t)t * n_q + h0 + r) * head_dim + c * 8);
-        *reinterpret_cast<uint4*>(qs + (size_t)r * ldq + c * 8) = v;
+        const bool there = h0 + r < n_q;
+        cp_async16(smem_address(qs + (size_t)r * ldq + c * 8), there ? q + ((size_t)t * n_q + h0 + r) * head_dim + c * 8 : q, there ? 16 : 0);
     }
-    if (tid < SK_ROWS) { m_run[tid] = -INFINITY; l_run[tid] = 0.f; corr[tid] = 1.f; }
+    cp_async_commit();
     float o[VB][4];
 #pragma unroll
     for (int b = 0; b < VB; ++b) o[b][0] = o[b][1] = o[b][2] = o[b][3] = 0.f;
     const int col0 = warp * VB * 8;                                 // this warp's value columns
 
     for (int it = it0; it < it1; ++it) {
-        const int j0 = (win0 + it) * KT;
-        __syncthreads();                                            // the tile before is done with K and P
-        if (tid < KT) {
-            const int j = j0 + tid;
-            int page = -1;
-            if (j >= first && j <= pos) {
-                page = j / page_size < table_width ? table[j / page_size] : -1;
-                if (page < 0) atomicExch(status, 3);
-            }
-            pg[tid] = page;
-            sl[tid] = j % page_size;
+        const int stage = stages == 2 ? (it - it0) & 1 : 0;
+        if (stages == 2) {                                          // the next tile is on its way
+            if (it + 1 < it1) fetch(it + 1, page_of(it + 1), stage ^ 1);
+            cp_async_commit();
+            cp_async_wait<1>();
+        } else {
+            if (it > it0) fetch(it, page_of(it), 0);
+            cp_async_commit();
+            cp_async_wait<0>();
         }
         __syncthreads();
-        for (int rr = tid >> 2; rr < KT; rr += SK_THREADS / 4) {    // four threads per key row
-            const bool ok = pg[rr] >= 0;
-            const bf16* src = ok ? k_pages + ((size_t)pg[rr] * page_size + sl[rr]) * head_dim : k_pages;
-            const uint32_t dst = smem_address(ks + (size_t)rr * ldq);
-            for (int c = tid & 3; c < chunks; c += 4) cp_async16(dst + c * 16, ok ? src + c * 8 : src, ok ? 16 : 0);
-        }
-        cp_async_commit();
-        cp_async_wait<0>();
-        __syncthreads();
+        const bf16* ks = reinterpret_cast<const bf16*>(raw + L.ks) + (size_t)stage * KT * ldq;
         // ---- S = Q K^T: this warp's 8 keys
         {
             float c[4] = {0.f, 0.f, 0.f, 0.f};
             const bf16* kr = ks + (size_t)(warp * 8 + gid) * ldq + tig * 2;
             const bf16* qa = qs + (size_t)gid * ldq + tig * 2;
+#pragma unroll 4
             for (int k0 = 0; k0 < head_dim; k0 += 16) {
                 uint32_t a[4];
                 a[0] = *reinterpret_cast<const uint32_t*>(qa + k0);
@@ -1047,12 +1056,12 @@ attention_shared_key_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
             sraw[(gid + 8) * lds + key + 1] = capped(c[3] * scale, ex.softcap);
         }
         __syncthreads();
-        head_rows_softmax(sraw, lds, phi, plo, ldp, m_run, l_run, corr, pg[lane] >= 0, warp, lane);
+        head_rows_softmax(sraw, lds, phi, plo, ldp, m_run, l_run, corr, pg[stage * KT + lane] >= 0, warp, lane);
         __syncthreads();
         // ---- O += P V: the value of a key is the head of its row
         head_rows_accumulate<VB>(o, phi, plo, ldp, corr, ks, ldq, col0, v_dim, gid, tig);
+        __syncthreads();                                            // this stage and the weights may be overwritten
     }
-    __syncthreads();
     // rows gid and gid + 8 are heads h0 + gid and h0 + gid + 8; a thread holds columns col + 2 tig, + 1
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
@@ -1088,7 +1097,13 @@ int launch_shared_key(void* out, const void* q, const void* k_pages, const int* 
                       const int* block_table, int table_width, int page_size, int tokens, int n_q, int head_dim,
                       int v_dim, float scale, int window, float out_scale, int runs, float* partial, int* status,
                       const MixExtras& ex, cudaStream_t s) {
-    const size_t smem = SharedKeySmem(head_dim).bytes;
+    const int split = runs > 1 ? 1 : 0;
+    const dim3 grid((unsigned)tokens, (unsigned)((n_q + SK_ROWS - 1) / SK_ROWS), (unsigned)(split ? runs : 1));
+    // Two stages of keys, the next tile on its way, where no more than two blocks an SM are there anyway (of 576 columns two
+    // stages leave room for two, one for four): one token of 300 keys, 16 heads: 12.5 us a launch, 15.2 with a tile's page, keys
+    // and products one after the other.
+    const int stages = (long long)grid.x * grid.y * grid.z <= 2 * 148 && SharedKeySmem(head_dim, 2).bytes <= SK_SMEM_MAX ? 2 : 1;
+    const size_t smem = SharedKeySmem(head_dim, stages).bytes;
     auto kernel = attention_shared_key_kernel<VB>;
     static size_t allowed = 0;
     if (smem > 48 * 1024 && smem > allowed) {
@@ -1096,11 +1111,9 @@ int launch_shared_key(void* out, const void* q, const void* k_pages, const int* 
         if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
         allowed = smem;
     }
-    const int split = runs > 1 ? 1 : 0;
-    const dim3 grid((unsigned)tokens, (unsigned)((n_q + SK_ROWS - 1) / SK_ROWS), (unsigned)(split ? runs : 1));
     int rc = kipp_launch(kernel, grid, dim3(SK_THREADS), smem, s, 1, (bf16*)out, (const bf16*)q, (const bf16*)k_pages,
                          positions, entry_of_token, block_table, table_width, page_size, n_q, head_dim, v_dim, scale,
-                         window, out_scale, split, partial, status, ex);
+                         window, out_scale, split, stages, partial, status, ex);
     if (rc || !split) return rc;
     return launch_merge<bf16>(out, partial, positions, tokens, n_q, v_dim, window, 0, runs, out_scale, ex, s);
 }
@@ -1216,6 +1229,7 @@ attention_group_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, const
             float c[4] = {0.f, 0.f, 0.f, 0.f};
             const bf16* kr = ks + (size_t)(warp * 8 + gid) * ldk + tig * 2;
             const bf16* qa = qs + (size_t)gid * ldk + tig * 2;
+#pragma unroll 4
             for (int k0 = 0; k0 < head_dim; k0 += 16) {
                 uint32_t a[4];
                 a[0] = *reinterpret_cast<const uint32_t*>(qa + k0);
@@ -1333,7 +1347,7 @@ extern "C" int kipp_attention_group(void* out, const void* q, const void* k_page
 // Whether the tensor-core kernel for one shared key row per token takes these sizes (bfloat16 only).
 extern "C" int kipp_attention_shared_key_ok(int n_q, int head_dim, int v_dim) {
     if (n_q <= 0 || head_dim <= 0 || v_dim <= 0 || head_dim % 16 || v_dim % 8 || v_dim > head_dim || v_dim > 512) return 0;
-    return SharedKeySmem(head_dim).bytes <= 200 * 1024 ? 1 : 0;
+    return SharedKeySmem(head_dim, 1).bytes <= SK_SMEM_MAX ? 1 : 0;
 }
 
 // n_q heads over one key row of head_dim per token whose first v_dim elements are its value.

@@ -1137,3 +1137,48 @@ def test_latent_expand(sizes, page):
                 if out is ko:
                     assert (got[:n, :, size:] == rows[:, None, rank:].double()).all(), (tc, e)
                 assert (got[n:end] == 0).all() and (got[end:] == 7).all(), (tc, e)
+
+
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("sizes", [(20, 96, 64), (16, 576, 512), (33, 1312, 24)])
+def test_attention_shared_key(sizes, window):
+    """One key row per token for all heads, its head the value: tokens at the edges of the tiles of 32 keys, in pages of any
+    order, as few blocks (two stages of keys where they fit; 1,312 columns leave room for one), as many (one stage) and cut
+    into runs.  Without runs a token has the same bits among few and among many; all stay within the bound of 16-bit inputs
+    and results (weights as pairs of bfloat16, sums in float32) around float64."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    n_q, D, V = sizes
+    page, width, scale = 16, 14, 0.05
+    g = torch.Generator().manual_seed(D + window)
+    at = [0, 1, 30, 31, 32, 63, 64, 95, 96, 200]
+    T = 300
+    pos = torch.tensor((at * T)[:T], dtype=torch.int32)
+    entry = torch.arange(T, dtype=torch.int32) % 3
+    table = torch.randperm(3 * width, generator=g).int().reshape(3, width)
+    pool = torch.randn(3 * width, page, D, generator=g).bfloat16()
+    q = torch.randn(T, n_q, D, generator=g).bfloat16()
+    fn = load_library("attention_mix").kipp_attention_shared_key
+    p, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    fn.argtypes = [p, p, p, p, p, p, i, i, i, i, i, i, f, i, f, i, p, p, p, p]
+    d = [x.to(DEV) for x in (q, pool, pos, entry, table)]
+    status = torch.zeros(8, dtype=torch.int32, device=DEV)
+
+    def run(tokens, runs):
+        out = torch.zeros(tokens, n_q, V, dtype=torch.bfloat16, device=DEV)
+        partial = torch.zeros(tokens * runs * n_q * (V + 2), device=DEV)
+        rc = fn(out.data_ptr(), d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), d[3].data_ptr(), d[4].data_ptr(), width, page, tokens,
+                n_q, D, V, scale, window, 1.0, runs, partial.data_ptr(), None, status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0 and status.abs().sum().item() == 0
+        return out
+
+    many, few, cut = run(T, 1), run(len(at), 1), run(len(at), 4)
+    assert torch.equal(many[:len(at)], few)
+    for t in range(len(at)):
+        lo = max(0, int(pos[t]) - window + 1) if window else 0
+        keys = torch.cat([pool[j] for j in table[int(entry[t])]])[lo:int(pos[t]) + 1].double()
+        w = torch.softmax(q[t].double() @ keys.t() * scale, -1)
+        want, size = w @ keys[:, :V], w @ keys[:, :V].abs()
+        for got in (few[t], cut[t]):
+            assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4 * size).all(), (t, window)
