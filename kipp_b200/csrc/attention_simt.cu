@@ -17,8 +17,7 @@
 // lane that walks its own key row in global memory waits a trip to the L2 for every few values, and every
 // head of a group fetched the same rows (four layers of 16 heads of 128 over prompts of 400 tokens and eight steps
 // of three tokens: 36 launches in 10.6 ms, 1.35 now; 1.63 while each 16 bytes copied looked its page up).  What bounds it
-// now is the chain of head_dim FMAs per key tile and the
-// 32 weighted rows after it.
+// now is the chain of head_dim FMAs per key tile and the 32 weighted rows after it.
 //
 // A window of w (0 = none) lets position p see keys j with p - w < j <= p.
 #include "common.cuh"
