@@ -833,15 +833,13 @@ public:
         using Fn = int (*)(void*, long long, const void*, long long, int, int, int, int, const float*, const float*, int,
                            const float*, const float*, const float*, const float*, int, float*, long long, const int*,
                            const int*, const int*, int, int, int, int, int, int, float, float*, float*, void*);
-        using Fc = int (*)(int, int, int, int, int, int);
         static Fn f = kernel_symbol<Fn>("recurrent", "kipp_ssd_scan");
-        static Fc by_chunks = kernel_symbol<Fc>("recurrent", "kipp_ssd_by_chunks");
         float* scratch = recurrent_scratch(tokens, heads, dim, v_dim, 4);
         float* conv_out = workspace->get<float>("state_space_conv", (size_t)tokens * ((size_t)heads * v_dim + 2 * (size_t)groups * dim));
         run(f(out, ld_out, proj, ld_proj, dtype, z_off, xbc_off, dt_off, conv_w, conv_b, taps, dt_bias, a_log, d_skip, norm_w,
               norm_groups, state, slot_stride, q_start, entry_of_token, slots, entries, tokens, heads, groups, dim, v_dim, eps,
               scratch, conv_out, stream),
-            "ssd_scan", tokens == entries ? 2 : (taps > 1 ? 4 : 3) + (by_chunks(entries, tokens, heads, groups, dim, v_dim) ? 3 : 0));
+            "ssd_scan", tokens == entries ? 2 : taps > 1 ? 4 : 3);
     }
 
     // The gated delta rule (recurrent.cu, kind 5): convolution, unit keys, decays, the recurrence, norm and gate.

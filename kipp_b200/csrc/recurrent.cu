@@ -58,8 +58,11 @@
 // Two kinds have scans of their own for the sizes that divide by four: ssd_scan_kernel (straight from the
 // convolved rows, no records), and for the gated delta rule gated_delta_scan_kernel (four columns a thread) and
 // gated_delta_column_kernel (one, where few blocks make the chain of a token what counts).  There a thread works on pairs of
-// float32 and the shuffles of one token's sums travel while the next token is worked on.  State space prompts go by
-// chunks of tokens instead where that pays (by_chunks): products within a chunk, the state from chunk to chunk.  For steps of one token per request
+// float32 and the shuffles of one token's sums travel while the next token is worked on.  (State space prompts by chunks of
+// 128 tokens, products within a chunk and the state from chunk to chunk, took 164 us instead of 477 for 2,048 tokens of 64
+// heads of 128 x 64 and are not used: their sums come in another order, which can turn a near tie of a router behind the
+// layer; the order hung on the step's other prompts; and the masked products carried an infinite token into the ones
+// before it.)  For steps of one token per request
 // ssd_token_kernel and gated_delta_token_kernel do the convolution, the state and the output in one launch.
 // A scan of many tokens starts when the kernel before it has left the GPU (kipp_launch_spread): blocks that
 // were placed early share few multiprocessors, and a scan lasts as long as its most crowded one.
@@ -1529,433 +1532,6 @@ int launch_scan_chunk(const ScanArgs& b, const float* vec, float* o_raw, int sli
 
 // scratch: float32 [heads][tokens][NV * dim + v_dim] for the records, then [tokens][heads * v_dim] for raw o
 // conv_out: float32 [tokens, channels] for the convolved rows of the state space layer and the gated delta rule (null for the other kinds)
-// ---------------------------------------------------------------------------
-// The state space recurrence by chunks of CHUNK tokens, for prompts.  In one chunk of one head, with p_t the product
-// of the decays up to t, q_s that of those after s, and l_ts that of those in (s, t]:
-//
-//   y_t = p_t C_t S_in + sum_{s <= t} (C_t . B_s) l_ts dt_s x_s        S_out = p_end S_in + sum_s q_s dt_s B_s x_s^T
-//
-// so the tokens no longer wait for one another: only the chunks' states do, and theirs is one multiply-add per
-// element and chunk.  Four launches: (1) C_t . B_s for the groups (all heads of a group share them), C transposed, and
-// the products of decays; (2) a chunk's own share of S_out, per head; (3) the states in front of the chunks, in
-// order; (4) the outputs.  All sums are float32 FMAs (in pairs) and every l_ts is a product of decays, never a
-// quotient or a difference of logarithms, so nothing is lost against the scan in order, whose sums are
-// longer.  (2) and (4) are products of 128 x 64 by 128 threads with 8 x 8 results each, operands in slices of
-// 32 through shared memory, both with the summed index outermost so that a slice's rows are read 16 bytes at a
-// time by neighbouring lanes.  CHUNK: at 64 the chunks' states are 67 MB written and read three times for
-// 2,048 tokens of 64 heads, at 256 the pairs (t, s) cost as much as the states save.
-//
-// 2,048 tokens, 64 heads of 128 x 64, one sequence: 164 us (19 + 48 + 10 + 87) against 477 us for the scan in
-// order, whose 128 blocks walk 0.23 us a token; the whole layer for four sequences of 511: 261 us against 412.
-constexpr int CHUNK = 128, CHUNK_COLS = 64, CHUNK_SLICE = 32;
-struct ChunkScratch {
-    float* states;      // [chunks][heads][dim][v_dim]: (2) leaves the chunk's own share, (3) the state before the chunk
-    float* pairs;       // [chunks][groups][CHUNK s][CHUNK t]: C_t . B_s where s <= t (64 x 64 corners above stay unwritten)
-    float* c_rows;      // [chunks][groups][dim][CHUNK]
-    float* up_to;       // [chunks][CHUNK][heads]: p_t
-    float* after;       // [chunks][CHUNK][heads]: q_s
-};
-inline long long chunk_count(int tokens, int entries) { return (long long)tokens / CHUNK + entries; }
-inline long long chunk_floats(int tokens, int entries, int heads, int groups, int dim, int v_dim) {
-    return chunk_count(tokens, entries) * ((long long)heads * dim * v_dim + (long long)groups * (CHUNK * CHUNK + dim * CHUNK) + 2LL * CHUNK * heads);
-}
-// Which tokens chunk i is: false beyond the last one.
-__device__ __forceinline__ bool chunk_at(const ScanArgs& a, int i, int& row0, int& n) {
-    for (int e = 0; e < a.entries; ++e) {
-        const int q0 = a.q_start[e], len = a.q_start[e + 1] - q0, k = (len + CHUNK - 1) / CHUNK;
-        if (i < k) {
-            row0 = q0 + i * CHUNK;
-            n = min(CHUNK, len - i * CHUNK);
-            return true;
-        }
-        i -= k;
-    }
-    return false;
-}
-
-// (1) blockIdx.y 1 + 3 g + z: the 64 x 64 part (s half, t half) = (0, 0), (0, 1), (1, 1) of group g; y 0: the decays.
-constexpr int PAIRS_ROW = CHUNK_SLICE + 4;
-__global__ void __launch_bounds__(128)
-ssd_chunk_pairs_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* __restrict__ dts, const ChunkScratch w) {
-    __shared__ __align__(16) float rows[2][128 * PAIRS_ROW];          // 64 rows of B, 64 of C
-    pdl_launch_dependents();
-    pdl_wait();
-    const int ci = blockIdx.x, tid = threadIdx.x, D = a.dim;
-    int row0, n;
-    if (!chunk_at(a, ci, row0, n)) return;
-    if (blockIdx.y == 0) {                                            // (first: its loops are the longest)
-        float* up = w.up_to + (size_t)ci * CHUNK * a.heads;
-        float* down = w.after + (size_t)ci * CHUNK * a.heads;
-        for (int h = tid; h < a.heads; h += 128) {
-            const float2* d = dts + (size_t)row0 * a.heads + h;
-            float p = 1.f, q = 1.f;
-            for (int t0 = 0; t0 < CHUNK; t0 += 32) {                  // (32 loads on their way at a time)
-                float x[32];
-#pragma unroll
-                for (int k = 0; k < 32; ++k) x[k] = t0 + k < n ? d[(size_t)(t0 + k) * a.heads].x : 1.f;
-#pragma unroll
-                for (int k = 0; k < 32; ++k) up[(size_t)(t0 + k) * a.heads + h] = p *= x[k];
-            }
-            for (int t0 = CHUNK - 32; t0 >= 0; t0 -= 32) {
-                float x[32];
-#pragma unroll
-                for (int k = 0; k < 32; ++k) x[k] = t0 + k < n ? d[(size_t)(t0 + k) * a.heads].x : 1.f;
-#pragma unroll
-                for (int k = 31; k >= 0; --k) {
-                    down[(size_t)(t0 + k) * a.heads + h] = q;
-                    q *= x[k];
-                }
-            }
-        }
-        return;
-    }
-    const int part = blockIdx.y - 1, g = part / 3, z = part % 3, s0 = z == 2 ? 64 : 0, t0 = z == 0 ? 0 : 64;
-    const int inner = a.heads * a.v_dim, slices = (D + CHUNK_SLICE - 1) / CHUNK_SLICE;
-    if (n <= t0) return;                                              // (rows past the last token are read by nobody)
-    auto fetch = [&](int slice, int buf) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int c = j * 128 + tid, row = c >> 3, k = slice * CHUNK_SLICE + (c & 7) * 4;
-            const int t = row < 64 ? s0 + row : t0 + row - 64;
-            const bool in = t < n && k < D;
-            const float* src = conv + (size_t)(row0 + (in ? t : 0)) * a.channels + inner + (size_t)(row < 64 ? g : a.groups + g) * D + (in ? k : 0);
-            cp_async16(smem_address(&rows[buf][row * PAIRS_ROW + (c & 7) * 4]), src, in ? 16 : 0);
-        }
-        cp_async_commit();
-    };
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    const int tx = tid & 15, ty = tid >> 4;
-    float* ct = w.c_rows + ((size_t)ci * a.groups + g) * D * CHUNK;
-    fetch(0, 0);
-    for (int sl = 0; sl < slices; ++sl) {
-        if (sl + 1 < slices) fetch(sl + 1, (sl + 1) & 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const float* b = rows[sl & 1];
-        const float* c = b + 64 * PAIRS_ROW;
-        if (z != 1)
-            for (int i = tid; i < CHUNK_SLICE * 64; i += 128) {
-                const int k = i >> 6, t = i & 63;
-                if (sl * CHUNK_SLICE + k < D) ct[(size_t)(sl * CHUNK_SLICE + k) * CHUNK + t0 + t] = c[t * PAIRS_ROW + k];
-            }
-#pragma unroll
-        for (int q = 0; q < CHUNK_SLICE; q += 4) {
-            float4 x[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) x[j] = *reinterpret_cast<const float4*>(c + (tx + 16 * j) * PAIRS_ROW + q);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float4 v = *reinterpret_cast<const float4*>(b + (ty + 8 * i) * PAIRS_ROW + q);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    acc[i][j] = fmaf(v.w, x[j].w, fmaf(v.z, x[j].z, fmaf(v.y, x[j].y, fmaf(v.x, x[j].x, acc[i][j]))));
-            }
-        }
-        __syncthreads();
-    }
-    float* out = w.pairs + ((size_t)ci * a.groups + g) * CHUNK * CHUNK;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) out[(size_t)(s0 + ty + 8 * i) * CHUNK + t0 + tx + 16 * j] = acc[i][j];
-}
-
-// acc[i][j] (rows 2 i, 2 i + 1 of a thread's eight: four at r, four at 64 + r; columns four at c, four at 32 + c) += the
-// slice's products: rows [k][128], cols [k][64].  FROM 2: the rows of the upper half only.
-template <int FROM>
-__device__ __forceinline__ void chunk_products(float2 (&acc)[4][8], const float* rows, const float* cols, int r, int c) {
-#pragma unroll 4
-    for (int k = 0; k < CHUNK_SLICE; ++k) {
-        float2 v[4];
-        if (FROM == 0) {
-            const float4 lo = *reinterpret_cast<const float4*>(rows + k * CHUNK + r);
-            v[0] = make_float2(lo.x, lo.y);
-            v[1] = make_float2(lo.z, lo.w);
-        }
-        const float4 hi = *reinterpret_cast<const float4*>(rows + k * CHUNK + 64 + r);
-        v[2] = make_float2(hi.x, hi.y);
-        v[3] = make_float2(hi.z, hi.w);
-        const float4 a = *reinterpret_cast<const float4*>(cols + k * CHUNK_COLS + c);
-        const float4 b = *reinterpret_cast<const float4*>(cols + k * CHUNK_COLS + 32 + c);
-        const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int i = FROM; i < 4; ++i) acc[i][j] = fma2(v[i], both(x[j]), acc[i][j]);
-    }
-}
-// x of a slice of tokens into [k][CHUNK_COLS]; the rows past n and the columns past v_dim become zeros
-__device__ __forceinline__ void chunk_fetch_x(const ScanArgs& a, const float* conv, float* to, int row0, int n, int s0, int h, int v0) {
-#pragma unroll
-    for (int j = 0; j < CHUNK_SLICE * CHUNK_COLS / 4 / 128; ++j) {
-        const int c = j * 128 + threadIdx.x, k = c >> 4, x = v0 + (c & 15) * 4;
-        const bool in = s0 + k < n && x < a.v_dim;
-        cp_async16(smem_address(to + k * CHUNK_COLS + (c & 15) * 4), conv + (in ? (size_t)(row0 + s0 + k) * a.channels + h * a.v_dim + x : 0), in ? 16 : 0);
-    }
-}
-// each row k of the slice times f(k); the caller synchronises before and after
-template <typename F> __device__ __forceinline__ void chunk_scale_x(float* x, F f) {
-#pragma unroll
-    for (int j = 0; j < CHUNK_SLICE * CHUNK_COLS / 4 / 128; ++j) {
-        const int c = j * 128 + threadIdx.x;
-        float4* at = reinterpret_cast<float4*>(x + (c >> 4) * CHUNK_COLS + (c & 15) * 4);
-        const float w = f(c >> 4);
-        float4 v = *at;
-        v.x *= w; v.y *= w; v.z *= w; v.w *= w;
-        *at = v;
-    }
-}
-
-constexpr int CHUNK_SMEM = 2 * CHUNK_SLICE * (CHUNK + CHUNK_COLS) * 4;
-// (2) a chunk's own share of the state: sum_s (q_s dt_s) B_s x_s^T
-__global__ void __launch_bounds__(128)
-ssd_chunk_state_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* __restrict__ dts, const ChunkScratch w) {
-    extern __shared__ __align__(16) float smem[];                     // two of [slice][CHUNK] B and [slice][CHUNK_COLS] x
-    __shared__ float weight[CHUNK];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int ci = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * CHUNK_COLS, tid = threadIdx.x, D = a.dim, V = a.v_dim;
-    int row0, n;
-    if (!chunk_at(a, ci, row0, n)) return;
-    const int g = h / (a.heads / a.groups), inner = a.heads * V, slices = (n + CHUNK_SLICE - 1) / CHUNK_SLICE;
-    weight[tid] = tid < n ? w.after[((size_t)ci * CHUNK + tid) * a.heads + h] * dts[(size_t)(row0 + tid) * a.heads + h].y : 0.f;
-    auto fetch = [&](int sl, int buf) {
-        float* to = smem + buf * CHUNK_SLICE * (CHUNK + CHUNK_COLS);
-#pragma unroll
-        for (int j = 0; j < CHUNK_SLICE * CHUNK / 4 / 128; ++j) {
-            const int c = j * 128 + tid, k = c >> 5, d = (c & 31) * 4, s = sl * CHUNK_SLICE + k;
-            const bool in = s < n && d < D;
-            cp_async16(smem_address(to + k * CHUNK + d), conv + (in ? (size_t)(row0 + s) * a.channels + inner + (size_t)g * D + d : 0), in ? 16 : 0);
-        }
-        chunk_fetch_x(a, conv, to + CHUNK_SLICE * CHUNK, row0, n, sl * CHUNK_SLICE, h, v0);
-        cp_async_commit();
-    };
-    float2 acc[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = both(0.f);
-    const int r = (tid >> 3) * 4, c = (tid & 7) * 4;
-    fetch(0, 0);
-    for (int sl = 0; sl < slices; ++sl) {
-        if (sl + 1 < slices) fetch(sl + 1, (sl + 1) & 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        float* rows = smem + (sl & 1) * CHUNK_SLICE * (CHUNK + CHUNK_COLS);
-        float* x = rows + CHUNK_SLICE * CHUNK;
-        chunk_scale_x(x, [&](int k) { return weight[sl * CHUNK_SLICE + k]; });
-        __syncthreads();
-        chunk_products<0>(acc, rows, x, r, c);
-        __syncthreads();
-    }
-    float* out = w.states + ((size_t)ci * a.heads + h) * D * V + v0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int d = (i < 4 ? r : 60 + r) + i;
-        if (d >= D) continue;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            if (v0 + 32 * half + c >= V) continue;
-            auto at = [&](int j) { return i & 1 ? acc[i >> 1][4 * half + j].y : acc[i >> 1][4 * half + j].x; };
-            *reinterpret_cast<float4*>(out + (size_t)d * V + 32 * half + c) = make_float4(at(0), at(1), at(2), at(3));
-        }
-    }
-}
-
-// (3) the chunks of an entry in order: each one's own share is replaced by the state before it, and the slot gets the last.
-__global__ void __launch_bounds__(256)
-ssd_chunk_carry_kernel(const ScanArgs a, const ChunkScratch w) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int e = blockIdx.y, per_head = a.dim * a.v_dim / 4, i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= a.heads * per_head) return;
-    const int h = i / per_head;
-    int first = 0;
-    for (int k = 0; k < e; ++k) first += (a.q_start[k + 1] - a.q_start[k] + CHUNK - 1) / CHUNK;
-    const int chunks = (a.q_start[e + 1] - a.q_start[e] + CHUNK - 1) / CHUNK;
-    float4* slot = reinterpret_cast<float4*>(a.state + (size_t)a.slots[e] * (size_t)a.slot_stride) + i;
-    float4* at = reinterpret_cast<float4*>(w.states) + (size_t)first * a.heads * per_head + i;
-    const float* end = w.up_to + ((size_t)first * CHUNK + CHUNK - 1) * a.heads + h;       // (past the last token p stays)
-    const size_t step = (size_t)a.heads * per_head, end_step = (size_t)CHUNK * a.heads;
-    float4 s = *slot;
-    constexpr int AHEAD = 8;                                          // chunks whose loads are on their way together
-    for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
-        float4 own[AHEAD];
-        float p[AHEAD];
-#pragma unroll
-        for (int k = 0; k < AHEAD; ++k)
-            if (c0 + k < chunks) {
-                own[k] = at[(size_t)(c0 + k) * step];
-                p[k] = end[(size_t)(c0 + k) * end_step];
-            }
-#pragma unroll
-        for (int k = 0; k < AHEAD; ++k)
-            if (c0 + k < chunks) {
-                at[(size_t)(c0 + k) * step] = s;
-                s.x = fmaf(p[k], s.x, own[k].x); s.y = fmaf(p[k], s.y, own[k].y);
-                s.z = fmaf(p[k], s.z, own[k].z); s.w = fmaf(p[k], s.w, own[k].w);
-            }
-    }
-    *slot = s;
-}
-
-// (4) the outputs.  Thread t makes row t of l_ts (C_t . B_s) in place, a slice of s at a time from the last to the first,
-// so that l grows by one factor per step.  (With the pairs read from global memory at that place, a trip for
-// every eight of them, the kernel took 106 us; 87 so.)
-__global__ void __launch_bounds__(128)
-ssd_chunk_output_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* __restrict__ dts, const ChunkScratch w,
-                        float* __restrict__ o_raw) {
-    extern __shared__ __align__(16) float smem[];
-    __shared__ float decay[CHUNK], dt[CHUNK], up[CHUNK];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int ci = blockIdx.x, h = blockIdx.y, v0 = blockIdx.z * CHUNK_COLS, tid = threadIdx.x, D = a.dim, V = a.v_dim;
-    int row0, n;
-    if (!chunk_at(a, ci, row0, n)) return;
-    const int g = h / (a.heads / a.groups), inner = a.heads * V;
-    const float2 kd = tid < n ? dts[(size_t)(row0 + tid) * a.heads + h] : make_float2(1.f, 0.f);
-    decay[tid] = kd.x;
-    dt[tid] = kd.y;
-    up[tid] = w.up_to[((size_t)ci * CHUNK + tid) * a.heads + h];
-    const float* ct = w.c_rows + ((size_t)ci * a.groups + g) * D * CHUNK;
-    const float* s_in = w.states + ((size_t)ci * a.heads + h) * D * V + v0;
-    const float* pairs = w.pairs + ((size_t)ci * a.groups + g) * CHUNK * CHUNK;
-    constexpr int BUF = CHUNK_SLICE * (CHUNK + CHUNK_COLS);
-    auto fetch = [&](int sl, int buf) {
-        float* to = smem + buf * BUF;
-#pragma unroll
-        for (int j = 0; j < CHUNK_SLICE * CHUNK / 4 / 128; ++j) {
-            const int c = j * 128 + tid, k = c >> 5, d = sl * CHUNK_SLICE + k;
-            cp_async16(smem_address(to + k * CHUNK + (c & 31) * 4), ct + (d < D ? (size_t)d * CHUNK + (c & 31) * 4 : 0), d < D ? 16 : 0);
-        }
-#pragma unroll
-        for (int j = 0; j < CHUNK_SLICE * CHUNK_COLS / 4 / 128; ++j) {
-            const int c = j * 128 + tid, k = c >> 4, d = sl * CHUNK_SLICE + k, x = (c & 15) * 4;
-            const bool in = d < D && v0 + x < V;
-            cp_async16(smem_address(to + CHUNK_SLICE * CHUNK + k * CHUNK_COLS + x), s_in + (in ? (size_t)d * V + x : 0), in ? 16 : 0);
-        }
-        cp_async_commit();
-    };
-    float2 acc[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = both(0.f);
-    const int r = (tid >> 3) * 4, c = (tid & 7) * 4, slices = (D + CHUNK_SLICE - 1) / CHUNK_SLICE;
-    fetch(0, 0);
-    for (int sl = 0; sl < slices; ++sl) {
-        if (sl + 1 < slices) fetch(sl + 1, (sl + 1) & 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const float* rows = smem + (sl & 1) * BUF;
-        chunk_products<0>(acc, rows, rows + CHUNK_SLICE * CHUNK, r, c);
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = (i < 2 ? r : 60 + r) + 2 * i;
-        const float2 p = make_float2(up[t], up[t + 1]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = mul2(acc[i][j], p);
-    }
-    // slices of s from the last that holds a token, the next one's pairs and x on their way
-    const int last = (n - 1) / CHUNK_SLICE;
-    auto fetch_pairs = [&](int sl) {
-        float* to = smem + (sl & 1) * BUF;
-#pragma unroll
-        for (int j = 0; j < CHUNK_SLICE * CHUNK / 4 / 128; ++j) {
-            const int i = 4 * (j * 128 + tid);
-            cp_async16(smem_address(to + i), pairs + (size_t)sl * CHUNK_SLICE * CHUNK + i, 16);
-        }
-        chunk_fetch_x(a, conv, to + CHUNK_SLICE * CHUNK, row0, n, sl * CHUNK_SLICE, h, v0);
-        cp_async_commit();
-    };
-    fetch_pairs(last);
-    float l = 1.f;
-    for (int sl = last; sl >= 0; --sl) {
-        if (sl > 0) fetch_pairs(sl - 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        float* rows = smem + (sl & 1) * BUF;
-        float* x = rows + CHUNK_SLICE * CHUNK;
-        // thread t's column, s from high to low (above the diagonal lies what nobody wrote)
-#pragma unroll 8
-        for (int k = CHUNK_SLICE - 1; k >= 0; --k) {
-            const int s = sl * CHUNK_SLICE + k;
-            float m = 0.f;
-            if (s <= tid) {
-                m = l * rows[k * CHUNK + tid];
-                l *= decay[s];
-            }
-            rows[k * CHUNK + tid] = m;
-        }
-        chunk_scale_x(x, [&](int k) { return dt[sl * CHUNK_SLICE + k]; });
-        __syncthreads();
-        if (sl * CHUNK_SLICE >= 64) chunk_products<2>(acc, rows, x, r, c);      // the rows below 64 see none of these
-        else chunk_products<0>(acc, rows, x, r, c);
-        __syncthreads();
-    }
-    float* out = o_raw + (size_t)row0 * inner + h * V + v0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int t = (i < 4 ? r : 60 + r) + i;
-        if (t >= n) continue;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            if (v0 + 32 * half + c >= V) continue;
-            auto at = [&](int j) { return i & 1 ? acc[i >> 1][4 * half + j].y : acc[i >> 1][4 * half + j].x; };
-            *reinterpret_cast<float4*>(out + (size_t)t * inner + 32 * half + c) = make_float4(at(0), at(1), at(2), at(3));
-        }
-    }
-}
-
-// Whether the form by chunks pays: heads whose rows and columns fill most of the products' tiles, 192 tokens an
-// entry on average (a partial chunk costs what a whole one does) and 320 in all (300 tokens of one sequence: 117 us the
-// layer against 111), few enough entries to look through.  What it keeps lies where the records of the general
-// form would; groups that are hardly shared by heads may not fit there.
-inline long long chunk_room(int tokens, int heads, int dim, int v_dim) {
-    return (long long)tokens * heads * (2LL * dim + 4 + v_dim) - (2LL * tokens * heads + 3) / 4 * 4;
-}
-inline bool by_chunks(int entries, int tokens, int heads, int groups, int dim, int v_dim) {
-    return dim <= CHUNK && dim > CHUNK / 2 && v_dim > CHUNK_COLS / 2 && tokens >= 192 * entries && tokens >= 320 && entries <= 64 && heads <= 65535 &&
-           chunk_floats(tokens, entries, heads, groups, dim, v_dim) <= chunk_room(tokens, heads, dim, v_dim);
-}
-inline int launch_ssd_chunks(const ScanArgs& a, const float* conv, const float2* dts, float* scratch, float* o_raw, int tokens,
-                             cudaStream_t stream) {
-    const long long chunks = chunk_count(tokens, a.entries);
-    ChunkScratch w;
-    w.states = scratch;
-    w.pairs = w.states + chunks * a.heads * a.dim * a.v_dim;
-    w.c_rows = w.pairs + chunks * a.groups * CHUNK * CHUNK;
-    w.up_to = w.c_rows + chunks * a.groups * a.dim * CHUNK;
-    w.after = w.up_to + chunks * CHUNK * a.heads;
-    const unsigned slices = (unsigned)((a.v_dim + CHUNK_COLS - 1) / CHUNK_COLS);
-    const dim3 per_head((unsigned)chunks, (unsigned)a.heads, slices);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(ssd_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(ssd_chunk_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
-    int rc = kipp_launch(ssd_chunk_pairs_kernel, dim3((unsigned)chunks, (unsigned)(3 * a.groups + 1)), dim3(128), 0, stream, 1, a, conv, dts, w);
-    if (rc) return rc;
-    rc = kipp_launch(ssd_chunk_state_kernel, per_head, dim3(128), CHUNK_SMEM, stream, 1, a, conv, dts, w);
-    if (rc) return rc;
-    rc = kipp_launch(ssd_chunk_carry_kernel, dim3((unsigned)((a.heads * a.dim * a.v_dim / 4 + 255) / 256), (unsigned)a.entries), dim3(256), 0,
-                     stream, 1, a, w);
-    if (rc) return rc;
-    return kipp_launch(ssd_chunk_output_kernel, per_head, dim3(128), CHUNK_SMEM, stream, 1, a, conv, dts, w, o_raw);
-}
-
 template <typename T, int DELTA>
 int launch_scan(const ScanArgs& a, int entries, int tokens, float* scratch, cudaStream_t stream, float* conv_out = nullptr) {
     const int D = a.dim, V = a.v_dim + Rec<DELTA>::XV;
@@ -2021,10 +1597,7 @@ int launch_scan(const ScanArgs& a, int entries, int tokens, float* scratch, cuda
         if (by_fours && (DELTA != SSD || direct)) {
             if constexpr (DELTA == SSD) {
                 const float* cv = conv_out;
-                float* rest = vec + (2 * (size_t)tokens * a.heads + 3) / 4 * 4;        // behind the decays and step sizes
-                if (by_chunks(entries, tokens, a.heads, a.groups, D, V))
-                    rc = launch_ssd_chunks(b, cv, dts, rest, o_raw, tokens, stream);
-                else if (D <= 32) rc = launch_ssd_scan<8, 4>(b, cv, dts, o_raw, entries, tokens, stream);
+                if (D <= 32) rc = launch_ssd_scan<8, 4>(b, cv, dts, o_raw, entries, tokens, stream);
                 else if (D <= 64) rc = launch_ssd_scan<16, 4>(b, cv, dts, o_raw, entries, tokens, stream);
                 else if (D <= 128) rc = launch_ssd_scan<32, 4>(b, cv, dts, o_raw, entries, tokens, stream);
                 else rc = launch_ssd_scan<32, 8>(b, cv, dts, o_raw, entries, tokens, stream);
@@ -2220,13 +1793,6 @@ extern "C" int kipp_wkv_scan(void* out, long long ld_out, const void* proj, long
 // last taps - 1 inputs of the heads * v_dim + 2 * groups * dim convolved channels.
 extern "C" long long kipp_ssd_state_floats(int heads, int groups, int dim, int v_dim, int taps) {
     return (long long)heads * dim * v_dim + (long long)(taps > 1 ? taps - 1 : 0) * ((long long)heads * v_dim + 2LL * groups * dim);
-}
-
-// Whether a step of these sizes goes by chunks (rows and states on 16 bytes as the general conditions ask): three
-// launches more than the scan in order.
-extern "C" int kipp_ssd_by_chunks(int entries, int tokens, int heads, int groups, int dim, int v_dim) {
-    return entries > 0 && tokens > 0 && heads > 0 && groups > 0 && dim % 4 == 0 && v_dim % 4 == 0 &&
-           by_chunks(entries, tokens, heads, groups, dim, v_dim);
 }
 
 // The state space layer (see the head of this file).  proj [T, ...] holds z [heads * v_dim] at z_off, the

@@ -5,7 +5,6 @@ again; keys far away and at the edges of pages; the sink; the first tokens; a st
 that remembers the first token through long decoding; long decoding through
 graphs; drawn configurations; greedy generation through the scheduler; the command
 line and the trace program."""
-import ctypes
 import json
 import math
 import os
@@ -140,16 +139,11 @@ def test_state_space_alone(name, layer, dtype):
     close(out, want, dtype, f"{name} layer {layer}")
 
 
-@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("state,vdim,heads,groups", [(128, 64, 4, 2), (68, 36, 12, 2), (100, 72, 6, 1)])
-def test_state_space_by_chunks(state, vdim, heads, groups, dtype):
-    """Prompts long enough for the form by chunks of 128 tokens: whole and partial chunks, one of a single token, an entry
-    that ends on a chunk's edge, columns in two slices, heads that share their group's pairs; two steps, so that the
-    second starts from the state that the first left.  Then the same step with one token fewer than the form asks for."""
+def _state_space_engine(state, vdim, heads, groups, dtype):
+    """An engine of one state space layer alone, its mixer's configuration and its weights."""
     from kipp_b200.config import config_from_dict
     from kipp_b200.config.registry import get_architecture
-    from kipp_b200.csrc.build import library_path
-    from kipp_b200.engine import Engine, StepEntry
+    from kipp_b200.engine import Engine
     from kipp_b200.weights.random_init import random_tensors
     mixer = {"heads": heads, "groups": groups, "vdim": vdim, "state": state, "conv": 4, "norm_groups": 1}
     cfg = {"architecture": "Zunilorn", "vocab": 64, "width": 64, "norm": {"eps": 1e-6},
@@ -158,15 +152,22 @@ def test_state_space_by_chunks(state, vdim, heads, groups, dtype):
     tensors = dict(random_tensors(spec.tensor_specs(), 5, sigma=0.1, dtype=torch.float32))
     if dtype == "bfloat16":                            # matrices lie in bfloat16 (the convolution stays 32-bit)
         tensors = {k: v.bfloat16().float() if v.dim() == 2 and "conv" not in k else v for k, v in tensors.items()}
-    eng = Engine(spec, tensors, dtype=dtype, cache_tokens=4096, max_requests=4, max_batch_tokens=1024, cuda_graphs=False)
+    return Engine(spec, tensors, dtype=dtype, cache_tokens=4096, max_requests=4, max_batch_tokens=1024, cuda_graphs=False), mixer, tensors
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("state,vdim,heads,groups", [(128, 64, 4, 2), (68, 36, 12, 2), (100, 72, 6, 1)])
+def test_state_space_long_prompts(state, vdim, heads, groups, dtype):
+    """Prompts of several hundred tokens beside others of one and of a few hundred, columns that end inside a block's, heads
+    that share their group's keys; two steps, so that the second starts from the state that the first left."""
+    from kipp_b200.engine import StepEntry
+    eng, mixer, tensors = _state_space_engine(state, vdim, heads, groups, dtype)
     w = {k: v.double() for k, v in tensors.items()}
     steps = [[("a", 385), ("b", 1), ("c", 256)], [("b", 300), ("a", 128), ("c", 200)], [("a", 191)]]
     total = {r: sum(n for st in steps for q, n in st if q == r) for r in "abc"}
     h = {r: torch.randn(n, 64, generator=torch.Generator().manual_seed(ord(r))).to("cuda", eng.dtype) for r, n in total.items()}
     want = {r: P.mamba2(mixer, w, "l0.mix.", x.double().cpu(), 1e-6) for r, x in h.items()}
     at = dict.fromkeys("abc", 0)
-    lib = ctypes.CDLL(library_path("recurrent"))
-    assert [lib.kipp_ssd_by_chunks(len(st), sum(n for _, n in st), heads, groups, state, vdim) for st in steps] == [1, 1, 0]
     for st in steps:
         rows = torch.cat([h[r][at[r]:at[r] + n] for r, n in st]).contiguous()
         out = torch.zeros(len(rows), 64, device="cuda")
@@ -174,6 +175,43 @@ def test_state_space_by_chunks(state, vdim, heads, groups, dtype):
         close(out, torch.cat([want[r][at[r]:at[r] + n] for r, n in st]), dtype, str(st))
         for r, n in st:
             at[r] += n
+
+
+@pytest.mark.parametrize("state,vdim,heads,groups", [(128, 64, 4, 2), (100, 72, 6, 1), (37, 9, 3, 1)])
+def test_a_state_space_row_hangs_on_its_own_tokens_only(state, vdim, heads, groups):
+    """A prompt's rows in 32-bit have the same bits alone, beside another prompt and cut into portions, and the rows before a
+    token that is not finite have the bits they have without it: a row comes from its own tokens up to it, in one
+    order of sums, whatever else the step holds."""
+    from kipp_b200.engine import StepEntry
+    eng, _, _ = _state_space_engine(state, vdim, heads, groups, "float32")
+    n, beside, bad = 420, 330, 411
+    h = torch.randn(n + beside, 64, generator=torch.Generator().manual_seed(9)).cuda()
+
+    def run(name, cuts, spoil=None, other=False):
+        got, at = [], 0
+        for c in cuts:
+            rows = h[at:at + c].clone()
+            if spoil is not None and at <= spoil < at + c:
+                rows[spoil - at] = float("inf")
+            if other:
+                rows = torch.cat([h[n:], rows])
+            out = torch.zeros(len(rows), 64, device="cuda")
+            first = [StepEntry(name + "/other", [0] * beside, [])] if other else []
+            eng.run_part(first + [StepEntry(name, [0] * c, [])], 0, "mixer", input=rows.contiguous(), residual=out)
+            got.append(out[-c:])
+            at += c
+        for r in [name] + [name + "/other"] * other:
+            eng.finish(r)
+        return torch.cat(got)
+
+    alone = run("alone", [n])
+    assert torch.isfinite(alone).all()
+    assert torch.equal(run("beside", [n], other=True), alone)
+    for cuts in ([200, 220], [319, 101], [2, 418]):
+        assert torch.equal(run(str(cuts), cuts), alone), cuts
+    spoiled = run("spoiled", [n], spoil=bad)
+    assert torch.equal(spoiled[:bad], alone[:bad])
+    assert not torch.isfinite(spoiled[bad]).all()
 
 
 def test_the_convolution_starts_from_zeros_in_a_slot_used_again():
