@@ -580,9 +580,10 @@ gated_delta_prepare_kernel(const ScanArgs a, const float* __restrict__ conv_out,
 }
 
 // After the scan: y = (o + D_h x) * silu(z), divided by the root mean square of its part of the row
-// (norm_groups equal parts of heads * v_dim), times the weight.  A block per (token, part), a thread W neighbouring
-// channels at a time (4 where rows, parts and heads go by fours and start accordingly: 2,048 tokens of 4,096
-// channels, 100 MB: 56 us a channel at a time, 28 so).
+// (norm_groups equal parts of heads * v_dim), times the weight.  A block per (token, part).  W: channels that a thread
+// forms at a time; 4 where rows, parts and heads go by fours, start accordingly and fit in shared memory, through which
+// the values then go, so that thread t adds the squares of channels t, t + threads, ... whatever W is (2,048 tokens of
+// 4,096 channels, 100 MB: 56 us a channel at a time, 29 so).
 // keep: every entry brought one token, and the blocks of its row also move its kept inputs on.
 template <int W> __device__ __forceinline__ void load_channels(float (&v)[W], const float* p) {
     if constexpr (W == 4) {
@@ -641,27 +642,45 @@ ssd_finish_kernel(const ScanArgs a, const float* __restrict__ conv_out, const fl
 #pragma unroll
         for (int j = 0; j < W; ++j) y[j] = fmaf(skip, x[j], y[j]) * (z[j] / (1.0f + expf(-z[j])));
     };
-    // a thread's first values stay in registers between the two passes (all of them for parts of up to 1,024)
-    constexpr int HELD = 8 / W;
+    constexpr int HELD = 8 / W;                                 // values formed together: their loads travel together
     float held[HELD][W];
     float ss = 0.f;
+    extern __shared__ __align__(16) float values[];             // W of 4: the part's n values
+    auto form = [&](int i0) {
 #pragma unroll
-    for (int k = 0; k < HELD; ++k) {
-        const int i = W * (threadIdx.x + k * blockDim.x);
-        if (i < n) {
-            value(held[k], part * n + i);
-        } else {
+        for (int k = 0; k < HELD; ++k) {
+            const int i = i0 + W * (threadIdx.x + k * blockDim.x);
+            if (i < n) {
+                value(held[k], part * n + i);
+            } else {
 #pragma unroll
-            for (int j = 0; j < W; ++j) held[k][j] = 0.f;
+                for (int j = 0; j < W; ++j) held[k][j] = 0.f;
+            }
         }
+    };
+    const int at_once = HELD * W * blockDim.x;
+    form(0);
+    if constexpr (W == 4) {
+        for (int i0 = 0; i0 < n; i0 += at_once) {
+            if (i0 > 0) form(i0);
 #pragma unroll
-        for (int j = 0; j < W; ++j) ss = fmaf(held[k][j], held[k][j], ss);
-    }
-    for (int i = W * (threadIdx.x + HELD * blockDim.x); i < n; i += W * blockDim.x) {
-        float y[W];
-        value(y, part * n + i);
+            for (int k = 0; k < HELD; ++k) {
+                const int i = i0 + W * (threadIdx.x + k * blockDim.x);
+                if (i < n) store_channels<W>(values + i, held[k]);
+            }
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int i = threadIdx.x; i < n; i += blockDim.x) ss = fmaf(values[i], values[i], ss);
+    } else {
+        // (a thread's first values stay in registers between the two passes: all of them for parts of up to 1,024)
 #pragma unroll
-        for (int j = 0; j < W; ++j) ss = fmaf(y[j], y[j], ss);
+        for (int k = 0; k < HELD; ++k) ss = fmaf(held[k][0], held[k][0], ss);
+        for (int i = threadIdx.x + at_once; i < n; i += blockDim.x) {
+            float y[W];
+            value(y, part * n + i);
+            ss = fmaf(y[0], y[0], ss);
+        }
     }
     ss = block_sum(ss, scratch);
     const float inv = 1.0f / sqrtf(ss / (float)n + a.eps);
@@ -678,15 +697,23 @@ ssd_finish_kernel(const ScanArgs a, const float* __restrict__ conv_out, const fl
         for (int j = 0; j < W; ++j) y[j] = y[j] * inv * w[j];
         store_channels<W>(out + ch, y);
     };
+    if constexpr (W == 4) {
+#pragma unroll 2
+        for (int i = W * threadIdx.x; i < n; i += W * blockDim.x) {
+            load_channels<W>(held[0], values + i);
+            put(held[0], part * n + i);
+        }
+    } else {
 #pragma unroll
-    for (int k = 0; k < HELD; ++k) {
-        const int i = W * (threadIdx.x + k * blockDim.x);
-        if (i < n) put(held[k], part * n + i);
-    }
-    for (int i = W * (threadIdx.x + HELD * blockDim.x); i < n; i += W * blockDim.x) {
-        float y[W];
-        value(y, part * n + i);
-        put(y, part * n + i);
+        for (int k = 0; k < HELD; ++k) {
+            const int i = threadIdx.x + k * blockDim.x;
+            if (i < n) put(held[k], part * n + i);
+        }
+        for (int i = threadIdx.x + at_once; i < n; i += blockDim.x) {
+            float y[W];
+            value(y, part * n + i);
+            put(y, part * n + i);
+        }
     }
 }
 
@@ -1631,11 +1658,10 @@ int launch_scan(const ScanArgs& a, int entries, int tokens, float* scratch, cuda
         const int es = (int)sizeof(T);
         const bool fours = per_part % 4 == 0 && a.v_dim % 4 == 0 && a.dim % 2 == 0 && a.z_off % 4 == 0 && a.ld_proj % 4 == 0 && a.ld_out % 4 == 0 &&
                            (((uintptr_t)conv_out | (uintptr_t)o_raw | (uintptr_t)a.norm_w) & 15) == 0 &&
-                           (((uintptr_t)a.proj | (uintptr_t)a.out) & (4 * es - 1)) == 0;
-        const int at_once = fours ? per_part / 4 : per_part;
+                           (((uintptr_t)a.proj | (uintptr_t)a.out) & (4 * es - 1)) == 0 && (per_part + 32) * sizeof(float) <= 48 * 1024;
         rc = kipp_launch(fours ? ssd_finish_kernel<T, 4> : ssd_finish_kernel<T, 1>, dim3((unsigned)parts),
-                         dim3(one_token ? 256 : at_once >= 128 ? 128 : (at_once + 31) / 32 * 32), 0, stream, 1, b, (const float*)conv_out,
-                         (const float*)o_raw, one_token && b.taps > 1 ? 1 : 0);
+                         dim3(one_token ? 256 : per_part >= 128 ? 128 : (per_part + 31) / 32 * 32), fours ? per_part * sizeof(float) : 0, stream, 1,
+                         b, (const float*)conv_out, (const float*)o_raw, one_token && b.taps > 1 ? 1 : 0);
     } else {
         rc = kipp_launch(recurrent_finish_kernel<T, DELTA>, wgrid, dim3(128), 0, stream, 1, b, (const float*)o_raw, tokens);
     }

@@ -1182,3 +1182,45 @@ def test_attention_shared_key(sizes, window):
         want, size = w @ keys[:, :V], w @ keys[:, :V].abs()
         for got in (few[t], cut[t]):
             assert ((got.double().cpu() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4 * size).all(), (t, window)
+
+
+@pytest.mark.parametrize("lens", [[37], [1, 1, 1]])
+@pytest.mark.parametrize("heads,v_dim,norm_groups", [(8, 64, 1), (8, 64, 8), (64, 64, 1), (192, 64, 1), (5, 36, 1), (6, 20, 3)])
+def test_gated_norm_adds_in_one_order(heads, v_dim, norm_groups, lens):
+    """The gate and grouped norm behind the state space scan take four channels at a time where the gate's rows start on
+    that, one channel elsewhere and in parts too long for shared memory: the same bits in 32-bit, for prompts and one-token
+    steps, in parts of fewer and of more channels than threads."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    lib = load_library("recurrent")
+    p, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+    lib.kipp_ssd_scan.argtypes = [p, ll, p, ll, i, i, i, i, p, p, i, p, p, p, p, i, p, ll, p, p, p, i, i, i, i, i, i, f, p, p, p]
+    lib.kipp_ssd_state_floats.restype = lib.kipp_recurrent_scratch_floats.restype = ll
+    D, taps, T, E = 16, 3, sum(lens), len(lens)
+    inner, channels = heads * v_dim, heads * v_dim + 2 * D
+    g = torch.Generator().manual_seed(heads + v_dim)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)                      # noqa: E731
+    x, z, dt = rnd(T, channels), rnd(T, inner), rnd(T, heads)
+    weights = [rnd(taps, channels) * 0.5, rnd(channels) * 0.1, rnd(heads), rnd(heads) * 0.5, rnd(heads), rnd(inner)]
+    stride = lib.kipp_ssd_state_floats(heads, 1, D, v_dim, taps)
+    state = rnd(E, stride)
+    q_start = torch.tensor([0] + np.cumsum(lens).tolist(), dtype=torch.int32, device=DEV)
+    entry = torch.repeat_interleave(torch.arange(E), torch.tensor(lens)).int().to(DEV)
+    slots = torch.arange(E, dtype=torch.int32, device=DEV)
+    results = []
+    for shift in (0, 1):
+        ld = channels + heads + (-heads) % 4 + inner + 4
+        z_off = ld - inner - 4 + shift
+        proj = torch.zeros(T, ld, device=DEV)
+        proj[:, :channels], proj[:, channels:channels + heads], proj[:, z_off:z_off + inner] = x, dt, z
+        out, s = torch.zeros(T, inner, device=DEV), state.clone()
+        scratch = torch.zeros(lib.kipp_recurrent_scratch_floats(T, heads, D, v_dim, 4), device=DEV)
+        conv = torch.zeros(T, channels, device=DEV)
+        w = [t.data_ptr() for t in weights]
+        rc = lib.kipp_ssd_scan(out.data_ptr(), inner, proj.data_ptr(), ld, 0, z_off, 0, channels, w[0], w[1], taps, w[2], w[3], w[4], w[5],
+                               norm_groups, s.data_ptr(), stride, q_start.data_ptr(), entry.data_ptr(), slots.data_ptr(), E, T, heads, 1, D,
+                               v_dim, 1e-5, scratch.data_ptr(), conv.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0 and torch.isfinite(out).all()
+        results.append((out, s))
+    assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
