@@ -12,7 +12,7 @@
 // their order, and so are then the up to four sums of those.  The runs are what lets a few tokens be multiplied by
 // many threads at once, the groups of four what lets a small product of many tokens be shared by more blocks.
 //
-// Three kernels, chosen by shape alone, with that one order:
+// Three kernels, chosen by shape and alignment alone, with that one order for 32-bit weights whose rows start on 16 bytes:
 //   few   float32, up to FEW_MAX tokens (16 of many features): bound by the weights' bytes (a token is 2 operations per 4 bytes).  A
 //         block holds 16 features, a thread one feature and one run, so a 2,048-feature matrix still
 //         gives 128 blocks of 256 chains; the weights travel by asynchronous copies, five chunks of 64 bytes
@@ -27,8 +27,9 @@
 //         are blocks of their own, a cluster that meets in its shared memory.
 //         407 tokens, 12,288 x 2,048: 608 us (943 before), 2,048 x 6,144: 392 us (866; 540 with
 //         tiles of 64 x 64, 8 x 4 per thread and k innermost); 64 tokens, 12,288 x 2,048: 106 us (387; 181).
-//   any   what is left: bfloat16 operands of shapes that the tensor-core kernels refuse, and float32 rows that do
-//         not start on 16 bytes.
+//   any   what is left: tokens whose float32 rows do not start on 16 bytes, in the order above; and what no other kernel
+//         here takes, bfloat16 operands of shapes that the tensor-core kernels refuse and float32 weights off 16 bytes: one chain of FMAs in the order of k, without the 38 registers and the extra sums of the runs (bfloat16, 2,050
+//         features of 2,056: 1 and 200 tokens 154 and 152 us, 186 and 180 in runs).
 //
 // Epilogues:
 //   STORE   C[m,n]    = acc                 (C in float32 or bfloat16)
@@ -60,7 +61,8 @@ __device__ __forceinline__ void put(TC* C, int ldc, int m, int n, float v) {
 }
 __device__ __forceinline__ float swiglu(float g, float u) { return g / (1.0f + expf(-g)) * u; }
 
-template <typename TA, typename TW, typename TC, int EPI>
+// RUNS: the sum in runs and groups of them (see the head of the file), else one chain.
+template <typename TA, typename TW, typename TC, int EPI, bool RUNS>
 __global__ void __launch_bounds__(256)
 gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restrict__ W,
                  int M, int N, int K, int lda, int ldw, int ldc) {
@@ -71,12 +73,15 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int run = run_length(K);
-    float acc[TM][TN], group[TM][TN], sum[TM][TN];
+    const int run = RUNS ? run_length(K) : 0;
+    float acc[TM][TN], group[RUNS ? TM : 1][TN], sum[RUNS ? TM : 1][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = group[i][j] = sum[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) {
+            acc[i][j] = 0.f;
+            if constexpr (RUNS) group[i][j] = sum[i][j] = 0.f;
+        }
 
     // 64x16 tile = 1024 elements, 256 threads -> 4 each; thread loads row
     // (tid / 4), k columns (tid % 4) * 4 .. + 3.
@@ -103,22 +108,28 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
                 for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
         __syncthreads();
-        if ((k0 + BK) % run == 0 || k0 + BK >= K) {
-            const bool whole = (k0 + BK) % (GROUP_RUNS * run) == 0 || k0 + BK >= K;
+        if constexpr (RUNS) {
+            if ((k0 + BK) % run == 0 || k0 + BK >= K) {
+                const bool whole = (k0 + BK) % (GROUP_RUNS * run) == 0 || k0 + BK >= K;
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+                for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    group[i][j] += acc[i][j];
-                    acc[i][j] = 0.f;
-                    if (whole) {
-                        sum[i][j] += group[i][j];
-                        group[i][j] = 0.f;
+                    for (int j = 0; j < TN; ++j) {
+                        group[i][j] += acc[i][j];
+                        acc[i][j] = 0.f;
+                        if (whole) {
+                            sum[i][j] += group[i][j];
+                            group[i][j] = 0.f;
+                        }
                     }
-                }
+            }
         }
     }
 
+    auto total = [&](int i, int j) {
+        if constexpr (RUNS) return sum[i][j];
+        else return acc[i][j];
+    };
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int m = m0 + ty * TM + i;
@@ -127,9 +138,9 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
         for (int j = 0; j < TN; ++j) {
             const int n = n0 + tx * TN + j;
             if (EPI == EPI_SWIGLU) {
-                if ((j & 1) == 0 && n + 1 < N) put<TC, EPI_STORE>(C, ldc, m, n >> 1, swiglu(sum[i][j], sum[i][j + 1]));
+                if ((j & 1) == 0 && n + 1 < N) put<TC, EPI_STORE>(C, ldc, m, n >> 1, swiglu(total(i, j), total(i, j + 1)));
             } else if (n < N) {
-                put<TC, EPI>(C, ldc, m, n, sum[i][j]);
+                put<TC, EPI>(C, ldc, m, n, total(i, j));
             }
         }
     }
@@ -449,21 +460,21 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, in
     return kipp_launch(gemm_tile_kernel<EPI>, grid, dim3(TILE_THREADS), TILE_SMEM, s, groups, C, A, W, M, N, K, lda, ldw, ldc);
 }
 
-template <typename TA, typename TW, typename TC>
+template <typename TA, typename TW, typename TC, bool RUNS>
 int launch(void* C, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldc,
            int epi, cudaStream_t s) {
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     if (grid.y > 65535) return KIPP_ERR_ARG;
     switch (epi) {
     case EPI_STORE:
-        return kipp_launch(gemm_simt_kernel<TA, TW, TC, EPI_STORE>, grid, dim3(256), 0, s, 1, (TC*)C, (const TA*)A,
+        return kipp_launch(gemm_simt_kernel<TA, TW, TC, EPI_STORE, RUNS>, grid, dim3(256), 0, s, 1, (TC*)C, (const TA*)A,
                            (const TW*)W, M, N, K, lda, ldw, ldc);
     case EPI_ADD:
-        return kipp_launch(gemm_simt_kernel<TA, TW, TC, EPI_ADD>, grid, dim3(256), 0, s, 1, (TC*)C, (const TA*)A,
+        return kipp_launch(gemm_simt_kernel<TA, TW, TC, EPI_ADD, RUNS>, grid, dim3(256), 0, s, 1, (TC*)C, (const TA*)A,
                            (const TW*)W, M, N, K, lda, ldw, ldc);
     case EPI_SWIGLU:
         if (N & 1) return KIPP_ERR_ARG;
-        return kipp_launch(gemm_simt_kernel<TA, TW, TC, EPI_SWIGLU>, grid, dim3(256), 0, s, 1, (TC*)C, (const TA*)A,
+        return kipp_launch(gemm_simt_kernel<TA, TW, TC, EPI_SWIGLU, RUNS>, grid, dim3(256), 0, s, 1, (TC*)C, (const TA*)A,
                            (const TW*)W, M, N, K, lda, ldw, ldc);
     default:
         return KIPP_ERR_ARG;
@@ -479,7 +490,9 @@ extern "C" int kipp_gemm_simt(void* C, int out_dtype, const void* A, const void*
     if (K <= 0) return KIPP_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     if (epilogue == EPI_ADD && out_dtype != KIPP_DT_F32) return KIPP_ERR_DTYPE;
-    const bool vectors = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    // `shared`: weights that all three kernels may be given, and so have one order of sums for
+    const bool shared = K % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)W & 15) == 0;
+    const bool vectors = shared && lda % 4 == 0 && ((uintptr_t)A & 15) == 0;
     if (in_dtype == KIPP_DT_F32 && out_dtype == KIPP_DT_F32 && vectors) {
         if (epilogue == EPI_STORE) return launch_f32<EPI_STORE>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, s);
         if (epilogue == EPI_ADD) return launch_f32<EPI_ADD>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, s);
@@ -487,10 +500,11 @@ extern "C" int kipp_gemm_simt(void* C, int out_dtype, const void* A, const void*
             return launch_f32<EPI_SWIGLU>((float*)C, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldc, s);
     }
     if (in_dtype == KIPP_DT_F32 && out_dtype == KIPP_DT_F32)
-        return launch<float, float, float>(C, A, W, M, N, K, lda, ldw, ldc, epilogue, s);
+        return shared ? launch<float, float, float, true>(C, A, W, M, N, K, lda, ldw, ldc, epilogue, s)
+                      : launch<float, float, float, false>(C, A, W, M, N, K, lda, ldw, ldc, epilogue, s);
     if (in_dtype == KIPP_DT_BF16 && out_dtype == KIPP_DT_F32)
-        return launch<bf16, bf16, float>(C, A, W, M, N, K, lda, ldw, ldc, epilogue, s);
+        return launch<bf16, bf16, float, false>(C, A, W, M, N, K, lda, ldw, ldc, epilogue, s);
     if (in_dtype == KIPP_DT_BF16 && out_dtype == KIPP_DT_BF16)
-        return launch<bf16, bf16, bf16>(C, A, W, M, N, K, lda, ldw, ldc, epilogue, s);
+        return launch<bf16, bf16, bf16, false>(C, A, W, M, N, K, lda, ldw, ldc, epilogue, s);
     return KIPP_ERR_DTYPE;
 }

@@ -152,6 +152,25 @@ def test_gemm_32_bit_kernels_agree(shape, epilogue):
     assert torch.equal(some, whole)
 
 
+@pytest.mark.parametrize("dtype,shape,w_rows", [(torch.bfloat16, (5, 70, 100), 100), (torch.bfloat16, (65, 130, 37), 40),
+                                                (torch.float32, (3, 66, 37), 37), (torch.float32, (70, 20, 60), 61)])
+def test_gemm_simt_chain(dtype, shape, w_rows):
+    """What only the general kernel takes (bfloat16, and 32-bit weights whose rows do not start on 16 bytes) is one chain
+    of FMAs in the order of k.  The products of 8-bit mantissas are exact in 32 bits, so a loop of rounded additions
+    gives every bit."""
+    M, N, K = shape
+    g = torch.Generator().manual_seed(K)
+    a, w = torch.randn(M, K, generator=g).bfloat16().float(), torch.randn(N, K, generator=g).bfloat16().float()
+    want = torch.zeros(M, N)
+    for k in range(K):
+        want = want + a[:, k:k + 1] * w[:, k]
+    held = torch.zeros(N, w_rows, dtype=dtype, device=DEV)
+    held[:, :K] = w
+    out = torch.zeros(M, N, device=DEV)
+    ops().gemm(out, a.to(dtype).to(DEV), held[:, :K], "store", impl="simt")
+    assert torch.equal(out.cpu(), want)
+
+
 @pytest.mark.parametrize("epilogue", ["store", "add", "swiglu"])
 @pytest.mark.parametrize("shape", [(1, 128, 64), (8, 256, 128), (17, 250, 192), (64, 1000, 136),
                                    (100, 384, 2568), (300, 640, 520), (5, 2560, 1216), (40, 14400, 136),
