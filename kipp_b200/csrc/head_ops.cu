@@ -58,6 +58,13 @@ struct SegmentArgs {
     int vec;                                 // every row of every segment starts on 16 bytes and holds whole 16-byte pieces
 };
 
+// One value of a rotated pair, u cos - v sin for the first and v cos + u sin for the second, rounded the same way whichever
+// form of the kernel turns it: the product with the sine, then one FMA.
+__device__ __forceinline__ float turned(float own, float other, float c, float s, bool first) {
+    const float across = __fmul_rn(other, s);
+    return fmaf(own, c, first ? -across : across);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
@@ -194,10 +201,10 @@ head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
                     for (int j = 0; j < VEC; j += 4) {
                         const float4 c = *reinterpret_cast<const float4*>(cs + (r + j) / 2);        // two pairs' (cos, sin)
                         const float u0 = v[j], u1 = v[j + 2];
-                        v[j] = u0 * c.x - v[j + 1] * c.y;
-                        v[j + 1] = v[j + 1] * c.x + u0 * c.y;
-                        v[j + 2] = u1 * c.z - v[j + 3] * c.w;
-                        v[j + 3] = v[j + 3] * c.z + u1 * c.w;
+                        v[j] = turned(u0, v[j + 1], c.x, c.y, true);
+                        v[j + 1] = turned(v[j + 1], u0, c.x, c.y, false);
+                        v[j + 2] = turned(u1, v[j + 3], c.z, c.w, true);
+                        v[j + 3] = turned(v[j + 3], u1, c.z, c.w, false);
                     }
                 } else {
                     const bool low = r < half;
@@ -206,8 +213,8 @@ head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
 #pragma unroll
                     for (int j = 0; j < VEC; j += 2) {
                         const float4 c = *reinterpret_cast<const float4*>(cs + (low ? r : r - half) + j);
-                        v[j] = low ? v[j] * c.x - other[j] * c.y : v[j] * c.x + other[j] * c.y;
-                        v[j + 1] = low ? v[j + 1] * c.z - other[j + 1] * c.w : v[j + 1] * c.z + other[j + 1] * c.w;
+                        v[j] = turned(v[j], other[j], c.x, c.y, low);
+                        v[j + 1] = turned(v[j + 1], other[j + 1], c.z, c.w, low);
                     }
                 }
             }
@@ -234,7 +241,7 @@ head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
             const bool low = g.interleaved ? (r & 1) == 0 : r < half;
             const float2 c = cs[g.interleaved ? r >> 1 : (low ? r : r - half)];
             const float other = value(g.interleaved ? (low ? i + 1 : i - 1) : (low ? i + half : i - half));
-            v = low ? v * c.x - other * c.y : v * c.x + other * c.y;
+            v = turned(v, other, c.x, c.y, low);
         }
         if (into_cache) {
             if (a.write_cache & 2) v = __bfloat162float(__float2bfloat16_rn(v));

@@ -1082,6 +1082,7 @@ def test_head_segments_rotated(dtype, D, rot_off, rot, interleaved):
     ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
     bound = ulp * v.abs() + (D + 8) * 2.0 ** -24 * v.abs().amax()
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    bits = []
     for src_shift, w_shift, cs_shift in ((0, 0, 0), (0, 1, 0), (0, 0, 2), (1, 0, 0)):
         held = torch.zeros(src_shift + x.numel(), dtype=dtype, device=DEV)
         held[src_shift:] = x.flatten()
@@ -1095,6 +1096,8 @@ def test_head_segments_rotated(dtype, D, rot_off, rot, interleaved):
         torch.cuda.synchronize()
         assert rc == 0 and status.item() == 0
         assert ((out.double().cpu() - v).abs() <= bound).all(), (src_shift, w_shift, cs_shift)
+        bits += [out] if src_shift == 0 else []                                  # (rows off 16 bytes add their squares otherwise)
+    assert all(torch.equal(b, bits[0]) for b in bits)                            # whichever form turned them
 
 
 @pytest.mark.parametrize("page", [8, 16, 64, 192, 24])
