@@ -1246,3 +1246,41 @@ def test_gated_norm_adds_in_one_order(heads, v_dim, norm_groups, lens):
         assert rc == 0 and torch.isfinite(out).all()
         results.append((out, s))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+@pytest.mark.parametrize("size", [1, 100, 128, 2048, 2049, 2560, 5000])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_row_dot(dtype, size):
+    """A weight's product with each row: thread t of 128 adds elements t, t + 128, ... in turn, then the threads' sums meet
+    lane by lane, the farthest first, and warp by warp: that order's bits, whatever the alignment."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    fn = load_library("elementwise").kipp_row_dot
+    p, i, ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
+    fn.argtypes = [p, p, ll, i, p, i, i, p]
+    rows = 3
+    g = torch.Generator().manual_seed(size)
+    # 8-bit mantissas: products are exact in 32 bits, so an FMA is a rounded addition
+    x, w = torch.randn(rows, size, generator=g).bfloat16().float(), torch.randn(size, generator=g).bfloat16().float()
+    prod = torch.zeros(rows, -(-size // 128) * 128)
+    prod[:, :size] = x * w
+    acc = torch.zeros(rows, 128)
+    for part in prod.reshape(rows, -1, 128).unbind(1):
+        acc = acc + part
+
+    def lanes(v):                                                                # [..., 32]: the butterfly of a warp
+        for o in (16, 8, 4, 2, 1):
+            v = v[..., :o] + v[..., o:2 * o]
+        return v[..., 0]
+
+    warps = torch.zeros(rows, 32)
+    warps[:, :4] = lanes(acc.reshape(rows, 4, 32))
+    want = lanes(warps)
+    for shift in (0, 1):
+        held = torch.zeros(rows, size + 3, dtype=dtype, device=DEV)
+        held[:, shift:shift + size] = x
+        wd, out = torch.zeros(size + 1, device=DEV), torch.zeros(rows, device=DEV)
+        wd[shift:shift + size] = w
+        rc = fn(out.data_ptr(), held[:, shift:].data_ptr(), size + 3, 0 if dtype == torch.float32 else 1, wd[shift:].data_ptr(), rows, size,
+                torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and torch.equal(out.cpu(), want)
