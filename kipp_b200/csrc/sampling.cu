@@ -272,6 +272,12 @@ __device__ void select(RowCtx& c, Shared& sh, int mode, unsigned long long targe
                 unsigned long long all = 0;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) all += sh.units_all[8 * threadIdx.x + j];
+                // Below an infinite largest value every member weighs e^(inf - inf).  Its conversion to units gives 2^63 and
+                // sums are taken modulo 2^64: with an odd number of members a share of the total lies behind all of them,
+                // so that the last is taken; with an even number it is 0.
+                if (isinf(c.smax))
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) all += (unsigned long long)sh.cnt_all[8 * threadIdx.x + j] << 63;
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
                 const double sum = (double)all * WEIGHT_UNIT;

@@ -1284,3 +1284,28 @@ def test_row_dot(dtype, size):
         rc = fn(out.data_ptr(), held[:, shift:].data_ptr(), size + 3, 0 if dtype == torch.float32 else 1, wd[shift:].data_ptr(), rows, size,
                 torch.cuda.current_stream().cuda_stream)
         assert rc == 0 and torch.equal(out.cpu(), want)
+
+
+@pytest.mark.parametrize("vocab", [51, 700, 40001])
+def test_sample_rows_below_an_infinite_value(vocab):
+    """Under a largest value that is not finite every candidate weighs e^(inf - inf).  Such a total counts 2^63 units a
+    candidate modulo 2^64, so of an odd number of candidates the last is drawn and of an even number the first (the last
+    without a nucleus); the sums of a NaN's weight in a draw are none."""
+    from kipp_b200.kernels import sampling as ks
+    x = torch.randn(6, vocab, generator=torch.Generator().manual_seed(vocab)) * 2
+    x[0, 7] = x[1, 7] = x[1, 9] = x[2, 7] = x[2, 9] = x[2, 40] = math.inf
+    x[3] = -math.inf
+    x[4] = 3e38                                                                  # infinite once divided by the temperature
+    x[5, ::2] = math.nan
+    x[5, 1] = math.inf
+    first = {0: 7, 1: 7, 2: 7, 3: 0, 4: 0, 5: 1}
+    last = {0: 7, 1: 9, 2: 40, 3: vocab - 1, 4: vocab - 1, 5: 1}
+    odd = {0: True, 1: False, 2: True, 3: vocab % 2 == 1, 4: vocab % 2 == 1, 5: True}
+    t = lambda v, d: torch.full((6,), v, dtype=d, device=DEV)                     # noqa: E731
+    for top_p, min_p in ((0.9, 0.0), (0.3, 0.5), (1.0, 0.0)):
+        for u in (0.0, 0.4, 0.999):
+            got = ks.sample_rows(x.to(DEV), t(1e-3, torch.float32), t(0, torch.int32), t(top_p, torch.float32), t(min_p, torch.float32),
+                                 t(u, torch.float64)).tolist()
+            assert got == [last[r] if odd[r] or top_p == 1.0 else first[r] for r in range(6)], (top_p, u)
+    got = ks.sample_rows(x.to(DEV), t(1e-3, torch.float32), t(5, torch.int32), t(0.9, torch.float32), t(0.0, torch.float32), t(0.4, torch.float64))
+    assert got.tolist()[3:5] == [4, 4]                                           # five candidates are left
