@@ -915,10 +915,11 @@ ssd_scan_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* 
 // The gated delta rule: a thread owns 4 columns x R rows, as above.  The decayed state meets k; the four columns' sums
 // over P lanes meet with every exchange halving the columns a lane is responsible for, the lane that ends up with a
 // column forms its u = beta (v - S^T k), and three more exchanges hand the four u to everybody.  The sums with q travel
-// while the next token is worked on, and the token's own write joins the output as (q . k) u.
+// while the next token is worked on, and the token's own write joins the output as (q . k) u.  A column's sum: a thread's
+// pairs of rows by turns into two sums (no chain is longer than a quarter of the rows), then the lanes, the farthest first.
 // (With one column per thread, as below, a token costs ten shuffles and three 16-byte reads of shared memory for FOUR
 // elements of the state, and many blocks on an SM are bound by those: sequences of 1,277, 700 and 753 tokens, 16 heads:
-// 712 us so, 431 us here.)
+// 712 us so, 445 us here.)
 template <int P, int R, int WARPS, bool EXACT>
 __global__ void __launch_bounds__(32 * WARPS)
 gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* __restrict__ o_raw, int v_slices, int tokens) {
@@ -933,8 +934,9 @@ gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* 
     const int row0 = a.q_start[e], n_tok = a.q_start[e + 1] - row0;
     const int cl = tid / P * SCAN_COLS, col = slice * COLS + cl;
     const bool live = col < V;                                      // (V is a multiple of 4: a group is whole or absent)
-    const bool odd_lane = p & 1, second = p & 2;
-    const int mine = 2 * (p & 1) + (p >> 1 & 1);                    // the column whose sums end up in this lane
+    constexpr int FAR = P / 2, NEAR = P / 4;                        // the lanes of the first two exchanges
+    const bool high = p & FAR, second = p & NEAR;
+    const int mine = 2 * (high ? 1 : 0) + (second ? 1 : 0);         // the column whose sums end up in this lane
     float* S_slot = a.state + (size_t)a.slots[e] * (size_t)a.slot_stride + (size_t)h * D * V;
     const float* recs = vec + ((size_t)h * tokens + row0) * rec;
     auto fetch = [&](int t0, float* buf) {
@@ -981,12 +983,12 @@ gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* 
     };
     // the four columns' sums over the P lanes: each lane gets column `mine`
     auto meet = [&](const float (&o)[SCAN_COLS]) {
-        float k0 = odd_lane ? o[2] : o[0], k1 = odd_lane ? o[3] : o[1];
-        k0 += __shfl_xor_sync(0xffffffffu, odd_lane ? o[0] : o[2], 1);
-        k1 += __shfl_xor_sync(0xffffffffu, odd_lane ? o[1] : o[3], 1);
-        float y = (second ? k1 : k0) + __shfl_xor_sync(0xffffffffu, second ? k0 : k1, 2);
+        float k0 = high ? o[2] : o[0], k1 = high ? o[3] : o[1];
+        k0 += __shfl_xor_sync(0xffffffffu, high ? o[0] : o[2], FAR);
+        k1 += __shfl_xor_sync(0xffffffffu, high ? o[1] : o[3], FAR);
+        float y = (second ? k1 : k0) + __shfl_xor_sync(0xffffffffu, second ? k0 : k1, NEAR);
 #pragma unroll
-        for (int x = 4; x < P; x <<= 1) y += __shfl_xor_sync(0xffffffffu, y, x);
+        for (int x = NEAR / 2; x > 0; x >>= 1) y += __shfl_xor_sync(0xffffffffu, y, x);
         return y;
     };
     fetch(0, smem);
@@ -999,40 +1001,39 @@ gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* 
         __syncthreads();
         const float* toks = smem + (size_t)buf * tb.tokens * tb.floats;
         float* out = o_raw + (size_t)(row0 + t0) * (a.heads * V) + h * V + col + mine;
-        const bool writes = live && p < SCAN_COLS;
+        const bool writes = live && p % NEAR == 0;
         Token even, odd;
         float last[SCAN_COLS] = {0.f, 0.f, 0.f, 0.f}, last_qk = 0.f, last_u = 0.f;      // the token before: its sums with q, q . k, u
         // one token from `now`; `next` is fetched meanwhile (the last token of a batch fetches itself again)
         auto step = [&](int t, const Token& now, Token& next) {
-            float2 us[SCAN_COLS];
+            float2 us[2][SCAN_COLS];
 #pragma unroll
             for (int i = 0; i < R / 2; ++i)
 #pragma unroll
                 for (int c = 0; c < SCAN_COLS; ++c) {
                     S[i][c] = mul2(S[i][c], now.g[i]);
-                    us[c] = i == 0 ? mul2(now.k[i], S[i][c]) : fma2(now.k[i], S[i][c], us[c]);
+                    us[i & 1][c] = i < 2 ? mul2(now.k[i], S[i][c]) : fma2(now.k[i], S[i][c], us[i & 1][c]);
                 }
             float sum[SCAN_COLS];
 #pragma unroll
-            for (int c = 0; c < SCAN_COLS; ++c) sum[c] = us[c].x + us[c].y;
+            for (int c = 0; c < SCAN_COLS; ++c) sum[c] = (us[0][c].x + us[0][c].y) + (us[1][c].x + us[1][c].y);
             const float uy = meet(sum);
             const float y = fmaf(last_qk, last_u, meet(last));
             if (writes && t > 0) {
                 *out = y;
                 out += a.heads * V;
             }
-            float2 os[SCAN_COLS];
+            float2 os[2][SCAN_COLS];
 #pragma unroll
             for (int i = 0; i < R / 2; ++i)
 #pragma unroll
-                for (int c = 0; c < SCAN_COLS; ++c) os[c] = i == 0 ? mul2(now.q[i], S[i][c]) : fma2(now.q[i], S[i][c], os[c]);
+                for (int c = 0; c < SCAN_COLS; ++c) os[i & 1][c] = i < 2 ? mul2(now.q[i], S[i][c]) : fma2(now.q[i], S[i][c], os[i & 1][c]);
             take(toks + (size_t)min(t + 1, nb - 1) * tb.floats, next);
             const float u = now.beta * (now.v - uy);
-            const float over2 = __shfl_xor_sync(0xffffffffu, u, 2);
-            const float lo = second ? over2 : u, hi = second ? u : over2;                 // the pair of columns of this parity
-            const float lo1 = __shfl_xor_sync(0xffffffffu, lo, 1), hi1 = __shfl_xor_sync(0xffffffffu, hi, 1);
-            const float2 u2[SCAN_COLS] = {both(odd_lane ? lo1 : lo), both(odd_lane ? hi1 : hi), both(odd_lane ? lo : lo1),
-                                          both(odd_lane ? hi : hi1)};
+            const float over2 = __shfl_xor_sync(0xffffffffu, u, NEAR);
+            const float lo = second ? over2 : u, hi = second ? u : over2;                 // the pair of columns of this half
+            const float lo1 = __shfl_xor_sync(0xffffffffu, lo, FAR), hi1 = __shfl_xor_sync(0xffffffffu, hi, FAR);
+            const float2 u2[SCAN_COLS] = {both(high ? lo1 : lo), both(high ? hi1 : hi), both(high ? lo : lo1), both(high ? hi : hi1)};
 #pragma unroll
             for (int i = 0; i < R / 2; ++i)
 #pragma unroll
@@ -1040,7 +1041,7 @@ gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* 
             last_qk = now.qk;
             last_u = u;
 #pragma unroll
-            for (int c = 0; c < SCAN_COLS; ++c) last[c] = os[c].x + os[c].y;
+            for (int c = 0; c < SCAN_COLS; ++c) last[c] = (os[0][c].x + os[0][c].y) + (os[1][c].x + os[1][c].y);
         };
         take(toks, even);
         int t = 0;
@@ -1132,20 +1133,20 @@ gated_delta_column_kernel(const ScanArgs a, const float* __restrict__ vec, float
         Token even, odd;
         // one token from `now`; `next` is fetched meanwhile (the last token of a batch fetches itself again)
         auto step = [&](int t, const Token& now, Token& next) {
-            float2 us, os;
+            float2 us[2], os[2];
 #pragma unroll
             for (int i = 0; i < R / 2; ++i) {
                 S[i] = mul2(S[i], now.g[i]);
-                us = i == 0 ? mul2(now.k[i], S[i]) : fma2(now.k[i], S[i], us);
+                us[i & 1] = i < 2 ? mul2(now.k[i], S[i]) : fma2(now.k[i], S[i], us[i & 1]);
             }
-            float uy = us.x + us.y;
+            float uy = (us[0].x + us[0].y) + (us[1].x + us[1].y);
 #pragma unroll
-            for (int x = 1; x < P; x <<= 1) uy += __shfl_xor_sync(0xffffffffu, uy, x);
+            for (int x = P / 2; x > 0; x >>= 1) uy += __shfl_xor_sync(0xffffffffu, uy, x);
 #pragma unroll
-            for (int i = 0; i < R / 2; ++i) os = i == 0 ? mul2(now.q[i], S[i]) : fma2(now.q[i], S[i], os);
-            float oy = os.x + os.y;
+            for (int i = 0; i < R / 2; ++i) os[i & 1] = i < 2 ? mul2(now.q[i], S[i]) : fma2(now.q[i], S[i], os[i & 1]);
+            float oy = (os[0].x + os[0].y) + (os[1].x + os[1].y);
 #pragma unroll
-            for (int x = 1; x < P; x <<= 1) oy += __shfl_xor_sync(0xffffffffu, oy, x);
+            for (int x = P / 2; x > 0; x >>= 1) oy += __shfl_xor_sync(0xffffffffu, oy, x);
             take(toks + (size_t)min(t + 1, nb - 1) * tb.floats, next);
             const float u = now.beta * (now.v - uy);
             const float2 u2 = both(u);

@@ -1309,3 +1309,63 @@ def test_sample_rows_below_an_infinite_value(vocab):
             assert got == [last[r] if odd[r] or top_p == 1.0 else first[r] for r in range(6)], (top_p, u)
     got = ks.sample_rows(x.to(DEV), t(1e-3, torch.float32), t(5, torch.int32), t(0.9, torch.float32), t(0.0, torch.float32), t(0.4, torch.float64))
     assert got.tolist()[3:5] == [4, 4]                                           # five candidates are left
+
+
+@pytest.mark.parametrize("entries", [1, 400])
+@pytest.mark.parametrize("D,V", [(32, 32), (64, 20), (128, 64), (100, 36), (256, 32)])
+def test_gated_delta_scans_add_in_one_order(D, V, entries):
+    """The output's sum over the key rows, with a thread per column (few blocks) and four columns per thread (many): a thread's
+    pairs of neighbouring rows by turns into two sums, those, then the lanes, the farthest first.  With equal queries, no
+    decay and no write a column of the state that holds 2^30, 1 and -2^30 gives the query's value or 0, as the order
+    meets the three; float32 sums of the state in that order say which."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    lib = load_library("recurrent")
+    p, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+    lib.kipp_gated_delta_scan.argtypes = [p, ll, p, ll, i, i, i, p, i, p, ll, p, p, p, ll, i, p, p, ll, p, p, p, i, i, i, i, i, i, f, f, f, p, p, p]
+    lib.kipp_recurrent_scratch_floats.restype = lib.kipp_gated_delta_state_floats.restype = ll
+    heads, T = 2, 2 * entries
+    blocks = entries * heads * -(-V // 8)
+    assert blocks <= 64 or blocks > 148 * 14
+    g = torch.Generator().manual_seed(D + V)
+    state = torch.zeros(entries, heads, D, V)
+    rows = torch.stack([torch.randperm(D, generator=g)[:3] for _ in range(entries * heads * V)]).reshape(entries, heads, V, 3)
+    for n, value in enumerate((2.0 ** 30, 1.0, -2.0 ** 30)):
+        state.scatter_(2, rows[..., n][:, :, None, :], value)
+    P, R = (8, 4) if D <= 32 else (16, 4) if D <= 64 else (32, 4) if D <= 128 else (32, 8)
+    padded = torch.zeros(entries, heads, P * R, V)
+    padded[:, :, :D] = state
+    by_lane = padded.reshape(entries, heads, R // 4, P, 2, 2, V)                  # row 4 (lane + P q) + 2 pair + half
+    sums = [0.0, 0.0]
+    for q in range(R // 4):
+        for pair in range(2):
+            sums[pair] = by_lane[:, :, q, :, pair] + sums[pair]                   # [.., lane, half, V]
+    v = (sums[0][..., 0, :] + sums[0][..., 1, :]) + (sums[1][..., 0, :] + sums[1][..., 1, :])
+    while v.shape[2] > 1:
+        half = v.shape[2] // 2
+        v = v[:, :, :half] + v[:, :, half:]
+    want = v[:, :, 0]
+    assert (want == 0).any() and (want == 1).any()
+    channels = 2 * D + heads * V
+    ld = channels + heads + (-channels - heads) % 4
+    proj = torch.ones(T, ld, device=DEV)
+    proj[:, channels:] = -200.0                                                   # write rates of 0
+    ones = torch.ones(max(heads * D, channels, heads * V, V), device=DEV)
+    a_raw, a_log = torch.full((T, heads * D), -300.0, device=DEV), torch.zeros(heads, device=DEV)      # decays of 1
+    g_raw = torch.ones(T, heads * V, device=DEV)
+    q_start = torch.arange(entries + 1, dtype=torch.int32, device=DEV) * 2
+    entry = (torch.arange(T, device=DEV) // 2).int()
+    slots = torch.arange(entries, dtype=torch.int32, device=DEV)
+    S = state.reshape(entries, -1).to(DEV).clone()
+    assert S.shape[1] == lib.kipp_gated_delta_state_floats(heads, 1, D, V, 1)
+    scratch = torch.zeros(lib.kipp_recurrent_scratch_floats(T, heads, D, V, 5), device=DEV)
+    conv, out = torch.zeros(T, channels, device=DEV), torch.zeros(T, heads, V, device=DEV)
+    rc = lib.kipp_gated_delta_scan(out.data_ptr(), heads * V, proj.data_ptr(), ld, 0, 0, channels, ones.data_ptr(), 1, a_raw.data_ptr(),
+                                   heads * D, ones.data_ptr(), a_log.data_ptr(), g_raw.data_ptr(), heads * V, 1, ones.data_ptr(), S.data_ptr(),
+                                   S.shape[1], q_start.data_ptr(), entry.data_ptr(), slots.data_ptr(), entries, T, heads, 1, D, V, 1.0, 1e-12, 1.0,
+                                   scratch.data_ptr(), conv.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert rc == 0 and torch.equal(S.cpu(), state.reshape(entries, -1))
+    got = out.cpu().reshape(entries, 2, heads, V)
+    for t in range(2):
+        assert torch.equal(got[:, t] != 0, want != 0)
