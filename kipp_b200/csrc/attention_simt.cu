@@ -16,12 +16,13 @@
 // The tiles go through shared memory, the next one on its way while the present one is worked on: a
 // lane that walks its own key row in global memory waits a trip to the L2 for every few values, and every
 // head of a group fetched the same rows (four layers of 16 heads of 128 over prompts of 400 tokens and eight steps
-// of three tokens: 36 launches in 10.6 ms, 1.35 now; 1.63 while each 16 bytes copied looked its page up).  What bounds it
+// of three tokens: 36 launches in 10.6 ms, 1.35 with two stages, 1.63 while each 16 bytes copied looked its page up).  What bounds it
 // now is the chain of head_dim FMAs per key tile and the 32 weighted rows after it.
 //
 // A window of w (0 = none) lets position p see keys j with p - w < j <= p.
 #include "common.cuh"
 #include <math.h>
+#include <algorithm>
 
 namespace {
 constexpr int MAX_ACC = 8;         // head_dim <= 256
@@ -59,8 +60,8 @@ paged_attention_simt_kernel(T* __restrict__ out, const T* __restrict__ q,
                             const T* __restrict__ k_pages, const T* __restrict__ v_pages,
                             const int* __restrict__ positions, const int* __restrict__ entry_of_token,
                             const int* __restrict__ block_table, int table_width, int page_size,
-                            int n_q, int n_kv, int head_dim, float scale, int window, int* __restrict__ status) {
-    extern __shared__ __align__(16) uint8_t smem[];   // q [warps][head_dim padded], then two stages of a key and a value tile
+                            int n_q, int n_kv, int head_dim, float scale, int window, int stages, int* __restrict__ status) {
+    extern __shared__ __align__(16) uint8_t smem[];   // q [warps][head_dim padded], then the stages, a key and a value tile each
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -118,15 +119,17 @@ paged_attention_simt_kernel(T* __restrict__ out, const T* __restrict__ q,
     long long row_next = row_of(begin + lane);
     fetch(row_next, 0);
     int stage = 0;
-    for (int j0 = begin; j0 <= pos; j0 += TILE, stage ^= 1) {
+    for (int j0 = begin; j0 <= pos; j0 += TILE, stage ^= stages - 1) {
         const long long row = row_next;
-        if (j0 + TILE <= pos) {
-            row_next = row_of(j0 + TILE + lane);
-            fetch(row_next, stage ^ 1);
+        const bool more = j0 + TILE <= pos;
+        if (more) row_next = row_of(j0 + TILE + lane);
+        if (stages == 1) {
+            cp_async_wait<0>();
         } else {
-            cp_async_commit();
+            if (more) fetch(row_next, stage ^ 1);
+            else cp_async_commit();
+            cp_async_wait<1>();
         }
-        cp_async_wait<1>();
         __syncthreads();
         const uint8_t* kt = tiles + (size_t)stage * 2 * TILE * row_bytes;
         const uint8_t* vt = kt + (size_t)TILE * row_bytes;
@@ -166,6 +169,7 @@ paged_attention_simt_kernel(T* __restrict__ out, const T* __restrict__ q,
             }
         }
         __syncthreads();                              // the tile is read: its place may be filled again
+        if (stages == 1 && more) fetch(row_next, 0);
     }
     cp_async_wait<0>();
     if (!live) return;
@@ -178,6 +182,17 @@ paged_attention_simt_kernel(T* __restrict__ out, const T* __restrict__ q,
     }
 }
 
+constexpr int SM_SMEM = 227 * 1024, SM_THREADS = 2048, SM_BLOCKS = 32;         // what an SM has for blocks
+int sm_count() {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    }
+    return sms;
+}
+
 template <typename T, bool VEC, int NACC>
 int launch(void* out, const void* q, const void* k_pages, const void* v_pages, const int* positions,
            const int* entry_of_token, const int* block_table, int table_width, int page_size, int tokens, int n_q,
@@ -185,7 +200,14 @@ int launch(void* out, const void* q, const void* k_pages, const void* v_pages, c
     const int group = n_q / n_kv, warps = group < MAX_HEADS ? group : MAX_HEADS;
     const long long blocks = (long long)tokens * n_kv * ((group + warps - 1) / warps);
     if (blocks > 0x7fffffffLL) return KIPP_ERR_ARG;
-    const size_t smem = (size_t)warps * ((head_dim + 3) & ~3) * 4 + (size_t)4 * TILE * tile_row_bytes<T>(head_dim);
+    const size_t queries = (size_t)warps * ((head_dim + 3) & ~3) * 4, tiles = (size_t)2 * TILE * tile_row_bytes<T>(head_dim);
+    // Two stages where every block is on an SM at once even so, and a block's chain of tiles is what the launch lasts; else
+    // one, which makes room for more blocks (float32 heads of 256 that share no keys, 16 of them, 400 tokens: 2,749 us with one
+    // block an SM and two stages, 952 with three and one; with 3 tokens of 1,000 keys, four heads of 128 a group, 158 us with two
+    // stages and 166 with one).
+    const int sms = sm_count(), fit = std::min(SM_SMEM / (int)(queries + 2 * tiles + 1024), SM_THREADS / (32 * warps));
+    const int stages = blocks <= (long long)sms * std::min(fit, SM_BLOCKS) ? 2 : 1;
+    const size_t smem = queries + stages * tiles;
     static size_t allowed = 48 * 1024;
     if (smem > allowed) {
         const cudaError_t e = cudaFuncSetAttribute(paged_attention_simt_kernel<T, VEC, NACC>,
@@ -195,7 +217,7 @@ int launch(void* out, const void* q, const void* k_pages, const void* v_pages, c
     }
     return kipp_launch(paged_attention_simt_kernel<T, VEC, NACC>, dim3((unsigned)blocks), dim3(warps * 32), smem, s, 1,
                        (T*)out, (const T*)q, (const T*)k_pages, (const T*)v_pages, positions, entry_of_token, block_table,
-                       table_width, page_size, n_q, n_kv, head_dim, scale, window, status);
+                       table_width, page_size, n_q, n_kv, head_dim, scale, window, stages, status);
 }
 
 template <typename T, typename... Args>
