@@ -857,15 +857,15 @@ public:
                           const float* conv_w, int taps, const float* a_raw, long long ld_a, const float* dt_bias,
                           const float* a_log, const float* g_raw, long long ld_g, int gate, const float* norm_w, float* state,
                           long long slot_stride, const int* q_start, const int* entry_of_token, const int* slots, int entries,
-                          int tokens, int heads, int kv_heads, int dim, int v_dim, float q_scale, float eps, float out_scale) {
+                          int tokens, int longest, int heads, int kv_heads, int dim, int v_dim, float q_scale, float eps, float out_scale) {
         using Fn = int (*)(void*, long long, const void*, long long, int, int, int, const float*, int, const float*, long long,
                            const float*, const float*, const float*, long long, int, const float*, float*, long long, const int*,
-                           const int*, const int*, int, int, int, int, int, int, float, float, float, float*, float*, void*);
+                           const int*, const int*, int, int, int, int, int, int, int, float, float, float, float*, float*, void*);
         static Fn f = kernel_symbol<Fn>("recurrent", "kipp_gated_delta_scan");
         float* scratch = recurrent_scratch(tokens, heads, dim, v_dim, 5);
         float* conv_out = workspace->get<float>("gated_delta_conv", (size_t)tokens * (2 * (size_t)kv_heads * dim + (size_t)heads * v_dim));
         run(f(out, ld_out, proj, ld_proj, dtype, qkv_off, b_off, conv_w, taps, a_raw, ld_a, dt_bias, a_log, g_raw, ld_g, gate, norm_w,
-              state, slot_stride, q_start, entry_of_token, slots, entries, tokens, heads, kv_heads, dim, v_dim, q_scale, eps, out_scale,
+              state, slot_stride, q_start, entry_of_token, slots, entries, tokens, longest, heads, kv_heads, dim, v_dim, q_scale, eps, out_scale,
               scratch, conv_out, stream),
             "gated_delta_scan", tokens == entries ? 1 : taps > 1 ? 5 : 4);
     }

@@ -931,9 +931,10 @@ public:
                  EPI_STORE);
         void* gated = ctx.workspace->buffer("gated_delta_out", (size_t)T * vv_ld_ * es);
         if (vv_ld_ != vv_) cuda_check(cudaMemsetAsync(gated, 0, (size_t)T * vv_ld_ * es, ctx.stream), "clearing the padding");
+        const int longest = m.shape.q_lens.empty() ? 0 : *std::max_element(m.shape.q_lens.begin(), m.shape.q_lens.end());
         ops.gated_delta_scan(gated, vv_ld_, proj, ld_, ctx.dtype, 0, b_off_, conv_, taps_, a_raw, heads_ * dim_, dt_bias_, a_log_, g_raw,
-                             vv_, gate_, norm_, state, state_floats(), m.q_start, m.entry_of_token, m.slots, m.shape.entries, T, heads_,
-                             kv_heads_, dim_, v_dim_, q_scale_, eps_, out_scale_);
+                             vv_, gate_, norm_, state, state_floats(), m.q_start, m.entry_of_token, m.slots, m.shape.entries, T, longest,
+                             heads_, kv_heads_, dim_, v_dim_, q_scale_, eps_, out_scale_);
         output_product(ctx, residual, gated, vv_ld_, w_o_, vv_ld_, dtype_, hidden_, vv_ld_);
     }
 

@@ -89,6 +89,7 @@ struct ScanArgs {
     float* state;                          // [slots, heads, dim, v_dim]
     const int* q_start; const int* slots;
     int heads, dim, v_dim, batch, entries;
+    int longest;                           // gated delta: the most tokens that an entry brings (0: not known)
     float k_scale, eps, out_scale;
     int gate;                              // 0 none, 1 silu, 2 sigmoid
     // gated memory: columns of the two gates in proj, their biases [heads], the cap, the scale of q
@@ -1063,8 +1064,8 @@ gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* 
 }
 
 // The same with one column per thread, the same sums in the same order: more blocks, whose tokens wait for a shorter chain
-// (five exchanges instead of seven, a quarter of the arithmetic).  For grids that leave no SM more than one of its
-// blocks (see launch_gated_delta_scan): 8 heads of 128 x 128, one sequence of 2,048 tokens: 0.19 us a token against 0.27.
+// (five exchanges instead of seven, a quarter of the arithmetic).  For grids that leave an SM few of its
+// warps (see launch_gated_delta_scan): 8 heads of 128 x 128, one sequence of 2,048 tokens: 0.19 us a token against 0.27.
 template <int P, int R, int WARPS, bool EXACT>
 __global__ void __launch_bounds__(32 * WARPS)
 gated_delta_column_kernel(const ScanArgs a, const float* __restrict__ vec, float* __restrict__ o_raw, int v_slices, int tokens) {
@@ -1295,9 +1296,13 @@ int launch_ssd_scan(const ScanArgs& a, const float* conv, const float2* dts, flo
                        dim3((unsigned)(entries * a.heads * slices)), dim3(32 * WARPS), (size_t)2 * tb.tokens * tb.floats * sizeof(float),
                        stream, a, conv, dts, o_raw, slices);
 }
-// 16 columns a block, or, where its blocks of 8 columns are no more than the SMs, a thread per column (measured with layers
-// of 128 x 128, the whole layer: one sequence of 2,048 tokens, 8 heads: 478 us against 623; 16 heads, 256 blocks: 697
-// against 661; four sequences of 511, 16 heads: 581 against 356).  The bits are the same.
+// 16 columns a block, or a thread per column where that leaves an SM at most COLUMN_WARPS warps: below, a token's chain is what
+// the scan lasts, above the SMs' issue slots are.  The warps are those that work for as long as the longest entry, tokens /
+// longest entries of them (an SM soon has only the long ones left).  Measured over heads of 32 to 256 x 32 to 128, 4 to 32 of
+// them, and up to eight entries of equal and unequal lengths, the layer: 7 warps (8 heads of 128 x 128, one entry of 400) 114 us
+// a column and 149 four; 14 warps (16 heads) 153 and 153; 28 warps (32 heads) 263 and 184; with entries of 300, 1 and 77 tokens
+// 16 heads of 64 x 64, 4 warps, 89 and 116.  The form chosen is within 6 % of the better one everywhere.  The bits are the same.
+constexpr double COLUMN_WARPS = 12.0;
 template <int P, int R>
 int launch_gated_delta_scan(const ScanArgs& a, const float* vec, float* o_raw, int entries, int tokens, cudaStream_t stream) {
     static int sms = 0;
@@ -1308,7 +1313,8 @@ int launch_gated_delta_scan(const ScanArgs& a, const float* vec, float* o_raw, i
     }
     constexpr int CHAINS = P / 4, CHAIN_COLS = 32 * CHAINS / P;
     const int chain_slices = (a.v_dim + CHAIN_COLS - 1) / CHAIN_COLS;
-    if ((long long)entries * a.heads * chain_slices <= sms) {
+    const double at_work = a.longest > 0 ? (double)tokens / a.longest : entries;
+    if (at_work * a.heads * chain_slices * CHAINS <= COLUMN_WARPS * sms) {
         const TokenBatch tb = token_batch(3 * a.dim + 4 + CHAIN_COLS);
         return launch_walk(a, tokens, a.dim == P * R ? gated_delta_column_kernel<P, R, CHAINS, true> : gated_delta_column_kernel<P, R, CHAINS, false>,
                            dim3((unsigned)(entries * a.heads * chain_slices)), dim3(32 * CHAINS),
@@ -1863,13 +1869,14 @@ extern "C" long long kipp_gated_delta_state_floats(int heads, int kv_heads, int 
 // [taps, channels] (the last tap meets the current token); a_raw [T, heads * dim] and g_raw [T, heads * v_dim]
 // float32 are the pre-activations of the decay and of the output's gate (1 silu, 2 sigmoid); dt_bias [heads * dim],
 // a_log [heads], norm_w [v_dim] float32.  A slot is kipp_gated_delta_state_floats floats.  conv_out: float32
-// [tokens, channels] of scratch.  At most 16 taps.
+// [tokens, channels] of scratch.  At most 16 taps.  longest: the most tokens that an entry brings, or 0; it
+// chooses between two forms with the same bits.
 extern "C" int kipp_gated_delta_scan(void* out, long long ld_out, const void* proj, long long ld_proj, int dtype, int qkv_off,
                                      int b_off, const float* conv_w, int taps, const float* a_raw, long long ld_a,
                                      const float* dt_bias, const float* a_log, const float* g_raw, long long ld_g, int gate,
                                      const float* norm_w, float* state, long long slot_stride, const int* q_start,
-                                     const int* entry_of_token, const int* slots, int entries, int tokens, int heads, int kv_heads,
-                                     int dim, int v_dim, float q_scale, float eps, float out_scale, float* scratch, float* conv_out,
+                                     const int* entry_of_token, const int* slots, int entries, int tokens, int longest, int heads,
+                                     int kv_heads, int dim, int v_dim, float q_scale, float eps, float out_scale, float* scratch, float* conv_out,
                                      void* stream) {
     if (entries <= 0 || tokens <= 0) return 0;
     if (!kipp_recurrent_scan_ok(dim, v_dim, GATED_DELTA) || heads <= 0 || kv_heads <= 0 || heads % kv_heads || taps < 1 ||
@@ -1880,6 +1887,7 @@ extern "C" int kipp_gated_delta_scan(void* out, long long ld_out, const void* pr
     ScanArgs a = {};
     a.out = out; a.ld_out = ld_out; a.proj = proj; a.ld_proj = ld_proj;
     a.xbc_off = qkv_off; a.b_off = b_off; a.conv_w = conv_w; a.taps = taps; a.groups = kv_heads;
+    a.longest = longest;
     a.a_raw = a_raw; a.ld_a = ld_a; a.dt_bias = dt_bias; a.a_log = a_log; a.g_raw = g_raw; a.ld_g = ld_g; a.gate = gate; a.norm_w = norm_w;
     a.state = state; a.slot_stride = slot_stride; a.q_start = q_start; a.entry_of_token = entry_of_token; a.slots = slots;
     a.heads = heads; a.dim = dim; a.v_dim = v_dim; a.q_scale = q_scale; a.eps = eps; a.k_scale = 1.f; a.out_scale = out_scale;

@@ -1333,10 +1333,11 @@ def test_sample_rows_below_an_infinite_value(vocab):
     assert got.tolist()[3:5] == [4, 4]                                           # five candidates are left
 
 
-@pytest.mark.parametrize("entries", [1, 400])
+@pytest.mark.parametrize("entries,longest", [(1, 0), (400, 0), (400, 2), (400, 800)])
 @pytest.mark.parametrize("D,V", [(32, 32), (64, 20), (128, 64), (100, 36), (256, 32)])
-def test_gated_delta_scans_add_in_one_order(D, V, entries):
-    """The output's sum over the key rows, with a thread per column (few blocks) and four columns per thread (many): a thread's
+def test_gated_delta_scans_add_in_one_order(D, V, entries, longest):
+    """The output's sum over the key rows, with a thread per column (few warps at work, or said to
+    be few by the longest entry's length) and four columns per thread (many): a thread's
     pairs of neighbouring rows by turns into two sums, those, then the lanes, the farthest first.  With equal queries, no
     decay and no write a column of the state that holds 2^30, 1 and -2^30 gives the query's value or 0, as the order
     meets the three; float32 sums of the state in that order say which."""
@@ -1344,11 +1345,11 @@ def test_gated_delta_scans_add_in_one_order(D, V, entries):
     from kipp_b200.csrc.build import load_library
     lib = load_library("recurrent")
     p, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
-    lib.kipp_gated_delta_scan.argtypes = [p, ll, p, ll, i, i, i, p, i, p, ll, p, p, p, ll, i, p, p, ll, p, p, p, i, i, i, i, i, i, f, f, f, p, p, p]
+    lib.kipp_gated_delta_scan.argtypes = [p, ll, p, ll, i, i, i, p, i, p, ll, p, p, p, ll, i, p, p, ll, p, p, p, i, i, i, i, i, i, i, f, f, f, p, p, p]
     lib.kipp_recurrent_scratch_floats.restype = lib.kipp_gated_delta_state_floats.restype = ll
     heads, T = 2, 2 * entries
     blocks = entries * heads * -(-V // 8)
-    assert blocks <= 64 or blocks > 148 * 14
+    assert blocks <= 64 or 2 * blocks > 148 * 12
     g = torch.Generator().manual_seed(D + V)
     state = torch.zeros(entries, heads, D, V)
     rows = torch.stack([torch.randperm(D, generator=g)[:3] for _ in range(entries * heads * V)]).reshape(entries, heads, V, 3)
@@ -1384,8 +1385,8 @@ def test_gated_delta_scans_add_in_one_order(D, V, entries):
     conv, out = torch.zeros(T, channels, device=DEV), torch.zeros(T, heads, V, device=DEV)
     rc = lib.kipp_gated_delta_scan(out.data_ptr(), heads * V, proj.data_ptr(), ld, 0, 0, channels, ones.data_ptr(), 1, a_raw.data_ptr(),
                                    heads * D, ones.data_ptr(), a_log.data_ptr(), g_raw.data_ptr(), heads * V, 1, ones.data_ptr(), S.data_ptr(),
-                                   S.shape[1], q_start.data_ptr(), entry.data_ptr(), slots.data_ptr(), entries, T, heads, 1, D, V, 1.0, 1e-12, 1.0,
-                                   scratch.data_ptr(), conv.data_ptr(), torch.cuda.current_stream().cuda_stream)
+                                   S.shape[1], q_start.data_ptr(), entry.data_ptr(), slots.data_ptr(), entries, T, longest, heads, 1, D, V, 1.0, 1e-12,
+                                   1.0, scratch.data_ptr(), conv.data_ptr(), torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     assert rc == 0 and torch.equal(S.cpu(), state.reshape(entries, -1))
     got = out.cpu().reshape(entries, 2, heads, V)
