@@ -70,7 +70,8 @@ __global__ void __launch_bounds__(128)
 head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
     pdl_launch_dependents();
     // (positions and the block table come with the step's lists, which a copy brought before any kernel of the step
-    // started: a head's place is looked up before the wait, and its weights are asked for)
+    // started: a head's place is looked up before the wait, and its weights are asked for.  Warps with nothing to write wait
+    // too: a launch of nothing else must not end, and let the kernel after it go on, before the one in front of it has.)
     const int lane = threadIdx.x & 31;
     const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wg >= (long long)a.tokens * a.total_heads) return;
@@ -87,10 +88,11 @@ head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
     if (g.target == 0) {
         dst = static_cast<T*>(g.dst) + (size_t)t * g.ld_dst + g.dst_off + (size_t)hh * g.dst_stride;
     } else {
-        if (!(a.write_cache & 1)) return;
+        if (!(a.write_cache & 1)) { pdl_wait(); return; }
         const int pos = a.positions[t], slot = pos / a.page_size;
         const int page = slot < a.table_width ? a.block_table[(size_t)a.entry_of_token[t] * a.table_width + slot] : -1;
         if (page < 0) {                       // unmapped page: refuse, never write
+            pdl_wait();
             if (lane == 0) atomicExch(status, 2);
             return;
         }
