@@ -335,8 +335,8 @@ attention_mix_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __re
 // The runs of a token merged in run order: o = sum_r acc_r e^(m_r - M) / sum_r l_r e^(m_r - M).  A block
 // takes MERGE_HEADS heads of a token: a warp per head forms the runs' weights once, then every
 // thread sums its elements over the runs.  What such a launch lasts is its trips to the L2, one after the other: so the
-// token's position comes before the dependency wait (it lies in the step's lists, which a copy brought before any kernel
-// of the step started), and a thread's first values, MERGE_AHEAD runs of them, are on their way beside the maxima and
+// token's position comes before the dependency wait (it is one of the step's lists, see pdl_wait()), and a thread's
+// first values, MERGE_AHEAD runs of them, are on their way beside the maxima and
 // sums (with the position behind the wait, maxima, sums and values in turn, and the values of fewer than eight runs
 // one by one: 8.5 us a launch at one token of 300 keys, 5.1 so).
 constexpr int MERGE_HEADS = 2, MERGE_AHEAD = 8;
@@ -977,7 +977,7 @@ attention_shared_key_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, 
     int* pg = reinterpret_cast<int*>(raw + L.pg);
     const int ldq = L.ldq, lds = L.lds, ldp = L.ldp;
     pdl_launch_dependents();
-    // (positions and tables come with the step's lists, which a copy brought before any kernel of the step started)
+    // (positions and tables are the step's lists, see pdl_wait())
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int gid = lane >> 2, tig = lane & 3;
     const int t = blockIdx.x, h0 = blockIdx.y * SK_ROWS;

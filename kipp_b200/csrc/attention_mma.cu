@@ -606,9 +606,8 @@ __global__ void __launch_bounds__(THREADS)
 attn_decode_kernel(const DecodeParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_launch_dependents();
-    // (What is read before the dependency wait comes with the step's lists, which a
-    // copy brought before any kernel of the step started, or lies in the cache since
-    // earlier steps.)
+    // (What is read before the dependency wait are the step's lists, see pdl_wait(), or lies in the
+    // cache since earlier steps.)
     // Grid (kv heads, tokens, splits): the splits are the slowest dimension, so the CTAs
     // that have work come first in launch order and all start at once; those of
     // splits a step does not use come after and leave at once.  (With the splits as
@@ -898,13 +897,12 @@ extern "C" int kipp_attn_decode_mma(void* out, const void* q, const void* k_page
 // context (so a token's result does not depend on its neighbours); else, for the whole step,
 // the number of 64-key tiles per split k with the least (waves of resident CTAs) x (k + a CTA's
 // fixed cost in tiles), on a tie the fewer splits.  One block; used between the steps of a
-// burst that runs without the host.
+// burst that runs without the host; lets nothing start before it has ended (see common.cuh).
 namespace {
 struct SplitRule { int pairs_per_entry, resident_ctas, fixed_tiles, max_splits, own_length; };
 __global__ void attn_decode_replan_kernel(int* split_keys, const int* context_len, const int* rows, int n,
                                           SplitRule rule) {
     __shared__ int shared_s;
-    pdl_launch_dependents();
     pdl_wait();
     if (threadIdx.x == 0) shared_s = 0;
     __syncthreads();

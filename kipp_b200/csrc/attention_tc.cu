@@ -331,14 +331,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     // A kernel that follows may take tensor memory while it waits for this grid, so where a CTA needs all of its
     // SM's it lets the next kernel's blocks start only once it has it (below).
     if constexpr (C::CTAS > 1) pdl_launch_dependents();
-    // (What is read before the dependency wait below comes with the step's lists, which a
-    // copy brought before any kernel of the step started: the loads, three in a row, run
-    // while the barriers and the tensor memory are set up.)
+    // (What is read before the dependency wait below are the step's lists, see pdl_wait(): the loads,
+    // three in a row, run while the barriers and the tensor memory are set up.)
     // Grid (heads, tiles), the last tile of the list first: within an entry the later
     // tiles see more keys, and the long ones should not be the last to start; the
     // heads of a tile, which share its keys and values, start together.
-    // (The X form also runs inside bursts of decoded steps, whose lengths a kernel of the same
-    // graph moves on: it waits first.)
+    // (The X form also reads lists that a kernel of the step makes, see kipp_latent_expand: it waits first.)
     if constexpr (X) pdl_wait();
     const int item = gridDim.y - 1 - blockIdx.y;
     const int entry = p.work[2 * item], tile_tok = p.work[2 * item + 1];
@@ -745,8 +743,8 @@ latent_expand_tc_kernel(const __grid_constant__ CUtensorMap map_pages, const __g
                         const __grid_constant__ CUtensorMap map_wv, const ExpandArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // (lists first: a burst's steps move them on.  The tensor memory is asked for after the wait too, when no earlier
-    // kernel holds any, and the next kernel is let in once this CTA has it: nobody waits for one who waits.)
+    // (The tensor memory is asked for after the wait, when no earlier kernel holds any, and the next kernel is let in
+    // once this CTA has it: nobody waits for one who waits.)
     pdl_wait();
     const int e = blockIdx.z, t0 = blockIdx.y * X_TOK;
     const int ft = (int)blockIdx.x - 1;                                // (the copy first: it is one block's work)

@@ -92,7 +92,13 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // tail.  The rule every kernel keeps: call pdl_wait() before the first access
 // to global memory that an earlier kernel may have written or may still read;
 // only set-up that touches nothing of the sort (barrier init, tensor-memory
-// allocation, loads of weights) may come before it.
+// allocation, loads of weights) may come before it.  Every grid has a block that waits, so
+// that a kernel which has ended has seen the ones before it end.
+// The step's lists (tokens, positions, entries, lengths, block tables, work lists) may be read
+// before it too: they change between two steps only, by the copy that brings a step's lists, which every kernel of the
+// step comes after, or, in a burst that runs without the host, by kernels at the end of a
+// step (kipp_burst_advance, kipp_attn_decode_replan).  Those do not let the kernel behind them start early, so that
+// whatever follows, in the same graph or another, finds the lists as they left them.
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

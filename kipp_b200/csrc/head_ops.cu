@@ -69,9 +69,9 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 head_segments_kernel(const SegmentArgs a, int* __restrict__ status) {
     pdl_launch_dependents();
-    // (positions and the block table come with the step's lists, which a copy brought before any kernel of the step
-    // started: a head's place is looked up before the wait, and its weights are asked for.  Warps with nothing to write wait
-    // too: a launch of nothing else must not end, and let the kernel after it go on, before the one in front of it has.)
+    // (positions and the block table are the step's lists, see pdl_wait(): a head's place is looked up before the wait, and
+    // its weights are asked for.  Warps with nothing to write wait too: a launch of nothing else must not end, and let the
+    // kernel after it go on, before the one in front of it has.)
     const int lane = threadIdx.x & 31;
     const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wg >= (long long)a.tokens * a.total_heads) return;

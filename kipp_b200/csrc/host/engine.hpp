@@ -1018,7 +1018,8 @@ inline Engine::StepGraph& Engine::graph_for(const std::string& key, bool feedbac
 }
 
 // argmax of the step's logits -> next tokens, ring row, positions + 1, then what each mixer's
-// kernels derive from the lengths.
+// kernels derive from the lengths.  The kernels that move the step's lists on come last, and none that
+// follows starts before they have ended: others read the lists before they wait (common.cuh).
 inline void Engine::feedback_tail(StepGraph& g) {
     const int n = g.meta.shape.entries;
     ops_.argmax_rows(g.logits, plan_->vocab_size, n, plan_->vocab_size, g.next_tokens.as<int>());

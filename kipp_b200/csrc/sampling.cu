@@ -603,11 +603,11 @@ __global__ void apply_penalties_kernel(float* __restrict__ logits, long long ld,
 // tokens and go into row `*counter` of the ring; every request moves on by one
 // position.  What a mixer's kernels derive from the lengths (the keys per split of
 // the decode attention) is made anew by that mixer's own kernel after this one.
-// One block.
+// One block.  What follows may read the lists before its dependency wait (see common.cuh), so this kernel lets
+// nothing start before it has ended.
 namespace {
 __global__ void burst_advance_kernel(int* tokens, int* positions, int* context_len, const int* next, int* ring,
                                      int* counter, int n, int ring_rows) {
-    pdl_launch_dependents();
     pdl_wait();                                      // the tokens are chosen, every kernel of the step is through
     const int c = *counter;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
