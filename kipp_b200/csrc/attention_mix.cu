@@ -406,12 +406,7 @@ int launch_merge(void* out, const float* partial, const int* positions, int toke
                  int keep_first, int runs, float out_scale, const MixExtras& ex, cudaStream_t s) {
     const size_t smem = ((size_t)MERGE_HEADS * (v_dim + runs + 1) + 3) * sizeof(float);
     auto merge = attention_mix_merge_kernel<T>;
-    static size_t allowed = 0;
-    if (smem > 48 * 1024 && smem > allowed) {
-        cudaError_t e = cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
-        allowed = smem;
-    }
+    if (const int e = kipp_allow_smem(merge, smem)) return e;
     const dim3 grid((unsigned)tokens, (unsigned)((n_q + MERGE_HEADS - 1) / MERGE_HEADS));
     return kipp_launch(merge, grid, dim3(THREADS), smem, s, 1, (T*)out, partial, positions, n_q, v_dim, window, keep_first,
                        runs, out_scale, ex);
@@ -435,12 +430,7 @@ int launch_mix(void* out, const void* q, const void* k_pages, const void* v_page
     if (smem > 200 * 1024) return KIPP_ERR_ARG;
     if (ex.values_in_keys && kv_stage < n_kv) return KIPP_ERR_ARG;     // the keys of a tile must still be there
     auto kernel = attention_mix_kernel<T>;
-    static size_t allowed = 0;
-    if (smem > 48 * 1024 && smem > allowed) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
-        allowed = smem;
-    }
+    if (const int e = kipp_allow_smem(kernel, smem)) return e;
     const int split = runs > 1 ? 1 : 0;
     int rc = kipp_launch(kernel, dim3((unsigned)tokens, (unsigned)(split ? runs : 1)), dim3(THREADS), smem, s, 1, (T*)out,
                          (const T*)q, (const T*)k_pages, (const T*)v_pages, head_mix, positions, entry_of_token,
@@ -831,12 +821,7 @@ attention_mix_mma_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, con
 template <int HPW, int VB, typename... Args>
 int launch_mix_mma(size_t smem, int items, int head_blocks, cudaStream_t s, Args... args) {
     auto kernel = attention_mix_mma_kernel<HPW, VB>;
-    static size_t allowed = 0;
-    if (smem > 48 * 1024 && smem > allowed) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
-        allowed = smem;
-    }
+    if (const int e = kipp_allow_smem(kernel, smem)) return e;
     return kipp_launch(kernel, dim3((unsigned)items, (unsigned)head_blocks), dim3(MMA_THREADS), smem, s, 1, args...);
 }
 
@@ -1105,12 +1090,7 @@ int launch_shared_key(void* out, const void* q, const void* k_pages, const int* 
     const int stages = (long long)grid.x * grid.y * grid.z <= 2 * 148 && SharedKeySmem(head_dim, 2).bytes <= SK_SMEM_MAX ? 2 : 1;
     const size_t smem = SharedKeySmem(head_dim, stages).bytes;
     auto kernel = attention_shared_key_kernel<VB>;
-    static size_t allowed = 0;
-    if (smem > 48 * 1024 && smem > allowed) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
-        allowed = smem;
-    }
+    if (const int e = kipp_allow_smem(kernel, smem)) return e;
     int rc = kipp_launch(kernel, grid, dim3(SK_THREADS), smem, s, 1, (bf16*)out, (const bf16*)q, (const bf16*)k_pages,
                          positions, entry_of_token, block_table, table_width, page_size, n_q, head_dim, v_dim, scale,
                          window, out_scale, split, stages, partial, status, ex);
@@ -1294,12 +1274,7 @@ int launch_group(void* out, const void* q, const void* k_pages, const void* v_pa
                  int* status, const MixExtras& ex, cudaStream_t s) {
     const size_t smem = GroupSmem(head_dim, v_dim).bytes;
     auto kernel = attention_group_kernel<VB>;
-    static size_t allowed = 0;
-    if (smem > 48 * 1024 && smem > allowed) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
-        allowed = smem;
-    }
+    if (const int e = kipp_allow_smem(kernel, smem)) return e;
     const int split = runs > 1 ? 1 : 0, per_kv = (n_q / n_kv + SK_ROWS - 1) / SK_ROWS;
     const dim3 grid((unsigned)tokens, (unsigned)(n_kv * per_kv), (unsigned)(split ? runs : 1));
     int rc = kipp_launch(kernel, grid, dim3(SK_THREADS), smem, s, 1, (bf16*)out, (const bf16*)q, (const bf16*)k_pages,

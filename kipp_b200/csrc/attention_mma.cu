@@ -784,12 +784,7 @@ attn_decode_merge_kernel(bf16* __restrict__ out, const float* __restrict__ part_
 
 template <int D> int launch_prefill(const PrefillParams& p, int items, cudaStream_t s) {
     constexpr int SMEM = 4 * TILE_KEYS * D * 2;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(attn_prefill_kernel<D>, SMEM)) return e;
     return kipp_launch(attn_prefill_kernel<D>, dim3(items, p.n_q), dim3(THREADS), SMEM, s, 1, p);
 }
 
@@ -803,19 +798,9 @@ template <int D> int launch_decode(const DecodeParams& p, int n, cudaStream_t s)
     constexpr int PIPE = 2 * DECODE_STAGES * TILE_KEYS * D * 2 + 16 * D * 2;   // tiles, and the group's queries
     constexpr int MERGE = (2 * WARPS * 16 + WARPS * 16 * (D + 8)) * 4;
     constexpr int SMEM = PIPE > MERGE ? PIPE : MERGE;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(attn_decode_kernel<D>, SMEM)) return e;
     if (p.n_splits_out != nullptr) {
-        static bool configured_stream = false;
-        if (!configured_stream) {
-            cudaError_t e = cudaFuncSetAttribute(attn_decode_stream_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-            if (e != cudaSuccess) return (int)e;
-            configured_stream = true;
-        }
+        if (const int e = kipp_allow_smem(attn_decode_stream_kernel<D>, SMEM)) return e;
         return kipp_launch(attn_decode_stream_kernel<D>, dim3(p.stream_ctas), dim3(THREADS), SMEM, s, 1, p, n);
     }
     if (n > 65535) return KIPP_ERR_ARG;

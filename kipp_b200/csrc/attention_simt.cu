@@ -208,13 +208,7 @@ int launch(void* out, const void* q, const void* k_pages, const void* v_pages, c
     const int sms = sm_count(), fit = std::min(SM_SMEM / (int)(queries + 2 * tiles + 1024), SM_THREADS / (32 * warps));
     const int stages = blocks <= (long long)sms * std::min(fit, SM_BLOCKS) ? 2 : 1;
     const size_t smem = queries + stages * tiles;
-    static size_t allowed = 48 * 1024;
-    if (smem > allowed) {
-        const cudaError_t e = cudaFuncSetAttribute(paged_attention_simt_kernel<T, VEC, NACC>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        allowed = smem;
-    }
+    if (const int e = kipp_allow_smem(paged_attention_simt_kernel<T, VEC, NACC>, smem)) return e;
     return kipp_launch(paged_attention_simt_kernel<T, VEC, NACC>, dim3((unsigned)blocks), dim3(warps * 32), smem, s, 1,
                        (T*)out, (const T*)q, (const T*)k_pages, (const T*)v_pages, positions, entry_of_token, block_table,
                        table_width, page_size, n_q, n_kv, head_dim, scale, window, stages, status);

@@ -988,13 +988,7 @@ int query_map(CUtensorMap* out, const void* ptr, int tokens, int n_q, int head_d
 template <int D, int DV, bool X> int launch(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mk4, const CUtensorMap& mv4,
                             const CUtensorMap& mq, const CUtensorMap& mo, const Params& p, int items, cudaStream_t s) {
     using C = Cfg<D, DV>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<D, DV, X>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)C::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(attn_prefill_tc_kernel<D, DV, X>, C::SMEM)) return e;
     return kipp_launch(attn_prefill_tc_kernel<D, DV, X>, dim3(p.n_q, items), dim3(THREADS), C::SMEM, s, 1, mk, mv, mk4, mv4, mq, mo, p);
 }
 }  // namespace
@@ -1146,12 +1140,7 @@ extern "C" int kipp_latent_expand_tc(const void* pages, int n_pages, const int* 
     if (rc == 0) rc = pool_map(&mk, w_k, (long long)heads * dim, rank, X_FEAT);
     if (rc == 0) rc = pool_map(&mv, w_v, (long long)heads * v_dim, rank, X_FEAT);
     if (rc) return rc;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err = cudaFuncSetAttribute(latent_expand_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)X_SMEM);
-        if (err != cudaSuccess) { cudaGetLastError(); return (int)err; }
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(latent_expand_tc_kernel, X_SMEM)) return e;
     const int tiles = (pages_per_entry * X_PAGE + X_TOK - 1) / X_TOK;
     if (tiles > 65535) return KIPP_ERR_ARG;
     return kipp_launch(latent_expand_tc_kernel, dim3((unsigned)(a.k_tiles + a.v_tiles + 1), (unsigned)tiles, (unsigned)entries),

@@ -7,6 +7,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "launch_limits.cuh"
 
 #define KIPP_ERR_ARG (-1)        // a size the kernel refuses
 #define KIPP_ERR_DTYPE (-2)      // unknown dtype code
@@ -133,6 +134,23 @@ static inline bool kipp_pdl_enabled() {
         cached = (e != nullptr && e[0] == '0') ? 0 : 1;
     }
     return cached == 1;
+}
+
+// Lets the current device launch `kernel` with `bytes` of dynamic shared memory (SmemLimits).
+static inline int kipp_allow_smem_of(const void* kernel, size_t bytes) {
+    if (bytes <= SmemLimits::WITHOUT_ASKING) return 0;
+    static SmemLimits limits;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return (int)e;
+    return limits.raise(device, kernel, bytes, [&](size_t most) {
+        const cudaError_t rc = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (rc != cudaSuccess) cudaGetLastError();
+        return (int)rc;
+    });
+}
+template <typename... KArgs> static inline int kipp_allow_smem(void (*kernel)(KArgs...), size_t bytes) {
+    return kipp_allow_smem_of(reinterpret_cast<const void*>(kernel), bytes);
 }
 
 // Launches `kernel` with the package's attributes; a cluster of more than one

@@ -914,7 +914,7 @@ extern "C" int kipp_hyper_connection(float* x, long long stride, int streams, fl
     const int wide = std::min(streams <= 4 ? 512 : 256, std::max(64, (size / per + 31) / 32 * 32));
     const dim3 grid((unsigned)rows), block((unsigned)(rows >= 1024 ? std::min(128, wide) : wide));
     auto go = [&](auto kernel) {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (const int e = kipp_allow_smem(kernel, smem)) return e;
         return kipp_launch(kernel, grid, block, smem, (cudaStream_t)stream, 1, a);
     };
     const bool f32 = h == nullptr || h_dtype == KIPP_DT_F32;

@@ -419,12 +419,7 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
 template <int MT, int EPI, bool PAIR>
 int launch_few_form(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
     using F = Few<PAIR>;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_few_kernel<MT, EPI, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(gemm_few_kernel<MT, EPI, PAIR>, F::SMEM)) return e;
     return kipp_launch(gemm_few_kernel<MT, EPI, PAIR>, dim3((N + F::F - 1) / F::F, (M + MT - 1) / MT), dim3(FEW_THREADS),
                        F::SMEM, s, 1, C, A, W, M, N, K, lda, ldw, ldc);
 }
@@ -451,12 +446,7 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, in
     const int groups = (K + GROUP_RUNS * run_length(K) - 1) / (GROUP_RUNS * run_length(K));
     const dim3 grid((N + TILE_F - 1) / TILE_F, (M + TILE_T - 1) / TILE_T, groups);
     if (grid.y > 65535) return KIPP_ERR_ARG;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_tile_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(gemm_tile_kernel<EPI>, TILE_SMEM)) return e;
     return kipp_launch(gemm_tile_kernel<EPI>, grid, dim3(TILE_THREADS), TILE_SMEM, s, groups, C, A, W, M, N, K, lda, ldw, ldc);
 }
 

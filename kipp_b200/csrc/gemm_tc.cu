@@ -1417,13 +1417,7 @@ int make_map(CUtensorMap* out, const void* ptr, int rows, int cols, long long ld
 template <int TILE_T, int TILE_F>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, dim3 grid, cudaStream_t s) {
     using C = Cfg<TILE_T, TILE_F>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<TILE_T, TILE_F>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(gemm_tc_kernel<TILE_T, TILE_F>, C::SMEM)) return e;
     return kipp_launch(gemm_tc_kernel<TILE_T, TILE_F>, grid, dim3(THREADS), C::SMEM, s, p.splits, mw, mx, p);
 }
 
@@ -1441,13 +1435,7 @@ template <int TILE_N, bool REDUCE>
 int launch_tokm(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, const Params& p, int total,
                 cudaStream_t s) {
     using C = CfgTok<TILE_N, REDUCE>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_tokm_kernel<TILE_N, REDUCE>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(gemm_tc_tokm_kernel<TILE_N, REDUCE>, C::SMEM)) return e;
     // persistent: at most one CTA per SM
     const int sms = sm_count();
     return kipp_launch(gemm_tc_tokm_kernel<TILE_N, REDUCE>, dim3(total < sms ? total : sms), dim3(THREADS), C::SMEM,
@@ -1470,13 +1458,7 @@ template <int TILE_N, bool REDUCE, bool HEADS = false>
 int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, const Params& p, int total,
                 cudaStream_t s) {
     using C = CfgPair<TILE_N, REDUCE>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<TILE_N, REDUCE, HEADS>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(gemm_tc_pair_kernel<TILE_N, REDUCE, HEADS>, C::SMEM)) return e;
     // persistent: at most one pair of CTAs per pair of SMs
     const int pairs = sm_count() / 2;
     // the two CTAs of an MMA pair are neighbours along x

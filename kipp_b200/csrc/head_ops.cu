@@ -717,12 +717,7 @@ extern "C" int kipp_latent_expand(const void* pages, const int* block_table, int
     a.k_out = (bf16*)k_out; a.v_out = (bf16*)v_out; a.table_out = table_out; a.pages_per_entry = pages_per_entry; a.status = status;
     a.k_tiles = (heads * dim + EN - 1) / EN;
     a.v_tiles = (heads * v_dim + EN - 1) / EN;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(latent_expand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)E_SMEM);
-        if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
-        configured = true;
-    }
+    if (const int e = kipp_allow_smem(latent_expand_kernel, E_SMEM)) return e;
     const int tiles = (pages_per_entry * E_PAGE + EM - 1) / EM;
     if (tiles > 65535) return KIPP_ERR_ARG;
     return kipp_launch(latent_expand_kernel, dim3((unsigned)(a.k_tiles + a.v_tiles + 1), (unsigned)tiles, (unsigned)entries),

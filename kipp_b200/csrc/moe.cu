@@ -412,29 +412,17 @@ static int moe_route_any(int* expert_of, float* weight_of, const void* h, long l
     const int warps = tok == 4 ? 8 : experts > 32 ? 32 : experts < 4 ? 4 : experts;
     const dim3 grid((unsigned)((tokens + tok - 1) / tok)), block((unsigned)(32 * warps));
     const size_t scores = (size_t)(by_scores ? 2 : 1) * tok * experts * sizeof(float), smem = scores + (size_t)tok * top * sizeof(float);
-    if (smem > 48 * 1024 && scores <= 48 * 1024) {
-        // (the chosen weights must not be what a size fails for)
-        const void* kernels[] = {(const void*)moe_route_kernel<float, 1>, (const void*)moe_route_kernel<float, 4>,
-                                 (const void*)moe_route_kernel<bf16, 1>, (const void*)moe_route_kernel<bf16, 4>};
-        for (const void* k : kernels) {
-            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-        }
-    }
-    if (dtype == KIPP_DT_F32) {
-        if (tok == 4)
-            return kipp_launch(moe_route_kernel<float, 4>, grid, block, smem, s, 1, expert_of, weight_of, (const float*)h,
-                               ldh, router, bias, tokens, hidden, experts, top, vec, by_scores, renormalize, real_experts, weight_scale);
-        return kipp_launch(moe_route_kernel<float, 1>, grid, block, smem, s, 1, expert_of, weight_of, (const float*)h, ldh,
-                           router, bias, tokens, hidden, experts, top, vec, by_scores, renormalize, real_experts, weight_scale);
-    }
-    if (dtype == KIPP_DT_BF16) {
-        if (tok == 4)
-            return kipp_launch(moe_route_kernel<bf16, 4>, grid, block, smem, s, 1, expert_of, weight_of, (const bf16*)h, ldh,
-                               router, bias, tokens, hidden, experts, top, vec, by_scores, renormalize, real_experts, weight_scale);
-        return kipp_launch(moe_route_kernel<bf16, 1>, grid, block, smem, s, 1, expert_of, weight_of, (const bf16*)h, ldh,
-                           router, bias, tokens, hidden, experts, top, vec, by_scores, renormalize, real_experts, weight_scale);
-    }
+    auto go = [&](auto kernel, auto rows) {
+        // (the chosen weights must not be what a size fails for, and what is too large without them is refused as it was)
+        if (scores > SmemLimits::WITHOUT_ASKING) return (int)cudaErrorInvalidValue;
+        if (const int e = kipp_allow_smem(kernel, smem)) return e;
+        return kipp_launch(kernel, grid, block, smem, s, 1, expert_of, weight_of, rows, ldh, router, bias, tokens, hidden, experts, top, vec,
+                           by_scores, renormalize, real_experts, weight_scale);
+    };
+    if (dtype == KIPP_DT_F32)
+        return tok == 4 ? go(moe_route_kernel<float, 4>, (const float*)h) : go(moe_route_kernel<float, 1>, (const float*)h);
+    if (dtype == KIPP_DT_BF16)
+        return tok == 4 ? go(moe_route_kernel<bf16, 4>, (const bf16*)h) : go(moe_route_kernel<bf16, 1>, (const bf16*)h);
     return KIPP_ERR_DTYPE;
 }
 extern "C" int kipp_moe_route(int* expert_of, float* weight_of, const void* h, long long ldh, int dtype, const float* router,
