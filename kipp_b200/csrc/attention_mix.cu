@@ -1087,7 +1087,7 @@ int launch_shared_key(void* out, const void* q, const void* k_pages, const int* 
     // Two stages of keys, the next tile on its way, where no more than two blocks an SM are there anyway (of 576 columns two
     // stages leave room for two, one for four): one token of 300 keys, 16 heads: 12.5 us a launch, 15.2 with a tile's page, keys
     // and products one after the other.
-    const int stages = (long long)grid.x * grid.y * grid.z <= 2 * 148 && SharedKeySmem(head_dim, 2).bytes <= SK_SMEM_MAX ? 2 : 1;
+    const int stages = (long long)grid.x * grid.y * grid.z <= 2 * kipp_sm_count() && SharedKeySmem(head_dim, 2).bytes <= SK_SMEM_MAX ? 2 : 1;
     const size_t smem = SharedKeySmem(head_dim, stages).bytes;
     auto kernel = attention_shared_key_kernel<VB>;
     if (const int e = kipp_allow_smem(kernel, smem)) return e;

@@ -183,15 +183,6 @@ paged_attention_simt_kernel(T* __restrict__ out, const T* __restrict__ q,
 }
 
 constexpr int SM_SMEM = 227 * 1024, SM_THREADS = 2048, SM_BLOCKS = 32;         // what an SM has for blocks
-int sm_count() {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    }
-    return sms;
-}
 
 template <typename T, bool VEC, int NACC>
 int launch(void* out, const void* q, const void* k_pages, const void* v_pages, const int* positions,
@@ -205,7 +196,7 @@ int launch(void* out, const void* q, const void* k_pages, const void* v_pages, c
     // one, which makes room for more blocks (float32 heads of 256 that share no keys, 16 of them, 400 tokens: 2,749 us with one
     // block an SM and two stages, 952 with three and one; with 3 tokens of 1,000 keys, four heads of 128 a group, 158 us with two
     // stages and 166 with one).
-    const int sms = sm_count(), fit = std::min(SM_SMEM / (int)(queries + 2 * tiles + 1024), SM_THREADS / (32 * warps));
+    const int sms = kipp_sm_count(), fit = std::min(SM_SMEM / (int)(queries + 2 * tiles + 1024), SM_THREADS / (32 * warps));
     const int stages = blocks <= (long long)sms * std::min(fit, SM_BLOCKS) ? 2 : 1;
     const size_t smem = queries + stages * tiles;
     if (const int e = kipp_allow_smem(paged_attention_simt_kernel<T, VEC, NACC>, smem)) return e;

@@ -136,6 +136,16 @@ static inline bool kipp_pdl_enabled() {
     return cached == 1;
 }
 
+// SMs of the current device (the devices of a process are alike).
+static inline int kipp_sm_count() {
+    static const int sms = [] {
+        int n = 0, device = 0;
+        cudaGetDevice(&device);
+        return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 148;
+    }();
+    return sms;
+}
+
 // Lets the current device launch `kernel` with `bytes` of dynamic shared memory (SmemLimits).
 static inline int kipp_allow_smem_of(const void* kernel, size_t bytes) {
     if (bytes <= SmemLimits::WITHOUT_ASKING) return 0;

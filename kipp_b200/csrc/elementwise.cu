@@ -76,7 +76,7 @@ __global__ void rmsnorm_kernel(TO* __restrict__ out, const float* __restrict__ x
 // while the present one is summed; the deferred form's row leaves before its sum is there.
 // (The deferred form one after another on one stream, against a row per block and the weights after the sum: 2,048 rows of
 // 2,560 6.15 -> 5.4 us, 407 rows 3.6 -> 2.1, 64 rows 1.97 -> 1.5, one row 1.84 -> 1.33.)
-constexpr int NORM_BLOCKS = 4 * 148;             // four blocks of 256 threads and about 60 registers on each SM
+constexpr int NORM_BLOCKS = 4;                   // of 256 threads and about 60 registers on each SM
 template <typename TO>
 __global__ void __launch_bounds__(256, 4)
 rmsnorm_vec_kernel(TO* __restrict__ out, const float* __restrict__ x, const void* __restrict__ w, int w_dtype,
@@ -145,11 +145,12 @@ static int rmsnorm_launch(void* out, int out_dtype, const float* x, const void* 
     if (w_dtype != KIPP_DT_F32 && w_dtype != KIPP_DT_BF16) return KIPP_ERR_DTYPE;
     cudaStream_t s = (cudaStream_t)stream;
     if (size % 4 == 0 && size <= 4096 && size >= 256 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)out & 15) == 0) {
+        const int blocks = std::min(n_rows, NORM_BLOCKS * kipp_sm_count());
         if (out_dtype == KIPP_DT_F32)
-            return kipp_launch(rmsnorm_vec_kernel<float>, dim3(n_rows < NORM_BLOCKS ? n_rows : NORM_BLOCKS), dim3(256), 0, s, 1,
+            return kipp_launch(rmsnorm_vec_kernel<float>, dim3(blocks), dim3(256), 0, s, 1,
                                (float*)out, x, w, w_dtype, rows, n_rows, size, eps, ssq_out);
         if (out_dtype == KIPP_DT_BF16)
-            return kipp_launch(rmsnorm_vec_kernel<bf16>, dim3(n_rows < NORM_BLOCKS ? n_rows : NORM_BLOCKS), dim3(256), 0, s, 1,
+            return kipp_launch(rmsnorm_vec_kernel<bf16>, dim3(blocks), dim3(256), 0, s, 1,
                                (bf16*)out, x, w, w_dtype, rows, n_rows, size, eps, ssq_out);
         return KIPP_ERR_DTYPE;
     }

@@ -13,23 +13,27 @@
 // many threads at once, the groups of four what lets a small product of many tokens be shared by more blocks.
 //
 // Three kernels, chosen by shape and alignment alone, with that one order for 32-bit weights whose rows start on 16 bytes:
-//   few   float32, up to FEW_MAX tokens (16 of many features): bound by the weights' bytes (a token is 2 operations per 4 bytes).  A
-//         block holds 16 features, a thread one feature and one run, so a 2,048-feature matrix still
-//         gives 128 blocks of 256 chains; the weights travel by asynchronous copies, five chunks of 64 bytes
-//         per thread on their way, the first of them before the wait for the kernel before.  12,288 x 2,048 with
-//         1, 3 and 16 tokens: 24, 28 and 95 us (100 MB: 15 us of copy rate; the kernel below, which ran before: 334, 339
-//         and 353); 2,048 x 6,144 with 3: 24 us (543).  From 17 tokens on it needs two passes, which still win where the
-//         features are few (32 tokens, 2,048 and 3,072 x 2,048: 31 and 48 us against 58 and 74 in tiles) and lose where
-//         they are many (12,288 and 32,000: 180 and 442 us against 104 and 260): from MANY_F on those are tiles'.
-//   tile  float32, more tokens: bound by the FMA pipes.  128 features x 64 tokens per block of 128 threads, 8 x 8 per
-//         thread in float32 pairs, operands in shared memory with k outermost, so that a k's 16 values cost a
-//         thread four 16-byte reads (with four bytes copied at a time: 24 copies per 1,024 FMAs); the groups of runs
-//         are blocks of their own, a cluster that meets in its shared memory.
+//   few   float32, up to FEW_MAX tokens (16 of many features): bound by the weights' bytes (a token is 2 operations per 4
+//         bytes).  A block holds 16 features, a thread one feature and one run, so a 2,048-feature matrix still gives 128
+//         blocks of 256 chains; the weights travel by asynchronous copies, four chunks of 64 bytes per thread on their way
+//         (three of two features where a thread has pairs), the first of them before the wait for the kernel before.
+//         12,288 x 2,048 with 1, 3 and 16 tokens: 24, 28 and 95 us (100 MB: 15 us of copy rate; the kernel below, which ran
+//         before: 334, 339 and 353); 2,048 x 6,144 with 3: 24 us (543).  From 17 tokens on it needs two passes, which still
+//         win where the features are few (32 tokens, 2,048 and 3,072 x 2,048: 31 and 48 us against 58 and 74 in tiles) and
+//         lose where they are many (12,288 and 32,000: 180 and 442 us against 104 and 260): from many_features() on those
+//         are tiles'.
+//   tile  float32, more tokens: bound by warps in flight.  At 407 tokens, 12,288 x 2,048 (608 us, 34 of 74 TFLOP/s) the FMA
+//         pipes are busy 57 % of the time and shared memory's data pipe 62 %; the three blocks of four warps that registers
+//         and shared memory leave an SM give a scheduler 2.8 warps, and one of them can issue in 46 % of the cycles.
+//         128 features x 64 tokens per block of 128 threads, 8 x 8 per thread in float32 pairs, operands in shared memory
+//         with k outermost, so that a k's 16 values cost a thread four 16-byte reads (with four bytes copied at a time: 24
+//         copies per 1,024 FMAs); the groups of runs are blocks of their own, a cluster that meets in its shared memory.
 //         407 tokens, 12,288 x 2,048: 608 us (943 before), 2,048 x 6,144: 392 us (866; 540 with
 //         tiles of 64 x 64, 8 x 4 per thread and k innermost); 64 tokens, 12,288 x 2,048: 106 us (387; 181).
 //   any   what is left: tokens whose float32 rows do not start on 16 bytes, in the order above; and what no other kernel
-//         here takes, bfloat16 operands of shapes that the tensor-core kernels refuse and float32 weights off 16 bytes: one chain of FMAs in the order of k, without the 38 registers and the extra sums of the runs (bfloat16, 2,050
-//         features of 2,056: 1 and 200 tokens 154 and 152 us, 186 and 180 in runs).
+//         here takes, bfloat16 operands of shapes that the tensor-core kernels refuse and float32 weights off 16 bytes: one
+//         chain of FMAs in the order of k, without the 38 registers and the extra sums of the runs (bfloat16, 2,050 features
+//         of 2,056: 1 and 200 tokens 154 and 152 us, 186 and 180 in runs).
 //
 // Epilogues:
 //   STORE   C[m,n]    = acc                 (C in float32 or bfloat16)
@@ -151,7 +155,8 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
 // features; a warp copies only what its own lanes read, so its ring needs no block-wide barrier.
 // PAIR: a thread has two features (f and f + 16 of the block's 32), so that a token's values, which every lane of a
 // run reads, serve both: of several tokens those reads are what an SM is busy with.
-constexpr int FEW_F = 16, FEW_THREADS = 16 * MAX_RUNS, FEW_MAX = 32, MANY_F = 64 * 148;
+constexpr int FEW_F = 16, FEW_THREADS = 16 * MAX_RUNS, FEW_MAX = 32;
+inline int many_features() { return 64 * kipp_sm_count(); }         // two blocks of pairs of features for each SM
 constexpr int FEW_CHUNK = BK * 4 + 16;              // 64 bytes of a feature's row, padded against bank conflicts
 template <bool PAIR> struct Few {
     static constexpr int PER = PAIR ? 2 : 1, F = FEW_F * PER, STAGES = PAIR ? 4 : 5, CHUNKS = 32 * PER;
@@ -428,14 +433,14 @@ int launch_few(float* C, const float* A, const float* W, int M, int N, int K, in
     // pairs of features where they still make two blocks for each SM (12,288 x 2,048 with 3 and 8 tokens: 28.3 and 37.9 us,
     // one feature per thread 32.9 and 47.2; 32,000: 59 and 88 against 78 and 106)
     constexpr bool MAY_PAIR = MT >= 2 && MT <= 8;
-    if (MAY_PAIR && N >= MANY_F) return launch_few_form<MT, EPI, MAY_PAIR>(C, A, W, M, N, K, lda, ldw, ldc, s);
+    if (MAY_PAIR && N >= many_features()) return launch_few_form<MT, EPI, MAY_PAIR>(C, A, W, M, N, K, lda, ldw, ldc, s);
     return launch_few_form<MT, EPI, false>(C, A, W, M, N, K, lda, ldw, ldc, s);
 }
 
 // float32 rows that start on 16 bytes and hold whole groups of four: the kernels that copy 16 bytes at a time.
 template <int EPI>
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
-    if (M <= (N >= MANY_F ? FEW_MAX / 2 : FEW_MAX)) {
+    if (M <= (N >= many_features() ? FEW_MAX / 2 : FEW_MAX)) {
         // tokens of a block: as many as there are, up to 16 (the accumulators of a thread)
         if (M == 1) return launch_few<1, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
         if (M == 2) return launch_few<2, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);

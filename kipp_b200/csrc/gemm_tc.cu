@@ -1421,23 +1421,13 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, dim3 g
     return kipp_launch(gemm_tc_kernel<TILE_T, TILE_F>, grid, dim3(THREADS), C::SMEM, s, p.splits, mw, mx, p);
 }
 
-int sm_count() {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    }
-    return sms;
-}
-
 template <int TILE_N, bool REDUCE>
 int launch_tokm(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, const Params& p, int total,
                 cudaStream_t s) {
     using C = CfgTok<TILE_N, REDUCE>;
     if (const int e = kipp_allow_smem(gemm_tc_tokm_kernel<TILE_N, REDUCE>, C::SMEM)) return e;
     // persistent: at most one CTA per SM
-    const int sms = sm_count();
+    const int sms = kipp_sm_count();
     return kipp_launch(gemm_tc_tokm_kernel<TILE_N, REDUCE>, dim3(total < sms ? total : sms), dim3(THREADS), C::SMEM,
                        s, 1, mw, mx, mc, p);
 }
@@ -1460,7 +1450,7 @@ int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap&
     using C = CfgPair<TILE_N, REDUCE>;
     if (const int e = kipp_allow_smem(gemm_tc_pair_kernel<TILE_N, REDUCE, HEADS>, C::SMEM)) return e;
     // persistent: at most one pair of CTAs per pair of SMs
-    const int pairs = sm_count() / 2;
+    const int pairs = kipp_sm_count() / 2;
     // the two CTAs of an MMA pair are neighbours along x
     return kipp_launch_cluster(gemm_tc_pair_kernel<TILE_N, REDUCE, HEADS>, dim3(2 * (total < pairs ? total : pairs)),
                                dim3(THREADS), C::SMEM, s, dim3(2, 1, 1), mw, mx, mc, p);
@@ -1489,7 +1479,7 @@ int launch_pair_n(int tile_n, const CUtensorMap& mw, const CUtensorMap& mx, cons
 // Tiles wider than 256 (pairs only) have one accumulator, so their epilogue is not hidden
 // behind the next tile's MMAs: they are taken only where they make the whole product one round.
 int pick_tile_n(int tokens, int features, bool pair = false, long long* cost_out = nullptr) {
-    const int units = pair ? sm_count() / 2 : sm_count();
+    const int units = pair ? kipp_sm_count() / 2 : kipp_sm_count();
     const int rows = pair ? 2 * UMMA_M : UMMA_M;
     const int m_tiles = (tokens + rows - 1) / rows;
     int best = 256;
@@ -1685,7 +1675,7 @@ int gemm_tc_run(void* C, int out_dtype, const void* X, const void* W, int tokens
     if (splits == 0 && want_tile == 0 && want_tile_f == 0 && tokens > 32 && tokens < 512 && epilogue != EPI_ADD) {
         const int n = pick_tile_n(tokens, features, false);
         const long long tiles = (long long)((tokens + UMMA_M - 1) / UMMA_M) * ((features + n - 1) / n);
-        mid_fills = 4 * tiles >= 3LL * sm_count();
+        mid_fills = 4 * tiles >= 3LL * kipp_sm_count();
     }
     if ((want_tile == 0 && want_tile_f == 0 && tokens >= 512 && c_map_ok) || want_tile_f < 0 || mid_fills) {
         const bool reduce = epilogue == EPI_ADD && c_map_ok;     // else a thread per token adds in place

@@ -1305,16 +1305,10 @@ int launch_ssd_scan(const ScanArgs& a, const float* conv, const float2* dts, flo
 constexpr double COLUMN_WARPS = 12.0;
 template <int P, int R>
 int launch_gated_delta_scan(const ScanArgs& a, const float* vec, float* o_raw, int entries, int tokens, cudaStream_t stream) {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    }
     constexpr int CHAINS = P / 4, CHAIN_COLS = 32 * CHAINS / P;
     const int chain_slices = (a.v_dim + CHAIN_COLS - 1) / CHAIN_COLS;
     const double at_work = a.longest > 0 ? (double)tokens / a.longest : entries;
-    if (at_work * a.heads * chain_slices * CHAINS <= COLUMN_WARPS * sms) {
+    if (at_work * a.heads * chain_slices * CHAINS <= COLUMN_WARPS * kipp_sm_count()) {
         const TokenBatch tb = token_batch(3 * a.dim + 4 + CHAIN_COLS);
         return launch_walk(a, tokens, a.dim == P * R ? gated_delta_column_kernel<P, R, CHAINS, true> : gated_delta_column_kernel<P, R, CHAINS, false>,
                            dim3((unsigned)(entries * a.heads * chain_slices)), dim3(32 * CHAINS),

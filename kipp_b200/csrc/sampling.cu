@@ -115,12 +115,10 @@ struct Shared {
     double total;
     float red_val[32];
     int red_idx[32];
-    double red_d[32];
-    unsigned long long red_u[32];
     // results broadcast
     unsigned sel_digit; unsigned long long sel_cnt_before; double sel_w_before;
     unsigned sel_bucket_cnt; int found;
-    int i_val; float f_val; double d_val; unsigned long long u_val;
+    int i_val; float f_val; double d_val;
 };
 
 enum { MODE_COUNT = 0, MODE_W_GE = 1, MODE_W_GT = 2 };
@@ -666,14 +664,8 @@ extern "C" int kipp_sample_rows(const float* logits, long long ld, int rows, int
     if (n <= 0) return KIPP_ERR_ARG;
     // long rows: a cluster of up to eight blocks a row (at most eight: the kernel's loops over the
     // team are unrolled to that), as many as keep all rows' blocks within one wave of the GPU
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    }
     int blocks = 1;
-    while (blocks < 8 && n >= 16384 * blocks && (long long)rows * blocks * 2 <= sms) blocks *= 2;
+    while (blocks < 8 && n >= 16384 * blocks && (long long)rows * blocks * 2 <= kipp_sm_count()) blocks *= 2;
     if ((long long)rows * blocks > 0x7fffffffLL) return KIPP_ERR_ARG;
     return kipp_launch_cluster(sample_rows_kernel, dim3((unsigned)(rows * blocks)), dim3(THREADS), 0, (cudaStream_t)stream,
                                dim3(blocks, 1, 1), logits, ld, n, temperature, top_k, top_p, min_p, uniform, out);
