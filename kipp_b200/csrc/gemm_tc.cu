@@ -314,22 +314,24 @@ struct Params {
     const float* glu_row_gate;
 };
 
-// A token's sum of squares out of its partial sums, in slot order (see Params::ssq_in).  Forty values are on their way
-// at a time: with the compiler's four or eight, the 80 slots of a 2,560-wide row were 10 to 20 trips to the L2, which
-// stood before the cluster's reduction of a few-token product and behind the last tile of a prompt's.
+// A token's sum of squares out of its partial sums, in slot order (see Params::ssq_in).  SSQ_AHEAD values are on their way
+// at a time, zeros past the last: with the compiler's four or eight, the 64 to 128 slots of rows of 2,048 to 4,096 values were 8 to
+// 32 trips to the L2, which stood before the cluster's reduction of a few-token product and behind the last tile of a
+// prompt's.  (With 40 and with 48 at a time, steps of 1, 13 and 64 tokens and a prompt of 2,048 take the same within 1 %.)
+constexpr int SSQ_AHEAD = 32;
 __device__ __forceinline__ float token_ssq(const Params& p, int t) {
     const float* row = p.ssq_in + (size_t)t * p.ssq_in_slots;
     const int n = p.ssq_in_slots;
     float sum = 0.f;
     int i = 0;
     if ((n & 3) == 0 && ((uintptr_t)p.ssq_in & 15) == 0) {
-        constexpr int AT_ONCE = 10;
-        for (; i + 4 * AT_ONCE <= n; i += 4 * AT_ONCE) {
-            float4 v[AT_ONCE];
+        for (; i < n; i += SSQ_AHEAD) {
+            float4 v[SSQ_AHEAD / 4];
 #pragma unroll
-            for (int j = 0; j < AT_ONCE; ++j) v[j] = *reinterpret_cast<const float4*>(row + i + 4 * j);
+            for (int j = 0; j < SSQ_AHEAD / 4; ++j)
+                v[j] = i + 4 * j < n ? *reinterpret_cast<const float4*>(row + i + 4 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int j = 0; j < AT_ONCE; ++j) sum = sum + v[j].x + v[j].y + v[j].z + v[j].w;
+            for (int j = 0; j < SSQ_AHEAD / 4; ++j) sum = sum + v[j].x + v[j].y + v[j].z + v[j].w;
         }
     }
 #pragma unroll 8
