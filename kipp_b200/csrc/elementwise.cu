@@ -76,17 +76,19 @@ __global__ void rmsnorm_kernel(TO* __restrict__ out, const float* __restrict__ x
 // while the present one is summed; the deferred form's row leaves before its sum is there.
 // (The deferred form one after another on one stream, against a row per block and the weights after the sum: 2,048 rows of
 // 2,560 6.15 -> 5.4 us, 407 rows 3.6 -> 2.1, 64 rows 1.97 -> 1.5, one row 1.84 -> 1.33.)
-constexpr int NORM_BLOCKS = 4;                   // of 256 threads and about 60 registers on each SM
-template <typename TO>
-__global__ void __launch_bounds__(256, 4)
+constexpr int NORM_BLOCKS = 4, NORM_BLOCKS_NARROW = 8;      // of 256 threads on each SM, with about 60 and 30 registers
+// PIECES: float4 pieces of a row per thread.  (Rows of at most one, with the registers for four: 2,048 rows of 256 5.9 us, 4.9 so;
+// a block for each of them was slower still.)  The squares' roundings are spelled out: both forms give the same bits.
+template <typename TO, int PIECES>
+__global__ void __launch_bounds__(256, PIECES == 1 ? NORM_BLOCKS_NARROW : NORM_BLOCKS)
 rmsnorm_vec_kernel(TO* __restrict__ out, const float* __restrict__ x, const void* __restrict__ w, int w_dtype,
                    const int* __restrict__ rows, int n_rows, int size, float eps, float* __restrict__ ssq_out) {
     __shared__ float scratch[32];
     pdl_launch_dependents();
     const int n4 = size >> 2;
-    float4 weight[4], v[4];
+    float4 weight[PIECES], v[PIECES];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < PIECES; ++j) {
         const int i = threadIdx.x + 256 * j;
         if (i < n4) {
             const size_t e = (size_t)i * 4;
@@ -94,20 +96,20 @@ rmsnorm_vec_kernel(TO* __restrict__ out, const float* __restrict__ x, const void
         }
     }
     pdl_wait();
-    auto fetch = [&](int r, float4 (&to)[4]) {
+    auto fetch = [&](int r, float4 (&to)[PIECES]) {
         const float4* src = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[r] : r) * size);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < PIECES; ++j)
             if (threadIdx.x + 256 * j < n4) to[j] = src[threadIdx.x + 256 * j];
     };
     fetch(blockIdx.x, v);
     for (int r = blockIdx.x; r < n_rows; r += gridDim.x) {
-        float4 next[4];
+        float4 next[PIECES];
         if (r + gridDim.x < n_rows) fetch(r + gridDim.x, next);
         TO* dst = out + (size_t)r * size;
         auto put = [&](float scale) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < PIECES; ++j) {
                 const int i = threadIdx.x + 256 * j;
                 if (i < n4) {
                     const size_t e = (size_t)i * 4;
@@ -128,13 +130,13 @@ rmsnorm_vec_kernel(TO* __restrict__ out, const float* __restrict__ x, const void
         if (ssq_out != nullptr) put(1.0f);
         float ss = 0.f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (threadIdx.x + 256 * j < n4) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+        for (int j = 0; j < PIECES; ++j)
+            if (threadIdx.x + 256 * j < n4) ss += fmaf(v[j].w, v[j].w, fmaf(v[j].z, v[j].z, fmaf(v[j].x, v[j].x, __fmul_rn(v[j].y, v[j].y))));
         ss = block_sum(ss, scratch);
         if (ssq_out == nullptr) put(1.0f / sqrtf(ss / (float)size + eps));
         else if (threadIdx.x == 0) ssq_out[r] = ss;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = next[j];
+        for (int j = 0; j < PIECES; ++j) v[j] = next[j];
     }
 }
 
@@ -145,12 +147,13 @@ static int rmsnorm_launch(void* out, int out_dtype, const float* x, const void* 
     if (w_dtype != KIPP_DT_F32 && w_dtype != KIPP_DT_BF16) return KIPP_ERR_DTYPE;
     cudaStream_t s = (cudaStream_t)stream;
     if (size % 4 == 0 && size <= 4096 && size >= 256 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)out & 15) == 0) {
-        const int blocks = std::min(n_rows, NORM_BLOCKS * kipp_sm_count());
+        const bool narrow = size <= 1024;
+        const int blocks = std::min(n_rows, (narrow ? NORM_BLOCKS_NARROW : NORM_BLOCKS) * kipp_sm_count());
         if (out_dtype == KIPP_DT_F32)
-            return kipp_launch(rmsnorm_vec_kernel<float>, dim3(blocks), dim3(256), 0, s, 1,
+            return kipp_launch(narrow ? rmsnorm_vec_kernel<float, 1> : rmsnorm_vec_kernel<float, 4>, dim3(blocks), dim3(256), 0, s, 1,
                                (float*)out, x, w, w_dtype, rows, n_rows, size, eps, ssq_out);
         if (out_dtype == KIPP_DT_BF16)
-            return kipp_launch(rmsnorm_vec_kernel<bf16>, dim3(blocks), dim3(256), 0, s, 1,
+            return kipp_launch(narrow ? rmsnorm_vec_kernel<bf16, 1> : rmsnorm_vec_kernel<bf16, 4>, dim3(blocks), dim3(256), 0, s, 1,
                                (bf16*)out, x, w, w_dtype, rows, n_rows, size, eps, ssq_out);
         return KIPP_ERR_DTYPE;
     }

@@ -81,10 +81,10 @@ def test_rmsnorm_deferred(size):
     assert torch.equal(out.cpu(), (x.cpu()[[6, 0, 3]] * w.float().cpu()).to(torch.bfloat16))
 
 
-@pytest.mark.parametrize("rows", [591, 592, 593, 1300])
-@pytest.mark.parametrize("size", [256, 2052, 4096])
+@pytest.mark.parametrize("rows", [591, 592, 593, 1183, 1184, 1185, 1300])
+@pytest.mark.parametrize("size", [256, 1024, 1028, 2052, 4096])
 def test_rmsnorm_of_many_rows(size, rows):
-    """From 593 rows on a block has several: each row's result has the bits it has alone."""
+    """From 593 rows on (1,185 of up to 1,024 values) a block has several: each row's result has the bits it has alone."""
     g = torch.Generator().manual_seed(size + rows)
     x, w = torch.randn(rows, size, generator=g).to(DEV), torch.randn(size, generator=g).to(DEV)
     out, ssq, normed = torch.empty(rows, size, dtype=torch.bfloat16, device=DEV), torch.empty(rows, device=DEV), torch.empty(rows, size, device=DEV)
