@@ -28,6 +28,7 @@
 // A pair's row is computed from its own token alone, in an order of sums that depends on the
 // sizes only: the result does not depend on which other tokens share its tile.
 #include "common.cuh"
+#include <type_traits>
 #include <math.h>
 #include <limits.h>
 
@@ -50,8 +51,9 @@ __device__ __forceinline__ void load4(float (&x)[4], const bf16* row, int i) {
 // place allow: `vec`), then the lanes are summed; a router row is read once for all TOK tokens.
 // The order of a token's sums depends on the sizes only, not on TOK or on the other tokens.
 // Then warp j chooses for token j.
-template <typename T, int TOK>
-__global__ void __launch_bounds__(TOK == 1 ? 1024 : 256)
+// WIDE: few tokens, whose blocks have an SM to themselves: up to 32 warps with eight loads on their way each.
+template <typename T, int TOK, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 1024 : 512)
 moe_route_kernel(int* __restrict__ expert_of, float* __restrict__ weight_of, const T* __restrict__ h, long long ldh,
                  const float* __restrict__ router, const float* __restrict__ bias, int tokens, int hidden, int experts,
                  int top, int vec, int by_scores, int renormalize, int real_experts, float weight_scale) {
@@ -60,7 +62,7 @@ moe_route_kernel(int* __restrict__ expert_of, float* __restrict__ weight_of, con
     extern __shared__ float z_all[];
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    if (TOK == 1) {
+    if (WIDE) {
         // few tokens: the router's rows come from memory, and a warp asks for its own before the wait
         for (int e = warp; e < experts; e += warps)
             for (int i = 32 * lane; i < hidden; i += 1024)
@@ -78,8 +80,7 @@ moe_route_kernel(int* __restrict__ expert_of, float* __restrict__ weight_of, con
 #pragma unroll
         for (int j = 0; j < TOK; ++j) acc[j] = 0.f;
         if (vec) {
-#pragma unroll TOK == 1 ? 8 : 4
-            for (int i = 4 * lane; i < hidden; i += 128) {
+            auto four = [&](int i) {
                 float wv[4];
                 load4(wv, w, i);
 #pragma unroll
@@ -89,7 +90,16 @@ moe_route_kernel(int* __restrict__ expert_of, float* __restrict__ weight_of, con
 #pragma unroll
                     for (int u = 0; u < 4; ++u) acc[j] = fmaf(wv[u], x[u], acc[j]);
                 }
+            };
+            int i = 4 * lane;
+            if (WIDE) {
+#pragma unroll 1
+                for (; i + 7 * 128 < hidden; i += 8 * 128)
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) four(i + 128 * u);
             }
+#pragma unroll 4
+            for (; i < hidden; i += 128) four(i);
         } else {
 #pragma unroll 4
             for (int i = lane; i < hidden; i += 32) {
@@ -408,8 +418,11 @@ static int moe_route_any(int* expert_of, float* weight_of, const void* h, long l
     const int tok = tokens >= 256 ? 4 : 1;
     // few: a warp an expert, up to 32 (8 tokens, 18 outputs, 2,560 wide: 23 us with sixteen warps, whose last two outputs were a
     // round of their own, the router's rows asked for behind the wait and the weights normalised in global memory;
-    // 9 us so)
-    const int warps = tok == 4 ? 8 : experts > 32 ? 32 : experts < 4 ? 4 : experts;
+    // 9 us so), as long as every token's block finds an SM of its own: two of 32 warps do not fit on one (255 tokens, 64
+    // outputs, 2,560 wide: 25.3 us with up to 32 warps, 19.5 with up to 16)
+    const int wide = experts > 32 ? 32 : experts < 4 ? 4 : experts, narrow = experts >= 16 ? 16 : experts > 8 ? 8 : 4;
+    const bool alone = tokens <= kipp_sm_count();
+    const int warps = tok == 4 ? 8 : alone ? wide : narrow;
     const dim3 grid((unsigned)((tokens + tok - 1) / tok)), block((unsigned)(32 * warps));
     const size_t scores = (size_t)(by_scores ? 2 : 1) * tok * experts * sizeof(float), smem = scores + (size_t)tok * top * sizeof(float);
     auto go = [&](auto kernel, auto rows) {
@@ -419,10 +432,12 @@ static int moe_route_any(int* expert_of, float* weight_of, const void* h, long l
         return kipp_launch(kernel, grid, block, smem, s, 1, expert_of, weight_of, rows, ldh, router, bias, tokens, hidden, experts, top, vec,
                            by_scores, renormalize, real_experts, weight_scale);
     };
-    if (dtype == KIPP_DT_F32)
-        return tok == 4 ? go(moe_route_kernel<float, 4>, (const float*)h) : go(moe_route_kernel<float, 1>, (const float*)h);
-    if (dtype == KIPP_DT_BF16)
-        return tok == 4 ? go(moe_route_kernel<bf16, 4>, (const bf16*)h) : go(moe_route_kernel<bf16, 1>, (const bf16*)h);
+    auto of_type = [&](auto rows) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(rows)>>;
+        return tok == 4 ? go(moe_route_kernel<T, 4, false>, rows) : alone ? go(moe_route_kernel<T, 1, true>, rows) : go(moe_route_kernel<T, 1, false>, rows);
+    };
+    if (dtype == KIPP_DT_F32) return of_type((const float*)h);
+    if (dtype == KIPP_DT_BF16) return of_type((const bf16*)h);
     return KIPP_ERR_DTYPE;
 }
 extern "C" int kipp_moe_route(int* expert_of, float* weight_of, const void* h, long long ldh, int dtype, const float* router,

@@ -1392,3 +1392,36 @@ def test_gated_delta_scans_add_in_one_order(D, V, entries, longest):
     got = out.cpu().reshape(entries, 2, heads, V)
     for t in range(2):
         assert torch.equal(got[:, t] != 0, want != 0)
+
+
+@pytest.mark.parametrize("hidden,outputs", [(512, 18), (1028, 64), (33, 5), (2560, 3)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_routing_of_a_token_among_others(dtype, hidden, outputs):
+    """A token's experts and weights have the same bits whether its block has an SM to itself with up to 32 warps (148 tokens), shares
+    one with up to 16 (149, 255) or holds four tokens (256, 257), by logits and by scores, in rows of whole fours and others; the
+    weights are the softmax of the chosen logits, whose sums of `hidden` products are float32."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    lib = load_library("moe")
+    p, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+    lib.kipp_moe_route.argtypes = [p, p, p, ll, i, p, p, i, i, i, i, p]
+    lib.kipp_moe_route_scores.argtypes = [p, p, p, ll, i, p, p, i, i, i, i, i, i, i, f, p]
+    g = torch.Generator().manual_seed(hidden)
+    h, w, b = torch.randn(257, hidden, generator=g).to(dtype).to(DEV), (torch.randn(outputs, hidden, generator=g) * 0.2).to(DEV), torch.randn(outputs, generator=g).to(DEV)
+    top, code = min(3, outputs), 0 if dtype == torch.float32 else 1
+    for scores in (False, True):
+        kept = None
+        for tokens in (257, 1, 33, 148, 149, 255, 256):
+            expert, weight = torch.full((tokens, top), -9, dtype=torch.int32, device=DEV), torch.zeros(tokens, top, device=DEV)
+            at = (expert.data_ptr(), weight.data_ptr(), h.data_ptr(), hidden, code, w.data_ptr(), b.data_ptr(), tokens, hidden, outputs)
+            stream = torch.cuda.current_stream().cuda_stream
+            rc = lib.kipp_moe_route_scores(*at, outputs, top, 1, 1, 1.5, stream) if scores else lib.kipp_moe_route(*at, top, stream)
+            assert rc == 0
+            kept = kept or (expert, weight)
+            assert torch.equal(expert, kept[0][:tokens]) and torch.equal(weight, kept[1][:tokens]), (scores, tokens)
+        if not scores:
+            logits = (h.double() @ w.double().t() + b.double()).cpu()
+            best = torch.gather(logits, 1, kept[0].long().cpu())
+            slack = hidden * 2.0 ** -23 * float((h.double().abs() @ w.double().abs().t()).max()) + 1e-6
+            assert (logits.topk(top).values - best <= 2 * slack).all()
+            assert torch.allclose(kept[1].double().cpu(), torch.softmax(best, -1), atol=2 * slack)
