@@ -1113,6 +1113,15 @@ extern "C" int kipp_attn_prefill_tc_ex(void* out, const void* q, int tokens, con
                       items, n_q, n_kv, head_dim, v_dim, scale, window, out_scale, ex, status, stream);
 }
 
+// Whether kipp_latent_expand_tc takes the pages and is the faster form for `keys` cached tokens, new ones among them.  Its
+// launch has a floor of 10 us, for setting up the tensor memory and for the way out, that the mma.sync form does not have (128 and
+// 256 columns of latents, 20 tokens: 6.4 and 9.0 us there, 9.7 and 11.2 here; level at 0.3 G products, 15 and 11 us at four times
+// as many).  With 512 columns entries of 20 tokens are 4 % behind here and of 40 to 70 up to 11 % ahead.  The bits are the same.
+extern "C" int kipp_latent_expand_tc_pays(int page_size, int rank, int features, int entries, long long keys) {
+    if (!kipp_attn_prefill_tc_page_ok(page_size)) return 0;
+    return rank > 256 ? keys > 32LL * entries : (double)keys * features * rank >= 0.3e9;
+}
+
 // kipp_latent_expand (head_ops.cu) for page sizes whose boxes fill whole swizzle groups (kipp_attn_prefill_tc_page_ok):
 // the same arguments and results, and the number of the pool's pages.
 extern "C" int kipp_latent_expand_tc(const void* pages, int n_pages, const int* block_table, int table_width, int page_size, int row,

@@ -423,8 +423,8 @@ public:
     static int expand_pages(const PagedCacheView& cache) {
         return (int)(((long long)cache.table_width * cache.page_size + expand_page() - 1) / expand_page());
     }
-    PagedCacheView latent_expand(const PagedCacheView& cache, const int* q_start, const int* context_len, int entries, const void* w_k,
-                                 const void* w_v, int rank, int dim, int rot, int v_dim, int heads) {
+    PagedCacheView latent_expand(const PagedCacheView& cache, const int* q_start, const int* context_len, int entries, long long keys,
+                                 const void* w_k, const void* w_v, int rank, int dim, int rot, int v_dim, int heads) {
         using Fn = int (*)(const void*, const int*, int, int, int, const int*, const int*, int, const void*, const void*, int, int, int,
                            int, int, void*, void*, int*, int, int*, void*);
         static Fn f = kernel_symbol<Fn>("head_ops", "kipp_latent_expand");
@@ -437,10 +437,10 @@ public:
         v.v_pages = workspace->buffer("latent_values", rows * v_dim * 2);
         int* table = workspace->get<int>("latent_table", (size_t)v.n_pages);
         v.block_table = table;
-        // on tcgen05 where a box of the pool's rows lies in one page, as the attention kernel itself needs it (attention_tc.cu)
-        using Pages = int (*)(int);
-        static Pages page_ok = kernel_symbol<Pages>("attention_tc", "kipp_attn_prefill_tc_page_ok");
-        if (page_ok(cache.page_size)) {
+        // on tcgen05 where a box of the pool's rows lies in one page and there is enough of it (attention_tc.cu)
+        using Pays = int (*)(int, int, int, int, long long);
+        static Pays pays = kernel_symbol<Pays>("attention_tc", "kipp_latent_expand_tc_pays");
+        if (pays(cache.page_size, rank, heads * (dim + v_dim), entries, keys)) {
             using Ft = int (*)(const void*, int, const int*, int, int, int, const int*, const int*, int, const void*, const void*, int, int,
                                int, int, int, void*, void*, int*, int, int*, void*);
             static Ft ft = kernel_symbol<Ft>("attention_tc", "kipp_latent_expand_tc");

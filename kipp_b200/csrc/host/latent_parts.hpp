@@ -211,8 +211,10 @@ private:
         const int T = ctx.tokens();
         Ops& ops = *ctx.ops;
         const StepMeta& m = *ctx.meta;
-        const PagedCacheView kv = ops.latent_expand(cache, m.q_start, m.context_len, m.shape.entries, w_uk_, w_uv_, kv_rank_, dim_, rot_,
-                                                    v_dim_, heads_);
+        long long keys = 0;
+        for (int e = 0; e < m.shape.entries; ++e) keys += m.shape.starts[(size_t)e] + m.shape.q_lens[(size_t)e];
+        const PagedCacheView kv = ops.latent_expand(cache, m.q_start, m.context_len, m.shape.entries, keys, w_uk_, w_uv_, kv_rank_, dim_,
+                                                    rot_, v_dim_, heads_);
         const void* qr = q;
         if (rot_ > 0) {
             HeadSegment r;

@@ -1156,6 +1156,7 @@ def test_latent_expand(sizes, page):
     dev = [x.to(DEV).contiguous() for x in (pool, table, wk, wv)]
     on_tc = load_library("attention_tc").kipp_attn_prefill_tc_page_ok(page)
     assert bool(on_tc) == (page != 24)
+    bits = []
     for tc in ([True, False] if on_tc else [False]):
         fn = load_library("attention_tc").kipp_latent_expand_tc if tc else load_library("head_ops").kipp_latent_expand
         fn.argtypes = [p] + ([i] if tc else []) + rest
@@ -1169,6 +1170,7 @@ def test_latent_expand(sizes, page):
         torch.cuda.synchronize()
         assert rc == 0 and status.abs().sum().item() == 0
         assert torch.equal(to.cpu().flatten(), torch.arange(len(lens) * width, dtype=torch.int32))
+        bits.append((ko, vo))
         for e, n in enumerate(lens):
             rows = torch.cat([pool[table[e, j]] for j in range(-(-n // page))])[:n]
             c = rows[:, :rank].double()
@@ -1181,6 +1183,7 @@ def test_latent_expand(sizes, page):
                 if out is ko:
                     assert (got[:n, :, size:] == rows[:, None, rank:].double()).all(), (tc, e)
                 assert (got[n:end] == 0).all() and (got[end:] == 7).all(), (tc, e)
+    assert all(torch.equal(b[k], bits[0][k]) for b in bits for k in (0, 1))          # the engine takes either by their sizes
 
 
 @pytest.mark.parametrize("window", [0, 40])
