@@ -70,8 +70,10 @@ __device__ __forceinline__ unsigned long long team_ld_u64(const void* p, int ran
 }
 
 constexpr int LIST_CAP = 4096;  // elements a block lists: 16 KB
+constexpr int FEW_ELEMENTS = 2048;
 constexpr int COPIES = 4;       // histograms of a block, one for every fourth warp: most elements of a first pass meet a
                                 // handful of buckets, and atomics on one word run one after the other
+constexpr int COPIES_FROM = 2048;   // elements from which a block has them; clearing and adding four costs a short row more
 
 struct RowCtx {
     const float* v;
@@ -79,6 +81,7 @@ struct RowCtx {
     int lo, hi;                 // this block's part of the row
     int* list;                  // [LIST_CAP] in shared memory
     int listed;                 // >= 0: the elements to walk are the first `listed` of the list
+    int copies;                 // histograms in use
     float inv_t, smax, cutoff;
     // filters
     bool has_topk;   unsigned topk_key, topk_tok;
@@ -148,6 +151,16 @@ template <typename F> __device__ __forceinline__ void walk(const RowCtx& c, F f)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const bool list = c.listed >= 0;
     const int n = list ? c.listed : c.hi - c.lo;
+    // (few elements one by one: eight copies of a pass's code are more to fetch than they save there; four rows of 700 with a nucleus
+    // of 0.9: 36 us with eight at a time and four histograms, 30 so)
+    if (n <= FEW_ELEMENTS) {
+#pragma unroll 1
+        for (int base = warp * 32; base < n; base += warps * 32) {
+            const int at = base + lane, i = at >= n ? -1 : list ? c.list[at] : c.lo + at;
+            f(i, i < 0 ? 0.f : c.v[i], i >= 0);
+        }
+        return;
+    }
     for (int base = warp * 32; base < n; base += warps * 32 * AT_ONCE) {
         int i[AT_ONCE]; float x[AT_ONCE];
 #pragma unroll
@@ -179,11 +192,11 @@ __device__ __forceinline__ void append(const RowCtx& c, Shared& sh, int i, bool 
 // Without `weigh` only the counts are formed (no min-p is in force then).
 __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned prefix_key,
                                unsigned prefix_tok, bool gather, bool weigh) {
-    for (int b = threadIdx.x; b < COPIES * 256; b += blockDim.x) { (&sh.cnt[0][0])[b] = 0; (&sh.wfix[0][0])[b] = 0ull; }
+    for (int b = threadIdx.x; b < c.copies * 256; b += blockDim.x) { (&sh.cnt[0][0])[b] = 0; (&sh.wfix[0][0])[b] = 0ull; }
     if (threadIdx.x == 0) sh.listed = 0;
     __syncthreads();
     // the lanes of a round that fall into one bucket are found with match.any and add as one
-    const int lane = threadIdx.x & 31, copy = (threadIdx.x >> 5) % COPIES;
+    const int lane = threadIdx.x & 31, copy = (threadIdx.x >> 5) & (c.copies - 1);
     walk(c, [&](int i, float x, bool there) {
         unsigned key = 0; float w = 0.f;
         unsigned digit = 256u;                                  // no bucket: not in the set at this level
@@ -209,8 +222,7 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
     });
     __syncthreads();
     for (int b = threadIdx.x; b < 256; b += blockDim.x) {
-#pragma unroll
-        for (int k = 1; k < COPIES; ++k) { sh.cnt[0][b] += sh.cnt[k][b]; sh.wfix[0][b] += sh.wfix[k][b]; }
+        for (int k = 1; k < c.copies; ++k) { sh.cnt[0][b] += sh.cnt[k][b]; sh.wfix[0][b] += sh.wfix[k][b]; }
     }
     // the team's histogram: every block adds the blocks' parts in block order
     team_sync();
@@ -501,7 +513,7 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
         return;
     }
     RowCtx c;
-    c.v = v; c.n = n; c.lo = lo; c.hi = hi; c.list = list; c.listed = -1;
+    c.v = v; c.n = n; c.lo = lo; c.hi = hi; c.list = list; c.listed = -1; c.copies = hi - lo > COPIES_FROM ? COPIES : 1;
     c.inv_t = 1.0f / T;
     c.smax = v[best_i] * c.inv_t;
     c.cutoff = c.smax - 20.0f;
