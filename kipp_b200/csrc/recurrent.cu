@@ -584,7 +584,7 @@ gated_delta_prepare_kernel(const ScanArgs a, const float* __restrict__ conv_out,
 // (norm_groups equal parts of heads * v_dim), times the weight.  A block per (token, part).  W: channels that a thread
 // forms at a time; 4 where rows, parts and heads go by fours, start accordingly and fit in shared memory, through which
 // the values then go, so that thread t adds the squares of channels t, t + threads, ... whatever W is (2,048 tokens of
-// 4,096 channels, 100 MB: 56 us a channel at a time, 29 so).
+// 4,096 channels, 100 MB: 56 us a channel at a time, 31 so).
 // keep: every entry brought one token, and the blocks of its row also move its kept inputs on.
 template <int W> __device__ __forceinline__ void load_channels(float (&v)[W], const float* p) {
     if constexpr (W == 4) {
@@ -920,7 +920,7 @@ ssd_scan_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* 
 // pairs of rows by turns into two sums (no chain is longer than a quarter of the rows), then the lanes, the farthest first.
 // (With one column per thread, as below, a token costs ten shuffles and three 16-byte reads of shared memory for FOUR
 // elements of the state, and many blocks on an SM are bound by those: sequences of 1,277, 700 and 753 tokens, 16 heads:
-// 712 us so, 445 us here.)
+// 712 us so, 464 us here.)
 template <int P, int R, int WARPS, bool EXACT>
 __global__ void __launch_bounds__(32 * WARPS)
 gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* __restrict__ o_raw, int v_slices, int tokens) {
