@@ -59,7 +59,7 @@
 // convolved rows, no records), and for the gated delta rule gated_delta_scan_kernel (four columns a thread) and
 // gated_delta_column_kernel (one, where few blocks make the chain of a token what counts).  There a thread works on pairs of
 // float32 and the shuffles of one token's sums travel while the next token is worked on.  (State space prompts by chunks of
-// 128 tokens, products within a chunk and the state from chunk to chunk, took 164 us instead of 477 for 2,048 tokens of 64
+// 128 tokens, products within a chunk and the state from chunk to chunk, took 164 us (292 here) for 2,048 tokens of 64
 // heads of 128 x 64 and are not used: their sums come in another order, which can turn a near tie of a router behind the
 // layer; the order hung on the step's other prompts; and the masked products carried an infinite token into the ones
 // before it.)  For steps of one token per request
@@ -763,11 +763,12 @@ int launch_walk(const ScanArgs& a, int tokens, void (*kernel)(KArgs...), dim3 gr
 // while the token before is worked on, so that only the recurrence itself is a chain.  The order of every sum
 // depends on the sizes only.
 //
-// State space: a thread owns 4 columns x R rows (P threads per group of columns, rows in groups of four dealt out in
-// turn), so that a token's C and B serve four columns per load; the four outputs' sums over P lanes meet in P's
-// logarithm plus one shuffles (every exchange also halves the columns a lane is responsible for).  C, B and x come
-// straight out of the convolved rows, decay and step size from dts [tokens][heads].
-// Rows go through the arithmetic in pairs (float32 pairs in one instruction).
+// State space: a thread owns 4 columns x LPT R rows, so that a token's C and B serve four columns per load.  A column's sum
+// with C is a tree of one shape: R rows in turn (leaf l: groups of four rows, 4 l and every 4 LEAVES further), then the leaves
+// by the bits of l, the lowest first.  A thread holds leaf p, or the leaves 2 p and 2 p + 1, whose sums meet without
+// an exchange; four tokens' sums go through the exchanges together, and each halves what a lane is responsible for, so that
+// sixteen sums take fifteen or sixteen of them.  C, B and x come straight out of the convolved rows, decay and step size
+// from dts [tokens][heads].  Rows go through the arithmetic in pairs (float32 pairs in one instruction).
 constexpr int SCAN_COLS = 4;
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     float2 d;
@@ -793,14 +794,48 @@ __host__ __device__ inline TokenBatch token_batch(int floats) {
     if (b.tokens < 1) b.tokens = 1;
     return b;
 }
-// EXACT: the P threads' rows are the head's, none too many.
-template <int P, int R, int WARPS, bool EXACT>
-__global__ void __launch_bounds__(32 * WARPS)
+// A ring of SSD_RING batches of whole groups of SSD_GROUP tokens: two batches are on their way while one is worked on.
+constexpr int SSD_GROUP = 4, SSD_RING = 3, SSD_COLS = 32;      // SSD_COLS columns a block
+__host__ __device__ inline TokenBatch ssd_batch(int floats) {
+    TokenBatch b;
+    b.floats = floats;
+    b.tokens = floats * 4 * 16 <= 19 * 1024 ? 16 : (19 * 1024) / (floats * 4) / SSD_GROUP * SSD_GROUP;
+    return b;
+}
+// Sums of N values over P lanes, in lane bits from the lowest: while a lane holds several, an exchange halves them (the
+// upper half stays where the lane's bit is set), then every lane gets the same.
+template <int P, int N> __device__ __forceinline__ void meet_lanes(float (&v)[N], int p) {
+    int n = N;
+#pragma unroll
+    for (int x = 1; x < P; x <<= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool up = p & x;
+#pragma unroll
+            for (int i = 0; i < N / 2; ++i) {
+                if (i >= n) break;
+                const float keep = up ? v[i + n] : v[i], send = up ? v[i] : v[i + n];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, x);
+            }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], x);
+        }
+    }
+}
+// EXACT: the leaves' rows are the head's, none too many.
+// What bounds it is a token's chain and the issue of what surrounds its multiply-adds: 32 columns of 64 x 128 heads are four
+// warps of two leaves or eight of one, on 128 blocks for 64 heads, and a scheduler has one or two warps.  One sequence of 2,048
+// tokens, 64 heads, in a model: 477 us token by token with six exchanges each, 438 with the groups, 333 with one leaf a thread and
+// the state's update before the sums, 292 with the sizes as constants.  The two forms alone, sizes not constant: that
+// sequence 349 us with two leaves and 287 with one (441 with each row's update and sum in turn); entries of 1,276, 636 and 600
+// tokens, 80 heads: 377 and 363; eight of 100: 111 and 140 (many blocks an SM: fewer instructions count).
+template <int LEAVES, int LPT, int R, bool EXACT>
+__global__ void __launch_bounds__(8 * LEAVES / LPT, (R == 4 ? 64 : 32) / (LEAVES / LPT))
 ssd_scan_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* __restrict__ dts, float* __restrict__ o_raw, int v_slices) {
     extern __shared__ __align__(16) float smem[];
-    constexpr int COLS = SCAN_COLS * 32 * WARPS / P, THREADS = 32 * WARPS;
-    const int D = a.dim, V = a.v_dim;
-    const TokenBatch tb = token_batch(2 * D + COLS + 4);
+    constexpr int P = LEAVES / LPT, THREADS = SSD_COLS / SCAN_COLS * P, WARPS = THREADS / 32, COLS = SSD_COLS, Q = R / 4;
+    const int D = EXACT ? LEAVES * R : a.dim, V = a.v_dim;      // (a constant: the copies' and loads' addresses are then cheap)
+    const TokenBatch tb = ssd_batch(2 * D + COLS + 4);
     pdl_launch_dependents();
     pdl_wait();
     const int tid = threadIdx.x, p = tid % P, slice = blockIdx.x % v_slices, eh = blockIdx.x / v_slices;
@@ -827,90 +862,131 @@ ssd_scan_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* 
             }
         }
         for (int t = tid; t < nb; t += THREADS)
-            *reinterpret_cast<float2*>(buf + (size_t)t * tb.floats + 2 * D + COLS) = dts[(size_t)(row0 + t0 + t) * a.heads + h];
-        cp_async_commit();
+            cp_async8(smem_address(buf + (size_t)t * tb.floats + 2 * D + COLS), dts + (size_t)(row0 + t0 + t) * a.heads + h);
     };
-    // row i of this thread: 4 (p + P (i / 4)) + i % 4; S[i / 2][c] holds rows i and i + 1 of column c
-    float2 S[R / 2][SCAN_COLS];
+    // Groups of four rows of this thread: number j = s Q + q belongs to leaf LPT p + (s ^ turn), rows 4 (leaf + LEAVES q) ...;
+    // `turn` lets eight neighbouring lanes' loads fall into different banks (two leaves' sums meet in either order).
+    const int turn = LPT == 2 ? (p >> 2) & 1 : 0;
+    int row[LPT * Q];
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int r = 4 * (p + P * (i >> 2)) + (i & 3);
-        const float4 s4 = live && r < D ? *reinterpret_cast<const float4*>(S_slot + (size_t)r * V + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float e[4] = {s4.x, s4.y, s4.z, s4.w};
+    for (int j = 0; j < LPT * Q; ++j) row[j] = 4 * (LPT * p + (j / Q ^ turn) + LEAVES * (j % Q));
+    float2 S[2 * LPT * Q][SCAN_COLS];        // S[2 j + i][c]: rows row[j] + 2 i and + 2 i + 1 of column c
 #pragma unroll
-        for (int c = 0; c < SCAN_COLS; ++c) (i & 1 ? S[i >> 1][c].y : S[i >> 1][c].x) = e[c];
-    }
-    float2 cv[R / 2], bv[R / 2], keep, tx[SCAN_COLS];
-    auto take = [&](const float* tok) {
+    for (int j = 0; j < LPT * Q; ++j)
 #pragma unroll
-        for (int q = 0; q < R / 4; ++q) {
-            const int r = 4 * (p + P * q);
-            float4 c4 = make_float4(0.f, 0.f, 0.f, 0.f), b4 = c4;
-            if (EXACT || r < D) {
-                c4 = *reinterpret_cast<const float4*>(tok + r);
-                b4 = *reinterpret_cast<const float4*>(tok + D + r);
-            }
-            cv[2 * q] = make_float2(c4.x, c4.y); cv[2 * q + 1] = make_float2(c4.z, c4.w);
-            bv[2 * q] = make_float2(b4.x, b4.y); bv[2 * q + 1] = make_float2(b4.z, b4.w);
+        for (int i = 0; i < 4; ++i) {
+            const float4 s4 = live && row[j] < D ? *reinterpret_cast<const float4*>(S_slot + (size_t)(row[j] + i) * V + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float e[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+            for (int c = 0; c < SCAN_COLS; ++c) (i & 1 ? S[2 * j + (i >> 1)][c].y : S[2 * j + (i >> 1)][c].x) = e[c];
         }
-        const float4 x4 = *reinterpret_cast<const float4*>(tok + 2 * D + cl);
-        const float2 kd = *reinterpret_cast<const float2*>(tok + 2 * D + COLS);
-        keep = both(kd.x);
-        tx[0] = both(kd.y * x4.x); tx[1] = both(kd.y * x4.y); tx[2] = both(kd.y * x4.z); tx[3] = both(kd.y * x4.w);
+    struct Token { float2 c[2 * LPT * Q], b[2 * LPT * Q], kd; float4 x; };
+    auto take = [&](const float* tok, Token& n) {
+#pragma unroll
+        for (int j = 0; j < LPT * Q; ++j) {
+            float4 c4 = make_float4(0.f, 0.f, 0.f, 0.f), b4 = c4;
+            if (EXACT || row[j] < D) {
+                c4 = *reinterpret_cast<const float4*>(tok + row[j]);
+                b4 = *reinterpret_cast<const float4*>(tok + D + row[j]);
+            }
+            n.c[2 * j] = make_float2(c4.x, c4.y); n.c[2 * j + 1] = make_float2(c4.z, c4.w);
+            n.b[2 * j] = make_float2(b4.x, b4.y); n.b[2 * j + 1] = make_float2(b4.z, b4.w);
+        }
+        n.x = *reinterpret_cast<const float4*>(tok + 2 * D + cl);
+        n.kd = *reinterpret_cast<const float2*>(tok + 2 * D + COLS);
     };
-    fetch(0, smem);
-    int buf = 0;
-    for (int t0 = 0; t0 < n_tok; t0 += tb.tokens, buf ^= 1) {
-        const int nb = min(tb.tokens, n_tok - t0);
-        if (t0 + tb.tokens < n_tok) fetch(t0 + tb.tokens, smem + (size_t)(buf ^ 1) * tb.tokens * tb.floats);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const float* toks = smem + (size_t)buf * tb.tokens * tb.floats;
-        take(toks);
-        // a token's sums travel while the next token is worked on: the chain of shuffles is nobody's wait
-        float last[SCAN_COLS] = {0.f, 0.f, 0.f, 0.f};
-        float* out = o_raw + (size_t)(row0 + t0) * inner + h * V + col + 2 * (p & 1) + (p >> 1);      // lanes p < 4
-        auto meet = [&](const float* o) {
-            // lane p of a group of P ends up with column 2 (p & 1) + (p >> 1 & 1)
-            const bool odd = p & 1, second = p & 2;
-            float k0 = odd ? o[2] : o[0], k1 = odd ? o[3] : o[1];
-            k0 += __shfl_xor_sync(0xffffffffu, odd ? o[0] : o[2], 1);
-            k1 += __shfl_xor_sync(0xffffffffu, odd ? o[1] : o[3], 1);
-            float y = (second ? k1 : k0) + __shfl_xor_sync(0xffffffffu, second ? k0 : k1, 2);
+    // one token: the state moves on, then the leaves' sums of the four columns (all of the update first: the sums' chains
+    // then find their terms ready)
+    auto step = [&](const Token& n, float (&sum)[SCAN_COLS]) {
+        const float2 keep = both(n.kd.x);
+        const float2 tx[SCAN_COLS] = {both(n.kd.y * n.x.x), both(n.kd.y * n.x.y), both(n.kd.y * n.x.z), both(n.kd.y * n.x.w)};
 #pragma unroll
-            for (int x = 4; x < P; x <<= 1) y += __shfl_xor_sync(0xffffffffu, y, x);
-            return y;
-        };
-        const bool writes = live && p < SCAN_COLS;
-        for (int t = 0; t < nb; ++t) {
-            float2 o[SCAN_COLS];
-            const float y = meet(last);
+        for (int i = 0; i < 2 * LPT * Q; ++i)
 #pragma unroll
-            for (int i = 0; i < R / 2; ++i)
+            for (int c = 0; c < SCAN_COLS; ++c) S[i][c] = fma2(n.b[i], tx[c], mul2(keep, S[i][c]));
+        float2 o[LPT][SCAN_COLS];
 #pragma unroll
-                for (int c = 0; c < SCAN_COLS; ++c) {
-                    S[i][c] = fma2(bv[i], tx[c], mul2(keep, S[i][c]));
-                    o[c] = i == 0 ? mul2(cv[i], S[i][c]) : fma2(cv[i], S[i][c], o[c]);
-                }
-            take(toks + (size_t)min(t + 1, nb - 1) * tb.floats);
-            if (writes && t > 0) {
-                *out = y;
+        for (int i = 0; i < 2 * LPT * Q; ++i)
+#pragma unroll
+            for (int c = 0; c < SCAN_COLS; ++c) {
+                float2& to = o[i / (2 * Q)][c];
+                to = i % (2 * Q) == 0 ? mul2(n.c[i], S[i][c]) : fma2(n.c[i], S[i][c], to);
+            }
+#pragma unroll
+        for (int c = 0; c < SCAN_COLS; ++c) {
+            sum[c] = o[0][c].x + o[0][c].y;
+            if constexpr (LPT == 2) sum[c] += o[1][c].x + o[1][c].y;
+        }
+    };
+    // Which sum ends up in this lane: the first two exchanges leave it a column, the next ones (a group's) tokens.
+    const int my_col = 2 * (p & 1) + (p >> 1 & 1);
+    constexpr int LEFT = 4 * SSD_GROUP > P ? 4 * SSD_GROUP / P : 1;      // tokens of a group a lane ends up with
+    const int my_token = P >= 16 ? 2 * (p >> 2 & 1) + (p >> 3 & 1) : P == 8 ? 2 * (p >> 2 & 1) : 0;
+    const bool writes_group = live && p < 16, writes_one = live && p < SCAN_COLS;
+
+    const int n_batches = (n_tok + tb.tokens - 1) / tb.tokens;
+    const size_t per_batch = (size_t)tb.tokens * tb.floats;
+#pragma unroll
+    for (int b = 0; b < SSD_RING - 1; ++b) {
+        if (b < n_batches) fetch(b * tb.tokens, smem + b * per_batch);
+        cp_async_commit();
+    }
+    float* out = o_raw + (size_t)row0 * inner + h * V + col + my_col;
+    float sums[SCAN_COLS * SSD_GROUP];       // the group before, [column][token]: met and written while the next one is worked on
+    bool held = false;
+    auto write_group = [&]() {
+        meet_lanes<P>(sums, p);
+        if (writes_group) {
+#pragma unroll
+            for (int u = 0; u < LEFT; ++u) out[(size_t)(my_token + u) * inner] = sums[u];
+        }
+        out += (size_t)SSD_GROUP * inner;
+    };
+    for (int b = 0; b < n_batches; ++b) {
+        const int t0 = b * tb.tokens, nb = min(tb.tokens, n_tok - t0);
+        cp_async_wait<SSD_RING - 2>();
+        __syncthreads();                     // this batch has landed, and nobody reads the one before it any more
+        if (b + SSD_RING - 1 < n_batches) fetch((b + SSD_RING - 1) * tb.tokens, smem + (size_t)((b + SSD_RING - 1) % SSD_RING) * per_batch);
+        cp_async_commit();
+        const float* toks = smem + (size_t)(b % SSD_RING) * per_batch;
+        Token even, odd;
+        take(toks, even);
+        int t = 0;
+        for (; t + SSD_GROUP <= nb; t += SSD_GROUP) {
+            float now[SSD_GROUP][SCAN_COLS];
+            if (held) write_group();
+#pragma unroll
+            for (int u = 0; u < SSD_GROUP; ++u) {
+                take(toks + (size_t)min(t + u + 1, nb - 1) * tb.floats, u & 1 ? even : odd);      // (a batch's last token fetches itself again)
+                step(u & 1 ? odd : even, now[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < SSD_GROUP; ++u)
+#pragma unroll
+                for (int c = 0; c < SCAN_COLS; ++c) sums[c * SSD_GROUP + u] = now[u][c];
+            held = true;
+        }
+        if (t < nb) {                        // the entry's last tokens, fewer than a group
+            if (held) write_group();
+            held = false;
+            for (; t < nb; ++t) {
+                float one[SCAN_COLS];
+                take(toks + (size_t)t * tb.floats, even);
+                step(even, one);
+                meet_lanes<P>(one, p);
+                if (writes_one) *out = one[0];
                 out += inner;
             }
-#pragma unroll
-            for (int c = 0; c < SCAN_COLS; ++c) last[c] = o[c].x + o[c].y;
         }
-        const float y = meet(last);
-        if (writes) *out = y;
-        __syncthreads();                    // the buffer is free for the batch after the next
     }
+    if (held) write_group();
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int r = 4 * (p + P * (i >> 2)) + (i & 3);
-        auto at = [&](int c) { return i & 1 ? S[i >> 1][c].y : S[i >> 1][c].x; };
-        if (live && r < D) *reinterpret_cast<float4*>(S_slot + (size_t)r * V + col) = make_float4(at(0), at(1), at(2), at(3));
-    }
+    for (int j = 0; j < LPT * Q; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            auto at = [&](int c) { return i & 1 ? S[2 * j + (i >> 1)][c].y : S[2 * j + (i >> 1)][c].x; };
+            if (live && row[j] < D) *reinterpret_cast<float4*>(S_slot + (size_t)(row[j] + i) * V + col) = make_float4(at(0), at(1), at(2), at(3));
+        }
 }
 
 // The gated delta rule: a thread owns 4 columns x R rows, as above.  The decayed state meets k; the four columns' sums
@@ -921,6 +997,7 @@ ssd_scan_kernel(const ScanArgs a, const float* __restrict__ conv, const float2* 
 // (With one column per thread, as below, a token costs ten shuffles and three 16-byte reads of shared memory for FOUR
 // elements of the state, and many blocks on an SM are bound by those: sequences of 1,277, 700 and 753 tokens, 16 heads:
 // 712 us so, 464 us here.)
+// EXACT: the P threads' rows are the head's, none too many.
 template <int P, int R, int WARPS, bool EXACT>
 __global__ void __launch_bounds__(32 * WARPS)
 gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* __restrict__ o_raw, int v_slices, int tokens) {
@@ -1286,15 +1363,24 @@ template <typename T> bool conv_run_ok(const ScanArgs& a) {
 inline bool scan_by_fours(const ScanArgs& a) {
     return a.dim % 4 == 0 && a.v_dim % 4 == 0 && a.dim <= 256 && a.slot_stride % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
 }
-// (32 columns a block)
-template <int P, int R>
+// Two leaves a thread where there are more blocks than this for each SM, one (twice the warps) elsewhere: see above for both.
+constexpr int SSD_CROWD = 4;
+template <int LEAVES, int LPT, int R>
+int launch_ssd_form(const ScanArgs& a, const float* conv, const float2* dts, float* o_raw, int entries, int tokens, cudaStream_t stream) {
+    const TokenBatch tb = ssd_batch(2 * a.dim + SSD_COLS + 4);
+    const int slices = (a.v_dim + SSD_COLS - 1) / SSD_COLS;
+    const auto kernel = a.dim == LEAVES * R ? ssd_scan_kernel<LEAVES, LPT, R, true> : ssd_scan_kernel<LEAVES, LPT, R, false>;
+    const size_t bytes = (size_t)SSD_RING * tb.tokens * tb.floats * sizeof(float);
+    if (const int rc = kipp_allow_smem(kernel, bytes)) return rc;
+    return launch_walk(a, tokens, kernel, dim3((unsigned)(entries * a.heads * slices)), dim3(SSD_COLS / SCAN_COLS * LEAVES / LPT), bytes, stream,
+                       a, conv, dts, o_raw, slices);
+}
+template <int LEAVES, int R>
 int launch_ssd_scan(const ScanArgs& a, const float* conv, const float2* dts, float* o_raw, int entries, int tokens, cudaStream_t stream) {
-    constexpr int WARPS = P / 4, COLS = SCAN_COLS * 32 * WARPS / P;
-    const TokenBatch tb = token_batch(2 * a.dim + COLS + 4);
-    const int slices = (a.v_dim + COLS - 1) / COLS;
-    return launch_walk(a, tokens, a.dim == P * R ? ssd_scan_kernel<P, R, WARPS, true> : ssd_scan_kernel<P, R, WARPS, false>,
-                       dim3((unsigned)(entries * a.heads * slices)), dim3(32 * WARPS), (size_t)2 * tb.tokens * tb.floats * sizeof(float),
-                       stream, a, conv, dts, o_raw, slices);
+    const int slices = (a.v_dim + SSD_COLS - 1) / SSD_COLS;
+    if ((long long)entries * a.heads * slices > (long long)SSD_CROWD * kipp_sm_count())
+        return launch_ssd_form<LEAVES, 2, R>(a, conv, dts, o_raw, entries, tokens, stream);
+    return launch_ssd_form<LEAVES, 1, R>(a, conv, dts, o_raw, entries, tokens, stream);
 }
 // 16 columns a block, or a thread per column where that leaves an SM at most COLUMN_WARPS warps: below, a token's chain is what
 // the scan lasts, above the SMs' issue slots are.  The warps are those that work for as long as the longest entry, tokens /

@@ -1273,6 +1273,45 @@ def test_gated_norm_adds_in_one_order(heads, v_dim, norm_groups, lens):
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
 
 
+@pytest.mark.parametrize("D,v_dim,heads,n", [(128, 64, 4, 53), (32, 36, 3, 16), (64, 32, 2, 18), (100, 64, 2, 5), (256, 20, 2, 35), (16, 64, 1, 6)])
+def test_state_space_scans_add_in_one_order(D, v_dim, heads, n):
+    """The scan has a leaf of rows a thread where there are few blocks and two where they crowd the SMs: an entry's outputs and
+    its state have the same bits alone and among as many as that takes, for whole groups of four tokens and rests, heads
+    of whole leaves and others, columns that end inside a block's."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    lib = load_library("recurrent")
+    p, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+    lib.kipp_ssd_scan.argtypes = [p, ll, p, ll, i, i, i, i, p, p, i, p, p, p, p, i, p, ll, p, p, p, i, i, i, i, i, i, f, p, p, p]
+    lib.kipp_ssd_state_floats.restype = lib.kipp_recurrent_scratch_floats.restype = ll
+    taps, inner = 2, heads * v_dim
+    channels, sms = inner + 2 * D, torch.cuda.get_device_properties(0).multi_processor_count
+    stride = lib.kipp_ssd_state_floats(heads, 1, D, v_dim, taps)
+    g = torch.Generator().manual_seed(D + n)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)                      # noqa: E731
+    z_off, ld = channels + heads + (-heads) % 4, channels + heads + (-heads) % 4 + inner
+    rows, first = rnd(n, ld), rnd(1, stride)
+    weights = [rnd(taps, channels) * 0.5, rnd(channels) * 0.1, rnd(heads), rnd(heads) * 0.5, rnd(heads), rnd(inner)]
+    w = [t.data_ptr() for t in weights]
+
+    def run(E):
+        T = E * n
+        proj, state = rows.repeat(E, 1).contiguous(), first.repeat(E, 1).contiguous()
+        q_start = torch.arange(0, T + 1, n, dtype=torch.int32, device=DEV)
+        entry, slots = torch.arange(E, device=DEV).repeat_interleave(n).int(), torch.arange(E, dtype=torch.int32, device=DEV)
+        out, conv = torch.zeros(T, inner, device=DEV), torch.zeros(T, channels, device=DEV)
+        scratch = torch.zeros(lib.kipp_recurrent_scratch_floats(T, heads, D, v_dim, 4), device=DEV)
+        rc = lib.kipp_ssd_scan(out.data_ptr(), inner, proj.data_ptr(), ld, 0, z_off, 0, channels, w[0], w[1], taps, w[2], w[3], w[4], w[5],
+                               1, state.data_ptr(), stride, q_start.data_ptr(), entry.data_ptr(), slots.data_ptr(), E, T, heads, 1, D,
+                               v_dim, 1e-5, scratch.data_ptr(), conv.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0 and torch.isfinite(out).all()
+        return out.reshape(E, n, inner), state
+    (one, kept), E = run(2), 4 * sms // heads + 1
+    many, states = run(E)
+    assert torch.equal(many, one[:1].expand_as(many)) and torch.equal(states, kept[:1].expand_as(states))
+
+
 @pytest.mark.parametrize("size", [1, 100, 128, 2048, 2049, 2560, 5000])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_row_dot(dtype, size):
