@@ -17,12 +17,14 @@
 //
 // Work split.  grid = (token tiles, feature tiles, K splits).  With few tokens
 // there are too few tiles to pull the whole HBM bandwidth, so K is split over
-// the CTAs of one thread-block cluster (up to 8, along grid z).  Each CTA puts
-// its partial accumulator into its own shared memory; after a cluster barrier
-// CTA r adds, in split order, the partial sums of its share of the tokens out
-// of all the CTAs' shared memory (distributed shared memory) and runs the
-// epilogue for them.  No global scratch, no atomics, and the order of the sum
-// is fixed.
+// the CTAs of one thread-block cluster (up to 8, along grid z).  CTA r adds, in
+// split order, the partial sums of its share of the tokens and runs the epilogue
+// for them.  Up to 16 tokens a CTA SENDS its partial sums (st.async) into the
+// shared memory of those that finish them, which wait for the bytes; more tokens
+// are put into a CTA's own shared memory and read by the others (distributed shared
+// memory) between two cluster barriers.  No global scratch, no atomics, and the order
+// of the sum is fixed.  (Sending takes the two barriers and a trip through the
+// cluster off a chain that is all latency.)
 //
 // Warp roles (320 threads): warp 0 issues TMA loads, warp 1 allocates tensor
 // memory and issues the MMAs, warps 2-9 run the epilogue (warp w reads the
@@ -99,6 +101,10 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
         ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
 }
+// Asks for a tensor map ahead of its first copy, which would fetch it from memory on its own path.
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
 // Adds a float32 box from shared memory into global memory (the adds happen at
 // the L2; nothing is read back).  Tracked by the thread's bulk-group.
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const void* src, int x, int y) {
@@ -151,6 +157,11 @@ __device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t rank)
     uint32_t remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(bar)), "r"(rank));
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+}
+// Stores a float at a shared address of the cluster; its bytes are counted on `bar` (of the same CTA).
+__device__ __forceinline__ void store_remote(uint32_t addr, float v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(__float_as_uint(v)), "r"(bar)
+                 : "memory");
 }
 // The address, in the cluster's shared window, of `bar` at the same offset in CTA `rank`.
 __device__ __forceinline__ uint32_t mbar_in_cta(uint64_t* bar, uint32_t rank) {
@@ -269,6 +280,14 @@ template <int TILE_T, int TILE_F> struct Cfg {
     static constexpr int CTAS = (TILE_T >= 128 || TILE_F > 128) ? 1 : 2;
     static constexpr int ACC_COLS = TILE_T * HALVES;
     static constexpr int TMEM_COLS = ACC_COLS < 32 ? 32 : ACC_COLS;   // 32, 64, 128, 256 or 512
+    // Split products of up to 16 tokens send their partial sums; the ring's last stage is then the mailbox: rows of 128
+    // sums, one per token and split (at most TILE_T + 7 of them).  Steps of 36 layers of 2,560: one token, 2,048 keys:
+    // 2,231 -> 2,055 us, eight of 8,100 keys 3,557 -> 3,469, 13 of up to 5,003 keys 3,271 -> 3,258 (with what the attention's
+    // kernel gave in the same measurement, see there).  (With 32 columns: 24 tokens level, 32 slower by 2.5 %: the stage is
+    // missed.  A kernel of its own for split products, with its stages as a constant, costs more than it saves: two kernels
+    // taking turns in a layer, one token: 2,189 us.)
+    static constexpr bool SEND = TILE_T == 16 && TILE_F == UMMA_M;
+    static_assert(!SEND || (TILE_T + 7) * UMMA_M * 4 <= STAGE_BYTES, "the mailbox is a stage");
     // epilogue warp groups: two groups of four warps split the token columns
     static constexpr int COL_GROUPS = TILE_T >= 32 ? 2 : 1;
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ +
@@ -462,7 +481,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     uint64_t* full = (uint64_t*)(tiles + (size_t)C::STAGES * C::STAGE_BYTES);
     uint64_t* empty = full + C::STAGES;
     uint64_t* acc_ready = empty + C::STAGES;
-    uint32_t* tmem_slot = (uint32_t*)(acc_ready + 1);
+    uint64_t* mail_ready = acc_ready + 1;
+    uint32_t* tmem_slot = (uint32_t*)(mail_ready + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     float* rstd_s = (float*)(tiles + (size_t)C::STAGES * C::STAGE_BYTES + 256);   // [TILE_T], see Params::ssq_in
 
@@ -486,17 +506,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         else n_kb = 0;
     }
 
+    const bool send = C::SEND && p.splits > 1;
+    const int stages = send ? C::STAGES - 1 : C::STAGES;
+    float* mailbox = (float*)(tiles + (size_t)(C::STAGES - 1) * C::STAGE_BYTES);    // [token][split][128], where sums are sent
+    // the tokens of the tile that this CTA of a split product finishes; where sums are sent, those there are
+    const int per = (TILE_T + p.splits - 1) / p.splits;
+    const int j_first = split * per, j_end = min(min(TILE_T, j_first + per), C::SEND ? p.tokens - t0 : TILE_T);
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         mbar_init(acc_ready, 1);
+        if (send) mbar_init(mail_ready, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (send && j_end > j_first) mbar_expect_tx(mail_ready, (uint32_t)((j_end - j_first) * p.splits * UMMA_M * 4));
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // (the CTAs of a cluster may send once all their barriers exist: waited for where the first value goes out)
+    if (send) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    bool may_send = false;                         // this warp has made that wait
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -504,8 +535,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             // Weights do not depend on the kernels before this one: the first
             // ring of weight tiles is on its way before the dependency wait; the
             // activation tiles follow after it.
-            const int ahead = min(n_kb, C::STAGES);
+            const int ahead = min(n_kb, stages);
             if (elect_one()) {
+                tma_prefetch_map(&map_x);
                 for (int i = 0; i < ahead; ++i) {
                     uint8_t* wt = tiles + (size_t)i * C::STAGE_BYTES;
                     mbar_expect_tx(&full[i], C::STAGE_BYTES);
@@ -521,10 +553,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             }
             __syncwarp();
+            int s = 0;                             // stage of K block i, and its phase: no division by the number of stages
+            uint32_t ph = 0;
             for (int i = ahead; i < n_kb; ++i) {
-                const int s = i % C::STAGES;
-                const uint32_t ph = (i / C::STAGES) & 1;
-                if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ph ^ 1, abort_flag))) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(&empty[s], ph, abort_flag))) break;
                 uint8_t* wt = tiles + (size_t)s * C::STAGE_BYTES;
                 uint8_t* xt = wt + C::W_BYTES;
                 const int k = (kb_begin + i) * TILE_K;
@@ -534,6 +566,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     tma_load_2d(xt, &map_x, &full[s], k, t0);
                 }
                 __syncwarp();
+                if (++s == stages) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
@@ -541,9 +574,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         {
             constexpr uint32_t idesc = umma_idesc(UMMA_M, TILE_T);
             bool ok = true;
+            int s = 0;
+            uint32_t ph = 0;
             for (int i = 0; i < n_kb && ok; ++i) {
-                const int s = i % C::STAGES;
-                const uint32_t ph = (i / C::STAGES) & 1;
                 if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
                 tcgen05_fence_after();
                 const uint32_t wa = smem_u32(tiles + (size_t)s * C::STAGE_BYTES);
@@ -562,6 +595,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     umma_commit(&empty[s]);            // stage reusable when these MMAs are done
                 }
                 __syncwarp();
+                if (++s == stages) { s = 0; ph ^= 1; }
             }
             if (ok && n_kb > 0 && elect_one()) umma_commit(acc_ready);   // nobody waits where there was no K block
             __syncwarp();
@@ -582,7 +616,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             asm volatile("bar.sync 1, 256;" ::: "memory");
         }
         const float* rstd_tile = p.ssq_in != nullptr ? rstd_s : nullptr;
-        bool ok = n_kb > 0 ? mbar_wait(acc_ready, 0, abort_flag) : true;
+        const bool ok = __all_sync(0xffffffffu, n_kb > 0 ? mbar_wait(acc_ready, 0, abort_flag) : true);
         tcgen05_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
         constexpr int COLS_PER_GROUP = TILE_T / C::COL_GROUPS;
@@ -601,6 +635,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         }
                         epilogue_chunk(p, v, t0 + c, f, lane, rstd_tile ? rstd_tile + c : nullptr);
                     }
+                }
+            } else if constexpr (C::SEND) {
+                asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+                may_send = true;
+                // the partial sums of every token there is straight to the CTA that finishes it
+                const uint32_t box = smem_u32(mailbox + split * UMMA_M + q * 32 + lane);
+                static_assert(COLS_PER_GROUP == 16, "a warp's share of the columns is read at once");
+                float v[16];
+                tmem_ld16(taddr + cg * 16, v);
+                uint32_t to = 0, bar = 0;
+                int dst = -1;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int j = cg * 16 + i;
+                    if (t0 + j >= p.tokens) break;
+                    if (j / per != dst) {
+                        dst = j / per;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(box), "r"(dst));
+                        bar = mbar_in_cta(mail_ready, (uint32_t)dst);
+                    }
+                    store_remote(to + (uint32_t)((j - dst * per) * p.splits * UMMA_M * 4), v[i], bar);
                 }
             } else {
                 // partial sums of this split into this CTA's shared memory, [token][feature]
@@ -627,8 +682,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         float next_norm_w = 0.f;
         if (warp >= 2 && p.epilogue == EPI_ADD) {
             const int f = f0 + (warp & 3) * 32 + lane;
-            const int per = (TILE_T + p.splits - 1) / p.splits;
-            const int j0 = split * per, j1 = min(TILE_T, j0 + per);
+            const int j0 = j_first, j1 = j_end;
             if (f < p.features) {
 #pragma unroll
                 for (int k = 0; k < PRE; ++k) {
@@ -638,15 +692,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (p.xn != nullptr) next_norm_w = load_w(p.norm_w, p.norm_w_dtype, f);
             }
         }
-        // all threads of all CTAs of the cluster: partial sums are visible afterwards
-        asm volatile("barrier.cluster.arrive.release.aligned;\n"
-                     "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-        if (warp >= 2 && !*abort_flag) {
+        bool there = true;
+        if constexpr (C::SEND) {
+            // What this CTA finishes arrives on its own barrier: nobody waits for a neighbour's threads, before or after, and a
+            // CTA with nothing to finish is through.
+            if (!may_send) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            if (warp >= 2 && j_end > j_first) there = __all_sync(0xffffffffu, mbar_wait(mail_ready, 0, abort_flag));
+        } else {
+            // all threads of all CTAs of the cluster: partial sums are visible afterwards
+            asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                         "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        }
+        if (warp >= 2 && there && !*abort_flag) {
             const int q = warp & 3;
             const int cg = (warp - 2) >> 2;                             // two warp groups share the tokens
             const int f = f0 + q * 32 + lane;
-            const int per = (TILE_T + p.splits - 1) / p.splits;       // tokens this CTA finishes
-            const int j0 = split * per, j1 = min(TILE_T, j0 + per);
+            const int j0 = j_first, j1 = j_end;
+            const float* box = mailbox + q * 32 + lane;
             const uint32_t local = smem_u32(reinterpret_cast<float*>(tiles) + q * 32 + lane);
             // this CTA's view of every split's partial tile (at most 8 splits)
             uint32_t remote[8];
@@ -661,7 +723,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
                 for (int s = 0; s < 8; ++s) {
                     part[s] = 0.f;
-                    if (s < p.splits)
+                    if constexpr (C::SEND) {
+                        if (s < p.splits) part[s] = box[((j - j0) * p.splits + s) * UMMA_M];
+                    } else if (s < p.splits)
                         asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part[s])
                                      : "r"(remote[s] + (uint32_t)(j * UMMA_M * 4)) : "memory");
                 }
@@ -709,9 +773,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             }
         }
-        // nobody's shared memory may go away while a neighbour still reads it
-        asm volatile("barrier.cluster.arrive.release.aligned;\n"
-                     "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        // nobody's shared memory may go away while a neighbour still reads it (what is sent goes to a CTA that waits for it)
+        if (!C::SEND)
+            asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                         "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     }
 
     tcgen05_fence_before();
@@ -1072,6 +1137,8 @@ gemm_tc_tokm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     mbar_expect_tx(&full[i], C::STAGE_BYTES);
                     tma_load_2d(tiles + (size_t)i * C::STAGE_BYTES + C::X_BYTES, &map_w, &full[i], i * TILE_K, f0);
                 }
+                tma_prefetch_map(&map_x);
+                if (REDUCE) tma_prefetch_map(&map_c);
                 pdl_wait();
                 for (int i = 0; i < ahead; ++i)
                     tma_load_2d(tiles + (size_t)i * C::STAGE_BYTES, &map_x, &full[i], i * TILE_K, t0);
@@ -1530,7 +1597,9 @@ extern "C" int kipp_gemm_tc_plan(int tokens, int features, int K, int want_split
     if (splits <= 0) {
         // Few tiles: split K so that tiles x splits comes close to, but stays
         // under, what is resident at once with clusters (measured: 48 tiles run
-        // fastest with 5 splits = 240 CTAs, slower with 6 = 288; 20 tiles with 8).
+        // fastest with 5 splits = 240 CTAs, slower with 6 = 288; 20 tiles with 8;
+        // again with sums that are sent: a step of one token 2,050 us, 2,095 with up to
+        // 192 CTAs, 2,114 with 160, 2,246 with 296).
         // Every split keeps at least 4 K blocks.
         const int tiles = f_tiles * t_tiles;
         splits = 1;

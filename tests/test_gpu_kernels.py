@@ -172,6 +172,26 @@ def test_gemm_simt_chain(dtype, shape, w_rows):
 
 
 @pytest.mark.parametrize("epilogue", ["store", "add", "swiglu"])
+@pytest.mark.parametrize("splits", [2, 3, 5, 6, 7, 8])
+def test_gemm_sends_partial_sums(splits, epilogue):
+    """Up to 16 tokens the CTAs of a split product send their sums to the one that finishes a token: every share of tokens
+    (some CTAs have none, the last ones fewer), features that end inside a tile; whole numbers come out exactly."""
+    from kipp_b200.kernels import gemm_bf16
+    N, K = 200, 64 * splits * 3
+    g = torch.Generator().manual_seed(splits)
+    a = torch.randint(-3, 4, (16, K), generator=g).to(torch.bfloat16).to(DEV)
+    w = torch.randint(-2, 3, (N, K), generator=g).to(torch.bfloat16).to(DEV)
+    for M in (1, 2, 3, 7, 8, 9, 15, 16):
+        out = torch.randint(-5, 6, (M, N // 2 if epilogue == "swiglu" else N), generator=g).float().to(DEV)
+        ref = gemm_ref(a[:M], w, epilogue, out)
+        gemm_bf16.run("tc", out, a[:M], w, epilogue, M, splits=splits)
+        if epilogue == "swiglu":
+            assert torch.allclose(out.double().cpu(), ref, rtol=1e-5, atol=1e-4), M       # (the silu's division and exponential)
+        else:
+            assert torch.equal(out.double().cpu(), ref), M
+
+
+@pytest.mark.parametrize("epilogue", ["store", "add", "swiglu"])
 @pytest.mark.parametrize("shape", [(1, 128, 64), (8, 256, 128), (17, 250, 192), (64, 1000, 136),
                                    (100, 384, 2568), (300, 640, 520), (5, 2560, 1216), (40, 14400, 136),
                                    (100, 14400, 72)])
