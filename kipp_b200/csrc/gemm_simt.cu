@@ -14,22 +14,18 @@
 //
 // Three kernels, chosen by shape and alignment alone, with that one order for 32-bit weights whose rows start on 16 bytes:
 //   few   float32, up to FEW_MAX tokens (16 of many features): bound by the weights' bytes (a token is 2 operations per 4
-//         bytes).  A block holds 16 features, a thread one feature and one run, so a 2,048-feature matrix still gives 128
-//         blocks of 256 chains; the weights travel by asynchronous copies, four chunks of 64 bytes per thread on their way
-//         (three of two features where a thread has pairs), the first of them before the wait for the kernel before.
-//         12,288 x 2,048 with 1, 3 and 16 tokens: 24, 28 and 95 us (100 MB: 15 us of copy rate; the kernel below, which ran
-//         before: 334, 339 and 353); 2,048 x 6,144 with 3: 24 us (543).  From 17 tokens on it needs two passes, which still
-//         win where the features are few (32 tokens, 2,048 and 3,072 x 2,048: 31 and 48 us against 58 and 74 in tiles) and
-//         lose where they are many (12,288 and 32,000: 180 and 442 us against 104 and 260): from many_features() on those
-//         are tiles'.
-//   tile  float32, more tokens: bound by warps in flight.  At 407 tokens, 12,288 x 2,048 (608 us, 34 of 74 TFLOP/s) the FMA
-//         pipes are busy 57 % of the time and shared memory's data pipe 62 %; the three blocks of four warps that registers
-//         and shared memory leave an SM give a scheduler 2.8 warps, and one of them can issue in 46 % of the cycles.
-//         128 features x 64 tokens per block of 128 threads, 8 x 8 per thread in float32 pairs, operands in shared memory
-//         with k outermost, so that a k's 16 values cost a thread four 16-byte reads (with four bytes copied at a time: 24
-//         copies per 1,024 FMAs); the groups of runs are blocks of their own, a cluster that meets in its shared memory.
-//         407 tokens, 12,288 x 2,048: 608 us (943 before), 2,048 x 6,144: 392 us (866; 540 with
-//         tiles of 64 x 64, 8 x 4 per thread and k innermost); 64 tokens, 12,288 x 2,048: 106 us (387; 181).
+//         bytes) and, of several tokens, by shared memory's reads.  A block holds 16 features, a thread one feature and one
+//         run, so a 2,048-feature matrix still gives 128 blocks of 256 chains; weights and tokens travel by asynchronous copies,
+//         the weights' first ones before the wait for the kernel before (few_stages).
+//         12,288 x 2,048 with 1, 3 and 16 tokens: 20, 27 and 48 us (100 MB: 15 us of copy rate; the kernel below, which ran
+//         once: 334, 339 and 353); 2,048 x 6,144 with 3: 17 us.  From 17 tokens on it needs two passes, which still
+//         win where the features are few and lose where they are many: from many_features() on those are tiles'.
+//   tile  float32, more tokens: 128 or 256 features x 64 tokens per block of 128 threads, 8 or 16 x 8 per thread in float32
+//         pairs, operands in shared memory with k outermost, so that a k's values cost a thread four or six 16-byte reads
+//         (with four bytes copied at a time); the groups of runs are blocks of their own, a cluster that meets in its
+//         shared memory.  Bound by the issue around the multiply-adds and shared memory's reads: 407 tokens,
+//         12,288 x 2,048 in tiles of 128: FMA pipes 57 % busy, shared memory's data pipe 62 %.  1,024 tokens: 37.7 of 74 TFLOP/s
+//         in tiles of 128, 40.2 in 256.
 //   any   what is left: tokens whose float32 rows do not start on 16 bytes, in the order above; and what no other kernel
 //         here takes, bfloat16 operands of shapes that the tensor-core kernels refuse and float32 weights off 16 bytes: one
 //         chain of FMAs in the order of k, without the 38 registers and the extra sums of the runs (bfloat16, 2,050 features
@@ -158,23 +154,40 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
 constexpr int FEW_F = 16, FEW_THREADS = 16 * MAX_RUNS, FEW_MAX = 32;
 inline int many_features() { return 64 * kipp_sm_count(); }         // two blocks of pairs of features for each SM
 constexpr int FEW_CHUNK = BK * 4 + 16;              // 64 bytes of a feature's row, padded against bank conflicts
-template <bool PAIR> struct Few {
-    static constexpr int PER = PAIR ? 2 : 1, F = FEW_F * PER, STAGES = PAIR ? 4 : 5, CHUNKS = 32 * PER;
-    static constexpr int SMEM = (FEW_THREADS / 32) * STAGES * CHUNKS * FEW_CHUNK;
+// A warp's stage: its chunks of weights, then 16 values of each of MT tokens for its two runs.  (The tokens' values came
+// from global memory before, four at a time and the next four on their way: a trip to the L2 for every four, since a
+// block reads each of them once.)
+template <bool PAIR, int MT> struct Few {
+    static constexpr int PER = PAIR ? 2 : 1, F = FEW_F * PER, CHUNKS = 32 * PER;
+    static constexpr int X_AT = CHUNKS * FEW_CHUNK, STAGE = X_AT + MT * 2 * BK * 4;
+    static constexpr int BLOCK_STAGE = (FEW_THREADS / 32) * STAGE;        // bytes of a stage of the block's eight warps
 };
 
-template <int MT, int EPI, bool PAIR>
+// Waits until at most `n` of the thread's groups of copies are on their way (n from 0 to 6).
+__device__ __forceinline__ void cp_async_wait_most(int n) {
+    switch (n) {
+    case 0: cp_async_wait<0>(); break;
+    case 1: cp_async_wait<1>(); break;
+    case 2: cp_async_wait<2>(); break;
+    case 3: cp_async_wait<3>(); break;
+    case 4: cp_async_wait<4>(); break;
+    case 5: cp_async_wait<5>(); break;
+    default: cp_async_wait<6>(); break;
+    }
+}
+// (One function for all epilogues: a layer's four products then find its code where the one before left it.)
+template <int MT, bool PAIR>
 __global__ void __launch_bounds__(FEW_THREADS)
 gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
-                int M, int N, int K, int lda, int ldw, int ldc) {
-    using Form = Few<PAIR>;
+                int M, int N, int K, int lda, int ldw, int ldc, int epi, int stages) {
+    using Form = Few<PAIR, MT>;
     extern __shared__ __align__(16) uint8_t ring[];
     __shared__ float parts[MAX_RUNS][MT][Form::F + 1];
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n0 = blockIdx.x * Form::F, m0 = blockIdx.y * MT;
     const int run = run_length(K), steps = run / BK;
-    uint8_t* mine = ring + (size_t)warp * Form::STAGES * Form::CHUNKS * FEW_CHUNK;
+    uint8_t* mine = ring + (size_t)warp * stages * Form::STAGE;
     // copy j of a step: 16 bytes (lane & 3) of chunk 8 j + lane / 4; chunk c is feature c & 15 (the second 32: 16 + c & 15)
     // of run 2 warp + c / 16 & 1
     auto fetch = [&](int step, int stage) {
@@ -183,64 +196,62 @@ gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
             const int c = 8 * j + (lane >> 2), n = n0 + (c & 15) + (c >> 5) * FEW_F;
             const int k = (2 * warp + (c >> 4 & 1)) * run + step * BK + (lane & 3) * 4;
             const bool in = n < N && k < K;
-            cp_async16(smem_address(mine + (size_t)(stage * Form::CHUNKS + c) * FEW_CHUNK + (lane & 3) * 16),
-                       in ? W + (size_t)n * ldw + k : W, in ? 16 : 0);
+            cp_async16(smem_address(mine + (size_t)stage * Form::STAGE + c * FEW_CHUNK + (lane & 3) * 16),
+                               in ? W + (size_t)n * ldw + k : W, in ? 16 : 0);
         }
     };
+    // piece i of a step's tokens: 16 bytes (i & 3) of run 2 warp + (i / 4 & 1) of token i / 8
+    auto fetch_x = [&](int step, int stage) {
 #pragma unroll
-    for (int s = 0; s < Form::STAGES - 1; ++s) {
-        if (s < steps) fetch(s, s);
-        cp_async_commit();
-    }
+        for (int j = 0; j < (MT * 8 + 31) / 32; ++j) {
+            const int i = lane + 32 * j, k = (2 * warp + (i >> 2 & 1)) * run + step * BK + (i & 3) * 4;
+            if (i >= MT * 8) break;
+            cp_async16(smem_address(mine + (size_t)stage * Form::STAGE + Form::X_AT + i * 16),
+                       k < K ? A + (size_t)min(m0 + (i >> 3), M - 1) * lda + k : A, k < K ? 16 : 0);
+        }
+    };
+    for (int s = 0; s < min(stages - 1, steps); ++s) fetch(s, s);
     pdl_wait();
     const int r = 2 * warp + (lane >> 4);                 // this thread's run of feature lane & 15
-    const float* x[MT];
-#pragma unroll
-    for (int m = 0; m < MT; ++m) x[m] = A + (size_t)min(m0 + m, M - 1) * lda;
+    for (int s = 0; s < stages - 1; ++s) {
+        if (s < steps) fetch_x(s, s);
+        cp_async_commit();                                // (the first group holds all the weights)
+    }
     float acc[Form::PER][MT];
 #pragma unroll
     for (int f = 0; f < Form::PER; ++f)
 #pragma unroll
         for (int m = 0; m < MT; ++m) acc[f][m] = 0.f;
-    // (the tokens' next four values are asked for while the present ones are multiplied; left to itself the compiler
-    // held back the loads of four tokens to save registers: 39 us against 34 for 3 tokens of 12,288 x 2,048)
-    constexpr bool AHEAD = MT <= 8;
-    float4 next[AHEAD ? MT : 1];
-    auto load_next = [&](int k) {
-        if constexpr (AHEAD) {
-#pragma unroll
-            for (int m = 0; m < MT; ++m) next[m] = k < K ? *reinterpret_cast<const float4*>(x[m] + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    };
-    load_next(r * run);
+    int stage_at = 0;
     for (int step = 0; step < steps; ++step) {
-        cp_async_wait<Form::STAGES - 2>();
+        cp_async_wait_most(stages - 2);
         __syncwarp();
         const int k0 = r * run + step * BK;
-        const uint8_t* chunk = mine + (size_t)((step % Form::STAGES) * Form::CHUNKS + lane) * FEW_CHUNK;
+        const uint8_t* stage = mine + (size_t)stage_at * Form::STAGE;
+        const uint8_t* chunk = stage + lane * FEW_CHUNK;
+        const uint8_t* x = stage + Form::X_AT + (lane >> 4) * (BK * 4);
 #pragma unroll
         for (int q = 0; q < BK / 4; ++q) {
             if (k0 + 4 * q >= K) break;                   // whole quarters: K is a multiple of 4
             float4 w[Form::PER];
 #pragma unroll
             for (int f = 0; f < Form::PER; ++f) w[f] = *reinterpret_cast<const float4*>(chunk + 32 * f * FEW_CHUNK + 16 * q);
-            float4 now[AHEAD ? MT : 1];
-            if constexpr (AHEAD) {
-#pragma unroll
-                for (int m = 0; m < MT; ++m) now[m] = next[m];
-                load_next(k0 + 4 * q + 4);
-            }
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                const float4 v = AHEAD ? now[AHEAD ? m : 0] : *reinterpret_cast<const float4*>(x[m] + k0 + 4 * q);
+                const float4 v = *reinterpret_cast<const float4*>(x + m * 2 * BK * 4 + 16 * q);
 #pragma unroll
                 for (int f = 0; f < Form::PER; ++f)
                     acc[f][m] = fmaf(v.w, w[f].w, fmaf(v.z, w[f].z, fmaf(v.y, w[f].y, fmaf(v.x, w[f].x, acc[f][m]))));
             }
         }
         __syncwarp();                                     // the stage before this one is read: fill it again
-        if (step + Form::STAGES - 1 < steps) fetch(step + Form::STAGES - 1, (step + Form::STAGES - 1) % Form::STAGES);
+        if (step + stages - 1 < steps) {
+            const int free = stage_at == 0 ? stages - 1 : stage_at - 1;
+            fetch(step + stages - 1, free);
+            fetch_x(step + stages - 1, free);
+        }
         cp_async_commit();
+        if (++stage_at == stages) stage_at = 0;
     }
     cp_async_wait<0>();
 #pragma unroll
@@ -261,23 +272,27 @@ gemm_few_kernel(float* __restrict__ C, const float* __restrict__ A, const float*
             }
             return v;
         };
-        if (EPI == EPI_SWIGLU) {
+        if (epi == EPI_SWIGLU) {
             if ((f & 1) || n + 1 >= N) continue;
             put<float, EPI_STORE>(C, ldc, m0 + m, n >> 1, swiglu(total(f), total(f + 1)));
         } else if (n < N) {
-            put<float, EPI>(C, ldc, m0 + m, n, total(f));
+            if (epi == EPI_ADD) put<float, EPI_ADD>(C, ldc, m0 + m, n, total(f));
+            else put<float, EPI_STORE>(C, ldc, m0 + m, n, total(f));
         }
     }
 }
 
 // ---------------------------------------------------------------------------------------
-// Many tokens.  Thread (r, c) has features r .. r + 3 and 64 + r .. of the block's 128, tokens c .. c + 3 and 32 + c .. of
-// its 64.  A block has one group of runs; the blocks of the groups are a cluster along z, and each of them finishes a
+// Many tokens.  Thread (r, c) has features r .. r + 3, 64 + r .., (128 + r .., 192 + r ..) of the block's 64 FG, tokens
+// c .. c + 3 and 32 + c .. of its 64.  A block has one group of runs; the blocks of the groups are a cluster along z, and each of them finishes a
 // share of the tokens.  A group's sums lie in shared memory (one word per thread and value: 64 registers fewer).
-constexpr int TILE_F = 128, TILE_T = 64, TILE_K = 16, TILE_STAGES = 3, TILE_THREADS = 128;
-constexpr int TILE_W = TILE_F + 4, TILE_X = TILE_T + 4;               // padded: eight k's of four rows meet every bank once
-constexpr int TILE_STAGE = TILE_K * (TILE_W + TILE_X), TILE_VALUES = 64;
-constexpr int TILE_SMEM = (TILE_STAGES * TILE_STAGE + TILE_VALUES * TILE_THREADS) * 4;
+constexpr int TILE_T = 64, TILE_K = 16, TILE_THREADS = 128;
+template <int FG> struct Tile {                                       // FG groups of four features a thread
+    static constexpr int F = 64 * FG, PER = 4 * FG, STAGES = FG == 2 ? 3 : 2, BLOCKS = FG == 2 ? 3 : 2;
+    static constexpr int W = F + 4, X = TILE_T + 4;                   // padded: eight k's of four rows meet every bank once
+    static constexpr int STAGE = TILE_K * (W + X), VALUES = 8 * PER;
+    static constexpr int SMEM = (STAGES * STAGE + VALUES * TILE_THREADS) * 4;
+};
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int src_bytes) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -289,10 +304,13 @@ __device__ __forceinline__ float2 fma_pair(float2 a, float2 b, float2 c) {
     return d;
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(TILE_THREADS, 3)
+template <int EPI, int FG>
+__global__ void __launch_bounds__(TILE_THREADS, Tile<FG>::BLOCKS)
 gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W,
                  int M, int N, int K, int lda, int ldw, int ldc) {
+    using Form = Tile<FG>;
+    constexpr int TILE_F = Form::F, TILE_W = Form::W, TILE_X = Form::X, TILE_STAGE = Form::STAGE, TILE_STAGES = Form::STAGES;
+    constexpr int PER = Form::PER, TILE_VALUES = Form::VALUES;
     extern __shared__ __align__(16) float tiles[];        // [stage][W by k, X by k], then [value][thread]: a group's sum
     float* sums = tiles + TILE_STAGES * TILE_STAGE;
     pdl_launch_dependents();
@@ -324,13 +342,13 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
         if (s < steps) fetch(s, s);
         cp_async_commit();
     }
-    // acc[i][j]: features 2 i, 2 i + 1 of the thread's eight, token j of its eight
-    float2 acc[4][8];
+    // acc[i][j]: features 2 i, 2 i + 1 of the thread's, token j of its eight
+    float2 acc[PER / 2][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < PER / 2; ++i)
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
-    // value v of a thread: token v / 8, feature v % 8
+    // value v of a thread: token v / PER, feature v % PER
 #pragma unroll
     for (int v = 0; v < TILE_VALUES; ++v) sums[v * TILE_THREADS + tid] = 0.f;
     const int r = (tid >> 3) * 4, c = (tid & 7) * 4;
@@ -341,24 +359,40 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
         cp_async_commit();
         const float* w = tiles + (step % TILE_STAGES) * TILE_STAGE;
         const float* x = w + TILE_K * TILE_W;
-#pragma unroll 4
-        for (int k = 0; k < TILE_K; ++k) {
-            const float4 w0 = *reinterpret_cast<const float4*>(w + k * TILE_W + r), w1 = *reinterpret_cast<const float4*>(w + k * TILE_W + 64 + r);
+        // (a k's values are on their way while the one before is multiplied)
+        struct Values { float2 f[PER / 2]; float t[8]; } even, odd;
+        auto take = [&](int k, Values& v) {
+#pragma unroll
+            for (int g = 0; g < FG; ++g) {
+                const float4 w4 = *reinterpret_cast<const float4*>(w + k * TILE_W + 64 * g + r);
+                v.f[2 * g] = make_float2(w4.x, w4.y);
+                v.f[2 * g + 1] = make_float2(w4.z, w4.w);
+            }
             const float4 x0 = *reinterpret_cast<const float4*>(x + k * TILE_X + c), x1 = *reinterpret_cast<const float4*>(x + k * TILE_X + 32 + c);
-            const float2 f[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
-            const float t[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+            v.t[0] = x0.x; v.t[1] = x0.y; v.t[2] = x0.z; v.t[3] = x0.w;
+            v.t[4] = x1.x; v.t[5] = x1.y; v.t[6] = x1.z; v.t[7] = x1.w;
+        };
+        auto multiply = [&](const Values& v) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[i][j] = fma_pair(f[i], make_float2(t[j], t[j]), acc[i][j]);
+                for (int i = 0; i < PER / 2; ++i) acc[i][j] = fma_pair(v.f[i], make_float2(v.t[j], v.t[j]), acc[i][j]);
+        };
+        take(0, even);
+#pragma unroll 2
+        for (int k = 0; k < TILE_K; k += 2) {
+            take(k + 1, odd);
+            multiply(even);
+            take(k + 2 < TILE_K ? k + 2 : k, even);
+            multiply(odd);
         }
         const int done = k_begin + (step + 1) * TILE_K;
         if (done % run == 0 || step + 1 == steps) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float* at = sums + (8 * j + 2 * i) * TILE_THREADS + tid;
+                for (int i = 0; i < PER / 2; ++i) {
+                    float* at = sums + (PER * j + 2 * i) * TILE_THREADS + tid;
                     at[0] += acc[i][j].x;
                     at[TILE_THREADS] += acc[i][j].y;
                     acc[i][j] = make_float2(0.f, 0.f);
@@ -376,18 +410,18 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
     const int per = (8 + groups - 1) / groups, j0 = (int)blockIdx.z * per, j1 = min(8, j0 + per);
     const bool vectors = (EPI == EPI_SWIGLU ? ldc % 2 == 0 && ((uintptr_t)C & 7) == 0 : ldc % 4 == 0 && ((uintptr_t)C & 15) == 0);
     for (int j = j0; j < j1; ++j) {
-        float g[8][MAX_RUNS / GROUP_RUNS];
+        float g[PER][MAX_RUNS / GROUP_RUNS];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < PER; ++i)
 #pragma unroll
             for (int z = 0; z < MAX_RUNS / GROUP_RUNS; ++z) {
                 g[i][z] = 0.f;
                 if (z < groups)
-                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(g[i][z]) : "r"(of[z] + (uint32_t)((8 * j + i) * TILE_THREADS * 4)) : "memory");
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(g[i][z]) : "r"(of[z] + (uint32_t)((PER * j + i) * TILE_THREADS * 4)) : "memory");
             }
-        float v[8];
+        float v[PER];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < PER; ++i) {
             v[i] = 0.f;
 #pragma unroll
             for (int z = 0; z < MAX_RUNS / GROUP_RUNS; ++z) v[i] += g[i][z];
@@ -395,7 +429,7 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
         const int m = m0 + (j < 4 ? c + j : 28 + c + j);
         if (m >= M) continue;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        for (int half = 0; half < FG; ++half) {
             const int n = n0 + 64 * half + r;
             const float* q = v + 4 * half;
             if (EPI == EPI_SWIGLU) {
@@ -421,20 +455,53 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
-template <int MT, int EPI, bool PAIR>
-int launch_few_form(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
-    using F = Few<PAIR>;
-    if (const int e = kipp_allow_smem(gemm_few_kernel<MT, EPI, PAIR>, F::SMEM)) return e;
-    return kipp_launch(gemm_few_kernel<MT, EPI, PAIR>, dim3((N + F::F - 1) / F::F, (M + MT - 1) / MT), dim3(FEW_THREADS),
-                       F::SMEM, s, 1, C, A, W, M, N, K, lda, ldw, ldc);
+// Stages of a warp's ring.  A block that has its SM to itself takes what shared memory there is, so that enough of the weights
+// is on its way; where blocks follow one another on an SM, several at once hide one's start and end behind the others', the
+// more of them the more follow.  us per launch with 2 / 3 / 4 / 5 stages and more, weights in rotation: 3 tokens, 2,048 x
+// 2,048: - / 9.1 / 8.7 / 7.3, x 6,144: - / 23.2 / 22.9 / 17.3, 12,288 x 2,048: - / 27.0 / 27.5 / 40.1, 32,000 x 2,048:
+// 53.9 / 60.8 / 61.2 / 96; one token, 12,288 and 32,000: 23.1 / 20.1 / 22.2 / 21.8 and 42.0 / 43.2 / 45.8 / 45.9.
+inline int few_stages(long long blocks, int stage_bytes, int static_bytes) {
+    const long long per_sm = (blocks + kipp_sm_count() - 1) / kipp_sm_count();
+    const int at_once = per_sm <= 1 ? 1 : per_sm <= 8 ? 2 : 4, most = per_sm <= 2 ? 6 : 3;
+    const int fit = (227 * 1024 / at_once - static_bytes - 1024) / stage_bytes;
+    return fit < 2 ? 2 : fit > most ? most : fit;
 }
-template <int MT, int EPI>
-int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
-    // pairs of features where they still make two blocks for each SM (12,288 x 2,048 with 3 and 8 tokens: 28.3 and 37.9 us,
-    // one feature per thread 32.9 and 47.2; 32,000: 59 and 88 against 78 and 106)
-    constexpr bool MAY_PAIR = MT >= 2 && MT <= 8;
-    if (MAY_PAIR && N >= many_features()) return launch_few_form<MT, EPI, MAY_PAIR>(C, A, W, M, N, K, lda, ldw, ldc, s);
-    return launch_few_form<MT, EPI, false>(C, A, W, M, N, K, lda, ldw, ldc, s);
+template <int MT, bool PAIR>
+int launch_few_form(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int epi, cudaStream_t s) {
+    using F = Few<PAIR, MT>;
+    const dim3 grid((N + F::F - 1) / F::F, (M + MT - 1) / MT);
+    const int stages = few_stages((long long)grid.x * grid.y, F::BLOCK_STAGE, MAX_RUNS * MT * (F::F + 1) * 4);
+    const size_t smem = (size_t)stages * F::BLOCK_STAGE;
+    constexpr int parts = MAX_RUNS * MT * (F::F + 1) * 4;                 // what the kernel declares beside the ring
+    if (const int e = kipp_allow_smem(gemm_few_kernel<MT, PAIR>, smem + parts)) return e;
+    return kipp_launch(gemm_few_kernel<MT, PAIR>, grid, dim3(FEW_THREADS), smem, s, 1, C, A, W, M, N, K, lda, ldw, ldc, epi, stages);
+}
+template <int MT>
+int launch_few(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int epi, cudaStream_t s) {
+    // pairs of features for 5 to 8 tokens of many features (6 tokens, 32,000 x 2,048: 58.0 us, 64.5 with one a thread; 12,288: level;
+    // 3 tokens: 55.3 and 53.9, 29.4 and 27.0)
+    constexpr bool MAY_PAIR = MT == 8;
+    if (MAY_PAIR && N >= many_features()) return launch_few_form<MT, MAY_PAIR>(C, A, W, M, N, K, lda, ldw, ldc, epi, s);
+    return launch_few_form<MT, false>(C, A, W, M, N, K, lda, ldw, ldc, epi, s);
+}
+
+template <int EPI, int FG>
+int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int groups, cudaStream_t s) {
+    using Form = Tile<FG>;
+    const dim3 grid((N + Form::F - 1) / Form::F, (M + TILE_T - 1) / TILE_T, groups);
+    if (grid.y > 65535) return KIPP_ERR_ARG;
+    if (const int e = kipp_allow_smem(gemm_tile_kernel<EPI, FG>, Form::SMEM)) return e;
+    return kipp_launch(gemm_tile_kernel<EPI, FG>, grid, dim3(TILE_THREADS), Form::SMEM, s, groups, C, A, W, M, N, K, lda, ldw, ldc);
+}
+// 128 or 256 features a block, by what the SM with the most blocks has to do: a block of 256 takes 1.88 of 128's time beside
+// another one, 2.3 alone.  us a product in tiles of 128 / 256: 399 tokens, 12,288 x 2,048: 617 / 588, 3,072 x 2,048: 173 / 175,
+// 2,048 x 6,144: 369 / 348; 64 tokens: 104 / 131, 58 / 70, 118 / 194; 1,024 tokens: 1,366 / 1,282, 355 / 338, 713 / 708.  The one
+// chosen is within 7 % of the better everywhere that was measured (64 to 1,024 tokens).
+inline int tile_features(int M, int N, int groups) {
+    const long long t_tiles = (M + TILE_T - 1) / TILE_T, sms = kipp_sm_count();
+    auto per_sm = [&](int f) { return (t_tiles * ((N + f - 1) / f) * groups + sms - 1) / sms; };
+    const double narrow = (double)per_sm(Tile<2>::F), wide = (double)per_sm(Tile<4>::F);
+    return (wide <= 1 ? 2.3 : 1.88 * wide) < narrow ? Tile<4>::F : Tile<2>::F;
 }
 
 // float32 rows that start on 16 bytes and hold whole groups of four: the kernels that copy 16 bytes at a time.
@@ -442,17 +509,15 @@ template <int EPI>
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
     if (M <= (N >= many_features() ? FEW_MAX / 2 : FEW_MAX)) {
         // tokens of a block: as many as there are, up to 16 (the accumulators of a thread)
-        if (M == 1) return launch_few<1, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
-        if (M == 2) return launch_few<2, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
-        if (M <= 4) return launch_few<4, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
-        if (M <= 8) return launch_few<8, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
-        return launch_few<16, EPI>(C, A, W, M, N, K, lda, ldw, ldc, s);
+        if (M == 1) return launch_few<1>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
+        if (M == 2) return launch_few<2>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
+        if (M <= 4) return launch_few<4>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
+        if (M <= 8) return launch_few<8>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
+        return launch_few<16>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
     }
     const int groups = (K + GROUP_RUNS * run_length(K) - 1) / (GROUP_RUNS * run_length(K));
-    const dim3 grid((N + TILE_F - 1) / TILE_F, (M + TILE_T - 1) / TILE_T, groups);
-    if (grid.y > 65535) return KIPP_ERR_ARG;
-    if (const int e = kipp_allow_smem(gemm_tile_kernel<EPI>, TILE_SMEM)) return e;
-    return kipp_launch(gemm_tile_kernel<EPI>, grid, dim3(TILE_THREADS), TILE_SMEM, s, groups, C, A, W, M, N, K, lda, ldw, ldc);
+    return tile_features(M, N, groups) == Tile<4>::F ? launch_tile<EPI, 4>(C, A, W, M, N, K, lda, ldw, ldc, groups, s)
+                                                     : launch_tile<EPI, 2>(C, A, W, M, N, K, lda, ldw, ldc, groups, s);
 }
 
 template <typename TA, typename TW, typename TC, bool RUNS>
