@@ -182,6 +182,190 @@ paged_attention_simt_kernel(T* __restrict__ out, const T* __restrict__ q,
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// The same for few blocks, where a block's chain of tiles is what the launch lasts: FEW_TILES tiles at a time and what of
+// them depends on nothing else side by side.  A warp scores a tile for every fourth head of the block (as many chains of FMAs
+// as it has heads, a key's 16 bytes read once for all of them); the tiles' maxima meet in shared memory, which gives each
+// tile the running maximum it has in the order of the tiles, and so its weights; then a thread per value of the
+// result walks the keys.  Every sum has the terms and the order it has in the kernel above: the same bits.  What is left of a
+// chain is a head's FMAs once per FEW_TILES tiles and one FMA per key.  The next tiles' keys travel beside the weighted
+// sums, their values beside the scores, and the first ones before the dependency wait.  Bound by the instructions of a block's
+// warps, one after the other: 3 tokens of up to 211 keys, 16 heads of 128: 11.5 us a launch, 35 in the kernel above.
+constexpr int FEW_TILES = 4, FEW_KEYS = FEW_TILES * TILE, FEW_THREADS = 512, FEW_WARPS = FEW_THREADS / 32;
+struct FewStats {
+    float tile_max[MAX_HEADS][FEW_TILES], running[MAX_HEADS][FEW_TILES], sum[MAX_HEADS][FEW_TILES];
+    unsigned seen[FEW_TILES];
+    long long rows[FEW_KEYS];
+};
+// heads of the block at most 4 NH; NACC as above: a thread's value is number tid % (32 NACC) of heads tid / (32 NACC), + HEAD_STEP, ...
+template <typename T, int NACC, int NH>
+__global__ void __launch_bounds__(FEW_THREADS, 1)
+paged_attention_few_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ k_pages, const T* __restrict__ v_pages,
+                           const int* __restrict__ positions, const int* __restrict__ entry_of_token, const int* __restrict__ block_table,
+                           int table_width, int page_size, int n_q, int n_kv, int head_dim, float scale, int window, int block_heads,
+                           int* __restrict__ status) {
+    extern __shared__ __align__(16) uint8_t smem[];   // q [heads][head_dim padded], weights [heads][FEW_KEYS], keys, values
+    __shared__ FewStats st;
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int group = n_q / n_kv, parts = (group + block_heads - 1) / block_heads;
+    const int t = (int)(blockIdx.x / (unsigned)(n_kv * parts)), rest = (int)(blockIdx.x % (unsigned)(n_kv * parts));
+    const int g = rest / parts, h0 = (rest % parts) * block_heads, heads = min(block_heads, group - h0);
+    const int pos = positions[t];                     // (the step's lists)
+    const int* table = block_table + (size_t)entry_of_token[t] * table_width;
+    const int first = window > 0 ? max(0, pos - window + 1) : 0, begin = first / TILE * TILE;
+    const int row_bytes = tile_row_bytes<T>(head_dim), q_stride = (head_dim + 3) & ~3;
+    float* qs = reinterpret_cast<float*>(smem);
+    float* weights = qs + (size_t)block_heads * q_stride;
+    uint8_t* kt = reinterpret_cast<uint8_t*>(weights + (size_t)block_heads * FEW_KEYS);
+    uint8_t* vt = kt + (size_t)FEW_KEYS * row_bytes;
+
+    // the page rows of FEW_KEYS keys from j0 on: -1 outside what the token sees, -2 not mapped
+    auto look_up = [&](int j0) {
+        if (tid < FEW_KEYS) {
+            const int j = j0 + tid;
+            long long row = -1;
+            if (j >= first && j <= pos) {
+                const int page = j / page_size < table_width ? table[j / page_size] : -1;
+                row = page < 0 ? -2 : (((long long)page * n_kv + g) * page_size + (j % page_size)) * head_dim;
+            }
+            st.rows[tid] = row;
+        }
+    };
+    // a warp takes whole rows; of keys [from, to) of the FEW_KEYS
+    auto fetch = [&](const T* pages, uint8_t* tile, int from, int to) {
+        for (int key = from + warp; key < to; key += FEW_WARPS) {
+            const long long row = st.rows[key];
+            const uint32_t dst = smem_address(tile + key * row_bytes);
+            const uint8_t* src = (const uint8_t*)pages + (row < 0 ? 0 : (size_t)row * sizeof(T));
+            for (int at = lane * 16; at < head_dim * (int)sizeof(T); at += 512) cp_async16(dst + at, src + (row < 0 ? 0 : at), row < 0 ? 0 : 16);
+        }
+    };
+    auto whole_tiles = [&](int j0) { return min(FEW_KEYS, (pos - j0) / TILE * TILE + TILE); };     // keys of the tiles from j0 on
+    // The first keys and values come before the dependency wait, all but those of this step's own tokens: the entry's tokens
+    // up to this one, which follow one another.
+    look_up(begin);
+    int own = pos;
+    for (int u = t - 1; u >= 0 && entry_of_token[u] == entry_of_token[t]; --u) own = positions[u];
+    const int n_first = whole_tiles(begin), kept = min(max(own - begin, 0), n_first);
+    __syncthreads();
+    fetch(k_pages, kt, 0, kept);
+    fetch(v_pages, vt, 0, kept);
+    pdl_wait();
+    fetch(k_pages, kt, kept, n_first);
+    cp_async_commit();
+    fetch(v_pages, vt, kept, n_first);
+    cp_async_commit();
+    const T* q_rows = q + ((size_t)t * n_q + g * group + h0) * head_dim;
+    for (int i = tid; i < heads * head_dim; i += FEW_THREADS) qs[i / head_dim * q_stride + i % head_dim] = to_f32(q_rows[i]);
+
+    constexpr int VALUES = 32 * NACC, HEAD_STEP = FEW_THREADS / VALUES, PER = (FEW_WARPS / FEW_TILES * NH + HEAD_STEP - 1) / HEAD_STEP;
+    const int d = tid % VALUES, my_head = tid / VALUES;
+    float acc[PER], m[PER], l[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) { acc[i] = 0.f; m[i] = -INFINITY; l[i] = 0.f; }
+    float m_before[NH];                               // the scoring warps' running maxima
+#pragma unroll
+    for (int i = 0; i < NH; ++i) m_before[i] = -INFINITY;
+    const int tile = warp & (FEW_TILES - 1), first_head = warp / FEW_TILES;
+    constexpr int SCORE_STEP = FEW_WARPS / FEW_TILES;
+
+    for (int j0 = begin; j0 <= pos; j0 += FEW_KEYS) {
+        const int tiles = whole_tiles(j0) / TILE;
+        cp_async_wait<1>();                           // the keys; the values may still be on their way
+        __syncthreads();
+        const long long row = st.rows[tile * TILE + lane];
+        float s[NH];
+#pragma unroll
+        for (int i = 0; i < NH; ++i) s[i] = -INFINITY;
+        if (tile < tiles) {
+            if (row == -2) atomicExch(status, 3);     // a needed key is not mapped
+            const T* krow = reinterpret_cast<const T*>(kt + (size_t)(tile * TILE + lane) * row_bytes);
+            float dot[NH];
+#pragma unroll
+            for (int i = 0; i < NH; ++i) dot[i] = 0.f;
+#pragma unroll 4
+            for (int x = 0; x < head_dim; x += 16 / (int)sizeof(T))
+#pragma unroll
+                for (int i = 0; i < NH; ++i) dot[i] = dot16(qs + min(first_head + SCORE_STEP * i, heads - 1) * q_stride + x, krow + x, dot[i]);
+#pragma unroll
+            for (int i = 0; i < NH; ++i) {
+                s[i] = row >= 0 ? dot[i] * scale : -INFINITY;
+                const float most = warp_max(s[i]);
+                if (lane == 0 && first_head + SCORE_STEP * i < heads) st.tile_max[first_head + SCORE_STEP * i][tile] = most;
+            }
+            const unsigned seen = __ballot_sync(0xffffffffu, row >= 0);
+            if (lane == 0) st.seen[tile] = seen;
+        }
+        __syncthreads();
+        const bool more = j0 + FEW_KEYS <= pos;
+        if (more) look_up(j0 + FEW_KEYS);
+#pragma unroll
+        for (int i = 0; i < NH; ++i) {
+            const int h = min(first_head + SCORE_STEP * i, heads - 1);
+            float m_new = m_before[i];
+            for (int x = 0; x < tiles; ++x) {
+                m_before[i] = fmaxf(m_before[i], st.tile_max[h][x]);
+                if (x <= tile) m_new = m_before[i];
+            }
+            const float p = m_new == -INFINITY || s[i] == -INFINITY ? 0.f : expf(s[i] - m_new);
+            const float sum = warp_sum(p);
+            if (tile < tiles && first_head + SCORE_STEP * i < heads) {
+                weights[h * FEW_KEYS + tile * TILE + lane] = p;
+                if (lane == 0) { st.sum[h][tile] = sum; st.running[h][tile] = m_new; }
+            }
+        }
+        cp_async_wait<0>();                           // the values
+        __syncthreads();
+        if (more) fetch(k_pages, kt, 0, whole_tiles(j0 + FEW_KEYS));
+        cp_async_commit();
+        for (int x = 0; x < tiles; ++x) {
+            const unsigned seen = st.seen[x];
+            const float* p[PER];
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const int h = min(my_head + HEAD_STEP * i, heads - 1);
+                p[i] = weights + h * FEW_KEYS + x * TILE;
+                const float m_new = st.running[h][x];
+                if (m_new == -INFINITY) continue;     // nothing visible yet: the weights are 0
+                const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+                l[i] = l[i] * corr + st.sum[h][x];
+                acc[i] *= corr;
+                m[i] = m_new;
+            }
+            const T* v = reinterpret_cast<const T*>(vt + (size_t)x * TILE * row_bytes) + min(d, head_dim - 1);
+            const size_t pitch = (size_t)row_bytes / sizeof(T);
+            if (seen == 0xffffffffu) {
+#pragma unroll 4
+                for (int jj = 0; jj < TILE; jj += 4) {
+                    const float value[4] = {to_f32(v[jj * pitch]), to_f32(v[(jj + 1) * pitch]), to_f32(v[(jj + 2) * pitch]), to_f32(v[(jj + 3) * pitch])};
+#pragma unroll
+                    for (int i = 0; i < PER; ++i) {
+                        const float4 w = *reinterpret_cast<const float4*>(p[i] + jj);
+                        acc[i] = fmaf(w.w, value[3], fmaf(w.z, value[2], fmaf(w.y, value[1], fmaf(w.x, value[0], acc[i]))));
+                    }
+                }
+            } else {
+                for (int jj = 0; jj < TILE; ++jj) {
+                    if (!(seen >> jj & 1u)) continue;
+                    const float value = to_f32(v[jj * pitch]);
+#pragma unroll
+                    for (int i = 0; i < PER; ++i) acc[i] = fmaf(p[i][jj], value, acc[i]);
+                }
+            }
+        }
+        __syncthreads();                              // the values, weights and maxima are read
+        if (more) fetch(v_pages, vt, 0, whole_tiles(j0 + FEW_KEYS));
+        cp_async_commit();
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int h = my_head + HEAD_STEP * i;
+        if (h < heads && d < head_dim)
+            out[((size_t)t * n_q + g * group + h0 + h) * head_dim + d] = from_f32<T>(acc[i] * (l[i] > 0.f ? 1.0f / l[i] : 0.f));
+    }
+}
+
 constexpr int SM_SMEM = 227 * 1024, SM_THREADS = 2048, SM_BLOCKS = 32;         // what an SM has for blocks
 
 template <typename T, bool VEC, int NACC>
@@ -191,6 +375,17 @@ int launch(void* out, const void* q, const void* k_pages, const void* v_pages, c
     const int group = n_q / n_kv, warps = group < MAX_HEADS ? group : MAX_HEADS;
     const long long blocks = (long long)tokens * n_kv * ((group + warps - 1) / warps);
     if (blocks > 0x7fffffffLL) return KIPP_ERR_ARG;
+    if constexpr (VEC && NACC <= 4) {
+        // a block for each SM at most: the chain of a block's tiles is all that counts
+        if (blocks <= kipp_sm_count()) {
+            const size_t few = ((size_t)warps * (((head_dim + 3) & ~3) + FEW_KEYS)) * 4 + (size_t)2 * FEW_KEYS * tile_row_bytes<T>(head_dim);
+            const auto kernel = warps <= 4 ? paged_attention_few_kernel<T, NACC, 1> : paged_attention_few_kernel<T, NACC, 2>;
+            if (const int e = kipp_allow_smem(kernel, few + sizeof(FewStats))) return e;      // (what it declares counts too)
+            return kipp_launch(kernel, dim3((unsigned)blocks), dim3(FEW_THREADS), few, s, 1, (T*)out, (const T*)q, (const T*)k_pages,
+                               (const T*)v_pages, positions, entry_of_token, block_table, table_width, page_size, n_q, n_kv, head_dim,
+                               scale, window, warps, status);
+        }
+    }
     const size_t queries = (size_t)warps * ((head_dim + 3) & ~3) * 4, tiles = (size_t)2 * TILE * tile_row_bytes<T>(head_dim);
     // Two stages where every block is on an SM at once even so, and a block's chain of tiles is what the launch lasts; else
     // one, which makes room for more blocks (float32 heads of 256 that share no keys, 16 of them, 400 tokens: 2,749 us with one

@@ -649,6 +649,30 @@ def test_attention_simt_stages(shape, dtype):
         assert torch.equal(among, out.repeat(times, 1, 1)) and st.tolist() == [0, 0, 0, 0]
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("shape", [dict(D=128, nq=16, nkv=2, page=16), dict(D=128, nq=4, nkv=1, page=8), dict(D=64, nq=2, nkv=2, page=16),
+                                   dict(D=40, nq=12, nkv=1, page=32), dict(D=128, nq=9, nkv=3, page=4)])
+def test_attention_simt_of_few_blocks(shape, dtype):
+    """A block for each SM at most: four tiles of keys at a time.  Contexts that end inside the first tile, at the ends of
+    tiles and of four of them, and windows that begin inside each: the bits that a token has among thousands, where
+    the tiles go one by one."""
+    D, nq, nkv, page = shape["D"], shape["nq"], shape["nkv"], shape["page"]
+    few, times = [(0, 1), (31, 1), (126, 3), (255, 2), (400, 1)], 500
+    for window in (None, 33, 150):
+        meta, table, q, kp, vp = attention_case(5, D, nq, nkv, page, few, dtype)
+        out, st = torch.zeros_like(q), status()
+        run = lambda o, x, m: ops().attention(o, x, kp, vp, m, meta.block_tables[0], page, nq, nkv, D, 1 / math.sqrt(D), window, st, impl="simt")   # noqa: E731
+        run(out, q, meta)
+        ref = attention_ref(meta, table, q, kp, vp, few, page, window, 1 / math.sqrt(D))
+        assert torch.allclose(out.double().cpu(), ref, **tol(dtype))
+        class Many:
+            tokens = meta.tokens * times
+            positions, entry_of_token = meta.positions[:meta.tokens].repeat(times), meta.entry_of_token[:meta.tokens].repeat(times)
+        among = torch.zeros(Many.tokens, nq, D, dtype=dtype, device=DEV)
+        run(among, q.repeat(times, 1, 1), Many)
+        assert torch.equal(among, out.repeat(times, 1, 1)) and st.tolist() == [0, 0, 0, 0]
+
+
 @pytest.mark.parametrize("window", [None, 37, 300])
 @pytest.mark.parametrize("shape", [dict(D=64, nq=4, nkv=2, page=16), dict(D=128, nq=8, nkv=2, page=16),
                                    dict(D=128, nq=16, nkv=1, page=8), dict(D=64, nq=3, nkv=3, page=32),
