@@ -315,22 +315,29 @@ struct DecodeParams {
 // The per-head norm and the rotation of one head vector, one warp: lane l holds
 // elements l, l + 32, ...; element e < D/2 pairs with e + D/2, which the same lane
 // holds.  Returns the values in x.
+template <int D> struct HeadInput { float x[D / 32], w[D / 32]; float2 cs[D / 64]; };
+// a norm's weights (they come before the dependency wait); ones where there is no norm
 template <int D>
-__device__ __forceinline__ void warp_norm_rope(float (&x)[D / 32], const void* norm_w, int norm_dtype, float eps,
-                                               const float2* cs_row, int lane) {
-    constexpr int NE = D / 32;
-    // the weights and the (cos, sin) pairs first: their loads travel while the sum is formed
-    float w[NE];
-    float2 cs[NE / 2];
-    if (norm_w != nullptr) {
+__device__ __forceinline__ void take_norm_weights(HeadInput<D>& in, const void* norm_w, int norm_dtype, int lane) {
 #pragma unroll
-        for (int j = 0; j < NE; ++j) w[j] = load_w(norm_w, norm_dtype, lane + 32 * j);
-    }
+    for (int j = 0; j < D / 32; ++j) in.w[j] = norm_w != nullptr ? load_w(norm_w, norm_dtype, lane + 32 * j) : 1.f;
+}
+template <int D>
+__device__ __forceinline__ void take_head(HeadInput<D>& in, const bf16* raw, const float2* cs_row, int lane) {
+#pragma unroll
+    for (int j = 0; j < D / 32; ++j) in.x[j] = __bfloat162float(raw[lane + 32 * j]);
     if (cs_row != nullptr) {
 #pragma unroll
-        for (int j = 0; j < NE / 2; ++j) cs[j] = cs_row[lane + 32 * j];
+        for (int j = 0; j < D / 64; ++j) in.cs[j] = cs_row[lane + 32 * j];
     }
-    if (norm_w != nullptr) {
+}
+template <int D>
+__device__ __forceinline__ void warp_norm_rope(HeadInput<D>& in, bool norm, float eps, bool turn) {
+    constexpr int NE = D / 32;
+    float (&x)[NE] = in.x;
+    const float (&w)[NE] = in.w;
+    const float2 (&cs)[NE / 2] = in.cs;
+    if (norm) {
         float ss = 0.f;
 #pragma unroll
         for (int j = 0; j < NE; ++j) ss += x[j] * x[j];
@@ -339,7 +346,7 @@ __device__ __forceinline__ void warp_norm_rope(float (&x)[D / 32], const void* n
 #pragma unroll
         for (int j = 0; j < NE; ++j) x[j] = x[j] * scale * w[j];
     }
-    if (cs_row != nullptr) {
+    if (turn) {
 #pragma unroll
         for (int j = 0; j < NE / 2; ++j) {
             const float a = x[j], b = x[j + NE / 2];
@@ -400,6 +407,12 @@ __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* sme
             cp_async_commit();
         }
     }
+    HeadInput<D> head, own;
+    const bool new_kv = p.qkv != nullptr && split == n_splits - 1 && p.k_write != nullptr && warp < 2;    // warp 0 the key, 1 the value
+    if (p.qkv != nullptr) {
+        take_norm_weights(head, p.q_norm_w, p.norm_dtype, lane);
+        if (new_kv && warp == 0) take_norm_weights(own, p.k_norm_w, p.norm_dtype, lane);
+    }
     if (first) pdl_wait();
     if (lo > hi) {                                         // split wholly behind the window
         for (int i = threadIdx.x; i < group; i += THREADS) {
@@ -414,37 +427,36 @@ __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* sme
         // Fused form: norm and rotation of the group's queries here, a warp per head, into
         // shared memory (behind the tiles); the split that holds the token's own position
         // also makes the new key and value and puts them into the cache.
+        // What a launch of few tokens lasts is the trips to the L2 one behind the other, so everything that comes out of the
+        // projection is asked for at once, the norms' weights before the wait (36 layers, one token behind 2,048 keys: 2,218 -> 2,189
+        // us a step; 4 layers, 77 keys: 179 -> 173).
         constexpr int NE = D / 32;
+        bf16* q_s = reinterpret_cast<bf16*>(smem + 2 * STAGES * TILE_BYTES);   // [16][D]
+        const bf16* raw = p.qkv + (size_t)tok * p.ld_qkv;
+        const float2* cs_row = p.cos_sin != nullptr ? p.cos_sin + (size_t)tok * (D / 2) : nullptr;
+        if (warp < group) take_head(head, raw + (size_t)(g * group + warp) * D, cs_row, lane);
+        if (new_kv) take_head(own, raw + (size_t)(p.n_q + (warp == 0 ? 0 : p.n_kv) + g) * D, warp == 0 ? cs_row : nullptr, lane);
         if (patch) {                                     // the tiles fetched early have landed, for every thread
             cp_async_wait<0>();
             __syncthreads();
         }
-        bf16* q_s = reinterpret_cast<bf16*>(smem + 2 * STAGES * TILE_BYTES);   // [16][D]
-        const bf16* raw = p.qkv + (size_t)tok * p.ld_qkv;
-        const float2* cs_row = p.cos_sin != nullptr ? p.cos_sin + (size_t)tok * (D / 2) : nullptr;
         for (int hh = warp; hh < group; hh += WARPS) {
-            float x[NE];
+            if (hh != warp) take_head(head, raw + (size_t)(g * group + hh) * D, cs_row, lane);
+            warp_norm_rope(head, p.q_norm_w != nullptr, p.eps, cs_row != nullptr);
 #pragma unroll
-            for (int j = 0; j < NE; ++j) x[j] = __bfloat162float(raw[(size_t)(g * group + hh) * D + lane + 32 * j]);
-            warp_norm_rope<D>(x, p.q_norm_w, p.norm_dtype, p.eps, cs_row, lane);
-#pragma unroll
-            for (int j = 0; j < NE; ++j) q_s[hh * D + lane + 32 * j] = __float2bfloat16_rn(x[j]);
+            for (int j = 0; j < NE; ++j) q_s[hh * D + lane + 32 * j] = __float2bfloat16_rn(head.x[j]);
         }
-        if (split == n_splits - 1 && p.k_write != nullptr && warp < 2) {
+        if (new_kv) {
             const int slot = pos / p.page_size;
             const int page = slot < p.table_width ? table[slot] : -1;
             if (page < 0) {                                        // unmapped page: refuse, never write
                 if (lane == 0) atomicExch(p.status, 2);
             } else {
                 const size_t at = (((size_t)page * p.n_kv + g) * p.page_size + (pos - slot * p.page_size)) * D;
-                float x[NE];
-                const bf16* src = raw + (size_t)(p.n_q + (warp == 0 ? 0 : p.n_kv) + g) * D;
-#pragma unroll
-                for (int j = 0; j < NE; ++j) x[j] = __bfloat162float(src[lane + 32 * j]);
-                if (warp == 0) warp_norm_rope<D>(x, p.k_norm_w, p.norm_dtype, p.eps, cs_row, lane);
+                if (warp == 0) warp_norm_rope(own, p.k_norm_w != nullptr, p.eps, cs_row != nullptr);
                 bf16* dst = (warp == 0 ? p.k_write : p.v_write) + at;
 #pragma unroll
-                for (int j = 0; j < NE; ++j) dst[lane + 32 * j] = __float2bfloat16_rn(cache_value(x[j]));
+                for (int j = 0; j < NE; ++j) dst[lane + 32 * j] = __float2bfloat16_rn(cache_value(own.x[j]));
                 if (patch) {
                     const int ti = pos / TILE_KEYS - first_tile, row = pos - (first_tile + ti) * TILE_KEYS;
                     uint8_t* tile = smem + (warp == 0 ? 0 : STAGES * TILE_BYTES) + ti * TILE_BYTES;
@@ -452,11 +464,11 @@ __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* sme
                     for (int j = 0; j < NE; ++j) {
                         const int e = lane + 32 * j;
                         *reinterpret_cast<bf16*>(tile + tile_offset<D>(row, e >> 3) + (e & 7) * 2) =
-                            __float2bfloat16_rn(cache_value(x[j]));
+                            __float2bfloat16_rn(cache_value(own.x[j]));
                     }
                 }
             }
-            __threadfence();                                       // before this CTA gathers that page
+            if (!patch) __threadfence();                           // before this CTA gathers that page (a patched tile is not gathered again)
         }
         __syncthreads();
         const bool v0 = g4 < group, v1 = g4 + 8 < group;
@@ -657,8 +669,9 @@ __device__ __forceinline__ StreamCut stream_cut(const DecodeParams& p, int n_tok
     return c;
 }
 
+// (three CTAs an SM, as the planner counts them)
 template <int D>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 3)
 attn_decode_stream_kernel(const DecodeParams p, int n_tokens) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ int cum[STREAM_MAX_TOKENS + 1];
