@@ -20,6 +20,7 @@
 //
 // Cache layout of one layer: [page][kv_head][slot][head_dim].
 #include "common.cuh"
+#include "mbarrier.cuh"
 #include <math.h>
 
 namespace {
@@ -367,12 +368,30 @@ __host__ __device__ __forceinline__ int decode_split_keys(int kv_len, int max_sp
     return keys;
 }
 
+// Where the splits of a pair are a cluster: each CTA finishes `share` of the pair's group x D values (the first ones the CTA of
+// split 0, and so on), out of partial values, maxima and sums that all splits send into its shared memory and count on
+// its barrier.
+struct DecodeMail {
+    float* values;              // [split][share]
+    float* max_sum;             // [split][head of the group][2]
+    uint64_t* ready;
+    int share, ctas;
+};
+__device__ __forceinline__ void send(float* to, float v, uint64_t* bar, int rank) {
+    uint32_t at, b;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(to)), "r"(rank));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(smem_u32(bar)), "r"(rank));
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(at), "r"(__float_as_uint(v)), "r"(b) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 // One split of one (token, kv head) pair: keys lo .. hi of entry `entry` (decoded token n of the
 // step), split `split` of `n_splits`.  `first`: the CTA's first piece of work (it may fetch tiles
 // before the dependency wait and makes that wait); all threads of the CTA call this together.
-template <int D>
+template <int D, bool CLUSTER = false>
 __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* smem, int n, int entry, int g, int lo,
-                                             int hi, int split, int n_splits, bool first) {
+                                             int hi, int split, int n_splits, bool first, const DecodeMail* mail = nullptr) {
     constexpr int TILE_BYTES = TILE_KEYS * D * 2;
     constexpr int STAGES = DECODE_STAGES;
     const uint32_t k_base = smem_u32(smem), v_base = k_base + STAGES * TILE_BYTES;
@@ -414,6 +433,22 @@ __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* sme
         if (new_kv && warp == 0) take_norm_weights(own, p.k_norm_w, p.norm_dtype, lane);
     }
     if (first) pdl_wait();
+    auto send_max_sum = [&](int row, float m, float l) {
+        for (int r = 0; r < mail->ctas && r * mail->share < group * D; ++r) {
+            float* at = mail->max_sum + (split * group + row) * 2;
+            send(at, m, mail->ready, r);
+            send(at + 1, l, mail->ready, r);
+        }
+    };
+    if (CLUSTER && lo > hi) {
+        cluster_wait();
+        for (int i = threadIdx.x; i < group * D; i += THREADS) {
+            const int r = i / mail->share;
+            send(mail->values + split * mail->share + i - r * mail->share, 0.f, mail->ready, r);
+            if (i % D == 0) send_max_sum(i / D, -INFINITY, 0.f);
+        }
+        return;
+    }
     if (lo > hi) {                                         // split wholly behind the window
         for (int i = threadIdx.x; i < group; i += THREADS) {
             my_ml[i * head_stride_ml] = -INFINITY;
@@ -586,6 +621,7 @@ __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* sme
         r1[0] = o[d][2]; r1[1] = o[d][3];
     }
     __syncthreads();
+    if (CLUSTER) cluster_wait();                            // (every CTA's barrier exists)
     for (int i = threadIdx.x; i < group * D; i += THREADS) {
         const int row = i / D, d = i % D;
         float m = -INFINITY;
@@ -602,6 +638,12 @@ __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* sme
         if (n_splits == 1) {
             // nothing to merge: this is the token's result
             p.out[((size_t)tok * p.n_q + g * group + row) * D + d] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
+            continue;
+        }
+        if (CLUSTER) {
+            const int r = i / mail->share;
+            send(mail->values + split * mail->share + i - r * mail->share, acc, mail->ready, r);
+            if (d == 0) send_max_sum(row, m, l);
             continue;
         }
         my_o[row * head_stride_o + d] = acc;
@@ -634,6 +676,88 @@ attn_decode_kernel(const DecodeParams p) {
     if (split >= n_splits) return;
     decode_split<D>(p, smem, n, entry, g, max(first_key, split * split_keys), min(pos, (split + 1) * split_keys - 1),
                     split, n_splits, true);
+}
+
+// The same with the splits of a pair as a cluster of at most 8 CTAs, which finish the pair among themselves: no scratch, no
+// merge behind it.  A merge launch costs a link of the chain (its wait, its loads, its stores) and every split's partial values a
+// way out and in; a send costs neither (36 layers, 16 tokens behind 1,000 keys: 2,803 -> 2,660 us a step; 4 layers, one behind
+// 77: 172.7 -> 169).  Where it pays: AttentionPlanner::cluster_splits.  The arithmetic of the merge is
+// attn_decode_merge_kernel's, value for value.  A CTA without a split (its token is shorter) finishes its share all the same.
+template <int D> constexpr int decode_smem() {
+    constexpr int PIPE = 2 * DECODE_STAGES * TILE_KEYS * D * 2 + 16 * D * 2;   // tiles, and the group's queries
+    constexpr int MERGE = (2 * WARPS * 16 + WARPS * 16 * (D + 8)) * 4;
+    return PIPE > MERGE ? PIPE : MERGE;
+}
+constexpr int MAIL_MAX = 8;                       // CTAs of a cluster
+__host__ __device__ inline int mail_share(int values, int ctas) { return (values + 2 * ctas - 1) / (2 * ctas) * 2; }
+template <int D>
+__global__ void __launch_bounds__(THREADS)
+attn_decode_cluster_kernel(const DecodeParams p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ uint64_t ready;
+    __shared__ int gave_up;
+    pdl_launch_dependents();
+    const int n = blockIdx.y, entry = p.rows[n], g = blockIdx.x, split = blockIdx.z, group = p.n_q / p.n_kv;
+    const int pos = p.context_len[entry];
+    const int kv_len = pos + 1;
+    const int first_key = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+    const int split_keys = decode_split_keys(kv_len, p.max_splits, __ldg(p.split_keys + n * p.split_stride));
+    const int n_splits = (kv_len + split_keys - 1) / split_keys;
+    DecodeMail mail;
+    mail.ctas = p.max_splits;
+    mail.share = mail_share(group * D, mail.ctas);
+    mail.values = reinterpret_cast<float*>(smem + decode_smem<D>());
+    mail.max_sum = mail.values + mail.ctas * mail.share;
+    mail.ready = &ready;
+    const int mine = n_splits > 1 ? max(0, min(mail.share, group * D - split * mail.share)) : 0;
+    if (threadIdx.x == 0) {
+        gave_up = 0;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&ready)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (mine > 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&ready)), "r"(n_splits * (mine + 2 * group) * 4) : "memory");
+    }
+    __syncthreads();
+    cluster_arrive();
+    if (split < n_splits) {
+        decode_split<D, true>(p, smem, n, entry, g, max(first_key, split * split_keys), min(pos, (split + 1) * split_keys - 1), split,
+                              n_splits, true, &mail);
+    } else {
+        pdl_wait();
+        cluster_wait();
+    }
+    if (mine == 0) return;
+    if (!__syncthreads_and(kipp_mbar_wait_limited(&ready, 0, &gave_up, KIPP_WAIT_LIMIT_CYCLES))) {
+        if (threadIdx.x == 0) atomicExch(&p.status[2], 1);
+        return;
+    }
+    bf16* out = p.out + ((size_t)p.q_start[entry] * p.n_q + g * group) * D + split * mail.share;
+    for (int i = 2 * threadIdx.x; i < mine; i += 2 * THREADS) {
+        const float* ml = mail.max_sum + (split * mail.share + i) / D * 2;           // (a pair of values has one head)
+        float m[MAIL_MAX], lw[MAIL_MAX], w[MAIL_MAX], mx = -INFINITY;
+#pragma unroll
+        for (int s = 0; s < MAIL_MAX; ++s) {
+            m[s] = s < n_splits ? ml[s * group * 2] : -INFINITY;
+            mx = fmaxf(mx, m[s]);
+        }
+#pragma unroll
+        for (int s = 0; s < MAIL_MAX; ++s) {
+            w[s] = m[s] == -INFINITY ? 0.f : exp2f(m[s] - mx);
+            lw[s] = s < n_splits ? ml[s * group * 2 + 1] * w[s] : 0.f;
+        }
+        // (the merge kernel's tree over lanes, of which the first eight hold something)
+        const float total = ((lw[0] + lw[4]) + (lw[2] + lw[6])) + ((lw[1] + lw[5]) + (lw[3] + lw[7]));
+        const float inv_sum = total > 0.f ? 1.f / total : 0.f;
+        float a = 0.f, b = 0.f;
+#pragma unroll
+        for (int s = 0; s < MAIL_MAX; ++s)
+            if (w[s] != 0.f) {
+                const float2 v = *reinterpret_cast<const float2*>(mail.values + s * mail.share + i);
+                a += v.x * w[s];
+                b += v.y * w[s];
+            }
+        *reinterpret_cast<__nv_bfloat162*>(out + i) = __floats2bfloat162_rn(a * inv_sum, b * inv_sum);
+    }
 }
 
 // The same work cut differently (DecodeParams::stream): the 64-key tiles of all (token, kv head)
@@ -808,9 +932,7 @@ inline int launch_merge(const DecodeParams& p, void* out, int n, int head_dim, c
 }
 
 template <int D> int launch_decode(const DecodeParams& p, int n, cudaStream_t s) {
-    constexpr int PIPE = 2 * DECODE_STAGES * TILE_KEYS * D * 2 + 16 * D * 2;   // tiles, and the group's queries
-    constexpr int MERGE = (2 * WARPS * 16 + WARPS * 16 * (D + 8)) * 4;
-    constexpr int SMEM = PIPE > MERGE ? PIPE : MERGE;
+    constexpr int SMEM = decode_smem<D>();
     if (const int e = kipp_allow_smem(attn_decode_kernel<D>, SMEM)) return e;
     if (p.n_splits_out != nullptr) {
         if (const int e = kipp_allow_smem(attn_decode_stream_kernel<D>, SMEM)) return e;
@@ -818,6 +940,14 @@ template <int D> int launch_decode(const DecodeParams& p, int n, cudaStream_t s)
     }
     if (n > 65535) return KIPP_ERR_ARG;
     return kipp_launch(attn_decode_kernel<D>, dim3(p.n_kv, n, p.max_splits), dim3(THREADS), SMEM, s, 1, p);
+}
+// The splits of a pair as a cluster (p.max_splits CTAs).
+template <int D> int launch_decode_cluster(const DecodeParams& p, int n, cudaStream_t s) {
+    const int group = p.n_q / p.n_kv, share = mail_share(group * D, p.max_splits);
+    const size_t smem = decode_smem<D>() + (size_t)p.max_splits * (share + 2 * group) * 4;
+    if (const int e = kipp_allow_smem(attn_decode_cluster_kernel<D>, smem)) return e;
+    if (n > 65535) return KIPP_ERR_ARG;
+    return kipp_launch(attn_decode_cluster_kernel<D>, dim3(p.n_kv, n, p.max_splits), dim3(THREADS), smem, s, p.max_splits, p);
 }
 }  // namespace
 
@@ -950,7 +1080,8 @@ extern "C" int kipp_attn_decode_replan(int* split_keys, const int* context_len, 
 // projection [tokens, (n_q + 2 n_kv) * head_dim]: per-head norm (weights or nullptr),
 // rotation by the step's (cos, sin) table (or nullptr) and the write of the new key and
 // value into the pools (write_cache) happen inside the attention kernel.
-extern "C" int kipp_attn_decode_mma_fused(void* out, const void* qkv, long long ld_qkv, void* k_pages,
+namespace {
+int decode_fused_run(bool cluster, void* out, const void* qkv, long long ld_qkv, void* k_pages,
                                           void* v_pages, const void* q_norm_w, const void* k_norm_w,
                                           int norm_dtype, float eps, const void* cos_sin, int write_cache,
                                           const int* q_start, const int* context_len, const int* block_table,
@@ -960,7 +1091,7 @@ extern "C" int kipp_attn_decode_mma_fused(void* out, const void* qkv, long long 
                                           int* status, void* stream) {
     if (n <= 0) return 0;
     if (!kipp_attn_decode_supported(head_dim, n_q, n_kv) || page_size <= 0 || window < 0 || max_splits <= 0 ||
-        max_splits > 64 || scratch == nullptr || ((uintptr_t)scratch & 15) || stream_ctas < 0 ||
+        max_splits > (cluster ? MAIL_MAX : 64) || (!cluster && (scratch == nullptr || ((uintptr_t)scratch & 15))) || stream_ctas < 0 ||
         (stream_ctas > 0 ? !kipp_attn_decode_stream_ok(n, max_splits) : split_keys == nullptr) ||
         ((uintptr_t)out & 7) || status == nullptr || qkv == nullptr ||
         ld_qkv < (long long)(n_q + 2 * n_kv) * head_dim || ld_qkv > 0x7fffffffLL ||
@@ -985,7 +1116,33 @@ extern "C" int kipp_attn_decode_mma_fused(void* out, const void* qkv, long long 
     p.stream_ctas = stream_ctas;
     p.n_splits_out = stream_ctas > 0 ? reinterpret_cast<int*>(p.part_ml + (size_t)n * n_q * max_splits * 2) : nullptr;
     cudaStream_t s = (cudaStream_t)stream;
+    if (cluster) return head_dim == 64 ? launch_decode_cluster<64>(p, n, s) : launch_decode_cluster<128>(p, n, s);
     int rc = head_dim == 64 ? launch_decode<64>(p, n, s) : launch_decode<128>(p, n, s);
     if (rc) return rc;
     return launch_merge(p, out, n, head_dim, s);
+}
+}  // namespace
+extern "C" int kipp_attn_decode_mma_fused(void* out, const void* qkv, long long ld_qkv, void* k_pages,
+                                          void* v_pages, const void* q_norm_w, const void* k_norm_w,
+                                          int norm_dtype, float eps, const void* cos_sin, int write_cache,
+                                          const int* q_start, const int* context_len, const int* block_table,
+                                          int table_width, int page_size, const int* rows, int n, int n_q,
+                                          int n_kv, int head_dim, float scale, int window, int max_splits,
+                                          const int* split_keys, int split_stride, int stream_ctas, float* scratch,
+                                          int* status, void* stream) {
+    return decode_fused_run(false, out, qkv, ld_qkv, k_pages, v_pages, q_norm_w, k_norm_w, norm_dtype, eps, cos_sin, write_cache, q_start, context_len, block_table,
+                            table_width, page_size, rows, n, n_q, n_kv, head_dim, scale, window, max_splits, split_keys, split_stride, stream_ctas,
+                            scratch, status, stream);
+}
+// The same with the splits of a (token, kv head) pair, at most `ctas` (1 to 8) of them, as a cluster that finishes the pair
+// itself: one launch, no scratch.  A token whose split length would make more splits has longer ones.
+extern "C" int kipp_attn_decode_cluster_fused(void* out, const void* qkv, long long ld_qkv, void* k_pages, void* v_pages,
+                                              const void* q_norm_w, const void* k_norm_w, int norm_dtype, float eps,
+                                              const void* cos_sin, int write_cache, const int* q_start, const int* context_len,
+                                              const int* block_table, int table_width, int page_size, const int* rows, int n,
+                                              int n_q, int n_kv, int head_dim, float scale, int window, int ctas,
+                                              const int* split_keys, int split_stride, int* status, void* stream) {
+    return decode_fused_run(true, out, qkv, ld_qkv, k_pages, v_pages, q_norm_w, k_norm_w, norm_dtype, eps, cos_sin, write_cache, q_start, context_len, block_table,
+                            table_width, page_size, rows, n, n_q, n_kv, head_dim, scale, window, ctas, split_keys, split_stride, 0,
+                            nullptr, status, stream);
 }

@@ -426,7 +426,7 @@ inline void AttentionMixer::forward(StepContext& ctx, const LayerRun& run, int m
         output_product(ctx, residual, attn, o_dim_, w_o_, o_dim_, dtype_, hidden_, o_dim_);
         return;
     }
-    const AttentionWork work = planner_->work_of(m);
+    const AttentionWork work = planner_->work_of(m, (long long)cache.table_width * cache.page_size);
     if (to_heads) {
         // a prompt-sized step: the projection's epilogue norms, rotates and writes the cache
         void* q = ctx.workspace->buffer("q", (size_t)T * q_dim_ * es);

@@ -21,6 +21,7 @@ struct AttentionWork {
     const int* decode_rows = nullptr;      // [n_decode] entries that bring one token
     int n_decode = 0;
     const int* split_keys = nullptr;       // [n_decode] keys per split of each decoded token
+    int cluster_ctas = 0;                  // > 0: in a step of decoded tokens only, a pair's splits are a cluster of that many CTAs
     int stream_ctas = 0;                   // > 0: the decoded tokens' key tiles are dealt out in equal runs to
                                            // that many CTAs instead (split_keys is not read)
     const int* prefill_work = nullptr;     // [(entry, first token)] per 64-token tile, entries of > 1 token
@@ -1055,6 +1056,19 @@ public:
         using Fn = int (*)(void*, const void*, long long, void*, void*, const void*, const void*, int, float, const void*,
                            int, const int*, const int*, const int*, int, int, const int*, int, int, int, int, float, int,
                            int, const int*, int, int, float*, int*, void*);
+        if (work.cluster_ctas > 0) {
+            using Fc = int (*)(void*, const void*, long long, void*, void*, const void*, const void*, int, float, const void*,
+                               int, const int*, const int*, const int*, int, int, const int*, int, int, int, int, float, int,
+                               int, const int*, int, int*, void*);
+            static Fc c = kernel_symbol<Fc>("attention_mma", "kipp_attn_decode_cluster_fused");
+            run(c(out, qkv, ld_qkv, cache.k_pages, cache.v_pages, q_norm_w, k_norm_w, norm_dtype, eps, cos_sin,
+                  write_cache ? 1 : 0, q_start, context_len, cache.block_table, cache.table_width, cache.page_size,
+                  work.decode_rows, work.n_decode, n_q, n_kv, head_dim, scale, window, work.cluster_ctas, work.split_keys, 1,
+                  status, stream),
+                "attn_decode_mma_fused");
+            ++fused_decode_launches;
+            return;
+        }
         static Fn f = kernel_symbol<Fn>("attention_mma", "kipp_attn_decode_mma_fused");
         float* scratch = decode_scratch(work.n_decode, n_q, head_dim);
         run(f(out, qkv, ld_qkv, cache.k_pages, cache.v_pages, q_norm_w, k_norm_w, norm_dtype, eps, cos_sin,

@@ -1040,6 +1040,52 @@ def test_decode_attention_fused_with_norm_rotation_and_cache_write(case):
     assert torch.allclose(got3.float(), want.float(), rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("ctas", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("shape", [dict(D=128, nq=8, nkv=2, page=16), dict(D=64, nq=6, nkv=3, page=8), dict(D=128, nq=16, nkv=1, page=32),
+                                   dict(D=64, nq=5, nkv=5, page=16)])
+def test_decode_attention_in_a_cluster(shape, ctas, window):
+    """A pair's splits as a cluster that finishes the pair: the bits and the cache of the same splits merged by a launch of
+    its own.  Tokens of one split and of all, splits wholly behind a window, more splits asked for than the cluster has."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    lib = load_library("attention_mma")
+    p, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+    head = [p, p, ll, p, p, p, p, i, f, p, i, p, p, p, i, i, p, i, i, i, i, f, i, i, p, i]
+    lib.kipp_attn_decode_mma_fused.argtypes = head + [i, p, p, p]
+    lib.kipp_attn_decode_cluster_fused.argtypes = head + [p, p]
+    D, nq, nkv, page = shape["D"], shape["nq"], shape["nkv"], shape["page"]
+    layout = [(700, 1), (15, 1), (63, 1), (64, 1), (1023, 1), (0, 1), (300, 1)]
+    meta, table, _, kp, vp = attention_case(78, D, nq, nkv, page, layout, torch.bfloat16)
+    T = meta.tokens
+    g = torch.Generator().manual_seed(6)
+    qkv = torch.randn(T, (nq + 2 * nkv) * D, generator=g).to(torch.bfloat16).to(DEV)
+    qw, kw = ((1 + 0.2 * torch.randn(D, generator=g)).to(DEV) for _ in range(2))
+    inv = torch.pow(torch.tensor(1e4, dtype=torch.float64), -(torch.arange(D // 2) * 2.0 / D).double()).float().to(DEV)
+    cos_sin = ops().rope_table(meta.positions, inv, T)
+    rows = torch.arange(T, dtype=torch.int32, device=DEV)
+    tables = meta.block_tables[0]
+    scratch = torch.full((T * nq * (ctas * (D + 2) + 1),), float("nan"), device=DEV)
+    for keys in (64, 128):
+        split_keys = torch.full((T,), keys, dtype=torch.int32, device=DEV)
+        results = []
+        for cluster in (False, True):
+            k, v, st = kp.clone(), vp.clone(), status()
+            out = torch.full((T, nq, D), 7.0, dtype=torch.bfloat16, device=DEV)
+            args = [out.data_ptr(), qkv.data_ptr(), qkv.stride(0), k.data_ptr(), v.data_ptr(), qw.data_ptr(), kw.data_ptr(), 0, 1e-6,
+                    cos_sin.data_ptr(), 1, meta.q_start.data_ptr(), meta.context_len.data_ptr(), tables.data_ptr(), tables.shape[1], page,
+                    rows.data_ptr(), T, nq, nkv, D, 1 / math.sqrt(D), window, ctas, split_keys.data_ptr(), 1]
+            stream = torch.cuda.current_stream().cuda_stream
+            if cluster:
+                rc = lib.kipp_attn_decode_cluster_fused(*args, st.data_ptr(), stream)
+            else:
+                rc = lib.kipp_attn_decode_mma_fused(*args, 0, scratch.data_ptr(), st.data_ptr(), stream)
+            assert rc == 0 and st.tolist() == [0, 0, 0, 0]
+            results.append((out, k, v))
+        assert all(torch.equal(a, b) for a, b in zip(*results)), keys
+        assert torch.isfinite(results[1][0].float()).all()
+
+
 @pytest.mark.parametrize("window", [None, 500])
 @pytest.mark.parametrize("shape", [dict(D=128, nq=8, nkv=2, page=16), dict(D=64, nq=6, nkv=3, page=32),
                                    dict(D=128, nq=16, nkv=1, page=16)])
