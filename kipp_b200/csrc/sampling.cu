@@ -27,10 +27,11 @@
 // gives the total that its target is a share of; its second pass, which looks at one bucket of the
 // first, puts that bucket's elements into a list in shared memory, and the passes after it walk the
 // list; what top-k leaves is listed once for everything that follows; a rank is looked for without weights; and the
-// draw within a nucleus takes its first pass from the selection that found the nucleus.  64 rows of 151,936, half of
-// them with top-k 50, top-p 0.95: 488 us (588 without the last two; 934 with all passes over the rows
-// and the loads one at a time); a single such row by eight blocks: 143 us (170; 221).  What is left is the aggregation
-// of equal buckets within a warp.
+// draw within a nucleus takes its first pass from the selection that found the nucleus; and a pass over a long part
+// that adds weights has a histogram for each lane.  64 rows of 151,936, top-p 0.95: 204 us, 159 with top-k 50 (520 and 158
+// before the histograms by lane; with half the rows of either kind 488, 934 with all passes over the rows and the loads
+// one at a time); a single such row by eight blocks: 98 and 86 us (158 and 85); 128 rows of 32,000: 115 and 82 (242 and 78, with
+// more of the SM's memory left to the L1).  What is left is six walks of some forty instructions an element.
 //
 // Also here: the penalties and logit bias the reference applies before
 // sampling (apply_bias_and_penalties, src/kipp.c:3386-3431).
@@ -75,7 +76,17 @@ constexpr int COPIES = 4;       // histograms of a block, one for every fourth w
                                 // handful of buckets, and atomics on one word run one after the other
 constexpr int COPIES_FROM = 2048;   // elements from which a block has them; clearing and adding four costs a short row more
 
+// A pass over a long part of a row: a histogram for each lane of a warp, shared by the block's warps ([what][bucket][lane]
+// words: counts, then the two pieces of the weights' units), so that no two lanes of an atomic meet in a word or a bank.
+// Finding the lanes of equal buckets and adding them as one, which serves lists and counts without weights, took most of a
+// long pass: the lanes' buckets are few in a selection's first pass and many in its second, and their groups add their
+// weights one after the other.  BY_LANE_FROM: 16 rows of 10,000 101 us with the groups, 64 so; below that a kernel that
+// clears and adds up 24,576 words a pass has little to win.  A lane's piece of the units must not pass
+// 2^32: BY_LANE_TO.  (Kernels of their own for the two: four rows of 700 in one kernel for both 37 us, 33 so.)
+constexpr int LANE_WORDS = 256 * 32, BY_LANE_BYTES = 3 * LANE_WORDS * 4;
+constexpr int BY_LANE_FROM = 8192, BY_LANE_TO = 32 * 4095;
 struct RowCtx {
+    unsigned* by_lane;          // [3][256][32] in shared memory (LONG)
     const float* v;
     int n;
     int lo, hi;                 // this block's part of the row
@@ -134,13 +145,18 @@ enum { MODE_COUNT = 0, MODE_W_GE = 1, MODE_W_GT = 2 };
 // so it keeps eleven bits and more; a row's sums stay below 2^58.  Against the reference's
 // running float64 sum a draw within 2^-23 of a boundary may pick the neighbour.
 constexpr double WEIGHT_UNIT = 1.0 / 1099511627776.0;      // 2^-40
+struct Units { unsigned whole, rest; };      // whole 2^20 + rest
+__device__ __forceinline__ Units units_of(float w) {
+    const float scaled = w * 1048576.0f;
+    const unsigned whole = (unsigned)scaled;
+    return Units{whole, (unsigned)((scaled - (float)whole) * 1048576.0f)};
+}
 // Sum of the units of `w` (0 <= w <= 1, cut to a whole number of them) over the lanes of `peers` (all of them call this
 // with the same mask).  The units leave the float in two pieces of 20 bits, every step exact.
 __device__ __forceinline__ unsigned long long peers_units(unsigned peers, float w) {
-    const float scaled = w * 1048576.0f;
-    const unsigned whole = (unsigned)scaled;
-    const unsigned hi = __reduce_add_sync(peers, whole);                                                    // 32 x 2^20 < 2^32
-    const unsigned lo = __reduce_add_sync(peers, (unsigned)((scaled - (float)whole) * 1048576.0f));
+    const Units u = units_of(w);
+    const unsigned hi = __reduce_add_sync(peers, u.whole);                                                  // 32 x 2^20 < 2^32
+    const unsigned lo = __reduce_add_sync(peers, u.rest);
     return ((unsigned long long)hi << 20) + lo;
 }
 
@@ -190,16 +206,22 @@ __device__ __forceinline__ void append(const RowCtx& c, Shared& sh, int i, bool 
 // One histogram pass.  level 0..3: value key digits (high to low); level 4..7:
 // token digits among elements whose key == prefix_key.  `gather`: what lies under the prefix is listed too.
 // Without `weigh` only the counts are formed (no min-p is in force then).
+template <bool LONG>
 __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned prefix_key,
                                unsigned prefix_tok, bool gather, bool weigh) {
-    for (int b = threadIdx.x; b < c.copies * 256; b += blockDim.x) { (&sh.cnt[0][0])[b] = 0; (&sh.wfix[0][0])[b] = 0ull; }
+    const bool by_lane = LONG && weigh && c.listed < 0;
+    if (by_lane) {
+        for (int i = threadIdx.x; i < 3 * LANE_WORDS / 4; i += blockDim.x) reinterpret_cast<uint4*>(c.by_lane)[i] = make_uint4(0, 0, 0, 0);
+    } else {
+        for (int b = threadIdx.x; b < c.copies * 256; b += blockDim.x) { (&sh.cnt[0][0])[b] = 0; (&sh.wfix[0][0])[b] = 0ull; }
+    }
     if (threadIdx.x == 0) sh.listed = 0;
     __syncthreads();
-    // the lanes of a round that fall into one bucket are found with match.any and add as one
     const int lane = threadIdx.x & 31, copy = (threadIdx.x >> 5) & (c.copies - 1);
-    walk(c, [&](int i, float x, bool there) {
-        unsigned key = 0; float w = 0.f;
+    auto digit_of = [&](int i, float x, bool there, float& w) {
+        unsigned key = 0;
         unsigned digit = 256u;                                  // no bucket: not in the set at this level
+        w = 0.f;
         if (there && candidate(c, i, x, key)) {
             if (level < 4) {
                 const int shift = 24 - 8 * level;
@@ -211,17 +233,53 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
             }
             if (weigh && digit < 256u && !weighs(c, x, w)) { digit = 256u; w = 0.f; }
         }
-        if (gather) append(c, sh, i, digit < 256u);
-        if (!__any_sync(0xffffffffu, digit < 256u)) return;
-        const unsigned peers = __match_any_sync(0xffffffffu, digit);
-        const unsigned long long units = weigh ? peers_units(peers, w) : 0ull;
-        if (digit < 256u && lane == __ffs(peers) - 1) {
-            atomicAdd(&sh.cnt[copy][digit], (unsigned)__popc(peers));
-            if (weigh) atomicAdd(&sh.wfix[copy][digit], units);
-        }
-    });
+        return digit;
+    };
+    // (two walks rather than one with both forms in it: 64 rows of 151,936 203 us instead of 239)
+    if (by_lane) {
+        walk(c, [&](int i, float x, bool there) {
+            float w;
+            const unsigned digit = digit_of(i, x, there, w);
+            if (gather) append(c, sh, i, digit < 256u);
+            if (digit < 256u) {
+                unsigned* at = c.by_lane + digit * 32 + lane;
+                const Units u = units_of(w);
+                atomicAdd(at, 1u);
+                atomicAdd(at + LANE_WORDS, u.whole);
+                atomicAdd(at + 2 * LANE_WORDS, u.rest);
+            }
+        });
+    } else {
+        // the lanes of a round that fall into one bucket are found with match.any and add as one
+        walk(c, [&](int i, float x, bool there) {
+            float w;
+            const unsigned digit = digit_of(i, x, there, w);
+            if (gather) append(c, sh, i, digit < 256u);
+            if (!__any_sync(0xffffffffu, digit < 256u)) return;
+            const unsigned peers = __match_any_sync(0xffffffffu, digit);
+            const unsigned long long units = weigh ? peers_units(peers, w) : 0ull;
+            if (digit < 256u && lane == __ffs(peers) - 1) {
+                atomicAdd(&sh.cnt[copy][digit], (unsigned)__popc(peers));
+                if (weigh) atomicAdd(&sh.wfix[copy][digit], units);
+            }
+        });
+    }
     __syncthreads();
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) {
+    if (by_lane) {
+        // four neighbouring threads a bucket, eight lanes' words each
+        for (int at = threadIdx.x; at < 1024; at += blockDim.x) {
+            unsigned long long sum[3] = {0ull, 0ull, 0ull};
+#pragma unroll
+            for (int what = 0; what < 3; ++what) {
+                const uint4* words = reinterpret_cast<const uint4*>(c.by_lane + what * LANE_WORDS + at * 8);
+                const uint4 x = words[0], y = words[1];
+                sum[what] = (unsigned long long)x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w;
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) sum[what] += __shfl_xor_sync(0xffffffffu, sum[what], o);
+            }
+            if ((at & 3) == 0) { sh.cnt[0][at >> 2] = (unsigned)sum[0]; sh.wfix[0][at >> 2] = (sum[1] << 20) + sum[2]; }
+        }
+    } else for (int b = threadIdx.x; b < 256; b += blockDim.x) {
         for (int k = 1; k < c.copies; ++k) { sh.cnt[0][b] += sh.cnt[k][b]; sh.wfix[0][b] += sh.wfix[k][b]; }
     }
     // the team's histogram: every block adds the blocks' parts in block order
@@ -253,6 +311,7 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
 // the one where the nucleus ends, in that one too much, which decides nothing (it is the last either way),
 // and none after it.
 // Outputs (uniform over the block): key, token, inclusive weight sum at it.
+template <bool LONG>
 __device__ void select(RowCtx& c, Shared& sh, int mode, unsigned long long target_count, double target_w, bool of_total,
                        bool again, unsigned& out_key, unsigned& out_tok, double& out_cum, double& total) {
     const int listed_before = c.listed;
@@ -270,7 +329,7 @@ __device__ void select(RowCtx& c, Shared& sh, int mode, unsigned long long targe
             }
             __syncthreads();
         } else {
-            histogram_pass(c, sh, level, prefix_key, prefix_tok, gather, mode != MODE_COUNT);
+            histogram_pass<LONG>(c, sh, level, prefix_key, prefix_tok, gather, mode != MODE_COUNT);
         }
         if (gather) c.listed = sh.listed;
         if (level == 0 && mode == MODE_W_GE)                      // (a bucket's own thread has formed all three)
@@ -479,6 +538,47 @@ __global__ void argmax_merge_kernel(const ArgmaxPart* __restrict__ parts, int n_
     if (threadIdx.x == 0) out[blockIdx.x] = bi == 0x7fffffff ? 0 : bi;
 }
 
+// The token drawn from a row (temperature above 0) whose first maximum is `best_i`.
+template <bool LONG>
+__device__ int draw(RowCtx& c, Shared& sh, int k, float tp, float mp, double uniform, int best_i) {
+    unsigned key, tok; double cum, total;
+    if (k > 0) {
+        // rank k in the order, or the last candidate when there are fewer
+        select<LONG>(c, sh, MODE_COUNT, (unsigned long long)k, 0.0, false, false, key, tok, cum, total);
+        c.has_topk = true; c.topk_key = key; c.topk_tok = tok;
+        if (k <= LIST_CAP) {                           // what is left is k elements at most
+            if (threadIdx.x == 0) sh.listed = 0;
+            __syncthreads();
+            walk(c, [&](int i, float x, bool there) {
+                unsigned kk;
+                append(c, sh, i, there && candidate(c, i, x, kk));
+            });
+            __syncthreads();
+            c.listed = sh.listed;
+            __syncthreads();                           // read by all before the next pass counts anew
+        }
+    }
+    if (mp > 0.0f) {
+        // The top weight is expf(smax - smax) = 1.
+        c.has_minp = true;
+        c.minp_threshold = (double)mp * (double)expf(0.0f);
+    }
+    // with a nucleus, the prefix that is kept, and a share of its weight; else a share of the set's
+    double kept;
+    if (tp < 1.0f) {
+        select<LONG>(c, sh, MODE_W_GE, 0, (double)tp, true, false, key, tok, cum, total);
+        c.has_nucleus = true; c.nuc_key = key; c.nuc_tok = tok;
+        kept = cum;
+        select<LONG>(c, sh, MODE_W_GT, 0, uniform * kept, false, true, key, tok, cum, total);
+    } else {
+        select<LONG>(c, sh, MODE_W_GT, 0, uniform, true, false, key, tok, cum, total);
+        kept = total;
+    }
+    return (key == 0xffffffffu && tok == 0 && kept == 0.0) ? best_i : (int)tok;
+}
+
+// LONG: a block's part of a row is long enough for the histograms by lane, and not too long.
+template <bool LONG>
 __global__ void __launch_bounds__(THREADS)
 sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
                    const float* __restrict__ temperature, const int* __restrict__ top_k,
@@ -486,6 +586,7 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
                    const double* __restrict__ uniform, int* __restrict__ out) {
     __shared__ Shared sh;
     __shared__ int list[LIST_CAP];
+    extern __shared__ __align__(16) unsigned by_lane[];     // BY_LANE_BYTES with LONG, else nothing
     pdl_launch_dependents();
     pdl_wait();
     const int blocks = team_size(), rank = team_rank();
@@ -513,6 +614,7 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
         return;
     }
     RowCtx c;
+    c.by_lane = by_lane;
     c.v = v; c.n = n; c.lo = lo; c.hi = hi; c.list = list; c.listed = -1; c.copies = hi - lo > COPIES_FROM ? COPIES : 1;
     c.inv_t = 1.0f / T;
     c.smax = v[best_i] * c.inv_t;
@@ -521,43 +623,12 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
     c.topk_key = c.topk_tok = c.nuc_key = c.nuc_tok = 0;
     c.minp_threshold = 0.0;
 
-    unsigned key, tok; double cum, total;
+    // (Rows whose top-k leaves no more than the list holds walk long parts without weights only: they take the code of the short
+    // parts.  Sharing the other's, with its second kind of walk, cost them another 2 to 3 us of code to fetch.)
     const int k = top_k[r];
-    if (k > 0) {
-        // rank k in the order, or the last candidate when there are fewer
-        select(c, sh, MODE_COUNT, (unsigned long long)k, 0.0, false, false, key, tok, cum, total);
-        c.has_topk = true; c.topk_key = key; c.topk_tok = tok;
-        if (k <= LIST_CAP) {                           // what is left is k elements at most
-            if (threadIdx.x == 0) sh.listed = 0;
-            __syncthreads();
-            walk(c, [&](int i, float x, bool there) {
-                unsigned kk;
-                append(c, sh, i, there && candidate(c, i, x, kk));
-            });
-            __syncthreads();
-            c.listed = sh.listed;
-            __syncthreads();                           // read by all before the next pass counts anew
-        }
-    }
-    const float mp = min_p[r];
-    if (mp > 0.0f) {
-        // The top weight is expf(smax - smax) = 1.
-        c.has_minp = true;
-        c.minp_threshold = (double)mp * (double)expf(0.0f);
-    }
-    // with a nucleus, the prefix that is kept, and a share of its weight; else a share of the set's
-    const float tp = top_p[r];
-    double kept;
-    if (tp < 1.0f) {
-        select(c, sh, MODE_W_GE, 0, (double)tp, true, false, key, tok, cum, total);
-        c.has_nucleus = true; c.nuc_key = key; c.nuc_tok = tok;
-        kept = cum;
-        select(c, sh, MODE_W_GT, 0, uniform[r] * kept, false, true, key, tok, cum, total);
-    } else {
-        select(c, sh, MODE_W_GT, 0, uniform[r], true, false, key, tok, cum, total);
-        kept = total;
-    }
-    if (threadIdx.x == 0 && rank == 0) out[r] = (key == 0xffffffffu && tok == 0 && kept == 0.0) ? best_i : (int)tok;
+    const int token = LONG && !(k > 0 && k <= LIST_CAP) ? draw<true>(c, sh, k, top_p[r], min_p[r], uniform[r], best_i)
+                                                        : draw<false>(c, sh, k, top_p[r], min_p[r], uniform[r], best_i);
+    if (threadIdx.x == 0 && rank == 0) out[r] = token;
 }
 
 // Logit bias, then repetition / presence / frequency penalties over each row's
@@ -679,7 +750,12 @@ extern "C" int kipp_sample_rows(const float* logits, long long ld, int rows, int
     int blocks = 1;
     while (blocks < 8 && n >= 16384 * blocks && (long long)rows * blocks * 2 <= kipp_sm_count()) blocks *= 2;
     if ((long long)rows * blocks > 0x7fffffffLL) return KIPP_ERR_ARG;
-    return kipp_launch_cluster(sample_rows_kernel, dim3((unsigned)(rows * blocks)), dim3(THREADS), 0, (cudaStream_t)stream,
+    const int part = ((n + blocks - 1) / blocks + 3) & ~3;                // (the last block of a row may have less)
+    const bool by_lane = part >= BY_LANE_FROM && part <= BY_LANE_TO;
+    const auto kernel = by_lane ? sample_rows_kernel<true> : sample_rows_kernel<false>;
+    const size_t smem = by_lane ? BY_LANE_BYTES : 0;
+    if (const int e = kipp_allow_smem(kernel, smem)) return e;
+    return kipp_launch_cluster(kernel, dim3((unsigned)(rows * blocks)), dim3(THREADS), smem, (cudaStream_t)stream,
                                dim3(blocks, 1, 1), logits, ld, n, temperature, top_k, top_p, min_p, uniform, out);
 }
 

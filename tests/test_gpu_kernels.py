@@ -925,6 +925,25 @@ def test_sample_rows_with_buckets_longer_than_a_blocks_list():
             assert c[at] >= draw - 1e-2 and (at == 0 or c[at - 1] <= draw + 1e-2), (u, r, got[r])
 
 
+@pytest.mark.parametrize("vocab", [8188, 8192, 8195, 65537, 131040, 131044])
+def test_sample_rows_alone_and_among_others(vocab):
+    """Long parts of a row are counted in a histogram for each lane, short and very long ones by groups of equal buckets: a
+    row's token is the same whether eight blocks share it or one walks it among 80, on both sides of either limit."""
+    from kipp_b200.kernels import sampling as ks
+    rows, some = 80, 8
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(some, vocab, generator=g) * torch.tensor([0.1, 1.0, 3.0, 10.0, 0.01, 2.0, 1.0, 5.0])[:, None]
+    logits[6, ::3] = 0.5
+    k = torch.tensor([0, 0, 50, 0, 5000, 0, 0, 0], dtype=torch.int32)
+    p = torch.tensor([0.95, 1.0, 0.9, 0.5, 0.99, 0.3, 0.7, 0.9999])
+    mp = torch.tensor([0.0, 0.0, 0.0, 0.01, 0.0, 0.2, 0.0, 0.0])
+    u = torch.rand(some, generator=g, dtype=torch.float64)
+    one = lambda t, n: t.repeat(n, *[1] * (t.dim() - 1)).to(DEV)                     # noqa: E731
+    draw = lambda n: ks.sample_rows(one(logits, n), torch.full((some * n,), 0.8, device=DEV), one(k, n), one(p, n), one(mp, n), one(u, n))  # noqa: E731
+    alone = draw(1).cpu()
+    assert draw(rows // some).cpu().equal(alone.repeat(rows // some))
+
+
 @pytest.mark.parametrize("vocab", [700, 151936])
 def test_sample_rows_at_the_ends_of_a_nucleus(vocab):
     """The draw takes its first pass from the selection that found the nucleus: 0 gives the nucleus's first token and the
