@@ -1003,7 +1003,8 @@ __global__ void __launch_bounds__(32 * WARPS)
 gated_delta_scan_kernel(const ScanArgs a, const float* __restrict__ vec, float* __restrict__ o_raw, int v_slices, int tokens) {
     extern __shared__ __align__(16) float smem[];
     constexpr int COLS = SCAN_COLS * 32 * WARPS / P;
-    const int D = a.dim, V = a.v_dim, nvd = 3 * D + 4, rec = nvd + V;
+    // (a constant where the threads' rows fill it: strides and bounds of a token's record drop out of its chain; 384 blocks of 3 prompts: 463 -> 431 us a launch)
+    const int D = EXACT ? P * R : a.dim, V = a.v_dim, nvd = 3 * D + 4, rec = nvd + V;
     const TokenBatch tb = token_batch(nvd + COLS);
     pdl_launch_dependents();
     pdl_wait();
@@ -1148,7 +1149,8 @@ __global__ void __launch_bounds__(32 * WARPS)
 gated_delta_column_kernel(const ScanArgs a, const float* __restrict__ vec, float* __restrict__ o_raw, int v_slices, int tokens) {
     extern __shared__ __align__(16) float smem[];
     constexpr int COLS = 32 * WARPS / P;
-    const int D = a.dim, V = a.v_dim, nvd = 3 * D + 4, rec = nvd + V;
+    // (a constant where the threads' rows fill it: strides and bounds of a token's record drop out of its chain; 128 blocks: 62.7 -> 60.5 us)
+    const int D = EXACT ? P * R : a.dim, V = a.v_dim, nvd = 3 * D + 4, rec = nvd + V;
     const TokenBatch tb = token_batch(nvd + COLS);
     pdl_launch_dependents();
     pdl_wait();
