@@ -28,10 +28,11 @@
 // first, puts that bucket's elements into a list in shared memory, and the passes after it walk the
 // list; what top-k leaves is listed once for everything that follows; a rank is looked for without weights; and the
 // draw within a nucleus takes its first pass from the selection that found the nucleus; and a pass over a long part
-// that adds weights has a histogram for each lane.  64 rows of 151,936, top-p 0.95: 204 us, 159 with top-k 50 (520 and 158
+// that adds weights has a histogram for each lane.  64 rows of 151,936, top-p 0.95: 207 us, 158 with top-k 50 (519 and 158
 // before the histograms by lane; with half the rows of either kind 488, 934 with all passes over the rows and the loads
-// one at a time); a single such row by eight blocks: 98 and 86 us (158 and 85); 128 rows of 32,000: 115 and 82 (242 and 78, with
-// more of the SM's memory left to the L1).  What is left is six walks of some forty instructions an element.
+// one at a time); a single such row by eight blocks: 92 and 86 us (138 and 85), 148 of them by a block each 351 and 231 (1,013 and
+// 225); 128 rows of 32,000 with top-k 50: 82 (78, with more of the SM's memory left to the L1).  What is left is six walks of
+// some forty instructions an element.
 //
 // Also here: the penalties and logit bias the reference applies before
 // sampling (apply_bias_and_penalties, src/kipp.c:3386-3431).
@@ -81,8 +82,9 @@ constexpr int COPIES_FROM = 2048;   // elements from which a block has them; cle
 // Finding the lanes of equal buckets and adding them as one, which serves lists and counts without weights, took most of a
 // long pass: the lanes' buckets are few in a selection's first pass and many in its second, and their groups add their
 // weights one after the other.  BY_LANE_FROM: 16 rows of 10,000 101 us with the groups, 64 so; below that a kernel that
-// clears and adds up 24,576 words a pass has little to win.  A lane's piece of the units must not pass
-// 2^32: BY_LANE_TO.  (Kernels of their own for the two: four rows of 700 in one kernel for both 37 us, 33 so.)
+// clears and adds up 24,576 words a pass has little to win.  A lane's sum of a piece of the units must not pass 2^32: after
+// BY_LANE_TO elements the lanes' sums are added up and start anew.  (Kernels of their own for the two: four rows of 700 in one
+// kernel for both 37 us, 33 so.)
 constexpr int LANE_WORDS = 256 * 32, BY_LANE_BYTES = 3 * LANE_WORDS * 4;
 constexpr int BY_LANE_FROM = 8192, BY_LANE_TO = 32 * 4095;
 struct RowCtx {
@@ -211,7 +213,7 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
                                unsigned prefix_tok, bool gather, bool weigh) {
     const bool by_lane = LONG && weigh && c.listed < 0;
     if (by_lane) {
-        for (int i = threadIdx.x; i < 3 * LANE_WORDS / 4; i += blockDim.x) reinterpret_cast<uint4*>(c.by_lane)[i] = make_uint4(0, 0, 0, 0);
+        for (int b = threadIdx.x; b < 256; b += blockDim.x) { sh.cnt[0][b] = 0; sh.wfix[0][b] = 0ull; }
     } else {
         for (int b = threadIdx.x; b < c.copies * 256; b += blockDim.x) { (&sh.cnt[0][0])[b] = 0; (&sh.wfix[0][0])[b] = 0ull; }
     }
@@ -237,18 +239,40 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
     };
     // (two walks rather than one with both forms in it: 64 rows of 151,936 203 us instead of 239)
     if (by_lane) {
-        walk(c, [&](int i, float x, bool there) {
-            float w;
-            const unsigned digit = digit_of(i, x, there, w);
-            if (gather) append(c, sh, i, digit < 256u);
-            if (digit < 256u) {
-                unsigned* at = c.by_lane + digit * 32 + lane;
-                const Units u = units_of(w);
-                atomicAdd(at, 1u);
-                atomicAdd(at + LANE_WORDS, u.whole);
-                atomicAdd(at + 2 * LANE_WORDS, u.rest);
+        RowCtx piece = c;
+#pragma unroll 1
+        for (piece.lo = c.lo; piece.lo < c.hi; piece.lo += BY_LANE_TO) {
+            piece.hi = min(c.hi, piece.lo + BY_LANE_TO);
+            for (int i = threadIdx.x; i < 3 * LANE_WORDS / 4; i += blockDim.x) reinterpret_cast<uint4*>(c.by_lane)[i] = make_uint4(0, 0, 0, 0);
+            __syncthreads();
+            walk(piece, [&](int i, float x, bool there) {
+                float w;
+                const unsigned digit = digit_of(i, x, there, w);
+                if (gather) append(c, sh, i, digit < 256u);
+                if (digit < 256u) {
+                    unsigned* at = c.by_lane + digit * 32 + lane;
+                    const Units u = units_of(w);
+                    atomicAdd(at, 1u);
+                    atomicAdd(at + LANE_WORDS, u.whole);
+                    atomicAdd(at + 2 * LANE_WORDS, u.rest);
+                }
+            });
+            __syncthreads();
+            // four neighbouring threads a bucket, eight lanes' words each
+            for (int at = threadIdx.x; at < 1024; at += blockDim.x) {
+                unsigned long long sum[3] = {0ull, 0ull, 0ull};
+#pragma unroll
+                for (int what = 0; what < 3; ++what) {
+                    const uint4* words = reinterpret_cast<const uint4*>(c.by_lane + what * LANE_WORDS + at * 8);
+                    const uint4 x = words[0], y = words[1];
+                    sum[what] = (unsigned long long)x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w;
+#pragma unroll
+                    for (int o = 1; o < 4; o <<= 1) sum[what] += __shfl_xor_sync(0xffffffffu, sum[what], o);
+                }
+                if ((at & 3) == 0) { sh.cnt[0][at >> 2] += (unsigned)sum[0]; sh.wfix[0][at >> 2] += (sum[1] << 20) + sum[2]; }
             }
-        });
+            __syncthreads();
+        }
     } else {
         // the lanes of a round that fall into one bucket are found with match.any and add as one
         walk(c, [&](int i, float x, bool there) {
@@ -265,21 +289,7 @@ __device__ void histogram_pass(const RowCtx& c, Shared& sh, int level, unsigned 
         });
     }
     __syncthreads();
-    if (by_lane) {
-        // four neighbouring threads a bucket, eight lanes' words each
-        for (int at = threadIdx.x; at < 1024; at += blockDim.x) {
-            unsigned long long sum[3] = {0ull, 0ull, 0ull};
-#pragma unroll
-            for (int what = 0; what < 3; ++what) {
-                const uint4* words = reinterpret_cast<const uint4*>(c.by_lane + what * LANE_WORDS + at * 8);
-                const uint4 x = words[0], y = words[1];
-                sum[what] = (unsigned long long)x.x + x.y + x.z + x.w + y.x + y.y + y.z + y.w;
-#pragma unroll
-                for (int o = 1; o < 4; o <<= 1) sum[what] += __shfl_xor_sync(0xffffffffu, sum[what], o);
-            }
-            if ((at & 3) == 0) { sh.cnt[0][at >> 2] = (unsigned)sum[0]; sh.wfix[0][at >> 2] = (sum[1] << 20) + sum[2]; }
-        }
-    } else for (int b = threadIdx.x; b < 256; b += blockDim.x) {
+    if (!by_lane) for (int b = threadIdx.x; b < 256; b += blockDim.x) {
         for (int k = 1; k < c.copies; ++k) { sh.cnt[0][b] += sh.cnt[k][b]; sh.wfix[0][b] += sh.wfix[k][b]; }
     }
     // the team's histogram: every block adds the blocks' parts in block order
@@ -577,7 +587,7 @@ __device__ int draw(RowCtx& c, Shared& sh, int k, float tp, float mp, double uni
     return (key == 0xffffffffu && tok == 0 && kept == 0.0) ? best_i : (int)tok;
 }
 
-// LONG: a block's part of a row is long enough for the histograms by lane, and not too long.
+// LONG: a block's part of a row is long enough for the histograms by lane.
 template <bool LONG>
 __global__ void __launch_bounds__(THREADS)
 sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
@@ -751,7 +761,7 @@ extern "C" int kipp_sample_rows(const float* logits, long long ld, int rows, int
     while (blocks < 8 && n >= 16384 * blocks && (long long)rows * blocks * 2 <= kipp_sm_count()) blocks *= 2;
     if ((long long)rows * blocks > 0x7fffffffLL) return KIPP_ERR_ARG;
     const int part = ((n + blocks - 1) / blocks + 3) & ~3;                // (the last block of a row may have less)
-    const bool by_lane = part >= BY_LANE_FROM && part <= BY_LANE_TO;
+    const bool by_lane = part >= BY_LANE_FROM;
     const auto kernel = by_lane ? sample_rows_kernel<true> : sample_rows_kernel<false>;
     const size_t smem = by_lane ? BY_LANE_BYTES : 0;
     if (const int e = kipp_allow_smem(kernel, smem)) return e;

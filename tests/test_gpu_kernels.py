@@ -925,10 +925,10 @@ def test_sample_rows_with_buckets_longer_than_a_blocks_list():
             assert c[at] >= draw - 1e-2 and (at == 0 or c[at - 1] <= draw + 1e-2), (u, r, got[r])
 
 
-@pytest.mark.parametrize("vocab", [8188, 8192, 8195, 65537, 131040, 131044])
+@pytest.mark.parametrize("vocab", [8188, 8192, 8195, 65537, 131040, 131044, 262200])
 def test_sample_rows_alone_and_among_others(vocab):
-    """Long parts of a row are counted in a histogram for each lane, short and very long ones by groups of equal buckets: a
-    row's token is the same whether eight blocks share it or one walks it among 80, on both sides of either limit."""
+    """Long parts of a row are counted in a histogram for each lane, 131,040 elements at a time, short ones by groups of equal
+    buckets: a row's token is the same whether eight blocks share it or one walks it among 80, on both sides of either limit."""
     from kipp_b200.kernels import sampling as ks
     rows, some = 80, 8
     g = torch.Generator().manual_seed(vocab)
