@@ -450,20 +450,18 @@ public:
         return stream_cost * STREAM_MARGIN < split_cost;
     }
 
-    // CTAs of the cluster that a pair's splits are in a step of decoded tokens only, or 0: where fewer and longer splits cost no
-    // more than the launch that would merge the planned ones, MERGE_TILES key tiles, and none has more than CLUSTER_TILES,
-    // above which what clusters cost in placing outweighs it (36 layers, us a step merged / in clusters: 16 tokens of 1,000 keys,
-    // 3 splits of 6 tiles: 2,803 / 2,660; 12 of 3,000, 4 of 12: 2,972 / 2,935; 8 of 8,100, 6 of 22: 3,469 / 3,653).
+    // CTAs of the cluster that a pair's splits are in a step of decoded tokens only, or 0: where no more than CLUSTER_MAX splits of
+    // at most CLUSTER_TILES key tiles are planned.  8 layers, us a step in clusters / merged: 12 tokens of 1,000 keys 569 / 584, 16 of
+    // 1,000 610 / 640, 24 of 700 630 / 679.  Clusters of up to eight, with splits made longer to fit, were level for 1 to 3
+    // tokens of 1,000 to 4,096 keys and slower for 6: 12 layers, 600 keys 808 / 722, 2,048 877 / 794, 4,096 1,005 / 868.
     // `room`: keys that the step's block tables have room for, so that a captured step, whose lengths move on under
     // the same tables, has clusters for all of them.
-    static constexpr int CLUSTER_MAX = 8, MERGE_TILES = 2, CLUSTER_TILES = 12;
+    static constexpr int CLUSTER_MAX = 4, CLUSTER_TILES = 12;
     int cluster_splits(const StepShape& s, long long room) const {
         if (own_length_ || room <= 0 || room > (1 << 30) || s.entries != s.tokens || stream_pays(s)) return 0;
         const int total = (int)((room + TILE - 1) / TILE), k = step_split_length(s.entries, (int)room) / TILE;
-        const int splits = (total + k - 1) / k, ctas = std::min(splits, CLUSTER_MAX), longer = (total + ctas - 1) / ctas;
-        const long long pairs = (long long)s.entries * kv_heads_;
-        auto cost = [&](int n, int tiles) { return (pairs * n + resident_ - 1) / resident_ * (tiles + CTA_FIXED_TILES); };
-        return longer <= CLUSTER_TILES && cost(ctas, longer) <= cost(splits, k) + MERGE_TILES ? ctas : 0;
+        const int splits = (total + k - 1) / k;
+        return splits <= CLUSTER_MAX && k <= CLUSTER_TILES ? splits : 0;
     }
 
     AttentionWork work_of(const StepMeta& meta, long long room = 0) const {
