@@ -353,6 +353,10 @@ paged_attention_few_kernel(T* __restrict__ out, const T* __restrict__ q, const T
                     for (int i = 0; i < PER; ++i) acc[i] = fmaf(p[i][jj], value, acc[i]);
                 }
             }
+            // (where a head has seen nothing yet the tile counts for nothing, infinite values and all)
+#pragma unroll
+            for (int i = 0; i < PER; ++i)
+                if (m[i] == -INFINITY) acc[i] = 0.f;
         }
         __syncthreads();                              // the values, weights and maxima are read
         if (more) fetch(v_pages, vt, 0, whole_tiles(j0 + FEW_KEYS));

@@ -673,6 +673,32 @@ def test_attention_simt_of_few_blocks(shape, dtype):
         assert torch.equal(among, out.repeat(times, 1, 1)) and st.tolist() == [0, 0, 0, 0]
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_attention_simt_before_the_first_visible_key(dtype):
+    """Tiles of keys whose scores are all -inf count for nothing before a score that is not, whatever their values: infinite ones do not
+    reach a result, neither where four tiles go at a time (few blocks) nor one by one.  They end with a tile, with
+    four of them, or with the context, and the result is then 0."""
+    D, nq, nkv, page = 128, 8, 2, 16
+    contexts, gone = [300, 170, 140, 31, 127, 200], [64, 128, 32, 32, 128, 201]          # a context's first keys score -inf
+    meta, table, q, kp, vp = attention_case(9, D, nq, nkv, page, [(c, 1) for c in contexts], dtype)
+    q = q.abs() + 0.5
+    for e, n in enumerate(gone):
+        for j in range(n):
+            at = int(table[e, j // page])
+            kp[at, :, j % page] = -3e38                                        # (the dot product overflows)
+            vp[at, :, j % page] = float("inf")
+    run = lambda o, x, m: ops().attention(o, x, kp, vp, m, meta.block_tables[0], page, nq, nkv, D, 1 / math.sqrt(D), None, status(), impl="simt")   # noqa: E731
+    few, times = torch.full_like(q, 7.0), 100
+    run(few, q, meta)
+    class Many:
+        tokens = meta.tokens * times
+        positions, entry_of_token = meta.positions[:meta.tokens].repeat(times), meta.entry_of_token[:meta.tokens].repeat(times)
+    among = torch.full((Many.tokens, nq, D), 7.0, dtype=dtype, device=DEV)
+    run(among, q.repeat(times, 1, 1), Many)
+    assert torch.isfinite(few.float()).all() and few[:3].any(dim=2).all() and not few[3:].any()
+    assert torch.equal(among, few.repeat(times, 1, 1))
+
+
 @pytest.mark.parametrize("window", [None, 37, 300])
 @pytest.mark.parametrize("shape", [dict(D=64, nq=4, nkv=2, page=16), dict(D=128, nq=8, nkv=2, page=16),
                                    dict(D=128, nq=16, nkv=1, page=8), dict(D=64, nq=3, nkv=3, page=32),
