@@ -189,7 +189,8 @@ paged_attention_simt_kernel(T* __restrict__ out, const T* __restrict__ q,
 // tile the running maximum it has in the order of the tiles, and so its weights; then a thread per value of the
 // result walks the keys.  Every sum has the terms and the order it has in the kernel above: the same bits.  What is left of a
 // chain is a head's FMAs once per FEW_TILES tiles and one FMA per key.  The next tiles' keys travel beside the weighted
-// sums, their values beside the scores, and the first ones before the dependency wait.  Bound by the instructions of a block's
+// sums, their values beside the scores, and the first ones before the dependency wait where the caller says that they are
+// there (`early`).  Bound by the instructions of a block's
 // warps, one after the other: 3 tokens of up to 211 keys, 16 heads of 128: 11.5 us a launch, 35 in the kernel above.
 constexpr int FEW_TILES = 4, FEW_KEYS = FEW_TILES * TILE, FEW_THREADS = 512, FEW_WARPS = FEW_THREADS / 32;
 struct FewStats {
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 1)
 paged_attention_few_kernel(T* __restrict__ out, const T* __restrict__ q, const T* __restrict__ k_pages, const T* __restrict__ v_pages,
                            const int* __restrict__ positions, const int* __restrict__ entry_of_token, const int* __restrict__ block_table,
                            int table_width, int page_size, int n_q, int n_kv, int head_dim, float scale, int window, int block_heads,
-                           int* __restrict__ status) {
+                           bool early, int* __restrict__ status) {
     extern __shared__ __align__(16) uint8_t smem[];   // q [heads][head_dim padded], weights [heads][FEW_KEYS], keys, values
     __shared__ FewStats st;
     pdl_launch_dependents();
@@ -242,11 +243,11 @@ paged_attention_few_kernel(T* __restrict__ out, const T* __restrict__ q, const T
         }
     };
     auto whole_tiles = [&](int j0) { return min(FEW_KEYS, (pos - j0) / TILE * TILE + TILE); };     // keys of the tiles from j0 on
-    // The first keys and values come before the dependency wait, all but those of this step's own tokens: the entry's tokens
-    // up to this one, which follow one another.
+    // With `early` the first keys and values come before the dependency wait, all but those of this step's own tokens: the
+    // entry's tokens up to this one, which follow one another.
     look_up(begin);
-    int own = pos;
-    for (int u = t - 1; u >= 0 && entry_of_token[u] == entry_of_token[t]; --u) own = positions[u];
+    int own = early ? pos : 0;
+    for (int u = t - 1; early && u >= 0 && entry_of_token[u] == entry_of_token[t]; --u) own = positions[u];
     const int n_first = whole_tiles(begin), kept = min(max(own - begin, 0), n_first);
     __syncthreads();
     fetch(k_pages, kt, 0, kept);
@@ -375,7 +376,7 @@ constexpr int SM_SMEM = 227 * 1024, SM_THREADS = 2048, SM_BLOCKS = 32;         /
 template <typename T, bool VEC, int NACC>
 int launch(void* out, const void* q, const void* k_pages, const void* v_pages, const int* positions,
            const int* entry_of_token, const int* block_table, int table_width, int page_size, int tokens, int n_q,
-           int n_kv, int head_dim, float scale, int window, int* status, cudaStream_t s) {
+           int n_kv, int head_dim, float scale, int window, bool early, int* status, cudaStream_t s) {
     const int group = n_q / n_kv, warps = group < MAX_HEADS ? group : MAX_HEADS;
     const long long blocks = (long long)tokens * n_kv * ((group + warps - 1) / warps);
     if (blocks > 0x7fffffffLL) return KIPP_ERR_ARG;
@@ -387,7 +388,7 @@ int launch(void* out, const void* q, const void* k_pages, const void* v_pages, c
             if (const int e = kipp_allow_smem(kernel, few + sizeof(FewStats))) return e;      // (what it declares counts too)
             return kipp_launch(kernel, dim3((unsigned)blocks), dim3(FEW_THREADS), few, s, 1, (T*)out, (const T*)q, (const T*)k_pages,
                                (const T*)v_pages, positions, entry_of_token, block_table, table_width, page_size, n_q, n_kv, head_dim,
-                               scale, window, warps, status);
+                               scale, window, warps, early, status);
         }
     }
     const size_t queries = (size_t)warps * ((head_dim + 3) & ~3) * 4, tiles = (size_t)2 * TILE * tile_row_bytes<T>(head_dim);
@@ -412,11 +413,10 @@ int launch_for(bool vec, int head_dim, Args... args) {
 }
 }  // namespace
 
-extern "C" int kipp_paged_attention_simt(
-    void* out, const void* q, const void* k_pages, const void* v_pages, int dtype,
-    const int* positions, const int* entry_of_token, const int* block_table, int table_width,
-    int page_size, int tokens, int n_q, int n_kv, int head_dim, float scale, int window,
-    int* status, void* stream) {
+namespace {
+int run_simt(void* out, const void* q, const void* k_pages, const void* v_pages, int dtype, const int* positions, const int* entry_of_token,
+             const int* block_table, int table_width, int page_size, int tokens, int n_q, int n_kv, int head_dim, float scale, int window,
+             bool early, int* status, void* stream) {
     if (tokens <= 0) return 0;
     if (head_dim <= 0 || head_dim > 32 * MAX_ACC || n_q <= 0 || n_kv <= 0 || n_q % n_kv ||
         page_size <= 0 || window < 0)
@@ -426,9 +426,31 @@ extern "C" int kipp_paged_attention_simt(
     const bool vec = head_dim * item % 16 == 0 && (((uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0;
     if (dtype == KIPP_DT_F32)
         return launch_for<float>(vec, head_dim, out, q, k_pages, v_pages, positions, entry_of_token, block_table, table_width,
-                                 page_size, tokens, n_q, n_kv, head_dim, scale, window, status, s);
+                                 page_size, tokens, n_q, n_kv, head_dim, scale, window, early, status, s);
     if (dtype == KIPP_DT_BF16)
         return launch_for<bf16>(vec, head_dim, out, q, k_pages, v_pages, positions, entry_of_token, block_table, table_width,
-                                page_size, tokens, n_q, n_kv, head_dim, scale, window, status, s);
+                                page_size, tokens, n_q, n_kv, head_dim, scale, window, early, status, s);
     return KIPP_ERR_DTYPE;
+}
+}  // namespace
+
+extern "C" int kipp_paged_attention_simt(
+    void* out, const void* q, const void* k_pages, const void* v_pages, int dtype,
+    const int* positions, const int* entry_of_token, const int* block_table, int table_width,
+    int page_size, int tokens, int n_q, int n_kv, int head_dim, float scale, int window,
+    int* status, void* stream) {
+    return run_simt(out, q, k_pages, v_pages, dtype, positions, entry_of_token, block_table, table_width, page_size, tokens, n_q, n_kv,
+                    head_dim, scale, window, false, status, stream);
+}
+// The same within a step of the engine, all of whose tokens of an entry are here and follow one another: the keys and values before
+// an entry's first token are from earlier steps, which ended before this step's lists came, so they may be read before
+// the kernel ahead in the stream has ended.  (The entry above takes whatever that kernel has written: a
+// few of the tokens it put into the cache, say.)
+extern "C" int kipp_paged_attention_simt_of_step(
+    void* out, const void* q, const void* k_pages, const void* v_pages, int dtype,
+    const int* positions, const int* entry_of_token, const int* block_table, int table_width,
+    int page_size, int tokens, int n_q, int n_kv, int head_dim, float scale, int window,
+    int* status, void* stream) {
+    return run_simt(out, q, k_pages, v_pages, dtype, positions, entry_of_token, block_table, table_width, page_size, tokens, n_q, n_kv,
+                    head_dim, scale, window, true, status, stream);
 }

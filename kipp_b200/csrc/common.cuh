@@ -100,6 +100,9 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // step comes after, or, in a burst that runs without the host, by kernels at the end of a
 // step (kipp_burst_advance, kipp_attn_decode_replan).  Those do not let the kernel behind them start early, so that
 // whatever follows, in the same graph or another, finds the lists as they left them.
+// So may keys and values that earlier steps left in the cache, which no kernel of a step writes and which were there before
+// its lists came; those of the step's own tokens only behind the wait.  (attn_decode_kernel and its kin, and
+// paged_attention_few_kernel by the entry for a step; whoever launches them outside the engine keeps to the same order.)
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

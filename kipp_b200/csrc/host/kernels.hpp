@@ -1031,7 +1031,7 @@ public:
         }
         using Fn = int (*)(void*, const void*, const void*, const void*, int, const int*, const int*, const int*, int,
                            int, int, int, int, int, float, int, int*, void*);
-        static Fn f = kernel_symbol<Fn>("attention_simt", "kipp_paged_attention_simt");
+        static Fn f = kernel_symbol<Fn>("attention_simt", "kipp_paged_attention_simt_of_step");
         run(f(out, q, cache.k_pages, cache.v_pages, dtype, positions, entry_of_token, cache.block_table,
               cache.table_width, cache.page_size, work.tokens, n_q, n_kv, head_dim, scale, window, status, stream),
             "attention_simt");

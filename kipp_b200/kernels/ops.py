@@ -284,7 +284,8 @@ def attention_decode_fused(out: torch.Tensor, qkv: torch.Tensor, k_pages: torch.
                            window: Optional[int], status: torch.Tensor) -> None:
     """``qk_norm_rope_write`` and ``attention`` of a step of decoded tokens in one pair of
     launches: the attention kernel normalises and rotates the raw queries and the new key
-    itself and writes the new key and value into the pages."""
+    itself and writes the new key and value into the pages.  The keys and values before them
+    must be there already: they are read before the kernel ahead in the stream has ended."""
     from . import attention_bf16
     attention_bf16.decode_fused(out, qkv, k_pages, v_pages, q_norm_w, k_norm_w, eps, cos_sin, write_cache, meta,
                                 block_table, page_size, n_q, n_kv, head_dim, scale, window, status)

@@ -699,6 +699,32 @@ def test_attention_simt_before_the_first_visible_key(dtype):
     assert torch.equal(among, few.repeat(times, 1, 1))
 
 
+@pytest.mark.parametrize("asked,of_step", [(1, False), (5, False), (40, False), (40, True)])
+def test_attention_simt_behind_the_cache_write(asked, of_step):
+    """Attention right behind the kernel that writes the keys and values: of the last of the tokens written (the general
+    entry, which waits for all of them), and of all of them beside a context that was there (a step's entry)."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    D, nq, nkv, page, scale = 64, 4, 2, 16, 1 / math.sqrt(64)
+    layout = [(100 if of_step else 0, 40)]
+    meta, table, _, kp, vp = attention_case(4, D, nq, nkv, page, layout, torch.float32)
+    g = torch.Generator().manual_seed(asked)
+    name = "kipp_paged_attention_simt" + ("_of_step" if of_step else "")
+    fn = getattr(load_library("attention_simt"), name)
+    p, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    fn.argtypes = [p, p, p, p, i, p, p, p, i, i, i, i, i, i, f, i, p, p]
+    bt, positions, entry = meta.block_tables[0], meta.positions[40 - asked:40].contiguous(), meta.entry_of_token[40 - asked:40].contiguous()
+    for _ in range(10):
+        qkv = torch.randn(40, (nq + 2 * nkv) * D, generator=g).to(DEV)
+        q, out, st = torch.zeros(40, nq, D, device=DEV), torch.zeros(asked, nq, D, device=DEV), status()
+        torch.cuda.synchronize()
+        ops().qk_norm_rope_write(qkv, q, kp, vp, None, None, 1e-6, None, 0, meta.positions, meta.entry_of_token, bt, page, 40, nq, nkv, D, True, st)
+        rc = fn(out.data_ptr(), q[40 - asked:].data_ptr(), kp.data_ptr(), vp.data_ptr(), 0, positions.data_ptr(), entry.data_ptr(), bt.data_ptr(),
+                bt.shape[1], page, asked, nq, nkv, D, scale, 0, st.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        ref = attention_ref(meta, table, q, kp, vp, layout, page, None, scale)[40 - asked:]
+        assert rc == 0 and st.tolist() == [0, 0, 0, 0] and torch.allclose(out.double().cpu(), ref, **tol(torch.float32))
+
+
 @pytest.mark.parametrize("window", [None, 37, 300])
 @pytest.mark.parametrize("shape", [dict(D=64, nq=4, nkv=2, page=16), dict(D=128, nq=8, nkv=2, page=16),
                                    dict(D=128, nq=16, nkv=1, page=8), dict(D=64, nq=3, nkv=3, page=32),
