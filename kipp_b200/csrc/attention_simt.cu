@@ -197,6 +197,7 @@ struct FewStats {
     float tile_max[MAX_HEADS][FEW_TILES], running[MAX_HEADS][FEW_TILES], sum[MAX_HEADS][FEW_TILES];
     unsigned seen[FEW_TILES];
     long long rows[FEW_KEYS];
+    int own[FEW_WARPS];          // by warp: the first position of the entry's tokens in this step
 };
 // heads of the block at most 4 NH; NACC as above: a thread's value is number tid % (32 NACC) of heads tid / (32 NACC), + HEAD_STEP, ...
 template <typename T, int NACC, int NH>
@@ -246,10 +247,17 @@ paged_attention_few_kernel(T* __restrict__ out, const T* __restrict__ q, const T
     // With `early` the first keys and values come before the dependency wait, all but those of this step's own tokens: the
     // entry's tokens up to this one, which follow one another.
     look_up(begin);
-    int own = early ? pos : 0;
-    for (int u = t - 1; early && u >= 0 && entry_of_token[u] == entry_of_token[t]; --u) own = positions[u];
-    const int n_first = whole_tiles(begin), kept = min(max(own - begin, 0), n_first);
+    if (early) {                                      // (a thread per token; walking back one by one, 148 tokens of one entry: 26.8 us, 15.3 so)
+        int own = pos;
+        for (int u = tid; u < t; u += FEW_THREADS)
+            if (entry_of_token[u] == entry_of_token[t]) own = min(own, positions[u]);
+        own = __reduce_min_sync(0xffffffffu, own);
+        if (lane == 0) st.own[warp] = own;
+    }
     __syncthreads();
+    int own = early ? pos : 0;
+    for (int w = 0; early && 32 * w < t && w < FEW_WARPS; ++w) own = min(own, st.own[w]);
+    const int n_first = whole_tiles(begin), kept = min(max(own - begin, 0), n_first);
     fetch(k_pages, kt, 0, kept);
     fetch(v_pages, vt, 0, kept);
     pdl_wait();
