@@ -101,6 +101,7 @@ int kipp_part_tensor_specs(const char* part_json, const char* prefix, const char
    context is `longest` keys (own_length: for one token of that context alone). */
 int kipp_attention_split_length(int decoded, int longest, int kv_heads, int sm_count, int own_length);
 int kipp_attention_stream_pays(int decoded, const int* keys, int kv_heads, int sm_count);
+int kipp_attention_cluster_splits(int decoded, const int* keys, int kv_heads, int sm_count, long long room);
 /* Names of the registered architectures and part kinds, as a JSON object of two lists. */
 const char* kipp_registered(void);
 

@@ -173,6 +173,18 @@ int kipp_attention_stream_pays(int decoded, const int* keys, int kv_heads, int s
     return AttentionPlanner(kv_heads, sm_count, false).stream_pays(s) ? 1 : 0;
 }
 
+// CTAs of the cluster that the planner makes of a (token, kv head) pair's splits in such a step, whose block tables have room
+// for `room` keys, or 0 where a launch of its own merges them.
+int kipp_attention_cluster_splits(int decoded, const int* keys, int kv_heads, int sm_count, long long room) {
+    StepShape s;
+    s.entries = s.tokens = decoded;
+    for (int i = 0; i < decoded; ++i) {
+        s.q_lens.push_back(1);
+        s.starts.push_back(keys[i] - 1);
+    }
+    return AttentionPlanner(kv_heads, sm_count, false).cluster_splits(s, room);
+}
+
 const char* kipp_registered(void) {
     ensure_registered();
     Json j = Json::object();

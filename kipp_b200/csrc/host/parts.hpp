@@ -450,18 +450,30 @@ public:
         return stream_cost * STREAM_MARGIN < split_cost;
     }
 
-    // CTAs of the cluster that a pair's splits are in a step of decoded tokens only, or 0: where no more than CLUSTER_MAX splits of
-    // at most CLUSTER_TILES key tiles are planned.  8 layers, us a step in clusters / merged: 12 tokens of 1,000 keys 569 / 584, 16 of
+    // CTAs of the cluster that a pair's splits are in a step of decoded tokens only, or 0.  Only where no length up to `room`, the
+    // keys that the step's block tables have room for, is planned as more than CLUSTER_MAX splits, and only up to CLUSTER_TILES key tiles
+    // a split at that length: a cluster has a place for every split then, and the bits are the merged ones, whether tables are
+    // rounded up (a captured step, whose lengths move on under them) or not (a plain launch), in a small page pool and a large one.
+    // 8 layers, us a step in clusters / merged: 12 tokens of 1,000 keys 569 / 584, 16 of
     // 1,000 610 / 640, 24 of 700 630 / 679.  Clusters of up to eight, with splits made longer to fit, were level for 1 to 3
     // tokens of 1,000 to 4,096 keys and slower for 6: 12 layers, 600 keys 808 / 722, 2,048 877 / 794, 4,096 1,005 / 868.
-    // `room`: keys that the step's block tables have room for, so that a captured step, whose lengths move on under
-    // the same tables, has clusters for all of them.
     static constexpr int CLUSTER_MAX = 4, CLUSTER_TILES = 12;
     int cluster_splits(const StepShape& s, long long room) const {
-        if (own_length_ || room <= 0 || room > (1 << 30) || s.entries != s.tokens || stream_pays(s)) return 0;
-        const int total = (int)((room + TILE - 1) / TILE), k = step_split_length(s.entries, (int)room) / TILE;
-        const int splits = (total + k - 1) / k;
-        return splits <= CLUSTER_MAX && k <= CLUSTER_TILES ? splits : 0;
+        if (own_length_ || room <= 0 || room > CLUSTER_MAX * CLUSTER_TILES * TILE || s.entries != s.tokens) return 0;
+        const int total = (int)((room + TILE - 1) / TILE);
+        auto known = cluster_of_.find({s.entries, total});           // (a few thousand divisions, and every layer asks)
+        if (known == cluster_of_.end()) known = cluster_of_.emplace(std::make_pair(s.entries, total), most_splits(s.entries, total)).first;
+        return known->second > 0 && !stream_pays(s) ? known->second : 0;
+    }
+    // The most splits that a length of 1 to `total` key tiles is planned as, or 0 where a cluster does not do.
+    int most_splits(int decoded, int total) const {
+        if (step_split_length(decoded, total * TILE) / TILE > CLUSTER_TILES) return 0;
+        int most = 0;
+        for (int tiles = 1; tiles <= total && most <= CLUSTER_MAX; ++tiles) {
+            const int k = step_split_length(decoded, tiles * TILE) / TILE;
+            most = std::max(most, (tiles + k - 1) / k);
+        }
+        return most <= CLUSTER_MAX ? most : 0;
     }
 
     AttentionWork work_of(const StepMeta& meta, long long room = 0) const {
@@ -489,6 +501,7 @@ public:
 private:
     int kv_heads_, resident_;
     bool own_length_;
+    mutable std::map<std::pair<int, int>, int> cluster_of_;           // (decoded tokens, key tiles of room) -> most_splits
 };
 
 // The work lists of the mixed-head attention's tensor-core prompt kernels: (entry, first token)

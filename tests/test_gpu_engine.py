@@ -72,6 +72,26 @@ def test_graph_steps_equal_plain_launches(dtype):
     assert torch.equal(outs[0], outs[1])             # same kernels, same order: bitwise
 
 
+@pytest.mark.parametrize("n,keys", [(40, 860), (48, 860), (30, 300)])
+def test_graph_steps_of_many_requests_equal_plain_launches(n, keys):
+    """A captured step's block tables are rounded up; its tokens are cut into the splits that a plain launch cuts them into, so
+    every bit is the same (40 of 860 keys and two key heads: five splits, where 1,024 keys would have four)."""
+    from kipp_b200.engine import StepEntry
+    seqs = [random_tokens("E", keys - i % 7, seed=i) for i in range(n)]
+    outs = []
+    for graphs in (True, False):
+        eng = engine("E", "bfloat16", cuda_graphs=graphs, cache_tokens=n * 1024, max_requests=n, max_batch_tokens=4096)
+        for i in range(0, n, 4):
+            eng.step([StepEntry(j, seqs[j][:-4], []) for j in range(i, min(i + 4, n))])
+        rows = []
+        for j in range(4, 0, -1):
+            rows.append(eng.step([StepEntry(i, [s[-j]], [0]) for i, s in enumerate(seqs)]).cpu().clone())
+        outs.append(torch.stack(rows))
+        if graphs:
+            assert eng.graph_replays == 3
+    assert torch.equal(outs[0], outs[1])
+
+
 def test_out_of_pages_leaves_every_request_unchanged():
     from kipp_b200.cache import OutOfPages
     from kipp_b200.engine import StepEntry

@@ -61,3 +61,28 @@ def test_split_rule_of_the_decode_attention():
         return lib.kipp_attention_stream_pays(n, arr, 8, 148)
     assert [stream(n, 2049) for n in (1, 8, 16, 64)] == [0, 0, 0, 1]      # 512 pairs on 444 places: four waves of splits
     assert stream(8, 8031) == 0 and stream(64, 4097) == 1
+
+
+def test_a_cluster_has_a_place_for_every_split():
+    """Where a token's splits are a cluster, no length that the block tables have room for is planned as more splits than it has
+    CTAs: a captured step, whose tables are rounded up, then cuts its tokens as a plain launch does."""
+    lib = N.lib()
+    taken = 0
+    for kv_heads in (1, 2, 4, 5, 8, 16):
+        for n in (*range(1, 70), 100, 128):
+            most = {}
+            for room in (64, 112, 320, 640, 960, 1008, 1024, 2048, 3072, 4096):
+                ctas = lib.kipp_attention_cluster_splits(n, (ctypes.c_int * n)(*[1] * n), kv_heads, 148, room)
+                assert 0 <= ctas <= 4
+                if ctas == 0:
+                    continue
+                taken += 1
+                for tiles in range(1, -(-room // 64) + 1):
+                    if tiles not in most:
+                        keys = lib.kipp_attention_split_length(n, 64 * tiles, kv_heads, 148, 0)
+                        most[tiles] = -(-64 * tiles // keys)
+                    assert most[tiles] <= ctas, (kv_heads, n, room, tiles)
+    assert taken > 500
+    tokens = lambda n, keys: (n, (ctypes.c_int * n)(*[keys] * n))                    # noqa: E731
+    assert lib.kipp_attention_cluster_splits(*tokens(16, 1000), 8, 148, 1024) == 3
+    assert lib.kipp_attention_cluster_splits(*tokens(11, 1000), 8, 148, 1024) == 0   # 900 keys are planned as five splits
