@@ -690,8 +690,9 @@ template <int D> constexpr int decode_smem() {
 }
 constexpr int MAIL_MAX = 8;                       // CTAs of a cluster
 __host__ __device__ inline int mail_share(int values, int ctas) { return (values + 2 * ctas - 1) / (2 * ctas) * 2; }
+// (three CTAs an SM, as the planner counts them: registers here, shared memory in kipp_attn_decode_cluster_fits)
 template <int D>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 3)
 attn_decode_cluster_kernel(const DecodeParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint64_t ready;
@@ -942,9 +943,11 @@ template <int D> int launch_decode(const DecodeParams& p, int n, cudaStream_t s)
     return kipp_launch(attn_decode_kernel<D>, dim3(p.n_kv, n, p.max_splits), dim3(THREADS), SMEM, s, 1, p);
 }
 // The splits of a pair as a cluster (p.max_splits CTAs).
+template <int D> size_t cluster_smem(int group, int ctas) {
+    return decode_smem<D>() + (size_t)ctas * (mail_share(group * D, ctas) + 2 * group) * 4;
+}
 template <int D> int launch_decode_cluster(const DecodeParams& p, int n, cudaStream_t s) {
-    const int group = p.n_q / p.n_kv, share = mail_share(group * D, p.max_splits);
-    const size_t smem = decode_smem<D>() + (size_t)p.max_splits * (share + 2 * group) * 4;
+    const size_t smem = cluster_smem<D>(p.n_q / p.n_kv, p.max_splits);
     if (const int e = kipp_allow_smem(attn_decode_cluster_kernel<D>, smem)) return e;
     if (n > 65535) return KIPP_ERR_ARG;
     return kipp_launch(attn_decode_cluster_kernel<D>, dim3(p.n_kv, n, p.max_splits), dim3(THREADS), smem, s, p.max_splits, p);
@@ -959,6 +962,15 @@ extern "C" int kipp_attn_mma_supported(int head_dim, int n_q, int n_kv) {
 }
 extern "C" int kipp_attn_decode_supported(int head_dim, int n_q, int n_kv) {
     return kipp_attn_mma_supported(head_dim, n_q, n_kv) && n_q / n_kv <= 16;
+}
+
+// Whether three CTAs of kipp_attn_decode_cluster_fused have room on an SM, which is what the planner counts its waves with:
+// heads of 128 in groups of more than 12 or 13 leave room for two, and a grid planned as one wave would run as two.
+extern "C" int kipp_attn_decode_cluster_fits(int head_dim, int n_q, int n_kv, int ctas) {
+    if (!kipp_attn_decode_supported(head_dim, n_q, n_kv) || ctas <= 0 || ctas > MAIL_MAX) return 0;
+    constexpr size_t SM = 228 * 1024, BESIDE = 1024 + 128;             // a CTA's reserve, and what the kernel declares
+    const int group = n_q / n_kv;
+    return 3 * ((head_dim == 64 ? cluster_smem<64>(group, ctas) : cluster_smem<128>(group, ctas)) + BESIDE) <= SM;
 }
 
 // Prompt portions: `work` lists (entry, first token) of every 64-token tile.

@@ -1016,6 +1016,13 @@ public:
         return work.stream_ctas > 0 && decode_stream_ok(work.n_decode) ? work.stream_ctas : 0;
     }
 
+    // Whether as many of the cluster's CTAs as the planner counts fit an SM (else a launch of its own merges the same splits).
+    static bool decode_cluster_fits(int head_dim, int n_q, int n_kv, int ctas) {
+        using Fn = int (*)(int, int, int, int);
+        static Fn f = kernel_symbol<Fn>("attention_mma", "kipp_attn_decode_cluster_fits");
+        return f(head_dim, n_q, n_kv, ctas) != 0;
+    }
+
     float* decode_scratch(int n, int n_q, int head_dim) {
         size_t floats = (size_t)n * n_q * DECODE_MAX_SPLITS * (head_dim + 2) + (size_t)n * n_q;
         if (floats < (1u << 20)) floats = 1u << 20;
@@ -1056,7 +1063,7 @@ public:
         using Fn = int (*)(void*, const void*, long long, void*, void*, const void*, const void*, int, float, const void*,
                            int, const int*, const int*, const int*, int, int, const int*, int, int, int, int, float, int,
                            int, const int*, int, int, float*, int*, void*);
-        if (work.cluster_ctas > 0) {
+        if (work.cluster_ctas > 0 && decode_cluster_fits(head_dim, n_q, n_kv, work.cluster_ctas)) {
             using Fc = int (*)(void*, const void*, long long, void*, void*, const void*, const void*, int, float, const void*,
                                int, const int*, const int*, const int*, int, int, const int*, int, int, int, int, float, int,
                                int, const int*, int, int*, void*);

@@ -86,3 +86,12 @@ def test_a_cluster_has_a_place_for_every_split():
     tokens = lambda n, keys: (n, (ctypes.c_int * n)(*[keys] * n))                    # noqa: E731
     assert lib.kipp_attention_cluster_splits(*tokens(16, 1000), 8, 148, 1024) == 3
     assert lib.kipp_attention_cluster_splits(*tokens(11, 1000), 8, 148, 1024) == 0   # 900 keys are planned as five splits
+
+
+def test_a_clusters_ctas_fit_an_sm_as_they_are_counted():
+    """The planner's waves hold three CTAs an SM; a kernel whose shared memory leaves room for two is not taken."""
+    fits = build.load_library("attention_mma").kipp_attn_decode_cluster_fits
+    assert all(fits(64, group, 1, ctas) for group in (1, 4, 16) for ctas in (1, 2, 3, 4, 8))
+    assert all(fits(128, 8 * group, 8, ctas) for group in (1, 4, 8, 12) for ctas in (1, 2, 3, 4))
+    assert not any(fits(128, group, 1, ctas) for group in (14, 16) for ctas in (1, 2, 3, 4))
+    assert not fits(128, 17, 1, 4) and not fits(96, 4, 1, 4) and not fits(128, 8, 1, 9) and not fits(128, 8, 1, 0)
