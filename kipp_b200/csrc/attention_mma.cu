@@ -729,6 +729,7 @@ attn_decode_cluster_kernel(const DecodeParams p) {
     }
     if (mine == 0) return;
     if (!__syncthreads_and(kipp_mbar_wait_limited(&ready, 0, &gave_up, KIPP_WAIT_LIMIT_CYCLES))) {
+        kipp_mail_drain(&ready, KIPP_WAIT_LIMIT_CYCLES);
         if (threadIdx.x == 0) atomicExch(&p.status[2], 1);
         return;
     }

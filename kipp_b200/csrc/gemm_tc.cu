@@ -773,7 +773,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 }
             }
         }
-        // nobody's shared memory may go away while a neighbour still reads it (what is sent goes to a CTA that waits for it)
+        // nobody's shared memory may go away while a neighbour still reads it (what is sent goes to a CTA that waits for it, or
+        // drains, below)
         if (!C::SEND)
             asm volatile("barrier.cluster.arrive.release.aligned;\n"
                          "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
@@ -781,7 +782,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
     tcgen05_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag) atomicExch(&p.status[1], 1);
+    if (*abort_flag) {
+        if (C::SEND && send) kipp_mail_drain(j_end > j_first ? mail_ready : nullptr, KIPP_WAIT_LIMIT_CYCLES);
+        if (threadIdx.x == 0) atomicExch(&p.status[1], 1);
+    }
     if (warp == 1) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 

@@ -32,3 +32,15 @@ __device__ __forceinline__ bool kipp_mbar_wait_limited(uint64_t* bar, uint32_t p
     *abort_flag = 1;
     return false;
 }
+
+// The end of a CTA of a cluster whose CTAs send into each other's shared memory (st.async, counted on the receiver's barrier
+// `mail`).  A CTA that got what it waited for may leave, since nothing else is on its way to it.  One that gave up calls this with
+// all its threads: it stays until every other thread of the cluster has left or come here too, which bounded waits make
+// certain (barrier.cluster.wait waits for the threads that have not exited), and until what was sent has landed: a
+// neighbour that was merely late still sends.  (One that gave up as well sends nothing: hence the limit.)
+// (With an arrival by every thread on its way out, eight tokens of 8,100 keys took 3,518 us a step instead of 3,462.)
+__device__ __noinline__ void kipp_mail_drain(uint64_t* mail, long long limit_cycles) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    int mine = 0;
+    if (mail != nullptr) kipp_mbar_wait_limited(mail, 0, &mine, limit_cycles);
+}

@@ -1229,6 +1229,24 @@ def test_a_bounded_wait_runs_out_and_reports():
     assert limit <= int(waited) < 200 * limit
 
 
+@pytest.mark.parametrize("late,limit,gives_up", [(0, 10_000_000, 0), (400_000, 10_000_000, 0), (9_000_000, 20_000, 1), (9_000_000, 0, 1)])
+def test_a_cluster_outlives_what_is_sent_late(late, limit, gives_up):
+    """A CTA whose wait for a neighbour's values ran out stays until the neighbour has sent them and they have landed
+    (csrc/mbarrier.cuh: the end of the split products' and the decode attention's clusters): the status word is set, the
+    word that came late lies in the mailbox, and the kernel returns by itself.  (A wait looks at its limit every 64 polls, which
+    block for a while each: the late word comes some 5 ms after the others.)"""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    fn = load_library("wait_probe").kipp_mail_probe
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]
+    st, landed = status(), torch.zeros(1, dtype=torch.int32, device=DEV)
+    for word in (77, 78, 79):
+        assert fn(st.data_ptr(), landed.data_ptr(), late, limit, word, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        assert landed.item() == word
+    assert st.tolist() == [0, gives_up, 0, 0]
+
+
 @pytest.mark.parametrize("interleaved", [0, 1])
 @pytest.mark.parametrize("D,rot_off,rot", [(64, 0, 64), (192, 128, 64), (192, 0, 16), (40, 8, 32), (72, 8, 24), (192, 128, 6), (48, 4, 40),
                                            (320, 24, 256)])
