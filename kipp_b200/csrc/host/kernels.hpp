@@ -829,16 +829,16 @@ public:
     void ssd_scan(void* out, long long ld_out, const void* proj, long long ld_proj, int dtype, int z_off, int xbc_off,
                   int dt_off, const float* conv_w, const float* conv_b, int taps, const float* dt_bias, const float* a_log,
                   const float* d_skip, const float* norm_w, int norm_groups, float* state, long long slot_stride,
-                  const int* q_start, const int* entry_of_token, const int* slots, int entries, int tokens, int heads,
+                  const int* q_start, const int* entry_of_token, const int* slots, int entries, int tokens, int longest, int heads,
                   int groups, int dim, int v_dim, float eps) {
         using Fn = int (*)(void*, long long, const void*, long long, int, int, int, int, const float*, const float*, int,
                            const float*, const float*, const float*, const float*, int, float*, long long, const int*,
-                           const int*, const int*, int, int, int, int, int, int, float, float*, float*, void*);
-        static Fn f = kernel_symbol<Fn>("recurrent", "kipp_ssd_scan");
+                           const int*, const int*, int, int, int, int, int, int, int, float, float*, float*, void*);
+        static Fn f = kernel_symbol<Fn>("recurrent", "kipp_ssd_scan_of");
         float* scratch = recurrent_scratch(tokens, heads, dim, v_dim, 4);
         float* conv_out = workspace->get<float>("state_space_conv", (size_t)tokens * ((size_t)heads * v_dim + 2 * (size_t)groups * dim));
         run(f(out, ld_out, proj, ld_proj, dtype, z_off, xbc_off, dt_off, conv_w, conv_b, taps, dt_bias, a_log, d_skip, norm_w,
-              norm_groups, state, slot_stride, q_start, entry_of_token, slots, entries, tokens, heads, groups, dim, v_dim, eps,
+              norm_groups, state, slot_stride, q_start, entry_of_token, slots, entries, tokens, longest, heads, groups, dim, v_dim, eps,
               scratch, conv_out, stream),
             "ssd_scan", tokens == entries ? 2 : taps > 1 ? 4 : 3);
     }

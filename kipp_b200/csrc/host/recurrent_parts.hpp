@@ -770,9 +770,10 @@ public:
                  fold_input(ctx, fold_in));
         void* gated = ctx.workspace->buffer("state_space_out", (size_t)T * inner_ld_ * es);
         if (inner_ld_ != inner_) cuda_check(cudaMemsetAsync(gated, 0, (size_t)T * inner_ld_ * es, ctx.stream), "clearing the padding");
+        const int longest = m.shape.q_lens.empty() ? 0 : *std::max_element(m.shape.q_lens.begin(), m.shape.q_lens.end());
         ops.ssd_scan(gated, inner_ld_, proj, proj_ld_, ctx.dtype, 0, inner_, inner_ + channels_, conv_, conv_b_, taps_, dt_bias_,
                      a_log_, d_, norm_, norm_groups_, state, state_floats(), m.q_start, m.entry_of_token, m.slots,
-                     m.shape.entries, T, heads_, groups_, state_, v_dim_, eps_);
+                     m.shape.entries, T, longest, heads_, groups_, state_, v_dim_, eps_);
         output_product(ctx, residual, gated, inner_ld_, w_o_, inner_ld_, dtype_, hidden_, inner_ld_);
     }
 

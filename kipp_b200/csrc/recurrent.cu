@@ -89,7 +89,7 @@ struct ScanArgs {
     float* state;                          // [slots, heads, dim, v_dim]
     const int* q_start; const int* slots;
     int heads, dim, v_dim, batch, entries;
-    int longest;                           // gated delta: the most tokens that an entry brings (0: not known)
+    int longest;                           // state space and gated delta: the most tokens that an entry brings (0: not known)
     float k_scale, eps, out_scale;
     int gate;                              // 0 none, 1 silu, 2 sigmoid
     // gated memory: columns of the two gates in proj, their biases [heads], the cap, the scale of q
@@ -1365,8 +1365,15 @@ template <typename T> bool conv_run_ok(const ScanArgs& a) {
 inline bool scan_by_fours(const ScanArgs& a) {
     return a.dim % 4 == 0 && a.v_dim % 4 == 0 && a.dim <= 256 && a.slot_stride % 4 == 0 && ((uintptr_t)a.state & 15) == 0;
 }
-// Two leaves a thread where there are more blocks than this for each SM, one (twice the warps) elsewhere: see above for both.
-constexpr int SSD_CROWD = 4;
+// Two leaves a thread where an SM has more than this many blocks at work, one (twice the warps) elsewhere: see above for both.  As in
+// launch_gated_delta_scan those are at work that last as long as the longest entry, tokens / longest entries of them.  us of the
+// layer with one leaf and with two, 64 heads of 128 x 64: 0.9 blocks at work (2,048 tokens) 348 and 412, (2,000 tokens beside seven of
+// one) 532 and 557, (400 beside 31 of one) 130 and 147; 1.7 (1,276, 636 and 600) 368 and 423; 2.6 (three of 300) 142 and 134;
+// 6.9 (eight of 100) 120 and 112; 24 heads of 256 x 32, 0.8 (five of 300) 88 and 103, 1.3 (eight of 100) 66 and 61; 128 heads of
+// 64 x 64, 2.2 (1,000 beside three of 100) 295 and 387, 6.9 (four of 300) 220 and 236, (four of 30) 49 and 44; 100 of 32 x 64, 4.1 (three
+// of 300) 98 and 107, 6.8 (five of 300) 147 and 142.  The form chosen is within 8 % of the better one over 103 sizes, head counts and
+// batches.
+template <int LEAVES, int R> constexpr double ssd_crowd() { return LEAVES < 32 ? 5.0 : R == 4 ? 2.4 : 1.0; }
 template <int LEAVES, int LPT, int R>
 int launch_ssd_form(const ScanArgs& a, const float* conv, const float2* dts, float* o_raw, int entries, int tokens, cudaStream_t stream) {
     const TokenBatch tb = ssd_batch(2 * a.dim + SSD_COLS + 4);
@@ -1377,10 +1384,13 @@ int launch_ssd_form(const ScanArgs& a, const float* conv, const float2* dts, flo
     return launch_walk(a, tokens, kernel, dim3((unsigned)(entries * a.heads * slices)), dim3(SSD_COLS / SCAN_COLS * LEAVES / LPT), bytes, stream,
                        a, conv, dts, o_raw, slices);
 }
+template <int LEAVES, int R> int ssd_leaves(int heads, int v_dim, int entries, int tokens, int longest) {
+    const double at_work = longest > 0 ? (double)tokens / longest : entries;
+    return at_work * heads * ((v_dim + SSD_COLS - 1) / SSD_COLS) > ssd_crowd<LEAVES, R>() * kipp_sm_count() ? 2 : 1;
+}
 template <int LEAVES, int R>
 int launch_ssd_scan(const ScanArgs& a, const float* conv, const float2* dts, float* o_raw, int entries, int tokens, cudaStream_t stream) {
-    const int slices = (a.v_dim + SSD_COLS - 1) / SSD_COLS;
-    if ((long long)entries * a.heads * slices > (long long)SSD_CROWD * kipp_sm_count())
+    if (ssd_leaves<LEAVES, R>(a.heads, a.v_dim, entries, tokens, a.longest) == 2)
         return launch_ssd_form<LEAVES, 2, R>(a, conv, dts, o_raw, entries, tokens, stream);
     return launch_ssd_form<LEAVES, 1, R>(a, conv, dts, o_raw, entries, tokens, stream);
 }
@@ -1914,14 +1924,15 @@ extern "C" long long kipp_ssd_state_floats(int heads, int groups, int dim, int v
 // channels to convolve [x | B | C] at xbc_off and dt [heads] at dt_off; conv_w [taps, channels] (the last
 // tap meets the current token), conv_b [channels], dt_bias, a_log, d_skip [heads], norm_w [heads * v_dim]
 // (or null) float32; `dim` is the size of B and C (the state's rows).  A slot is kipp_ssd_state_floats floats.
-// conv_out: float32 [tokens, channels] of scratch for the convolved rows.  At most 16 taps.
+// conv_out: float32 [tokens, channels] of scratch for the convolved rows.  At most 16 taps.  longest: the most tokens that
+// an entry brings, or 0; it chooses between two forms with the same bits.
 extern "C" int kipp_ssd_max_taps() { return 16; }
-extern "C" int kipp_ssd_scan(void* out, long long ld_out, const void* proj, long long ld_proj, int dtype, int z_off,
-                             int xbc_off, int dt_off, const float* conv_w, const float* conv_b, int taps,
-                             const float* dt_bias, const float* a_log, const float* d_skip, const float* norm_w,
-                             int norm_groups, float* state, long long slot_stride, const int* q_start,
-                             const int* entry_of_token, const int* slots, int entries, int tokens, int heads, int groups,
-                             int dim, int v_dim, float eps, float* scratch, float* conv_out, void* stream) {
+extern "C" int kipp_ssd_scan_of(void* out, long long ld_out, const void* proj, long long ld_proj, int dtype, int z_off,
+                                int xbc_off, int dt_off, const float* conv_w, const float* conv_b, int taps,
+                                const float* dt_bias, const float* a_log, const float* d_skip, const float* norm_w,
+                                int norm_groups, float* state, long long slot_stride, const int* q_start,
+                                const int* entry_of_token, const int* slots, int entries, int tokens, int longest, int heads,
+                                int groups, int dim, int v_dim, float eps, float* scratch, float* conv_out, void* stream) {
     if (entries <= 0 || tokens <= 0) return 0;
     if (!kipp_recurrent_scan_ok(dim, v_dim, SSD) || heads <= 0 || groups <= 0 || heads % groups || taps < 1 || taps > MAX_TAPS ||
         norm_groups <= 0 || (heads * v_dim) % norm_groups || conv_w == nullptr || conv_b == nullptr || dt_bias == nullptr ||
@@ -1933,11 +1944,30 @@ extern "C" int kipp_ssd_scan(void* out, long long ld_out, const void* proj, long
     a.z_off = z_off; a.xbc_off = xbc_off; a.dt_off = dt_off; a.taps = taps; a.groups = groups; a.norm_groups = norm_groups;
     a.conv_w = conv_w; a.conv_b = conv_b; a.dt_bias = dt_bias; a.a_log = a_log; a.d_skip = d_skip; a.norm_w = norm_w;
     a.state = state; a.slot_stride = slot_stride; a.q_start = q_start; a.entry_of_token = entry_of_token; a.slots = slots;
-    a.heads = heads; a.dim = dim; a.v_dim = v_dim; a.eps = eps; a.k_scale = 1.f; a.out_scale = 1.f;
+    a.heads = heads; a.dim = dim; a.v_dim = v_dim; a.eps = eps; a.k_scale = 1.f; a.out_scale = 1.f; a.longest = longest;
     a.channels = heads * v_dim + 2 * groups * dim; a.kept_off = (long long)heads * dim * v_dim;
     if (dtype == KIPP_DT_F32) return launch_scan<float, SSD>(a, entries, tokens, scratch, (cudaStream_t)stream, conv_out);
     if (dtype == KIPP_DT_BF16) return launch_scan<bf16, SSD>(a, entries, tokens, scratch, (cudaStream_t)stream, conv_out);
     return KIPP_ERR_DTYPE;
+}
+
+// The same where nobody says how long the entries are: as if they were alike.
+extern "C" int kipp_ssd_scan(void* out, long long ld_out, const void* proj, long long ld_proj, int dtype, int z_off,
+                             int xbc_off, int dt_off, const float* conv_w, const float* conv_b, int taps,
+                             const float* dt_bias, const float* a_log, const float* d_skip, const float* norm_w,
+                             int norm_groups, float* state, long long slot_stride, const int* q_start,
+                             const int* entry_of_token, const int* slots, int entries, int tokens, int heads, int groups,
+                             int dim, int v_dim, float eps, float* scratch, float* conv_out, void* stream) {
+    return kipp_ssd_scan_of(out, ld_out, proj, ld_proj, dtype, z_off, xbc_off, dt_off, conv_w, conv_b, taps, dt_bias, a_log, d_skip, norm_w,
+                            norm_groups, state, slot_stride, q_start, entry_of_token, slots, entries, tokens, 0, heads, groups, dim, v_dim,
+                            eps, scratch, conv_out, stream);
+}
+// Leaves of rows a thread has in the scan of such entries (1 or 2).
+extern "C" int kipp_ssd_scan_leaves(int dim, int v_dim, int heads, int entries, int tokens, int longest) {
+    if (dim <= 32) return ssd_leaves<8, 4>(heads, v_dim, entries, tokens, longest);
+    if (dim <= 64) return ssd_leaves<16, 4>(heads, v_dim, entries, tokens, longest);
+    if (dim <= 128) return ssd_leaves<32, 4>(heads, v_dim, entries, tokens, longest);
+    return ssd_leaves<32, 8>(heads, v_dim, entries, tokens, longest);
 }
 
 // float32 values of state one request slot of the gated delta rule holds: S [heads, dim, v_dim], then the last

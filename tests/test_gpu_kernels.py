@@ -1491,6 +1491,42 @@ def test_state_space_scans_add_in_one_order(D, v_dim, heads, n):
     assert torch.equal(many, one[:1].expand_as(many)) and torch.equal(states, kept[:1].expand_as(states))
 
 
+@pytest.mark.parametrize("D,v_dim,heads,lens", [(128, 64, 20, [53, 1, 7]), (64, 36, 64, [16, 40]), (100, 64, 30, [21]), (256, 32, 40, [9, 30]),
+                                                (32, 32, 130, [6, 33, 1])])
+def test_state_space_scans_of_either_form(D, v_dim, heads, lens):
+    """A leaf of rows a thread and two, as the longest entry's length chooses: the same bits."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    lib = load_library("recurrent")
+    p, i, ll, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+    lib.kipp_ssd_scan_of.argtypes = [p, ll, p, ll, i, i, i, i, p, p, i, p, p, p, p, i, p, ll, p, p, p, i, i, i, i, i, i, i, f, p, p, p]
+    lib.kipp_ssd_state_floats.restype = lib.kipp_recurrent_scratch_floats.restype = ll
+    taps, inner, E, T = 2, heads * v_dim, len(lens), sum(lens)
+    channels = inner + 2 * D
+    stride = lib.kipp_ssd_state_floats(heads, 1, D, v_dim, taps)
+    g = torch.Generator().manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)                      # noqa: E731
+    z_off = channels + heads + (-heads) % 4
+    ld = z_off + inner
+    proj, first = rnd(T, ld), rnd(E, stride)
+    weights = [rnd(taps, channels) * 0.5, rnd(channels) * 0.1, rnd(heads), rnd(heads) * 0.5, rnd(heads), rnd(inner)]
+    w = [t.data_ptr() for t in weights]
+    q_start = torch.tensor([0] + lens).cumsum(0).int().to(DEV)
+    entry, slots = torch.arange(E).repeat_interleave(torch.tensor(lens)).int().to(DEV), torch.arange(E, dtype=torch.int32, device=DEV)
+    results = []
+    for longest, leaves in ((T, 1), (1, 2)):
+        assert lib.kipp_ssd_scan_leaves(D, v_dim, heads, E, T, longest) == leaves
+        state, out, conv = first.clone(), torch.zeros(T, inner, device=DEV), torch.zeros(T, channels, device=DEV)
+        scratch = torch.zeros(lib.kipp_recurrent_scratch_floats(T, heads, D, v_dim, 4), device=DEV)
+        rc = lib.kipp_ssd_scan_of(out.data_ptr(), inner, proj.data_ptr(), ld, 0, z_off, 0, channels, w[0], w[1], taps, w[2], w[3], w[4], w[5],
+                                  1, state.data_ptr(), stride, q_start.data_ptr(), entry.data_ptr(), slots.data_ptr(), E, T, longest, heads, 1,
+                                  D, v_dim, 1e-5, scratch.data_ptr(), conv.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        assert rc == 0 and torch.isfinite(out).all()
+        results.append((out, state))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 @pytest.mark.parametrize("size", [1, 100, 128, 2048, 2049, 2560, 5000])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_row_dot(dtype, size):

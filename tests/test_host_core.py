@@ -95,3 +95,15 @@ def test_a_clusters_ctas_fit_an_sm_as_they_are_counted():
     assert all(fits(128, 8 * group, 8, ctas) for group in (1, 4, 8, 12) for ctas in (1, 2, 3, 4))
     assert not any(fits(128, group, 1, ctas) for group in (14, 16) for ctas in (1, 2, 3, 4))
     assert not fits(128, 17, 1, 4) and not fits(96, 4, 1, 4) and not fits(128, 8, 1, 9) and not fits(128, 8, 1, 0)
+
+
+def test_state_space_scans_count_the_work_that_lasts():
+    """The scan's form follows the blocks that last as long as the longest entry: one long prompt beside many single
+    tokens is scanned as the prompt alone, entries alike as all of them."""
+    leaves = build.load_library("recurrent").kipp_ssd_scan_leaves
+    for dim, heads in ((128, 64), (128, 80), (64, 32), (256, 24), (32, 100)):
+        alone = leaves(dim, 64, heads, 1, 2000, 2000)
+        assert alone == 1
+        for others in (1, 7, 31, 200):
+            assert leaves(dim, 64, heads, 1 + others, 2000 + others, 2000) == alone
+        assert leaves(dim, 64, heads, 64, 64 * 100, 100) == leaves(dim, 64, heads, 64, 64 * 100, 0) == 2
