@@ -1384,8 +1384,8 @@ inline void Engine::sample(const kipp_sample_params* params, uint64_t* rng_state
     cuda_check(cudaSetDevice(opt_.device), "cudaSetDevice");
     const int vocab = plan_->vocab_size;
     float* logits = const_cast<float*>(last_logits_);
-    bool any_penalty = false, any_bias = false, any_random = false;
-    int recent_width = 0, bias_width = 0;
+    bool any_penalty = false, any_bias = false, any_random = false, all_top_k = true;
+    int recent_width = 0, bias_width = 0, largest_top_k = 0;
     for (int i = 0; i < n_rows; ++i) {
         const kipp_sample_params& p = params[i];
         if (!(p.top_p > 0.f && p.top_p <= 1.f)) fail(KIPP_E_ARGUMENT, "top_p must be greater than 0 and at most 1");
@@ -1402,7 +1402,11 @@ inline void Engine::sample(const kipp_sample_params* params, uint64_t* rng_state
             any_bias = true;
             bias_width = std::max(bias_width, p.logit_bias_count);
         }
-        any_random = any_random || p.temperature > 0.f;
+        if (p.temperature > 0.f) {
+            any_random = true;
+            all_top_k = all_top_k && p.top_k > 0;
+            largest_top_k = std::max(largest_top_k, p.top_k);
+        }
     }
     // host block: [recent n x rw][recent_count n][rep n][pres n][freq n][bias tok n x bw][bias val n x bw]
     //             [bias count n][temperature n][top_k n][top_p n][min_p n][uniform n (double)]
@@ -1466,7 +1470,8 @@ inline void Engine::sample(const kipp_sample_params* params, uint64_t* rng_state
         ops_.argmax_rows(logits, vocab, n_rows, vocab, out_dev);
     else
         ops_.sample_rows(logits, vocab, n_rows, vocab, (const float*)at(temperature), (const int*)at(top_k),
-                         (const float*)at(top_p), (const float*)at(min_p), (const double*)at(uniform), out_dev);
+                         (const float*)at(top_p), (const float*)at(min_p), (const double*)at(uniform),
+                         all_top_k ? largest_top_k : 0, out_dev);
     cuda_check(cudaMemcpyAsync(out_host, out_dev, n * sizeof(int), cudaMemcpyDeviceToHost, stream_), "sampled tokens");
     cuda_check(cudaStreamSynchronize(stream_), "synchronize");
 }

@@ -1098,11 +1098,11 @@ public:
         run(f(logits, ld, rows, n, out, scratch, need, stream), "argmax_rows", need > 0 ? 2 : 1);
     }
     void sample_rows(const float* logits, long long ld, int rows, int n, const float* temperature, const int* top_k,
-                     const float* top_p, const float* min_p, const double* uniform, int* out) {
+                     const float* top_p, const float* min_p, const double* uniform, int largest_top_k, int* out) {
         using Fn = int (*)(const float*, long long, int, int, const float*, const int*, const float*, const float*,
-                           const double*, int*, void*);
-        static Fn f = kernel_symbol<Fn>("sampling", "kipp_sample_rows");
-        run(f(logits, ld, rows, n, temperature, top_k, top_p, min_p, uniform, out, stream), "sample_rows");
+                           const double*, int, int*, void*);
+        static Fn f = kernel_symbol<Fn>("sampling", "kipp_sample_rows_of");
+        run(f(logits, ld, rows, n, temperature, top_k, top_p, min_p, uniform, largest_top_k, out, stream), "sample_rows");
     }
     void apply_penalties(float* logits, long long ld, int rows, int n, const int* recent, int recent_width,
                          const int* recent_count, const float* repetition, const float* presence,

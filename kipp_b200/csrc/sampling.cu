@@ -30,9 +30,9 @@
 // draw within a nucleus takes its first pass from the selection that found the nucleus; and a pass over a long part
 // that adds weights has a histogram for each lane.  64 rows of 151,936, top-p 0.95: 207 us, 158 with top-k 50 (519 and 158
 // before the histograms by lane; with half the rows of either kind 488, 934 with all passes over the rows and the loads
-// one at a time); a single such row by eight blocks: 92 and 86 us (138 and 85), 148 of them by a block each 351 and 231 (1,013 and
-// 225); 128 rows of 32,000 with top-k 50: 82 (78, with more of the SM's memory left to the L1).  What is left is six walks of
-// some forty instructions an element.
+// one at a time); a single such row by eight blocks: 92 us (138), 148 of them by a block each 351 (1,013).  Rows that all have a top-k
+// that fits the list go without (kipp_sample_rows_of): as before them.  What is left is six walks of some forty instructions an
+// element.
 //
 // Also here: the penalties and logit bias the reference applies before
 // sampling (apply_bias_and_penalties, src/kipp.c:3386-3431).
@@ -548,9 +548,10 @@ __global__ void argmax_merge_kernel(const ArgmaxPart* __restrict__ parts, int n_
     if (threadIdx.x == 0) out[blockIdx.x] = bi == 0x7fffffff ? 0 : bi;
 }
 
-// The token drawn from a row (temperature above 0) whose first maximum is `best_i`.
+// The token drawn from a row (temperature above 0) whose first maximum is `best_i`.  (Its options are read where they are used: held
+// from the start they cost the kernel its last registers, and 64 rows of 151,936 with top-k 4,096 191 us instead of 187.)
 template <bool LONG>
-__device__ int draw(RowCtx& c, Shared& sh, int k, float tp, float mp, double uniform, int best_i) {
+__device__ int draw(RowCtx& c, Shared& sh, int k, const float* top_p, const float* min_p, const double* uniform, int best_i) {
     unsigned key, tok; double cum, total;
     if (k > 0) {
         // rank k in the order, or the last candidate when there are fewer
@@ -568,20 +569,22 @@ __device__ int draw(RowCtx& c, Shared& sh, int k, float tp, float mp, double uni
             __syncthreads();                           // read by all before the next pass counts anew
         }
     }
+    const float mp = *min_p;
     if (mp > 0.0f) {
         // The top weight is expf(smax - smax) = 1.
         c.has_minp = true;
         c.minp_threshold = (double)mp * (double)expf(0.0f);
     }
     // with a nucleus, the prefix that is kept, and a share of its weight; else a share of the set's
+    const float tp = *top_p;
     double kept;
     if (tp < 1.0f) {
         select<LONG>(c, sh, MODE_W_GE, 0, (double)tp, true, false, key, tok, cum, total);
         c.has_nucleus = true; c.nuc_key = key; c.nuc_tok = tok;
         kept = cum;
-        select<LONG>(c, sh, MODE_W_GT, 0, uniform * kept, false, true, key, tok, cum, total);
+        select<LONG>(c, sh, MODE_W_GT, 0, *uniform * kept, false, true, key, tok, cum, total);
     } else {
-        select<LONG>(c, sh, MODE_W_GT, 0, uniform, true, false, key, tok, cum, total);
+        select<LONG>(c, sh, MODE_W_GT, 0, *uniform, true, false, key, tok, cum, total);
         kept = total;
     }
     return (key == 0xffffffffu && tok == 0 && kept == 0.0) ? best_i : (int)tok;
@@ -636,8 +639,8 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int n,
     // (Rows whose top-k leaves no more than the list holds walk long parts without weights only: they take the code of the short
     // parts.  Sharing the other's, with its second kind of walk, cost them another 2 to 3 us of code to fetch.)
     const int k = top_k[r];
-    const int token = LONG && !(k > 0 && k <= LIST_CAP) ? draw<true>(c, sh, k, top_p[r], min_p[r], uniform[r], best_i)
-                                                        : draw<false>(c, sh, k, top_p[r], min_p[r], uniform[r], best_i);
+    const int token = LONG && !(k > 0 && k <= LIST_CAP) ? draw<true>(c, sh, k, top_p + r, min_p + r, uniform + r, best_i)
+                                                        : draw<false>(c, sh, k, top_p + r, min_p + r, uniform + r, best_i);
     if (threadIdx.x == 0 && rank == 0) out[r] = token;
 }
 
@@ -750,23 +753,44 @@ extern "C" int kipp_argmax_rows_split(const float* logits, long long ld, int row
                        (const ArgmaxPart*)scratch, shares, out);
 }
 
-extern "C" int kipp_sample_rows(const float* logits, long long ld, int rows, int n,
-                                const float* temperature, const int* top_k, const float* top_p,
-                                const float* min_p, const double* uniform, int* out, void* stream) {
-    if (rows <= 0) return 0;
-    if (n <= 0) return KIPP_ERR_ARG;
-    // long rows: a cluster of up to eight blocks a row (at most eight: the kernel's loops over the
-    // team are unrolled to that), as many as keep all rows' blocks within one wave of the GPU
+namespace {
+// Long rows: a cluster of up to eight blocks a row (at most eight: the kernel's loops over the team are unrolled to that), as many as
+// keep all rows' blocks within one wave of the GPU.
+int sample_blocks(int rows, int n) {
     int blocks = 1;
     while (blocks < 8 && n >= 16384 * blocks && (long long)rows * blocks * 2 <= kipp_sm_count()) blocks *= 2;
+    return blocks;
+}
+}  // namespace
+
+// Whether kipp_sample_rows_of launches the kernel with histograms by lane: where a block's part of a row is long and a row may be
+// without a top-k that fits the list.  (Rows that all have one walk long parts without weights only, and the kernel's 96 KB of shared
+// memory and second kind of walk cost them for nothing: top-k 50, 128 rows of 32,000 79.0 us, 76.9 without; 148 of 151,936 222 and 217, 8
+// of 10,000 57.8 and 55.6.)
+extern "C" int kipp_sample_rows_by_lane(int rows, int n, int largest_top_k) {
+    const int blocks = sample_blocks(rows, n), part = ((n + blocks - 1) / blocks + 3) & ~3;                // (the last block of a row may have less)
+    return part >= BY_LANE_FROM && !(largest_top_k > 0 && largest_top_k <= LIST_CAP);
+}
+// largest_top_k: the largest top_k of the rows that are drawn from (temperature above 0) where each of them has one; 0 where one has
+// none, or where nobody says.  It chooses between two forms with the same draws.
+extern "C" int kipp_sample_rows_of(const float* logits, long long ld, int rows, int n, const float* temperature, const int* top_k,
+                                   const float* top_p, const float* min_p, const double* uniform, int largest_top_k, int* out,
+                                   void* stream) {
+    if (rows <= 0) return 0;
+    if (n <= 0) return KIPP_ERR_ARG;
+    const int blocks = sample_blocks(rows, n);
     if ((long long)rows * blocks > 0x7fffffffLL) return KIPP_ERR_ARG;
-    const int part = ((n + blocks - 1) / blocks + 3) & ~3;                // (the last block of a row may have less)
-    const bool by_lane = part >= BY_LANE_FROM;
+    const bool by_lane = kipp_sample_rows_by_lane(rows, n, largest_top_k) != 0;
     const auto kernel = by_lane ? sample_rows_kernel<true> : sample_rows_kernel<false>;
     const size_t smem = by_lane ? BY_LANE_BYTES : 0;
     if (const int e = kipp_allow_smem(kernel, smem)) return e;
     return kipp_launch_cluster(kernel, dim3((unsigned)(rows * blocks)), dim3(THREADS), smem, (cudaStream_t)stream,
                                dim3(blocks, 1, 1), logits, ld, n, temperature, top_k, top_p, min_p, uniform, out);
+}
+extern "C" int kipp_sample_rows(const float* logits, long long ld, int rows, int n,
+                                const float* temperature, const int* top_k, const float* top_p,
+                                const float* min_p, const double* uniform, int* out, void* stream) {
+    return kipp_sample_rows_of(logits, ld, rows, n, temperature, top_k, top_p, min_p, uniform, 0, out, stream);
 }
 
 extern "C" int kipp_apply_penalties(float* logits, long long ld, int rows, int n, const int* recent,

@@ -996,6 +996,32 @@ def test_sample_rows_alone_and_among_others(vocab):
     assert draw(rows // some).cpu().equal(alone.repeat(rows // some))
 
 
+@pytest.mark.parametrize("rows,vocab", [(1, 151936), (80, 32000), (3, 8192)])
+def test_sample_rows_of_either_form(rows, vocab):
+    """A row's token is the same whether the caller says that every row has a top-k (no histograms by lane) or not, greedy rows
+    among them."""
+    import ctypes
+    from kipp_b200.csrc.build import load_library
+    fn = load_library("sampling").kipp_sample_rows_of
+    p, i, ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
+    fn.argtypes = [p, ll, i, i, p, p, p, p, p, i, p, p]
+    g = torch.Generator().manual_seed(rows)
+    logits = (torch.randn(rows, vocab, generator=g) * 2).to(DEV)
+    t = torch.full((rows,), 0.9, device=DEV)
+    t[2::5] = 0
+    k = (torch.arange(rows) * 613 % 4096 + 1).int().to(DEV)
+    tp, mp = torch.rand(rows, generator=g).clamp(0.05, 1).to(DEV), (torch.rand(rows, generator=g) * 0.01).to(DEV)
+    u = torch.rand(rows, generator=g, dtype=torch.float64).to(DEV)
+    tokens = []
+    for largest in (0, 4096):
+        out = torch.full((rows,), -1, dtype=torch.int32, device=DEV)
+        assert fn(logits.data_ptr(), vocab, rows, vocab, t.data_ptr(), k.data_ptr(), tp.data_ptr(), mp.data_ptr(), u.data_ptr(), largest,
+                  out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        tokens.append(out)
+    assert torch.equal(*tokens) and tokens[0].min() >= 0 and tokens[0].max() < vocab
+    assert torch.equal(tokens[0][2::5].long(), logits[2::5].argmax(dim=1))
+
+
 @pytest.mark.parametrize("vocab", [700, 151936])
 def test_sample_rows_at_the_ends_of_a_nucleus(vocab):
     """The draw takes its first pass from the selection that found the nucleus: 0 gives the nucleus's first token and the

@@ -107,3 +107,12 @@ def test_state_space_scans_count_the_work_that_lasts():
         for others in (1, 7, 31, 200):
             assert leaves(dim, 64, heads, 1 + others, 2000 + others, 2000) == alone
         assert leaves(dim, 64, heads, 64, 64 * 100, 100) == leaves(dim, 64, heads, 64, 64 * 100, 0) == 2
+
+
+def test_rows_with_a_top_k_are_sampled_without_histograms_by_lane():
+    """Only rows that may weigh a long part need them: not where every row's top-k fits the list."""
+    by_lane = build.load_library("sampling").kipp_sample_rows_by_lane
+    for rows, n in ((1, 151936), (64, 151936), (148, 151936), (128, 32000), (8, 10000)):
+        assert by_lane(rows, n, 0) == by_lane(rows, n, 4097) == 1
+        assert by_lane(rows, n, 1) == by_lane(rows, n, 50) == by_lane(rows, n, 4096) == 0
+    assert by_lane(4, 8000, 0) == 0
