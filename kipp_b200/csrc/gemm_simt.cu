@@ -18,8 +18,9 @@
 //         run, so a 2,048-feature matrix still gives 128 blocks of 256 chains; weights and tokens travel by asynchronous copies,
 //         the weights' first ones before the wait for the kernel before (few_stages).
 //         12,288 x 2,048 with 1, 3 and 16 tokens: 20, 27 and 48 us (100 MB: 15 us of copy rate; the kernel below, which ran
-//         once: 334, 339 and 353); 2,048 x 6,144 with 3: 17 us.  From 17 tokens on it needs two passes, which still
-//         win where the features are few and lose where they are many: from many_features() on those are tiles'.
+//         once: 334, 339 and 353); 2,048 x 6,144 with 3: 17 us.  From 17 tokens on it needs two passes, which win where the features
+//         are few: 32 tokens, 2,048 and 3,072 x 2,048 16 and 30 us, 8,192 x 2,048 60, 2,048 x 6,144 43 (33 tokens in tiles: 49,
+//         57, 93 and 128); from many_features() on they are tiles'.
 //   tile  float32, more tokens: 128 or 256 features x 64 tokens per block of 128 threads, 8 or 16 x 8 per thread in float32
 //         pairs, operands in shared memory with k outermost, so that a k's values cost a thread four or six 16-byte reads
 //         (with four bytes copied at a time); the groups of runs are blocks of their own, a cluster that meets in its
@@ -153,6 +154,7 @@ gemm_simt_kernel(TC* __restrict__ C, const TA* __restrict__ A, const TW* __restr
 // run reads, serve both: of several tokens those reads are what an SM is busy with.
 constexpr int FEW_F = 16, FEW_THREADS = 16 * MAX_RUNS, FEW_MAX = 32;
 inline int many_features() { return 64 * kipp_sm_count(); }         // two blocks of pairs of features for each SM
+inline bool few_tokens(int M, int N) { return M <= (N >= many_features() ? FEW_MAX / 2 : FEW_MAX); }
 constexpr int FEW_CHUNK = BK * 4 + 16;              // 64 bytes of a feature's row, padded against bank conflicts
 // A warp's stage: its chunks of weights, then 16 values of each of MT tokens for its two runs.  (The tokens' values came
 // from global memory before, four at a time and the next four on their way: a trip to the L2 for every four, since a
@@ -163,16 +165,16 @@ template <bool PAIR, int MT> struct Few {
     static constexpr int BLOCK_STAGE = (FEW_THREADS / 32) * STAGE;        // bytes of a stage of the block's eight warps
 };
 
-// Waits until at most `n` of the thread's groups of copies are on their way (n from 0 to 6).
+constexpr int FEW_STAGES_MAX = 6;
+// Waits until at most `n` of the thread's groups of copies are on their way, n from 0 to FEW_STAGES_MAX - 2 (else for all).
 __device__ __forceinline__ void cp_async_wait_most(int n) {
+    static_assert(FEW_STAGES_MAX - 2 == 4, "the cases below");
     switch (n) {
-    case 0: cp_async_wait<0>(); break;
     case 1: cp_async_wait<1>(); break;
     case 2: cp_async_wait<2>(); break;
     case 3: cp_async_wait<3>(); break;
     case 4: cp_async_wait<4>(); break;
-    case 5: cp_async_wait<5>(); break;
-    default: cp_async_wait<6>(); break;
+    default: cp_async_wait<0>(); break;
     }
 }
 // (One function for all epilogues: a layer's four products then find its code where the one before left it.)
@@ -462,7 +464,7 @@ gemm_tile_kernel(float* __restrict__ C, const float* __restrict__ A, const float
 // 53.9 / 60.8 / 61.2 / 96; one token, 12,288 and 32,000: 23.1 / 20.1 / 22.2 / 21.8 and 42.0 / 43.2 / 45.8 / 45.9.
 inline int few_stages(long long blocks, int stage_bytes, int static_bytes) {
     const long long per_sm = (blocks + kipp_sm_count() - 1) / kipp_sm_count();
-    const int at_once = per_sm <= 1 ? 1 : per_sm <= 8 ? 2 : 4, most = per_sm <= 2 ? 6 : 3;
+    const int at_once = per_sm <= 1 ? 1 : per_sm <= 8 ? 2 : 4, most = per_sm <= 2 ? FEW_STAGES_MAX : 3;
     const int fit = (227 * 1024 / at_once - static_bytes - 1024) / stage_bytes;
     return fit < 2 ? 2 : fit > most ? most : fit;
 }
@@ -470,9 +472,9 @@ template <int MT, bool PAIR>
 int launch_few_form(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, int epi, cudaStream_t s) {
     using F = Few<PAIR, MT>;
     const dim3 grid((N + F::F - 1) / F::F, (M + MT - 1) / MT);
-    const int stages = few_stages((long long)grid.x * grid.y, F::BLOCK_STAGE, MAX_RUNS * MT * (F::F + 1) * 4);
-    const size_t smem = (size_t)stages * F::BLOCK_STAGE;
     constexpr int parts = MAX_RUNS * MT * (F::F + 1) * 4;                 // what the kernel declares beside the ring
+    const int stages = few_stages((long long)grid.x * grid.y, F::BLOCK_STAGE, parts);
+    const size_t smem = (size_t)stages * F::BLOCK_STAGE;
     if (const int e = kipp_allow_smem(gemm_few_kernel<MT, PAIR>, smem + parts)) return e;
     return kipp_launch(gemm_few_kernel<MT, PAIR>, grid, dim3(FEW_THREADS), smem, s, 1, C, A, W, M, N, K, lda, ldw, ldc, epi, stages);
 }
@@ -497,6 +499,7 @@ int launch_tile(float* C, const float* A, const float* W, int M, int N, int K, i
 // another one, 2.3 alone.  us a product in tiles of 128 / 256: 399 tokens, 12,288 x 2,048: 617 / 588, 3,072 x 2,048: 173 / 175,
 // 2,048 x 6,144: 369 / 348; 64 tokens: 104 / 131, 58 / 70, 118 / 194; 1,024 tokens: 1,366 / 1,282, 355 / 338, 713 / 708.  The one
 // chosen is within 7 % of the better everywhere that was measured (64 to 1,024 tokens).
+inline int run_groups(int K) { return (K + GROUP_RUNS * run_length(K) - 1) / (GROUP_RUNS * run_length(K)); }
 inline int tile_features(int M, int N, int groups) {
     const long long t_tiles = (M + TILE_T - 1) / TILE_T, sms = kipp_sm_count();
     auto per_sm = [&](int f) { return (t_tiles * ((N + f - 1) / f) * groups + sms - 1) / sms; };
@@ -507,7 +510,7 @@ inline int tile_features(int M, int N, int groups) {
 // float32 rows that start on 16 bytes and hold whole groups of four: the kernels that copy 16 bytes at a time.
 template <int EPI>
 int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t s) {
-    if (M <= (N >= many_features() ? FEW_MAX / 2 : FEW_MAX)) {
+    if (few_tokens(M, N)) {
         // tokens of a block: as many as there are, up to 16 (the accumulators of a thread)
         if (M == 1) return launch_few<1>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
         if (M == 2) return launch_few<2>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
@@ -515,7 +518,7 @@ int launch_f32(float* C, const float* A, const float* W, int M, int N, int K, in
         if (M <= 8) return launch_few<8>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
         return launch_few<16>(C, A, W, M, N, K, lda, ldw, ldc, EPI, s);
     }
-    const int groups = (K + GROUP_RUNS * run_length(K) - 1) / (GROUP_RUNS * run_length(K));
+    const int groups = run_groups(K);
     return tile_features(M, N, groups) == Tile<4>::F ? launch_tile<EPI, 4>(C, A, W, M, N, K, lda, ldw, ldc, groups, s)
                                                      : launch_tile<EPI, 2>(C, A, W, M, N, K, lda, ldw, ldc, groups, s);
 }
@@ -543,6 +546,11 @@ int launch(void* C, const void* A, const void* W, int M, int N, int K, int lda, 
 }  // namespace
 
 // in_dtype: dtype of A and W (both float32 or both bfloat16); out_dtype: dtype of C.
+// Features of the tiles that a 32-bit product of this size is made in (128 or 256), or 0 where the kernel for few tokens makes it.
+extern "C" int kipp_gemm_simt_tile_features(int M, int N, int K) {
+    if (few_tokens(M, N)) return 0;
+    return tile_features(M, N, run_groups(K));
+}
 extern "C" int kipp_gemm_simt(void* C, int out_dtype, const void* A, const void* W, int in_dtype,
                               int M, int N, int K, int lda, int ldw, int ldc, int epilogue,
                               void* stream) {

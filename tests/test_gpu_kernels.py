@@ -129,8 +129,8 @@ def test_gemm_32_bit_kernels_agree(shape, epilogue):
     """The 32-bit product's three kernels add in one order: the rows of a batch have the same bits whether 1, 3,
     16, 17, 32 (the kernel for few tokens, at its block sizes and the last count it takes), 33 or 70 of them (tiles)
     are multiplied at once, and where rows do not start on 16 bytes; from 9,472 features on a thread of the kernel for
-    few tokens has two of them, and tiles take over at 17 tokens.  The K reach from one run of 16 to runs that
-    end inside a tile; the error against float64 stays under that of one chain of K roundings, K eps |a| |w|."""
+    few tokens has two of them where there are 5 to 8 tokens, and tiles take over at 17.  The K reach from one run of 16 to
+    runs that end inside a tile; the error against float64 stays under that of one chain of K roundings, K eps |a| |w|."""
     N, K = shape
     M = 70
     g = torch.Generator().manual_seed(N + K)
@@ -141,7 +141,7 @@ def test_gemm_32_bit_kernels_agree(shape, epilogue):
     if epilogue != "swiglu":
         bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()) + 2.0 ** -23 * whole.double().abs()
         assert ((whole.double().cpu() - gemm_ref(a, w, epilogue, base)).abs() <= bound.cpu()).all()
-    for m in (1, 2, 3, 5, 16, 17, 32, 33):
+    for m in (1, 2, 3, 5, 7, 8, 9, 16, 17, 32, 33):
         some = base[:m].clone()
         ops().gemm(some, a[:m], w, epilogue, impl="simt")
         assert torch.equal(some, whole[:m]), m
@@ -150,6 +150,28 @@ def test_gemm_32_bit_kernels_agree(shape, epilogue):
     some = base.clone()
     ops().gemm(some, odd, w, epilogue, impl="simt")
     assert torch.equal(some, whole)
+
+
+@pytest.mark.parametrize("epilogue", ["store", "add", "swiglu"])
+@pytest.mark.parametrize("M,N,K", [(70, 12418, 2048), (200, 6206, 1028), (400, 3140, 520)])
+def test_gemm_32_bit_tiles_of_256_features(M, N, K, epilogue):
+    """Tiles of 256 features, the last of which ends in its upper half or its lower one, and of 128 for the first rows (or the kernel
+    for few tokens): the same bits, within K eps |a| |w| of float64."""
+    from kipp_b200.csrc.build import load_library
+    features = load_library("gemm_simt").kipp_gemm_simt_tile_features
+    assert features(M, N, K) == 256 and features(16, N, K) == 0 and features(64, N, K) == 128
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    base = torch.randn(M, N // 2 if epilogue == "swiglu" else N, generator=g).to(DEV)
+    whole = base.clone()
+    ops().gemm(whole, a, w, epilogue, impl="simt")
+    if epilogue != "swiglu":
+        bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t()) + 2.0 ** -23 * whole.double().abs()
+        assert ((whole.double() - (a.double() @ w.double().t() + (base.double() if epilogue == "add" else 0))).abs() <= bound).all()
+    for m in (8, 16, 64):
+        some = base[:m].clone()
+        ops().gemm(some, a[:m], w, epilogue, impl="simt")
+        assert torch.equal(some, whole[:m]), m
 
 
 @pytest.mark.parametrize("dtype,shape,w_rows", [(torch.bfloat16, (5, 70, 100), 100), (torch.bfloat16, (65, 130, 37), 40),
