@@ -678,17 +678,17 @@ attn_decode_kernel(const DecodeParams p) {
                     split, n_splits, true);
 }
 
-// The same with the splits of a pair as a cluster of at most 8 CTAs, which finish the pair among themselves: no scratch, no
+// The same with the splits of a pair as a cluster of up to MAIL_MAX CTAs, which finish the pair among themselves: no scratch, no
 // merge behind it.  A merge launch costs a link of the chain (its wait, its loads, its stores) and every split's partial values a
-// way out and in; a send costs neither (36 layers, 16 tokens behind 1,000 keys: 2,803 -> 2,660 us a step; 4 layers, one behind
-// 77: 172.7 -> 169).  Where it pays: AttentionPlanner::cluster_splits.  The arithmetic of the merge is
+// way out and in; a send costs neither (36 layers, 16 tokens behind 1,000 keys: 2,803 -> 2,660 us a step).  Where it pays, and
+// with how many CTAs (four at most): AttentionPlanner::cluster_splits.  The arithmetic of the merge is
 // attn_decode_merge_kernel's, value for value.  A CTA without a split (its token is shorter) finishes its share all the same.
 template <int D> constexpr int decode_smem() {
     constexpr int PIPE = 2 * DECODE_STAGES * TILE_KEYS * D * 2 + 16 * D * 2;   // tiles, and the group's queries
     constexpr int MERGE = (2 * WARPS * 16 + WARPS * 16 * (D + 8)) * 4;
     return PIPE > MERGE ? PIPE : MERGE;
 }
-constexpr int MAIL_MAX = 8;                       // CTAs of a cluster
+constexpr int MAIL_MAX = 8;                       // CTAs of a cluster (the portable limit)
 __host__ __device__ inline int mail_share(int values, int ctas) { return (values + 2 * ctas - 1) / (2 * ctas) * 2; }
 // (three CTAs an SM, as the planner counts them: registers here, shared memory in kipp_attn_decode_cluster_fits)
 template <int D>

@@ -281,9 +281,9 @@ template <int TILE_T, int TILE_F> struct Cfg {
     static constexpr int ACC_COLS = TILE_T * HALVES;
     static constexpr int TMEM_COLS = ACC_COLS < 32 ? 32 : ACC_COLS;   // 32, 64, 128, 256 or 512
     // Split products of up to 16 tokens send their partial sums; the ring's last stage is then the mailbox: rows of 128
-    // sums, one per token and split (at most TILE_T + 7 of them).  Steps of 36 layers of 2,560: one token, 2,048 keys:
-    // 2,231 -> 2,055 us, eight of 8,100 keys 3,557 -> 3,469, 13 of up to 5,003 keys 3,271 -> 3,258 (with what the attention's
-    // kernel gave in the same measurement, see there).  (With 32 columns: 24 tokens level, 32 slower by 2.5 %: the stage is
+    // sums, one per token and split (at most TILE_T + 7 of them).  Steps of 36 layers of 2,560, together with the attention's loads
+    // (attention_mma.cu; those alone: one token 2,218 -> 2,189): one token, 2,048 keys: 2,231 -> 2,055 us, eight of 8,100
+    // keys 3,557 -> 3,469, 13 of up to 5,003 keys 3,271 -> 3,258.  (With 32 columns: 24 tokens level, 32 slower by 2.5 %: the stage is
     // missed.  A kernel of its own for split products, with its stages as a constant, costs more than it saves: two kernels
     // taking turns in a layer, one token: 2,189 us.)
     static constexpr bool SEND = TILE_T == 16 && TILE_F == UMMA_M;

@@ -454,9 +454,11 @@ public:
     // keys that the step's block tables have room for, is planned as more than CLUSTER_MAX splits, and only up to CLUSTER_TILES key tiles
     // a split at that length: a cluster has a place for every split then, and the bits are the merged ones, whether tables are
     // rounded up (a captured step, whose lengths move on under them) or not (a plain launch), in a small page pool and a large one.
-    // 8 layers, us a step in clusters / merged: 12 tokens of 1,000 keys 569 / 584, 16 of
-    // 1,000 610 / 640, 24 of 700 630 / 679.  Clusters of up to eight, with splits made longer to fit, were level for 1 to 3
-    // tokens of 1,000 to 4,096 keys and slower for 6: 12 layers, 600 keys 808 / 722, 2,048 877 / 794, 4,096 1,005 / 868.
+    // 8 layers, us a step in clusters / merged, with room for 1,024 keys: 12 tokens of 1,000 keys 572 / 579, 16 of 300 556 / 588, of 1,000
+    // 610 / 637, 20 of 500 595 / 629, 24 of 700 627 / 677, 30 of 300 642 / 646 (8 key heads).  Up to 11 are planned as more splits at some
+    // length below that room and are merged, one token behind any context too, unless the page pool itself has no room for more
+    // (4 layers, one behind 77 keys in a pool of 112: 169 / 172.7).  Clusters of up to eight, with splits made longer to fit, were level
+    // for 1 to 3 tokens of 1,000 to 4,096 keys and slower for 6: 12 layers, 600 keys 808 / 722, 2,048 877 / 794, 4,096 1,005 / 868.
     static constexpr int CLUSTER_MAX = 4, CLUSTER_TILES = 12;
     int cluster_splits(const StepShape& s, long long room) const {
         if (own_length_ || room <= 0 || room > CLUSTER_MAX * CLUSTER_TILES * TILE || s.entries != s.tokens) return 0;

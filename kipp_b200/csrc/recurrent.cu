@@ -823,8 +823,10 @@ template <int P, int N> __device__ __forceinline__ void meet_lanes(float (&v)[N]
     }
 }
 // EXACT: the leaves' rows are the head's, none too many.
-// What bounds it is a token's chain and the issue of what surrounds its multiply-adds: 32 columns of 64 x 128 heads are four
-// warps of two leaves or eight of one, on 128 blocks for 64 heads, and a scheduler has one or two warps.  One sequence of 2,048
+// What bounds it is the issue of what surrounds its multiply-adds: a warp takes 72 instructions a token, 24 of which multiply (each
+// for two cycles of its pipe).  One block of 32 columns of 64 x 128 heads, eight warps of one leaf, fills 50 % of an SM's issue slots and 43
+// % of its FMA pipes (two warps a scheduler, mostly in the fixed latency of the instruction before); a second block on the SM
+// needs the other half, and two then last nearly twice as long as one.  One sequence of 2,048
 // tokens, 64 heads, in a model: 477 us token by token with six exchanges each, 438 with the groups, 333 with one leaf a thread and
 // the state's update before the sums, 292 with the sizes as constants.  The two forms alone, sizes not constant: that
 // sequence 349 us with two leaves and 287 with one (441 with each row's update and sum in turn); entries of 1,276, 636 and 600
