@@ -782,11 +782,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
     tcgen05_fence_before();
     __syncthreads();
-    if (*abort_flag) {
-        if (C::SEND && send) kipp_mail_drain(j_end > j_first ? mail_ready : nullptr, KIPP_WAIT_LIMIT_CYCLES);
-        if (threadIdx.x == 0) atomicExch(&p.status[1], 1);
-    }
     if (warp == 1) tmem_dealloc(tmem_base, C::TMEM_COLS);
+    if (*abort_flag) {
+        if (threadIdx.x == 0) atomicExch(&p.status[1], 1);
+        if (C::SEND && send) kipp_mail_drain(j_end > j_first ? mail_ready : nullptr, KIPP_WAIT_LIMIT_CYCLES);
+    }
 }
 
 // ---------------------------------------------------------------------------------------
